@@ -130,7 +130,7 @@ def config(case):
 
 def build(case, seed):
     """The model with random weights: 0.02 as at the start of training; in the families with a fixed residual stream the
-    embedding and the decays are spread as in a trained model."""
+    embedding and the decays are spread as in a trained model, where the stream is several times what a layer adds to it."""
     from easyllm_b200.models.hf_models import CausalLM, arch_from_hf_config
     torch.manual_seed(seed)
     with torch.device("cuda"):
@@ -142,7 +142,7 @@ def build(case, seed):
             elif name.endswith(".sink"):
                 p.normal_()
             elif "embed" in name and case["model"] != "llama":
-                p.mul_(12 if case["model"] == "pafodra" else 25)
+                p.mul_(12 if case["model"] == "pafodra" else 100)
     return model
 
 
