@@ -142,7 +142,7 @@ def build(case, seed):
             elif name.endswith(".sink"):
                 p.normal_()
             elif "embed" in name and case["model"] != "llama":
-                p.mul_(12 if case["model"] == "pafodra" else 100)
+                p.mul_(30 if case["model"] == "pafodra" else 100)
     return model
 
 
