@@ -364,6 +364,9 @@ class MLP(nn.Module):
         self.up_proj = nn.Linear(a.hidden_size, a.intermediate_size, bias=False, dtype=dtype)
         self.down_proj = nn.Linear(a.intermediate_size, a.hidden_size, bias=False, dtype=dtype)
 
+    def fused_groups(self):
+        return [[self.gate_proj.weight, self.up_proj.weight]]
+
     def forward(self, x):
         gu = ops.linear_parts(x, (self.gate_proj.weight, self.up_proj.weight))
         return ops.linear(ops.glu(gu, "silu"), self.down_proj.weight)
