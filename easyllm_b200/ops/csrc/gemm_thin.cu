@@ -1,0 +1,469 @@
+// bf16 GEMM for few rows of activations (decoding, short prompts), sm_100a:  out[T, N] (+)= x[T, K] · W^T (+ bias).
+//
+// With few rows the product is bound by the bytes of W, and a grid of 128 x 256 output tiles leaves most SMs idle (16 tiles
+// for N = 4096).  Here W is the M side of tcgen05.mma: a tile is 128 rows of W by BN rows of x (16 to 128), so 16 rows of x
+// cost a sixteenth of a 256-wide tile, and the reduction is split over the CTAs of a cluster (1, 2, 4 or 8, picked by
+// thin_split so that the tiles fill the SMs evenly).  The partial sums meet in shared memory: every CTA sends the fp32
+// columns that a peer finishes to that peer (distributed shared memory, an mbarrier per direction), and each sums its
+// columns in the order of the cluster's ranks, so results do not depend on timing and no workspace exists.
+//   warp 0     TMA producer: a [128 x 64] box of W and a [BN x 64] box of x per stage
+//   warp 1     one thread issues tcgen05.mma (128 x BN x 16); two accumulators in TMEM
+//   warps 2-5  TMEM -> peers' shared memory -> sum -> bias -> global; a warp stores 32 consecutive columns of a row
+// W_MN: W is stored [K, N] (the input gradient of a linear layer reads its weight in place).
+#include "gemm_fuse.cuh"
+
+namespace ell {
+
+constexpr int kThRows = 128;               // rows of W of a tile
+constexpr int kThWBytes = kThRows * kBK * 2;
+
+template <int BN>
+struct ThinCfg {
+  static constexpr int kStageBytes = kThWBytes + BN * kBK * 2;
+  static constexpr int kStages = BN >= 128 ? 4 : (BN >= 64 ? 6 : 8);
+  static constexpr int kExCols = BN < 64 ? BN : 64;        // columns of an exchange between CTAs
+  static constexpr int kExBytes = kThRows * kExCols * 4;   // of each direction
+  static constexpr int kTmemCols = 2 * BN < 32 ? 32 : 2 * BN;
+  static constexpr int kSmemBytes = kStages * kStageBytes + 2 * kExBytes + 1024 + 256;
+};
+
+struct ThinShared {
+  uint64_t full[8], empty[8], tmem_full[2], tmem_empty[2], recv_full, recv_free;
+  uint32_t tmem_base;
+  int abort_flag;
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+// Shared memory of this CTA -> shared memory of a peer, whose mbarrier counts the bytes.
+__device__ __forceinline__ void bulk_copy_to_peer(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "r"(smem_u32(src)), "r"(bytes), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+// As mbar_wait, for a barrier that other CTAs of the cluster arrive on.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  const unsigned long long t0 = globaltimer_ns();
+  uint32_t spins = 0;
+  while (true) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    if (ok) return true;
+    if ((++spins & 255u) == 0 && (*abort_flag || globaltimer_ns() - t0 > kWaitTimeoutNs)) return false;
+  }
+}
+
+// Barrier of the epilogue that tells every thread whether any of them failed.
+__device__ __forceinline__ bool epi_any(bool failed) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "bar.red.or.pred p, 1, %2, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(any) : "r"((uint32_t)failed), "n"(kEpiThreads) : "memory");
+  return any != 0;
+}
+
+// 32 lanes x 16 consecutive fp32 columns.
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+
+// Rows of x of a tile.
+__host__ __device__ __forceinline__ int thin_bn(int T) { return T <= 16 ? 16 : (T <= 32 ? 32 : (T <= 64 ? 64 : 128)); }
+
+struct ThinArgs {
+  void* out;
+  const __nv_bfloat16* bias;
+  int T, N, K, ldo, out_mode, split, split_log2;
+  int* err;
+};
+
+// k-blocks [first, last) of CTA r out of `split`
+__host__ __device__ __forceinline__ int thin_first_block(int blocks, int split, int r) { return (int)((long long)blocks * r / split); }
+
+// Sums of `cols` columns over the CTAs of the cluster, in the order of their ranks; CH columns at a time so that their loads
+// are in flight together.
+template <int CH, typename Old, typename Put>
+__device__ __forceinline__ void sum_columns(const float* mine, const float* theirs, int cols, int rank, int split, int t, int T,
+                                            const Old& old, const Put& put) {
+#pragma unroll 1
+  for (int j = 0; j < cols && t + j < T; j += CH) {
+    float s[CH], before[CH];
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+      s[i] = 0.f;
+      before[i] = t + j + i < T ? old(t + j + i) : 0.f;
+    }
+#pragma unroll 1
+    for (int p = 0; p < split; ++p) {
+      const float* src = (p == rank ? mine : theirs + (size_t)(p - (p > rank)) * cols * kThRows) + j * kThRows;
+#pragma unroll
+      for (int i = 0; i < CH; ++i) s[i] += src[i * kThRows];
+    }
+#pragma unroll
+    for (int i = 0; i < CH; ++i)
+      if (t + j + i < T) put(t + j + i, before[i] + s[i]);
+  }
+}
+
+template <int BN, bool W_MN>
+__global__ void __launch_bounds__(kGemmThreads, 1)
+gemm_thin_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const ThinArgs a) {
+  using Cfg = ThinCfg<BN>;
+  extern __shared__ uint8_t smem_raw[];
+  // the same offset in every CTA of the cluster: the dynamic shared memory starts at the same address in each
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* sW = smem;
+  uint8_t* sX = smem + Cfg::kStages * kThWBytes;
+  float* send = reinterpret_cast<float*>(smem + Cfg::kStages * Cfg::kStageBytes);   // [column][row]
+  float* recv = send + Cfg::kExBytes / 4;                                            // [peer][column][row]
+  ThinShared* sh = reinterpret_cast<ThinShared*>(recv + Cfg::kExBytes / 4);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int split = a.split, rank = split > 1 ? (int)cluster_rank() : 0;
+  const int tiles_t = (a.T + BN - 1) / BN, tiles = tiles_t * ((a.N + kThRows - 1) / kThRows);
+  const int blocks = (a.K + kBK - 1) / kBK;
+  const int kb0 = thin_first_block(blocks, split, rank), kb1 = thin_first_block(blocks, split, rank + 1);
+  const int first = blockIdx.x / split, step = gridDim.x / split;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < Cfg::kStages; ++s) {
+      mbar_init(&sh->full[s], 1);
+      mbar_init(&sh->empty[s], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&sh->tmem_full[i], 1);
+      mbar_init(&sh->tmem_empty[i], kEpiThreads);
+    }
+    mbar_init(&sh->recv_full, 1);                    // and the peers' bytes
+    mbar_init(&sh->recv_free, 4 * (split - 1) + (split == 1));   // one arrival per epilogue warp of a peer
+    sh->abort_flag = 0;
+    fence_barrier_init();
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+  }
+  if (warp == 1) tmem_alloc<Cfg::kTmemCols>(&sh->tmem_base);
+  tc_fence_before();
+  __syncthreads();
+  if (split > 1) cluster_sync_all();                 // the peers' barriers exist
+  tc_fence_after();
+  const uint32_t tmem_base = sh->tmem_base;
+  volatile int* abort_flag = &sh->abort_flag;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int tile = first; tile < tiles && ok; tile += step) {
+        const int n0 = tile / tiles_t * kThRows, t0 = tile % tiles_t * BN;
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!mbar_wait(&sh->empty[stage], phase ^ 1, abort_flag)) {
+            ok = false;
+            break;
+          }
+          mbar_expect_tx(&sh->full[stage], Cfg::kStageBytes);
+          uint8_t* w = sW + stage * kThWBytes;
+          if (!W_MN) {
+            tma_load_2d(w, &tmW, &sh->full[stage], kb * kBK, n0);
+          } else {
+            tma_load_2d(w, &tmW, &sh->full[stage], n0, kb * kBK);
+            tma_load_2d(w + 64 * kBK * 2, &tmW, &sh->full[stage], n0 + 64, kb * kBK);
+          }
+          tma_load_2d(sX + stage * (BN * kBK * 2), &tmX, &sh->full[stage], kb * kBK, t0);
+          if (++stage == Cfg::kStages) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+      if (!ok) {
+        sh->abort_flag = 1;
+        atomicCAS(a.err, 0, kErrProducer);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc_bf16(kThRows, BN, W_MN, false);
+      constexpr uint32_t w_lbo = W_MN ? 64 * kBK * 2 : 16, w_kstep = W_MN ? 2048 : 32;
+      int stage = 0, it = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int tile = first; tile < tiles && ok; tile += step, ++it) {
+        const int acc = it & 1;
+        if (!mbar_wait(&sh->tmem_empty[acc], ((it >> 1) & 1) ^ 1, abort_flag)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!mbar_wait(&sh->full[stage], phase, abort_flag)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t w = smem_u32(sW + stage * kThWBytes), x = smem_u32(sX + stage * (BN * kBK * 2));
+#pragma unroll
+          for (int k = 0; k < kBK / 16; ++k)
+            umma_bf16(tmem_base + acc * BN, make_smem_desc(w + k * w_kstep, w_lbo, 1024), make_smem_desc(x + k * 32, 16, 1024),
+                      idesc, kb > kb0 || k > 0);
+          umma_commit(&sh->empty[stage]);
+          if (++stage == Cfg::kStages) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+        if (ok) umma_commit(&sh->tmem_full[acc]);
+      }
+      if (!ok) {
+        sh->abort_flag = 1;
+        atomicCAS(a.err, 0, kErrMma);
+      }
+    }
+  } else {
+    const int q = warp & 3, row = q * 32 + lane;     // TMEM lane = row of W in the tile
+    constexpr int EX = Cfg::kExCols;
+    const int cols = EX >> a.split_log2;             // columns (rows of x) of an exchange this CTA finishes
+    const uint32_t block = (uint32_t)cols * kThRows * 4;
+    int it = 0, ex = 0;
+    bool failed = false;
+    for (int tile = first; tile < tiles && !failed; tile += step, ++it) {
+      const int n0 = tile / tiles_t * kThRows, t0 = tile % tiles_t * BN, n = n0 + row;
+      const int acc = it & 1;
+      failed = epi_any(!mbar_wait(&sh->tmem_full[acc], (it >> 1) & 1, abort_flag));
+      if (failed) break;                             // uniform across the epilogue
+      tc_fence_after();
+      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
+      const float bias = a.bias != nullptr && n < a.N ? __bfloat162float(a.bias[n]) : 0.f;
+      auto put = [&](int t, float v) {
+        const size_t at = (size_t)t * a.ldo + n;
+        if (a.out_mode == kOutBf16) reinterpret_cast<__nv_bfloat16*>(a.out)[at] = __float2bfloat16_rn(v + bias);
+        else reinterpret_cast<float*>(a.out)[at] = v;
+      };
+      auto old = [&](int t) {
+        return a.out_mode == kOutF32Accum ? reinterpret_cast<const float*>(a.out)[(size_t)t * a.ldo + n] : 0.f;
+      };
+      if (split == 1) {
+#pragma unroll 1
+        for (int c = 0; c < BN && t0 + c < a.T; c += 16) {
+          uint32_t v[16];
+          tmem_ld_32x16(t_row + c, v);
+          tmem_ld_wait();
+          if (n >= a.N) continue;
+          float before[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) before[i] = t0 + c + i < a.T ? old(t0 + c + i) : 0.f;
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if (t0 + c + i < a.T) put(t0 + c + i, before[i] + __uint_as_float(v[i]));
+        }
+        tc_fence_before();
+        mbar_arrive(&sh->tmem_empty[acc]);
+        continue;
+      }
+      for (int c0 = 0; c0 < BN; c0 += EX, ++ex) {
+        // the peers are done with the exchange before: its bytes have left `send`, and their `recv` may be written
+        if (ex > 0) failed = !mbar_wait_cluster(&sh->recv_free, (ex - 1) & 1, abort_flag);
+#pragma unroll 1
+        for (int c = 0; c < EX; c += 16) {
+          uint32_t v[16];
+          tmem_ld_32x16(t_row + c0 + c, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) send[(c + i) * kThRows + row] = __uint_as_float(v[i]);
+        }
+        if (c0 + EX == BN) {
+          tc_fence_before();
+          mbar_arrive(&sh->tmem_empty[acc]);
+        }
+        fence_proxy_async_smem();
+        failed = epi_any(failed);
+        if (failed) break;
+        if (threadIdx.x == 64) {
+          mbar_expect_tx(&sh->recv_full, (split - 1) * block);
+          for (int d = 1; d < split; ++d) {          // slot of this CTA at peer p: its rank among the others
+            const int p = (rank + d) & (split - 1);
+            bulk_copy_to_peer(map_to_rank(smem_u32(recv), p) + (rank - (rank > p)) * block, send + (size_t)p * cols * kThRows,
+                              block, map_to_rank(smem_u32(&sh->recv_full), p));
+          }
+        }
+        failed = !mbar_wait_cluster(&sh->recv_full, ex & 1, abort_flag);
+        if (!failed && n < a.N) {
+          const int tc = t0 + c0 + rank * cols;
+          const float *mine = send + (size_t)rank * cols * kThRows + row, *theirs = recv + row;
+          if (cols >= 8) sum_columns<8>(mine, theirs, cols, rank, split, tc, a.T, old, put);
+          else if (cols == 4) sum_columns<4>(mine, theirs, cols, rank, split, tc, a.T, old, put);
+          else sum_columns<2>(mine, theirs, cols, rank, split, tc, a.T, old, put);
+        }
+        fence_proxy_async_smem();                    // these reads before the peers' next copies
+        __syncwarp();
+        if (lane < split && lane != rank) mbar_arrive_cluster(map_to_rank(smem_u32(&sh->recv_free), lane));
+      }
+    }
+    if (failed) {
+      sh->abort_flag = 1;
+      atomicCAS(a.err, 0, kErrEpilogue);
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag && threadIdx.x == 0) {
+    // error path: give copies and MMAs in flight time to land before shared memory and TMEM go away
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) {
+    }
+  }
+  __syncthreads();
+  if (split > 1) cluster_sync_all();                 // no peer writes here any more
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc<Cfg::kTmemCols>(tmem_base);
+  }
+}
+
+int make_tmap_bf16_2d(CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t outer, uint64_t row_stride_bytes,
+                      uint32_t box_inner, uint32_t box_outer);
+
+// Estimated time of a launch with `s` CTAs per reduction, in us.  From trains of launches on weights that L2 does not hold:
+// a launch costs 4.5; a k-block 0.27 plus what its rows of x add, 0.05 more with the traffic of more CTAs; a tile's end 0.3,
+// or 1.2 with the exchange, plus the columns it writes, half of it hidden behind the next tile's loads.  Within 10 % of what was measured for N 1024 .. 11264, K 1024 .. 11008.
+static float thin_us(int T, int N, int K, int s, int clusters) {
+  const int bn = thin_bn(T), tiles = (T + bn - 1) / bn * ((N + kThRows - 1) / kThRows), blocks = (K + kBK - 1) / kBK;
+  const int rounds = (tiles + clusters - 1) / clusters, own = (blocks + s - 1) / s;
+  const float end = s > 1 ? 1.2f + 0.03f * bn : 0.3f + 0.01f * bn;
+  const float us = 4.5f + rounds * own * (0.27f + 0.0004f * bn + (s > 1 ? 0.05f : 0.f)) + end * (rounds + 1) / 2;
+  return fmaxf(us, 4.5f + (float)N * K * 2 / 6e6f);
+}
+
+static int thin_split(int T, int N, int K, const int* clusters, float* us) {
+  int best = 1;
+  *us = 1e30f;
+  for (int i = 0, s = 1; i < 4 && s <= (K + kBK - 1) / kBK && clusters[i] > 0; s *= 2, ++i) {
+    const float t = thin_us(T, N, K, s, clusters[i]);
+    if (t < *us) {
+      *us = t;
+      best = s;
+    }
+  }
+  return best;
+}
+
+template <int BN, bool W_MN>
+static int launch_thin(const CUtensorMap& tw, const CUtensorMap& tx, ThinArgs a, cudaStream_t stream) {
+  auto kern = gemm_thin_kernel<BN, W_MN>;
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(kGemmThreads);
+  cfg.dynamicSmemBytes = ThinCfg<BN>::kSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  // clusters of 1, 2, 4, 8 CTAs that are resident together: a cluster lies within one GPC, so fewer than SMs / size
+  static int clusters[4] = {0, 0, 0, 0};
+  if (clusters[0] == 0) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ThinCfg<BN>::kSmemBytes);
+    if (e != cudaSuccess) return (int)e;
+    int found[4] = {0, 0, 0, 0}, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&found[0], cudaDevAttrMultiProcessorCount, dev);
+    for (int i = 1; i < 4; ++i) {
+      at[0].val.clusterDim.x = 1 << i;
+      cfg.gridDim = dim3(1 << i);
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&found[i], kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        found[i] = 0;
+      }
+    }
+    for (int i = 3; i >= 0; --i) clusters[i] = found[i];
+  }
+  const int tiles = (a.T + BN - 1) / BN * ((a.N + kThRows - 1) / kThRows);
+  float us;
+  if (a.split == 0) a.split = thin_split(a.T, a.N, a.K, clusters, &us);
+  a.split_log2 = __builtin_ctz(a.split);
+  const int fit = clusters[a.split_log2];
+  if (fit < 1) return -2;
+  cfg.gridDim = dim3((tiles < fit ? tiles : fit) * a.split);
+  at[0].val.clusterDim.x = a.split;
+  cfg.numAttrs = a.split > 1 ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tw, tx, a);
+  return e != cudaSuccess ? (int)e : launch_status();
+}
+
+}  // namespace ell
+
+using namespace ell;
+
+// The kernel for a product of T rows with an N x K weight: 0 the 128 x 256 tiles (or CTA pairs), 1 this file's, 2 the
+// matrix-vector kernel (16 rows and fewer).  Estimates in us, fitted to the same trains of launches as thin_us:
+//   tiles        4 + 0.39 a k-block and round of 148 tiles, at least 4 + the weight at 5.3 TB/s
+//   matrix-vector  3 + 2.6 per 1024 of K (its warps split K no further than 8 ways), at least 3 + the weight at 4.7 TB/s, 3.6
+//                with more than 8 rows; with so few columns that its CTAs do not fill the GPU it is the launch alone
+// E.g. 1 row, 4096 x 11008: 20.7 here, 34 matrix-vector, 68 tiles; 2048 x 1024: 6.7, 4.9, 10.8; 64 rows of 22016 x 4096: 41.8
+// here, 38.7 tiles.
+ELL_API int ell_gemm_thin_route(int T, int N, int K) {
+  // clusters of 1, 2, 4, 8 CTAs that fit on a B200
+  static const int clusters[4] = {148, 74, 36, 16};
+  if (T <= 0 || N <= 0 || K <= 0 || T > 256) return 0;
+  float thin;
+  thin_split(T, N, K, clusters, &thin);
+  const float bytes = (float)N * K * 2;
+  const int tiles = (T + 127) / 128 * ((N + 255) / 256), rounds = (tiles + kNumSMs - 1) / kNumSMs;
+  const float tiled = fmaxf(4.f + 0.39f * rounds * ((K + kBK - 1) / kBK), 4.f + bytes / 5.3e6f);
+  if (T <= 16) {
+    const float mv = N < 512 ? 3.f : fmaxf(3.f + 2.6e-3f * K, 3.f + bytes / (T <= 8 ? 4.7e6f : 3.6e6f));
+    if (mv <= thin && mv <= tiled) return 2;
+  }
+  return thin < tiled ? 1 : 0;
+}
+
+// out [T, N] rows of ldo = x [T, K] rows of ldx · W^T (+ bias [N], bf16 output only); W [N, K] (w_mn 0) or [K, N] (w_mn 1),
+// rows of ldw.  out_mode: 0 bf16, 1 fp32 +=, 2 fp32 =.  K, ldx, ldw multiples of 8, x and W on 16-byte boundaries.
+// split: CTAs per reduction, 0 for the rule above.
+ELL_API int ell_gemm_thin(const void* x, const void* W, void* out, const void* bias, int T, int N, int K, int ldx, int ldw,
+                          int ldo, int w_mn, int out_mode, int split, int* err, cudaStream_t stream) {
+  if (T <= 0 || N <= 0 || K <= 0) return 0;
+  if (out_mode < kOutBf16 || out_mode > kOutF32 || (bias && out_mode != kOutBf16)) return -2;
+  if (split != 0 && split != 1 && split != 2 && split != 4 && split != 8) return -2;
+  const int BN = thin_bn(T);
+  CUtensorMap tw, tx;
+  int rc = w_mn ? make_tmap_bf16_2d(&tw, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw * 2, 64, kBK)
+                : make_tmap_bf16_2d(&tw, W, (uint64_t)K, (uint64_t)N, (uint64_t)ldw * 2, kBK, kThRows);
+  if (!rc) rc = make_tmap_bf16_2d(&tx, x, (uint64_t)K, (uint64_t)T, (uint64_t)ldx * 2, kBK, BN);
+  if (rc) return rc;
+  if (split > (K + kBK - 1) / kBK) return -2;
+  const ThinArgs a{out, (const __nv_bfloat16*)bias, T, N, K, ldo, out_mode, split, 0, err};
+#define ELL_THIN(BN_)                                                                     \
+  if (BN == BN_) return w_mn ? launch_thin<BN_, true>(tw, tx, a, stream) : launch_thin<BN_, false>(tw, tx, a, stream);
+  ELL_THIN(16)
+  ELL_THIN(32)
+  ELL_THIN(64)
+  ELL_THIN(128)
+#undef ELL_THIN
+  return -3;
+}

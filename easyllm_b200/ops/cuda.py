@@ -8,6 +8,7 @@ this library (benchmarks report it).
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 import threading
 from ctypes import c_float, c_int, c_longlong, c_void_p
@@ -320,6 +321,35 @@ def _use_pair(M, N, bn):
     return _GEMM_PAIR and bn == 0 and M >= 256 and N >= 256 and (M % 256 == 0 or M >= 2048)
 
 
+@functools.lru_cache(maxsize=4096)
+def thin_route(T, N, K):
+    """The kernel of ``[T, K] x [N, K]ᵀ`` (``csrc/gemm_thin.cu``): 0 the tiled GEMMs, 1 the GEMM for few rows, 2 the
+    matrix-vector kernel."""
+    return lib().ell_gemm_thin_route(c_int(T), c_int(N), c_int(K))
+
+
+def matvec(x, ldx, w, bias, out, ldo, out_f32=False, accumulate=False, act_tanh=False, batch=1, strides=(0, 0, 0)):
+    if x.dtype not in (torch.bfloat16, torch.float32):
+        raise TypeError(f"matvec: bf16 or fp32 rows, got {x.dtype}")
+    _check(lib().ell_matvec(_p(x), _p(w), _p(bias), _p(out), *(c_longlong(s) for s in strides), c_int(batch),
+                            c_int(x.shape[-2]), c_int(w.shape[-2]), c_int(x.shape[-1]), c_int(ldx), c_int(ldo),
+                            c_int(out_f32), c_int(accumulate), c_int(act_tanh), c_int(x.dtype == torch.bfloat16), _stream()),
+           "matvec")
+    return out
+
+
+def gemm_thin(x, w, out, bias=None, ldx=None, ldw=None, ldo=None, w_mn=False, out_mode=0, split=0):
+    """``out [T, N] (+)= x [T, K] Wᵀ (+ bias)`` for few rows of ``x``; ``w [N, K]``, or ``[K, N]`` with ``w_mn``.  ``split``:
+    CTAs that share a reduction (0: chosen from the sizes)."""
+    T, K = x.shape
+    N = w.shape[1] if w_mn else w.shape[0]
+    rc = lib().ell_gemm_thin(_p(x), _p(w), _p(out), _p(bias), c_int(T), c_int(N), c_int(K), c_int(ldx or x.shape[1]),
+                             c_int(ldw or w.shape[1]), c_int(ldo or N), c_int(w_mn), c_int(out_mode), c_int(split),
+                             _p(err_flag(x.device)), _stream())
+    _check(rc, "gemm_thin")
+    return out
+
+
 def gemm(a, b, out=None, bias=None, a_mn=False, b_mn=False, out_mode=0, bn=0, pair=None):
     """``C = op(A) · op(B)ᵀ`` on tcgen05.  K-major operands are row-major ``[rows, K]``; MN-major
     operands are row-major ``[K, rows]``.  out_mode 0: bf16 C; 1: fp32 C += ; 2: fp32 C =.
@@ -342,6 +372,12 @@ def gemm(a, b, out=None, bias=None, a_mn=False, b_mn=False, out_mode=0, bn=0, pa
     want = torch.bfloat16 if out_mode == 0 else torch.float32
     if out.dtype != want or not out.is_contiguous() or tuple(out.shape) != (M, N):
         raise ValueError("gemm: bad output tensor")
+    if pair is None and bn == 0 and not a_mn and not (a.data_ptr() | b.data_ptr()) & 15:
+        route = thin_route(M, N, K)
+        if route == 2 and not b_mn and (bias is None or out_mode == 0):
+            return matvec(a, K, b, bias, out, N, out_f32=out_mode == 2, accumulate=out_mode == 1)
+        if route:
+            return gemm_thin(a, b, out, bias, w_mn=b_mn, out_mode=out_mode)
     if _use_pair(M, N, bn) if pair is None else pair:
         rc = lib().ell_gemm_bf16_pair(_p(a), _p(b), _p(out), _p(bias), c_int(M), c_int(N), c_int(K), c_int(a.shape[1]),
                                       c_int(b.shape[1]), c_int(N), c_int(1 if a_mn else 0), c_int(1 if b_mn else 0),

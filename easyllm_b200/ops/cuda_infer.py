@@ -43,8 +43,10 @@ def _gemm_fits(x, ldx, w, ldc, elem):
 
 
 def _gemm(x, ldx, w, bias, out, ldc, out_mode):
-    """Plain tcgen05 GEMM with explicit row strides."""
+    """tcgen05 GEMM with explicit row strides."""
     M, K, N = x.shape[0], x.shape[1], w.shape[0]
+    if cu.thin_route(M, N, K):
+        return cu.gemm_thin(x, w, out, bias, ldx, K, ldc, out_mode=out_mode)
     args = (_p(x), _p(w), _p(out), _p(bias), c_int(M), c_int(N), c_int(K), c_int(ldx), c_int(K), c_int(ldc), c_int(0),
             c_int(0), c_int(out_mode))
     if cu._use_pair(M, N, 0):
@@ -54,11 +56,9 @@ def _gemm(x, ldx, w, bias, out, ldc, out_mode):
     _check(lib().ell_gemm_bf16(*args, c_int(0), _p(err_flag(x.device)), _stream()), "gemm_bf16")
 
 
-def _matvec(x, ldx, w, bias, out, ldo, out_f32=False, accumulate=False, act_tanh=False, batch=1, strides=(0, 0, 0)):
-    _check(lib().ell_matvec(_p(x), _p(w), _p(bias), _p(out), *(c_longlong(s) for s in strides), c_int(batch),
-                            c_int(x.shape[-2]), c_int(w.shape[-2]), c_int(x.shape[-1]), c_int(ldx), c_int(ldo),
-                            c_int(out_f32), c_int(accumulate), c_int(act_tanh), _bf(x.dtype), _stream()), "matvec")
-    return out
+def _tensor_gemm(M, N, K, dtype):
+    """Whether the product runs on a TMA-fed GEMM where the operands allow it: not for a few rows of a small weight."""
+    return M > MATVEC_ROWS or (dtype == torch.bfloat16 and cu.thin_route(M, N, K) != 2)
 
 
 def linear(x, w, bias=None, out_f32=False, act=None):
@@ -73,7 +73,8 @@ def linear(x, w, bias=None, out_f32=False, act=None):
     if M > MATVEC_ROWS and x.dtype == torch.float32:
         y = torch.nn.functional.linear(x, w, bias)
         return torch.tanh(y) if act == "tanh" else y
-    if M > MATVEC_ROWS and _gemm_fits(x, ldx, w, ld, 4 if out_f32 or act else 2) and (bias is None or N % 8 == 0):
+    gemm = _tensor_gemm(M, N, x.shape[1], x.dtype) and (M > MATVEC_ROWS or not (act or (out_f32 and bias is not None)))
+    if gemm and _gemm_fits(x, ldx, w, ld, 4 if out_f32 or act else 2) and (bias is None or N % 8 == 0):
         if act == "tanh":
             z = torch.empty(M, ld, dtype=torch.float32, device=x.device)
             _gemm(x, ldx, w, bias, z, ld, 2)
@@ -84,7 +85,7 @@ def linear(x, w, bias=None, out_f32=False, act=None):
         _gemm(x, ldx, w, bias, y, ld, 2 if out_f32 else 0)
         return y[:, :N]
     y = torch.empty(M, ld, dtype=dt, device=x.device)
-    return _matvec(x, ldx, w, bias, y, ld, out_f32=out_f32, act_tanh=act == "tanh")[:, :N]
+    return cu.matvec(x, ldx, w, bias, y, ld, out_f32=out_f32, act_tanh=act == "tanh")[:, :N]
 
 
 def linear_batch(xs, w):
@@ -93,7 +94,7 @@ def linear_batch(xs, w):
     N = w.shape[1]
     y = torch.empty(n, M, N, dtype=xs.dtype, device=xs.device)
     if M <= MATVEC_ROWS or (xs.dtype == torch.bfloat16 and not _gemm_fits(xs[0], K, w[0], N, 2)):
-        return _matvec(xs, K, w, None, y, N, batch=n, strides=(M * K, N * K, M * N))
+        return cu.matvec(xs, K, w, None, y, N, batch=n, strides=(M * K, N * K, M * N))
     if xs.dtype == torch.float32:
         return torch.bmm(xs, w.transpose(1, 2), out=y)
     for i in range(n):
@@ -119,10 +120,10 @@ def linear_add_(acc, x, w):
         raise ValueError(f"linear_add_: {tuple(acc.shape)} += [{M}, {N}]")
     if M > MATVEC_ROWS and x.dtype == torch.float32:
         return acc.addmm_(x, w.t())
-    if M > MATVEC_ROWS and _gemm_fits(x, ldx, w, N, 4):
+    if _tensor_gemm(M, N, x.shape[1], x.dtype) and _gemm_fits(x, ldx, w, N, 4):
         _gemm(x, ldx, w, None, acc, N, 1)
         return acc
-    return _matvec(x, ldx, w, None, acc, N, accumulate=True)
+    return cu.matvec(x, ldx, w, None, acc, N, accumulate=True)
 
 
 # ---- elementwise -------------------------------------------------------------------------------

@@ -192,3 +192,56 @@ def test_lm_head_ce_autograd_matches_unfused(cu):
     torch.testing.assert_close(outs[0][2], outs[1][2], rtol=2e-2, atol=1e-5)
     ref_loss = torch.nn.functional.cross_entropy(x.float() @ w.float().t(), tgt, reduction="none")
     torch.testing.assert_close(outs[0][0], ref_loss, rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("split", [0, 1, 2, 4, 8])
+@pytest.mark.parametrize("T,N,K", [(1, 8, 8), (1, 128, 512), (16, 136, 520), (17, 4096, 1024), (32, 127, 640), (33, 264, 576),
+                                   (64, 11264, 512), (65, 256, 1032), (129, 384, 4096), (256, 1000, 768)])
+def test_gemm_for_few_rows(cu, T, N, K, split):
+    """Every width of the row tile and its remainders, weights in both orders, all outputs, rows inside wider ones; the split
+    reduction has the precision of the tiled kernel or better, and the same bits every time."""
+    if split > -(-K // 64):
+        pytest.skip("fewer k-blocks than CTAs")
+    torch.manual_seed(T * N + K)
+    wide = torch.randn(T, K + 24, device="cuda", dtype=torch.bfloat16)
+    x, w = wide[:, 8:8 + K], torch.randn(N, K, device="cuda", dtype=torch.bfloat16)
+    bias = torch.randn(N, device="cuda", dtype=torch.bfloat16)
+    ref = x.double() @ w.double().t()
+    ld = N + 16
+    out = torch.full((T, ld), 3.0, device="cuda", dtype=torch.bfloat16)
+    cu.gemm_thin(x, w, out, bias, ldx=wide.shape[1], ldo=ld, split=split)
+    _check(out[:, :N], (ref + bias.double()).float(), K)
+    assert (out[:, N:] == 3.0).all()
+    # fp32 sums of the tensor core: an ulp of the running sum for each 16 products (round towards zero)
+    bound = max(1, K // 16) * 2.0 ** -23
+    o32 = torch.empty(T, N, device="cuda")
+    cu.gemm_thin(x, w, o32, ldx=wide.shape[1], out_mode=2, split=split)
+    assert (o32.double() - ref).norm() <= bound * ref.norm()
+    acc = torch.randn(T, N, device="cuda")
+    want = acc.double() + ref
+    cu.gemm_thin(x, w, acc, ldx=wide.shape[1], out_mode=1, split=split)
+    assert (acc.double() - want).norm() <= bound * want.norm()
+    again = torch.empty_like(o32)
+    cu.gemm_thin(x, w, again, ldx=wide.shape[1], out_mode=2, split=split)
+    assert torch.equal(o32, again)
+    if N % 8 == 0:
+        cu.gemm_thin(x, w.t().contiguous(), again, ldx=wide.shape[1], w_mn=True, out_mode=2, split=split)
+        assert (again.double() - ref).norm() <= bound * ref.norm()
+    cu.check_err_flag()
+
+
+@pytest.mark.parametrize("T", [1, 16, 17, 100, 256])
+@pytest.mark.parametrize("N,K", [(1024, 2816), (256, 1024), (2048, 512)])
+def test_gemm_routes_agree(cu, T, N, K):
+    """What ``gemm`` picks by size gives what the tiled kernel gives, for every form it takes."""
+    torch.manual_seed(T + N)
+    a, w = (torch.randn(*s, device="cuda", dtype=torch.bfloat16) for s in ((T, K), (N, K)))
+    bias = torch.randn(N, device="cuda", dtype=torch.bfloat16)
+    wt = w.t().contiguous()
+    for kw in ({}, {"bias": bias}, {"out_mode": 2}, {"b_mn": True}, {"b_mn": True, "out_mode": 2}):
+        b = wt if kw.get("b_mn") else w
+        _check(cu.gemm(a, b, **kw), cu.gemm(a, b, pair=False, **kw).float(), K)
+    acc = torch.randn(T, N, device="cuda")
+    want = cu.gemm(a, w, out=acc.clone(), out_mode=1, pair=False)
+    _check(cu.gemm(a, w, out=acc, out_mode=1), want, K)
+    cu.check_err_flag()
