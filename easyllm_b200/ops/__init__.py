@@ -89,9 +89,15 @@ def _kern(x):
     return _BACKEND == "b200" and x.is_cuda and x.dtype == torch.bfloat16
 
 
+_CU = None
+
+
 def _cu():
-    from . import cuda
-    return cuda
+    global _CU
+    if _CU is None:
+        from . import cuda
+        _CU = cuda
+    return _CU
 
 
 def kernel_launches():
@@ -162,6 +168,8 @@ def _norm_ok(x, op):
 
 def rmsnorm(x, weight, eps=1e-6):
     if _norm_ok(x, "rmsnorm"):
+        if _cu().nothing_to_record():
+            return _cu().rmsnorm_fwd(x.reshape(-1, x.shape[-1]).contiguous(), None, weight, eps)[0].view(x.shape)
         return _RMSNorm.apply(x.reshape(-1, x.shape[-1]).contiguous(), weight, eps).view(x.shape)
     return ref.rmsnorm(x, weight, eps)
 
@@ -170,7 +178,8 @@ def add_rmsnorm(x, residual, weight, eps=1e-6):
     """Returns (norm(x + residual), x + residual)."""
     if _norm_ok(x, "add_rmsnorm"):
         H = x.shape[-1]
-        y, h = _AddRMSNorm.apply(x.reshape(-1, H).contiguous(), residual.reshape(-1, H).contiguous(), weight, eps)
+        x2, r2 = x.reshape(-1, H).contiguous(), residual.reshape(-1, H).contiguous()
+        y, h = _cu().rmsnorm_fwd(x2, r2, weight, eps)[:2] if _cu().nothing_to_record() else _AddRMSNorm.apply(x2, r2, weight, eps)
         return y.view(x.shape), h.view(x.shape)
     return ref.add_rmsnorm(x, residual, weight, eps)
 
@@ -238,10 +247,11 @@ def _gemm_ok(op, a, *dims):
     return True
 
 
-def matmul_nt(a, b, bias=None):
-    """a [M,K] · b [N,K]ᵀ → [M,N] (bf16)."""
+def matmul_nt(a, b, bias=None, few_rows=True):
+    """a [M,K] · b [N,K]ᵀ → [M,N] (bf16).  ``few_rows`` False keeps a short ``a`` on the tiled kernels too: the recorded
+    forward pass does, so that a loss does not change in its last bits with the number of tokens in the batch."""
     if _gemm_ok("matmul_nt", a, a.shape[-1], b.shape[-1], b.shape[0]):
-        return _cu().gemm(a, b, bias=bias)
+        return _cu().gemm(a, b, bias=bias, few_rows=few_rows)
     return F.linear(a, b, bias)
 
 
@@ -286,7 +296,7 @@ class _Linear(torch.autograd.Function):
     def forward(ctx, x, w, bias):
         ctx.save_for_backward(x, w)
         ctx.wref, ctx.bref = w, bias
-        return matmul_nt(x, w, bias)
+        return matmul_nt(x, w, bias, few_rows=False)
 
     @staticmethod
     def backward(ctx, dy):
@@ -308,7 +318,8 @@ class _Linear(torch.autograd.Function):
 
 def linear(x, w, bias=None):
     if _kern(x):
-        y = _Linear.apply(x.reshape(-1, x.shape[-1]).contiguous(), w, bias)
+        x2 = x.reshape(-1, x.shape[-1]).contiguous()
+        y = matmul_nt(x2, w, bias) if _cu().nothing_to_record() else _Linear.apply(x2, w, bias)
         return y if x.dim() == 2 else y.view(*x.shape[:-1], w.shape[0])
     return F.linear(x, w, bias)
 
@@ -335,13 +346,17 @@ class _LinearParts(torch.autograd.Function):
     an alias — nothing is concatenated, and the wgrad GEMM accumulates into the fused ``main_grad`` in one call."""
 
     @staticmethod
-    def forward(ctx, x, bias, *weights):
+    def fused(weights):
         alias = _adjacent_alias([w.detach() for w in weights])
-        W = alias if alias is not None else torch.cat([w.detach() for w in weights], 0)
+        return alias if alias is not None else torch.cat([w.detach() for w in weights], 0)
+
+    @staticmethod
+    def forward(ctx, x, bias, *weights):
+        W = _LinearParts.fused(weights)
         ctx.save_for_backward(x, W)
         ctx.wrefs = weights
         ctx.has_bias = bias is not None
-        return matmul_nt(x, W, bias)
+        return matmul_nt(x, W, bias, few_rows=False)
 
     @staticmethod
     def backward(ctx, dy):
@@ -373,7 +388,9 @@ def linear_parts(x, weights, biases=None):
     if biases is not None and all(b is not None for b in biases):
         bias = torch.cat(list(biases), 0)
     if _kern(x):
-        y = _LinearParts.apply(x.reshape(-1, x.shape[-1]).contiguous(), bias, *weights)
+        x2 = x.reshape(-1, x.shape[-1]).contiguous()
+        y = matmul_nt(x2, _LinearParts.fused(weights), bias) if _cu().nothing_to_record() else \
+            _LinearParts.apply(x2, bias, *weights)
         return y if x.dim() == 2 else y.view(*x.shape[:-1], y.shape[-1])
     return F.linear(x, torch.cat(list(weights), 0), bias)
 
@@ -441,7 +458,8 @@ def rope_packed(qkv, cos, sin, pos, n_q_heads, n_kv_heads, head_dim):
     if _kern(qkv):
         if head_dim % 16 == 0:
             pos32 = pos if pos.dtype == torch.int32 else pos.to(torch.int32)
-            return _RopePacked.apply(qkv, cos, sin, pos32, n_q_heads + n_kv_heads, head_dim)
+            rotate = _cu().rotate_ if _cu().nothing_to_record() else _RopePacked.apply
+            return rotate(qkv, cos, sin, pos32, n_q_heads + n_kv_heads, head_dim)
         note_fallback("rope", qkv, f"head_dim {head_dim} must be a multiple of 16")
     T = qkv.shape[0]
     nq, nk = n_q_heads * head_dim, n_kv_heads * head_dim
@@ -468,7 +486,8 @@ def glu(gate_up, activation="silu"):
     if _kern(gate_up):
         if activation in ("silu", "swiglu") and gate_up.shape[-1] % 16 == 0:
             W = gate_up.shape[-1]
-            return _SwiGLU.apply(gate_up.reshape(-1, W).contiguous()).view(*gate_up.shape[:-1], W // 2)
+            act = _cu().swiglu_fwd if _cu().nothing_to_record() else _SwiGLU.apply
+            return act(gate_up.reshape(-1, W).contiguous()).view(*gate_up.shape[:-1], W // 2)
         note_fallback("glu", gate_up, f"activation {activation!r} / width must be silu and a multiple of 16")
     F_ = gate_up.shape[-1] // 2
     return ref.GLU_ACTIVATIONS[activation](gate_up[..., :F_], gate_up[..., F_:])

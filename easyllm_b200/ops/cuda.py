@@ -54,13 +54,14 @@ _tls = threading.local()
 def _stream():
     """Current torch stream; also makes the device's context current on this thread for the
     library's own CUDA runtime (worker threads such as autograd's start without one)."""
-    dev = torch.cuda.current_device()
+    dev = torch._C._cuda_getDevice()
     if getattr(_tls, "dev", None) != dev:
         rc = lib().ell_set_device(c_int(dev))
         if rc != 0:
             raise KernelError(f"cudaSetDevice({dev}) failed with code {rc}")
         _tls.dev = dev
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    # torch.cuda.current_stream() builds a Stream object around this number: 8 us of the 25 that a launch cost here
+    return c_void_p(torch._C._cuda_getCurrentRawStream(dev))
 
 
 def _check(rc, name):
@@ -124,6 +125,13 @@ def scratch(nelem, dtype=torch.float32, tag="default"):
         b = torch.empty(max(int(nelem), 1), dtype=dtype, device=torch.device("cuda", dev))
         _scratch[key] = b
     return b
+
+
+def nothing_to_record():
+    """Whether a call may skip its autograd function (25 us of host time): no gradients are recorded, and neither a function
+    transform nor forward-mode differentiation is active, which the functions refuse."""
+    return not torch.is_grad_enabled() and not torch._C._are_functorch_transforms_active() and \
+        torch.autograd.forward_ad._current_level < 0
 
 
 # ---- norm ------------------------------------------------------------------------------------
@@ -201,6 +209,13 @@ def rope_(qkv, cos, sin, pos, n_rot_heads, head_dim, backward=False):
                         c_int(head_dim), c_int(1 if backward else 0), c_int(cos.shape[0]), _p(err_flag(qkv.device)),
                         _stream())
     _check(rc, "rope")
+    return qkv
+
+
+def rotate_(qkv, cos, sin, pos, n_rot_heads, head_dim):
+    """``rope_`` as an in-place operation that autograd's version check sees."""
+    rope_(qkv, cos, sin, pos, n_rot_heads, head_dim)
+    torch.autograd.graph.increment_version(qkv)
     return qkv
 
 
@@ -350,10 +365,11 @@ def gemm_thin(x, w, out, bias=None, ldx=None, ldw=None, ldo=None, w_mn=False, ou
     return out
 
 
-def gemm(a, b, out=None, bias=None, a_mn=False, b_mn=False, out_mode=0, bn=0, pair=None):
+def gemm(a, b, out=None, bias=None, a_mn=False, b_mn=False, out_mode=0, bn=0, pair=None, few_rows=True):
     """``C = op(A) · op(B)ᵀ`` on tcgen05.  K-major operands are row-major ``[rows, K]``; MN-major
     operands are row-major ``[K, rows]``.  out_mode 0: bf16 C; 1: fp32 C += ; 2: fp32 C =.
-    ``pair`` forces (True) or forbids (False) the CTA-pair kernel; None lets the shape decide."""
+    ``pair`` forces (True) or forbids (False) the CTA-pair kernel; None lets the shape decide, also on the kernels for few
+    rows unless ``few_rows`` is False."""
     _bf16c(a, "a"); _bf16c(b, "b")
     if a_mn:
         K, M = a.shape
@@ -372,7 +388,7 @@ def gemm(a, b, out=None, bias=None, a_mn=False, b_mn=False, out_mode=0, bn=0, pa
     want = torch.bfloat16 if out_mode == 0 else torch.float32
     if out.dtype != want or not out.is_contiguous() or tuple(out.shape) != (M, N):
         raise ValueError("gemm: bad output tensor")
-    if pair is None and bn == 0 and not a_mn and not (a.data_ptr() | b.data_ptr()) & 15:
+    if few_rows and pair is None and bn == 0 and not a_mn and not (a.data_ptr() | b.data_ptr()) & 15:
         route = thin_route(M, N, K)
         if route == 2 and not b_mn and (bias is None or out_mode == 0):
             return matvec(a, K, b, bias, out, N, out_f32=out_mode == 2, accumulate=out_mode == 1)
@@ -680,6 +696,12 @@ class _FlashAttnPacked(torch.autograd.Function):
 def flash_attention_packed(qkv, hq, hk, D, cu_seqlens, max_seqlen, scale, rope=None, row_start=None,
                            alibi_slopes=None):
     cos, sin, pos = rope if rope is not None else (None, None, None)
+    if nothing_to_record():
+        T = qkv.shape[0]
+        if cos is not None:
+            rotate_(qkv, cos, sin, pos, hq + hk, D)
+        rs = row_start if row_start is not None else _row_start(cu_seqlens, T, qkv.device)
+        return flash_attn_fwd(*_split_packed(qkv, hq, hk, D), rs, scale, alibi_slopes)[0].view(T, hq * D)
     return _FlashAttnPacked.apply(qkv, hq, hk, D, cu_seqlens, max_seqlen, scale, cos, sin, pos, row_start,
                                   alibi_slopes)
 
