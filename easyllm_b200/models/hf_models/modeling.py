@@ -265,12 +265,14 @@ class Attention(nn.Module):
         elif cache is not None:
             o = iops.attention_rows(q, cache.k.view(-1, self.hk, self.d), cache.v.view(-1, self.hk, self.dv),
                                     meta["kv_base"], meta["kv_len"], meta.get("kv_bound", meta["max_position"]),
-                                    self.scale, sink, sl)
+                                    self.scale, sink, sl, cu_seqlens=None if meta["one_token"] else meta["cu_seqlens"],
+                                    max_q=meta["max_seqlen"])
         else:
             cu = meta["cu_seqlens"].long()
             start = torch.repeat_interleave(cu[:-1], cu[1:] - cu[:-1], output_size=T)
             n = torch.arange(T, device=q.device) - start + 1
-            o = iops.attention_rows(q, k, v, start.int(), n.int(), meta["max_seqlen"], self.scale, sink, sl)
+            o = iops.attention_rows(q, k, v, start.int(), n.int(), meta["max_seqlen"], self.scale, sink, sl,
+                                    cu_seqlens=meta["cu_seqlens"], max_q=meta["max_seqlen"])
         return o.reshape(T, self.hq * self.dv)
 
     def forward(self, x, meta, cache=None, residual=None):

@@ -31,6 +31,7 @@ struct AttnRowsArgs {
   const void* gate;               // [n, ldg] of the activation type, or null
   int ldg;
   int* err;                       // error word (latent kernel)
+  int all_ranges;                 // every range has a triple of every row
 };
 
 // Keys row t sees: the last min(len, window) of its rows.
@@ -280,7 +281,7 @@ __global__ void __launch_bounds__(kArThreads) attn_rows_merge_kernel(const AttnR
   __shared__ float weight[kArMaxSplits];
   const int t = blockIdx.x, h = blockIdx.y, step = a.dv + 2;
   const float* pt = a.part + ((size_t)t * a.H + h) * a.splits * step;
-  const int used = min(a.splits, (row_keys(a, t).len + a.range - 1) / a.range);
+  const int used = a.all_ranges ? a.splits : min(a.splits, (row_keys(a, t).len + a.range - 1) / a.range);
   if (threadIdx.x < 32) {
     const int s0 = threadIdx.x, s1 = threadIdx.x + 32;
     const float m0 = s0 < used ? pt[(size_t)s0 * step] : -INFINITY, m1 = s1 < used ? pt[(size_t)s1 * step] : -INFINITY;
@@ -565,6 +566,538 @@ attn_latent_kernel(const __grid_constant__ CUtensorMap tmK, const AttnRowsArgs a
     }
 }
 
+// ---- bf16 rows over cached keys on mma.sync ------------------------------------------------------------
+// Decoding reads every cached key and value once for a few query rows: bound by those bytes, if the arithmetic keeps up.
+// On the FMA pipe it did not (230 us for 64 rows x 2048 keys x 8 key heads, 537 MB, which take 81; 134 here); and a continued prompt read its whole
+// context once per token (1060 us for 301 tokens over 3000, 50 here).  Here a tile of 16 rows is the consecutive tokens of one
+// sequence times the query heads of one key head, and m16n8k16 does the products:
+//   scores  exact bf16 products, fp32 sums, scale and bias applied in fp32
+//   values  the fp32 weights go in as two bf16 parts (value and remainder), so they keep 16 bits of mantissa
+//   attn_few_kernel   up to 16 rows (decoding).  Keys are the M side of both products and rows the N side, so 8 rows cost
+//                     half of 16: S^T = K q^T, O^T = V^T P^T.  The four warps take units of 16 keys in turn, each with a
+//                     softmax, accumulators and a ring of cp.async stages of its own; no barrier until their results meet.
+//                     Rows on the M side took 977 instructions a unit and 232 registers, and stayed at 162 us, bound by
+//                     the latency of eight warps an SM.
+//   attn_tile_kernel  more rows (continued prompts): a warp owns 16 of the CTA's 64 rows, tiles of 64 keys are shared
+// Ranges of keys and their merge are those of attn_rows_kernel.
+constexpr int kAtThreads = 128, kAtKRow = 256, kAtStages = 3;      // bytes of a key / value row in shared memory (up to 128)
+constexpr int kAtHeads = 16;                                       // most query heads of a CTA
+constexpr int kAtTile = 64, kAtUnit = 32, kAtRows = 64;            // attn_tile_kernel: keys of a stage, of a softmax step; rows
+constexpr int kAtStage = 2 * kAtTile * kAtKRow, kAtSmem = kAtStages * kAtStage;
+constexpr int kAfKeys = 16, kAfStage = 2 * kAfKeys * kAtKRow;      // attn_few_kernel: keys of a warp's unit
+constexpr int kAfSmem = 4 * kAtStages * kAfStage;
+
+__device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ uint32_t at_place(int row, int piece) {       // 16-byte piece of a row, no bank conflicts in ldmatrix
+  return (uint32_t)(row * kAtKRow + ((piece ^ (row & 7)) << 4));
+}
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+// x as a bf16 pair and the pair of what is left
+__device__ __forceinline__ void split_bf16(float x, float y, uint32_t& part, uint32_t& rest) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+  part = *reinterpret_cast<const uint32_t*>(&v);
+  rest = pack_bf16(x - __low2float(v), y - __high2float(v));
+}
+
+// What a thread keeps of its rows g and g + 8 (g = lane / 4).
+struct AtRows {
+  float m[2], l[2];                 // maximum; this lane's share of the sum
+  int first[2], end[2];             // keys the row sees, counted from the sequence's first row
+  float slope[2];
+};
+
+template <int UK>
+__device__ __forceinline__ void at_unit(const uint8_t* ks, const uint8_t* vs, int key0, bool mask, bool bias, float scale,
+                                        int ksteps, int vtiles, const uint32_t (&q)[8][4], AtRows& r, float (&acc)[16][4]) {
+  const int lane = threadIdx.x & 31, quad = lane >> 3, l8 = lane & 7, t = lane & 3;
+  float s[UK / 8][4];
+#pragma unroll
+  for (int n = 0; n < UK / 8; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s[n][i] = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    if (k < ksteps) {
+#pragma unroll
+      for (int n = 0; n < UK / 16; ++n) {
+        uint32_t b[4];
+        ldsm4(b, ks + at_place(n * 16 + (quad >> 1) * 8 + l8, k * 2 + (quad & 1)));
+        mma_bf16(s[2 * n], q[k], b[0], b[1]);
+        mma_bf16(s[2 * n + 1], q[k], b[2], b[3]);
+      }
+    }
+  }
+  float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+  for (int n = 0; n < UK / 8; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int h = i >> 1, key = key0 + n * 8 + 2 * t + (i & 1);
+      float x = s[n][i] * scale;
+      if (bias) x += r.slope[h] * (float)(key - (r.end[h] - 1));
+      if (mask && (key < r.first[h] || key >= r.end[h])) x = -INFINITY;
+      s[n][i] = x;
+      mx[h] = fmaxf(mx[h], x);
+    }
+  float al[2];
+  bool grew = false;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
+    mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
+    const float m = fmaxf(r.m[h], mx[h]);
+    grew |= m > r.m[h];
+    al[h] = m == -INFINITY ? 1.f : expf(r.m[h] - m);               // no key yet: nothing to rescale
+    r.m[h] = m;
+    r.l[h] *= al[h];
+  }
+  if (__any_sync(0xffffffffu, grew)) {
+#pragma unroll
+    for (int n = 0; n < 16; ++n) {
+      acc[n][0] *= al[0];
+      acc[n][1] *= al[0];
+      acc[n][2] *= al[1];
+      acc[n][3] *= al[1];
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < UK / 8; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int h = i >> 1;
+      s[n][i] = r.m[h] == -INFINITY ? 0.f : expf(s[n][i] - r.m[h]);
+      r.l[h] += s[n][i];
+    }
+#pragma unroll
+  for (int k = 0; k < UK / 16; ++k) {
+    uint32_t hi[4], lo[4];
+    split_bf16(s[2 * k][0], s[2 * k][1], hi[0], lo[0]);
+    split_bf16(s[2 * k][2], s[2 * k][3], hi[1], lo[1]);
+    split_bf16(s[2 * k + 1][0], s[2 * k + 1][1], hi[2], lo[2]);
+    split_bf16(s[2 * k + 1][2], s[2 * k + 1][3], hi[3], lo[3]);
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      if (n < vtiles) {
+        uint32_t b[4];
+        ldsm4_t(b, vs + at_place(k * 16 + (quad & 1) * 8 + l8, n * 2 + (quad >> 1)));
+        mma_bf16(acc[2 * n], hi, b[0], b[1]);
+        mma_bf16(acc[2 * n + 1], hi, b[2], b[3]);
+        mma_bf16(acc[2 * n], lo, b[0], b[1]);
+        mma_bf16(acc[2 * n + 1], lo, b[2], b[3]);
+      }
+    }
+  }
+}
+
+// One warp copies or four do: sixteen lanes take a row of KEYS keys and values, a 16-byte piece each.  Rows past the range are
+// zero-filled: their weight is 0, and 0 times what lies there must be 0.
+template <int KEYS, int THREADS>
+struct AtLoader {
+  const __nv_bfloat16 *kb, *vb;      // first row of the range
+  int piece, row_in, keys, ldk, ldv;
+  bool k_in, v_in;
+  __device__ __forceinline__ AtLoader(const AttnRowsArgs& a, size_t base, int g, int k0, int k1, int who) {
+    piece = who & 15;
+    row_in = who >> 4;
+    kb = reinterpret_cast<const __nv_bfloat16*>(a.k) + (base + k0) * a.ldk + (size_t)g * a.d + piece * 8;
+    vb = reinterpret_cast<const __nv_bfloat16*>(a.v) + (base + k0) * a.ldv + (size_t)g * a.dv + piece * 8;
+    keys = k1 - k0;
+    ldk = a.ldk;
+    ldv = a.ldv;
+    k_in = piece < a.d / 8;
+    v_in = piece < a.dv / 8;
+  }
+  __device__ __forceinline__ void load(int tile, uint8_t* stage) const {
+    const int first = tile * KEYS;
+    if (first < keys) {
+#pragma unroll
+      for (int i = 0; i < KEYS * 16 / THREADS; ++i) {
+        const int row = row_in + i * (THREADS / 16);
+        const bool in = first + row < keys;
+        const size_t at = in ? first + row : 0;
+        uint8_t* dst = stage + at_place(row, piece);
+        if (k_in) cp_async16_zfill(dst, kb + at * ldk, in);
+        if (v_in) cp_async16_zfill(dst + KEYS * kAtKRow, vb + at * ldv, in);
+      }
+    }
+    cp_async_commit();
+  }
+};
+
+// The tokens, heads and keys of a CTA.  blockIdx.x: tile of `tt` tokens of a sequence (cu null: one token each), y: key head
+// and group of its query heads, z: range of keys.
+struct AtTile {
+  int r0, r1, g, h0, nh, rows, k0, k1, len0, last_first;
+  size_t base;
+  __device__ __forceinline__ bool init(const AttnRowsArgs& a, const int* cu, int tiles, int tt) {
+    if (cu != nullptr) {
+      const int seq = blockIdx.x / tiles;
+      r0 = cu[seq] + blockIdx.x % tiles * tt;
+      r1 = min(r0 + tt, cu[seq + 1]);
+      if (r0 >= r1) return false;
+    } else {
+      r0 = blockIdx.x;
+      r1 = r0 + 1;
+    }
+    const int rep = a.H / a.G, groups = (rep + kAtHeads - 1) / kAtHeads;
+    g = blockIdx.y / groups;
+    h0 = g * rep + blockIdx.y % groups * kAtHeads;
+    nh = min(kAtHeads, (g + 1) * rep - h0);
+    rows = (r1 - r0) * nh;
+    base = a.base[r0];
+    len0 = a.len[r0];
+    const int len1 = a.len[r1 - 1];
+    last_first = max(0, len1 - a.window);
+    k0 = max(0, len0 - a.window) + (int)blockIdx.z * a.range;
+    k1 = min(k0 + a.range, len1);
+    return true;
+  }
+  __device__ __forceinline__ int token(int m) const { return r0 + m / nh; }
+  __device__ __forceinline__ int head(int m) const { return h0 + m % nh; }
+  // where row m goes: its place in `out` (with the factor of its sums), or the triple of this range
+  __device__ __forceinline__ __nv_bfloat16* place(const AttnRowsArgs& a, int m, float mx, float l, float& f, float*& part) const {
+    const size_t th = (size_t)token(m) * a.H + head(m);
+    part = nullptr;
+    f = 1.f;
+    if (a.splits > 1) {
+      part = a.part + (th * a.splits + blockIdx.z) * (a.dv + 2);
+      return nullptr;
+    }
+    float den = l;
+    if (a.sink != nullptr) {
+      const float sk = a.sink[head(m)], mm = fmaxf(mx, sk);
+      f = expf(mx - mm);
+      den = l * f + expf(sk - mm);
+    }
+    f = f / den * row_gate<__nv_bfloat16>(a, token(m), head(m));
+    return reinterpret_cast<__nv_bfloat16*>(a.out) + th * a.dv;
+  }
+};
+
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
+  uint32_t y;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+  return y;
+}
+
+// NB: groups of 8 rows.
+template <int NB>
+__global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const AttnRowsArgs a, const int* __restrict__ cu, int tiles, int tt) {
+  extern __shared__ __align__(128) uint8_t atsm[];
+  AtTile T;
+  if (!T.init(a, cu, tiles, tt)) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, t = lane & 3, quad = lane >> 3, l8 = lane & 7;
+  const AtLoader<kAfKeys, 32> loader(a, T.base, T.g, T.k0, T.k1, lane);
+  uint8_t* ring = atsm + warp * kAfStage * kAtStages;
+  const int n_units = T.k1 > T.k0 ? (T.k1 - T.k0 + kAfKeys - 1) / kAfKeys : 0;
+#pragma unroll
+  for (int i = 0; i < kAtStages - 1; ++i) loader.load(warp + i * 4, ring + i * kAfStage);
+
+  const int ksteps = a.d / 16, vtiles = a.dv / 16;
+  uint32_t q[NB][8][2];                              // B operand: row gr of the group
+  float m[NB][2], l[NB][2], slope[NB][2];            // of rows 2 t, 2 t + 1: maximum, this lane's share of the sum
+  int first[NB][2], end[NB][2];                      // keys they see
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    const int r = min(b * 8 + gr, T.rows - 1);       // rows past the end repeat the last
+    const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(a.q) + (size_t)T.token(r) * a.ldq + (size_t)T.head(r) * a.d + 2 * t;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) q[b][k][c] = k < ksteps ? *reinterpret_cast<const uint32_t*>(src + k * 16 + c * 8) : 0u;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int n = min(b * 8 + 2 * t + j, T.rows - 1);
+      end[b][j] = a.len[T.token(n)];
+      first[b][j] = max(0, end[b][j] - a.window);
+      slope[b][j] = a.slopes != nullptr ? a.slopes[T.head(n)] : 0.f;
+      m[b][j] = -INFINITY;
+      l[b][j] = 0.f;
+    }
+  }
+  float acc[8][NB][4];                               // 16 value columns x 8 rows each
+#pragma unroll
+  for (int n = 0; n < 8; ++n)
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[n][b][i] = 0.f;
+
+  const uint32_t k_row = (quad & 1) * 8 + l8, v_row = (quad >> 1) * 8 + l8;          // & 7 = l8
+  int stage = 0;
+  for (int u = warp; u < n_units; u += 4) {
+    cp_async_wait<kAtStages - 2>();
+    __syncwarp();
+    loader.load(u + (kAtStages - 1) * 4, ring + (stage == 0 ? kAtStages - 1 : stage - 1) * kAfStage);   // free since the step before
+    const uint8_t* ks = ring + stage * kAfStage + k_row * kAtKRow;
+    const uint8_t* vs = ring + stage * kAfStage + kAfKeys * kAtKRow + v_row * kAtKRow;
+    stage = stage == kAtStages - 1 ? 0 : stage + 1;
+    float s[NB][4], s2[NB][4];                       // two chains of sums
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s[b][i] = s2[b][i] = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (k < ksteps) {
+        uint32_t x[4];
+        ldsm4(x, ks + (((k * 2 + (quad >> 1)) ^ l8) << 4));
+#pragma unroll
+        for (int b = 0; b < NB; ++b) mma_bf16(k & 1 ? s2[b] : s[b], x, q[b][k][0], q[b][k][1]);
+      }
+    }
+    const int key0 = T.k0 + u * kAfKeys;
+    const bool mask = key0 + kAfKeys > min(T.len0, T.k1) || key0 < T.last_first;
+    float al[NB][2];
+    bool grew = false;
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s[b][i] = (s[b][i] + s2[b][i]) * a.scale;
+      if (a.slopes != nullptr || mask) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int j = i & 1, key = key0 + gr + (i >> 1) * 8;
+          s[b][i] += slope[b][j] * (float)(key - (end[b][j] - 1));
+          if (key < first[b][j] || key >= end[b][j]) s[b][i] = -INFINITY;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        float mx = fmaxf(s[b][j], s[b][j + 2]);
+#pragma unroll
+        for (int o = 4; o <= 16; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float now = fmaxf(m[b][j], mx);
+        grew |= now > m[b][j];
+        al[b][j] = now == -INFINITY ? 1.f : expf(m[b][j] - now);       // no key yet: nothing to rescale
+        m[b][j] = now;
+        const float ref = now == -INFINITY ? 0.f : now;
+        s[b][j] = expf(s[b][j] - ref);
+        s[b][j + 2] = expf(s[b][j + 2] - ref);
+        l[b][j] = l[b][j] * al[b][j] + (s[b][j] + s[b][j + 2]);
+      }
+    }
+    if (__any_sync(0xffffffffu, grew)) {
+#pragma unroll
+      for (int n = 0; n < 8; ++n)
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) acc[n][b][i] *= al[b][i & 1];
+    }
+    uint32_t hi[NB][2], lo[NB][2];                   // weights as the B operand: keys 2 t .. of row gr
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        split_bf16(s[b][2 * c], s[b][2 * c + 1], hi[b][c], lo[b][c]);
+        hi[b][c] = transpose_8x8(hi[b][c]);
+        lo[b][c] = transpose_8x8(lo[b][c]);
+      }
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      if (n < vtiles) {
+        uint32_t x[4];
+        ldsm4_t(x, vs + (((n * 2 + (quad & 1)) ^ l8) << 4));
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          mma_bf16(acc[n][b], x, hi[b][0], hi[b][1]);
+          mma_bf16(acc[n][b], x, lo[b][0], lo[b][1]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int b = 0; b < NB; ++b)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int o = 4; o <= 16; o <<= 1) l[b][j] += __shfl_xor_sync(0xffffffffu, l[b][j], o);
+
+  cp_async_wait<0>();
+  __syncthreads();
+  float* stat = reinterpret_cast<float*>(atsm);      // [warp][16 rows] maximum | sum
+  float* sums = stat + 128;                          // [warp][16 rows][ld]
+  const int ld = a.dv + 8;
+  if (gr == 0) {
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        stat[warp * 16 + b * 8 + 2 * t + j] = m[b][j];
+        stat[64 + warp * 16 + b * 8 + 2 * t + j] = l[b][j];
+      }
+  }
+#pragma unroll
+  for (int n = 0; n < 8; ++n) {
+    if (n < vtiles) {
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          sums[(size_t)(warp * 16 + b * 8 + 2 * t + (i & 1)) * ld + n * 16 + gr + (i >> 1) * 8] = acc[n][b][i];
+    }
+  }
+  __syncthreads();
+  for (int r = warp; r < T.rows; r += 4) {
+    float mx = -INFINITY, sum = 0.f, w[4], f;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) mx = fmaxf(mx, stat[x * 16 + r]);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const float mw = stat[x * 16 + r];
+      w[x] = mw == -INFINITY ? 0.f : expf(mw - mx);
+      sum += w[x] * stat[64 + x * 16 + r];
+    }
+    float* part;
+    __nv_bfloat16* out = T.place(a, r, mx, sum, f, part);
+    if (part != nullptr && lane == 0) {
+      part[0] = mx;
+      part[1] = sum;
+    }
+    for (int c = lane * 2; c < a.dv; c += 64) {
+      float2 o = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const float2 v = *reinterpret_cast<const float2*>(sums + (size_t)(x * 16 + r) * ld + c);
+        o.x = fmaf(w[x], v.x, o.x);
+        o.y = fmaf(w[x], v.y, o.y);
+      }
+      if (part != nullptr) *reinterpret_cast<float2*>(part + 2 + c) = o;
+      else *reinterpret_cast<__nv_bfloat162*>(out + c) = __floats2bfloat162_rn(o.x * f, o.y * f);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kAtThreads, 2) attn_tile_kernel(const AttnRowsArgs a, const int* __restrict__ cu, int tiles, int tt) {
+  extern __shared__ __align__(128) uint8_t atsm[];
+  AtTile T;
+  if (!T.init(a, cu, tiles, tt)) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, t = lane & 3;
+  const int ksteps = a.d / 16, vtiles = a.dv / 16, row0 = warp * 16;
+  const AtLoader<kAtTile, kAtThreads> loader(a, T.base, T.g, T.k0, T.k1, threadIdx.x);
+#pragma unroll
+  for (int i = 0; i < kAtStages - 1; ++i) loader.load(i, atsm + i * kAtStage);
+  uint32_t q[8][4];
+  AtRows r;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int m = min(row0 + gr + 8 * h, T.rows - 1), tok = T.token(m), head = T.head(m);      // rows past the end repeat the last
+    const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(a.q) + (size_t)tok * a.ldq + (size_t)head * a.d + 2 * t;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) q[k][2 * c + h] = k < ksteps ? *reinterpret_cast<const uint32_t*>(src + k * 16 + c * 8) : 0u;
+    r.end[h] = a.len[tok];
+    r.first[h] = max(0, r.end[h] - a.window);
+    r.slope[h] = a.slopes != nullptr ? a.slopes[head] : 0.f;
+    r.m[h] = -INFINITY;
+    r.l[h] = 0.f;
+  }
+  float acc[16][4];
+#pragma unroll
+  for (int n = 0; n < 16; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
+  const int n_tiles = T.k1 > T.k0 ? (T.k1 - T.k0 + kAtTile - 1) / kAtTile : 0;
+  for (int tile = 0; tile < n_tiles; ++tile) {
+    cp_async_wait<kAtStages - 2>();
+    __syncthreads();
+    loader.load(tile + kAtStages - 1, atsm + (tile + kAtStages - 1) % kAtStages * kAtStage);   // free since the step before
+    const uint8_t* ks = atsm + tile % kAtStages * kAtStage;
+    const uint8_t* vs = ks + kAtTile * kAtKRow;
+    if (row0 < T.rows) {
+#pragma unroll 1
+      for (int u = 0; u < kAtTile; u += kAtUnit) {
+        const int key = T.k0 + tile * kAtTile + u;
+        if (key >= T.k1) break;
+        const bool mask = key + kAtUnit > min(T.len0, T.k1) || key < T.last_first;
+        at_unit<kAtUnit>(ks + u * kAtKRow, vs + u * kAtKRow, key, mask, a.slopes != nullptr, a.scale, ksteps, vtiles, q, r, acc);
+      }
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    r.l[h] += __shfl_xor_sync(0xffffffffu, r.l[h], 1);
+    r.l[h] += __shfl_xor_sync(0xffffffffu, r.l[h], 2);
+    const int m = row0 + gr + 8 * h;
+    if (m >= T.rows) continue;
+    float f, *part;
+    __nv_bfloat16* out = T.place(a, m, r.m[h], r.l[h], f, part);
+    if (part != nullptr && t == 0) {
+      part[0] = r.m[h];
+      part[1] = r.l[h];
+    }
+#pragma unroll
+    for (int n = 0; n < 16; ++n) {
+      if (n < 2 * vtiles) {
+        const int c = n * 8 + 2 * t;
+        if (part != nullptr) *reinterpret_cast<float2*>(part + 2 + c) = make_float2(acc[n][2 * h], acc[n][2 * h + 1]);
+        else *reinterpret_cast<__nv_bfloat162*>(out + c) = __floats2bfloat162_rn(acc[n][2 * h] * f, acc[n][2 * h + 1] * f);
+      }
+    }
+  }
+}
+
+// How a call runs on these kernels: tokens and CTAs of a tile, ranges of keys.  One sequence per `cu` entry, or one token
+// each.  Ranges are of 128 keys at least.
+struct AtPlan {
+  bool fits, few;
+  int tt, tiles, splits, range;
+};
+static AtPlan at_plan(int n, int n_seq, int max_q, int H, int G, int d, int dv, int max_len, int window, bool is_bf16) {
+  AtPlan p{};
+  p.fits = is_bf16 && d % 16 == 0 && dv % 16 == 0 && d <= 128 && dv <= 128 && d > 0 && dv > 0;
+  if (!p.fits) return p;
+  const int rep = H / G, groups = (rep + kAtHeads - 1) / kAtHeads, nh = rep < kAtHeads ? rep : kAtHeads;
+  const bool one = n_seq <= 0 || max_q <= 1;
+  p.few = one || max_q * nh <= 16;
+  p.tt = one ? 1 : (p.few ? 16 : kAtRows) / nh;
+  p.tiles = one ? 1 : (max_q + p.tt - 1) / p.tt;
+  const long long ctas = (long long)(one ? n : n_seq * p.tiles) * G * groups;
+  if (window > 0 && max_len > window) max_len = window;
+  max_len += p.tt - 1;                                  // a tile's rows see windows that start apart
+  // the two CTAs that fit an SM: one round of long ranges (8 x 4096 keys x 8 heads: 41.5 us at 5 ranges, 55 at 3, 50 at 28);
+  // the tiles of continued prompts differ in length, so they are dealt finer
+  long long s = p.few ? (2LL * kNumSMs + ctas / 2) / ctas : (4LL * kNumSMs + ctas - 1) / ctas;
+  const long long most = (max_len + 127) / 128;
+  if (s > most) s = most;
+  if (s > kArMaxSplits) s = kArMaxSplits;
+  p.splits = s < 1 ? 1 : (int)s;
+  p.range = ((max_len + p.splits - 1) / p.splits + 63) / 64 * 64;
+  return p;
+}
+
+template <typename Kernel>
+static int launch_at(Kernel kern, int smem, bool& configured, const AttnRowsArgs& a, const AtPlan& p, const int* cu, int n_seq,
+                     cudaStream_t stream) {
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  const int rep = a.H / a.G, groups = (rep + kAtHeads - 1) / kAtHeads;
+  const bool one = p.tt == 1;
+  dim3 grid(one ? a.n : n_seq * p.tiles, a.G * groups, p.splits);
+  if (grid.y > 65535) return -2;
+  kern<<<grid, kAtThreads, smem, stream>>>(a, one ? nullptr : cu, p.tiles, p.tt);
+  if (a.splits > 1) attn_rows_merge_kernel<__nv_bfloat16><<<dim3(a.n, a.H), kArThreads, 0, stream>>>(a);
+  return launch_status();
+}
+static int launch_attn_tile(const AttnRowsArgs& a, const AtPlan& p, const int* cu, int n_seq, cudaStream_t stream) {
+  static bool few8 = false, few16 = false, tile = false;
+  if (!p.few) return launch_at(attn_tile_kernel, kAtSmem, tile, a, p, cu, n_seq, stream);
+  const int rep = a.H / a.G;
+  return p.tt * (rep < kAtHeads ? rep : kAtHeads) <= 8 ? launch_at(attn_few_kernel<1>, kAfSmem, few8, a, p, cu, n_seq, stream)
+                                                       : launch_at(attn_few_kernel<2>, kAfSmem, few16, a, p, cu, n_seq, stream);
+}
+
 static int al_mt(int H) { return H > 16 ? 2 : 1; }
 
 // Ranges per row of the latent kernel: one CTA an SM, at least one tile each.
@@ -643,32 +1176,45 @@ static int launch_attn_rows(const AttnRowsArgs& a, dim3 grid, bool vec, cudaStre
 
 using namespace ell;
 
-// Scratch floats a call needs (0: none).
-ELL_API long long ell_attn_rows_scratch(int n, int H, int G, int dv, int max_len) {
-  const int s = attn_rows_splits(n, H, G, max_len);
+// Scratch floats a call needs (0: none).  The sizes are those of ell_attn_rows.
+ELL_API long long ell_attn_rows_scratch(int n, int H, int G, int d, int dv, int max_len, int window, int n_seq, int max_q,
+                                        int is_bf16) {
+  const AtPlan p = at_plan(n, n_seq, max_q, H, G, d, dv, max_len, window, is_bf16);
+  const int most = window > 0 && max_len > window ? window : max_len, rows = attn_rows_splits(n, H, G, most);
+  const int s = p.fits && p.splits > rows ? p.splits : rows;       // enough for either kernel
   return s == 1 ? 0 : (long long)n * H * s * (dv + 2);
 }
 
 // Rows of ldq / ldk / ldv elements; max_len bounds len[] (it sets the number of ranges, longer rows would be cut).
 // window: keys a row sees (<= 0: all).  gate: rows of ldg elements of the activation type, or null.
+// cu [n_seq + 1] (or null): rows cu[i] .. cu[i + 1] - 1 are consecutive tokens of one sequence, with one base and lengths that
+// grow by one; max_q bounds their number.
 ELL_API int ell_attn_rows(const void* q, const void* k, const void* v, void* out, float* part, const int* base,
                           const int* len, const float* sink, const float* slopes, const void* gate, int n, int H, int G,
                           int d, int dv, int ldq, int ldk, int ldv, int ldg, int max_len, int window, float scale,
-                          int is_bf16, cudaStream_t stream) {
+                          const int* cu, int n_seq, int max_q, int is_bf16, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (H % G || dv > 8 * kArThreads || H > 65535) return -2;
+  const AtPlan p = at_plan(n, cu != nullptr ? n_seq : 0, max_q, H, G, d, dv, max_len, window, is_bf16);
   if (window <= 0) window = 0x7fffffff;
   if (max_len > window) max_len = window;
-  AttnRowsArgs a{q, k, v, out, part, base, len, sink, slopes, n, H, G, d, dv, ldq, ldk, ldv, 1, 0, scale, window, gate, ldg, nullptr};
+  AttnRowsArgs a{q, k, v, out, part, base, len, sink, slopes, n, H, G, d, dv, ldq, ldk, ldv, 1, 0, scale, window, gate, ldg, nullptr, 0};
+  const int esz = is_bf16 ? 2 : 4;
+  const bool vec = (d * esz) % 16 == 0 && (dv * esz) % 16 == 0 && (ldk * esz) % 16 == 0 && (ldv * esz) % 16 == 0 &&
+                   aligned_to(k, 16) && aligned_to(v, 16);
+  if (p.fits && vec && ldq % 2 == 0 && aligned_to(q, 4)) {
+    a.splits = p.splits;
+    a.range = p.range;
+    a.all_ranges = p.tt > 1;
+    if (a.splits > 1 && part == nullptr) return -2;
+    return launch_attn_tile(a, p, cu, n_seq, stream);
+  }
   a.splits = attn_rows_splits(n, H, G, max_len);
   a.range = ((max_len + a.splits - 1) / a.splits + 63) / 64 * 64;
   if (a.splits > 1 && part == nullptr) return -2;
   const int rep = H / G, per = ar_rep(rep);
   dim3 grid(n, G * ((rep + per - 1) / per), a.splits);
-  const int esz = is_bf16 ? 2 : 4;
   if (ar_layout(d, dv, esz, 16, per).bytes > 227 * 1024) return -2;
-  const bool vec = (d * esz) % 16 == 0 && (dv * esz) % 16 == 0 && (ldk * esz) % 16 == 0 && (ldv * esz) % 16 == 0 &&
-                   aligned_to(k, 16) && aligned_to(v, 16);
   if (is_bf16)
     return per == 4 ? launch_attn_rows<__nv_bfloat16, 4>(a, grid, vec, stream) : launch_attn_rows<__nv_bfloat16, 8>(a, grid, vec, stream);
   return per == 4 ? launch_attn_rows<float, 4>(a, grid, vec, stream) : launch_attn_rows<float, 8>(a, grid, vec, stream);
@@ -678,7 +1224,7 @@ ELL_API int ell_attn_rows(const void* q, const void* k, const void* v, void* out
 // the value -> out [n, H, dv].  bf16 shapes the mma kernel takes run there, others on attn_rows.
 ELL_API long long ell_attn_latent_scratch(const void* k, int n, int H, int d, int dv, int ldq, int ldk, int max_len, int window, int is_bf16) {
   if (window > 0 && max_len > window) max_len = window;
-  if (!(is_bf16 && attn_latent_fits(k, d, dv, ldq, ldk, H))) return ell_attn_rows_scratch(n, H, 1, dv, max_len);
+  if (!(is_bf16 && attn_latent_fits(k, d, dv, ldq, ldk, H))) return ell_attn_rows_scratch(n, H, 1, d, dv, max_len, window, 0, 1, is_bf16);
   const int s = attn_latent_splits(n, H, max_len);
   return s == 1 ? 0 : (long long)n * H * s * (dv + 2);
 }
@@ -689,11 +1235,11 @@ ELL_API int ell_attn_latent(const void* q, const void* k, void* out, float* part
   if (n <= 0) return 0;
   if (!(is_bf16 && attn_latent_fits(k, d, dv, ldq, ldk, H)))
     return ell_attn_rows(q, k, k, out, part, base, len, nullptr, nullptr, gate, n, H, 1, d, dv, ldq, ldk, ldk, ldg, max_len,
-                         window, scale, is_bf16, stream);
+                         window, scale, nullptr, 0, 1, is_bf16, stream);
   if (!aligned_to(q, 16) || !aligned_to(k, 16) || !aligned_to(out, 16) || rows > 0x7fffffff) return -2;
   if (window <= 0) window = 0x7fffffff;
   if (max_len > window) max_len = window;
-  AttnRowsArgs a{q, k, k, out, part, base, len, nullptr, nullptr, n, H, 1, d, dv, ldq, ldk, ldk, 1, 0, scale, window, gate, ldg, err};
+  AttnRowsArgs a{q, k, k, out, part, base, len, nullptr, nullptr, n, H, 1, d, dv, ldq, ldk, ldk, 1, 0, scale, window, gate, ldg, err, 0};
   a.splits = attn_latent_splits(n, H, max_len);
   a.range = ((max_len + a.splits - 1) / a.splits + kAlKeys - 1) / kAlKeys * kAlKeys;
   if (a.splits > 1 && part == nullptr) return -2;

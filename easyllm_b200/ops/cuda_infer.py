@@ -218,19 +218,24 @@ def _gate(gate, like):
     return _p(gate), c_int(_rows(gate, "gate"))
 
 
-def attention_rows(q, k, v, base, length, max_len, scale, sink=None, alibi_slopes=None, window=None, gate=None):
+def attention_rows(q, k, v, base, length, max_len, scale, sink=None, alibi_slopes=None, window=None, gate=None, cu_seqlens=None,
+                   max_q=None):
     T, H, d = q.shape
     G, dv = k.shape[1], v.shape[2]
-    max_len = min(max_len, window) if window else max_len
+    if cu_seqlens is not None and (cu_seqlens.dtype != torch.int32 or not cu_seqlens.is_contiguous()):
+        raise ValueError("attention_rows: int32 sequence borders")
+    n_seq, max_q = (0, 1) if cu_seqlens is None else (cu_seqlens.numel() - 1, max_q)
     out = torch.empty(T, H, dv, dtype=q.dtype, device=q.device)
-    need = lib().ell_attn_rows_scratch(c_int(T), c_int(H), c_int(G), c_int(dv), c_int(max_len))
+    need = lib().ell_attn_rows_scratch(c_int(T), c_int(H), c_int(G), c_int(d), c_int(dv), c_int(max_len), c_int(window or 0),
+                                       c_int(n_seq), c_int(max_q), _bf(q.dtype))
     part = torch.empty(need, dtype=torch.float32, device=q.device) if need else None
     sl = cu._slopes(alibi_slopes, H, q.device)
     _check(lib().ell_attn_rows(_p(q), _p(k), _p(v), _p(out), _p(part), _p(base), _p(length),
                                _p(None if sink is None else _f32(sink, "sink")), _p(sl), _gate(gate, q)[0], c_int(T),
                                c_int(H), c_int(G), c_int(d), c_int(dv), c_int(_heads(q, "q")), c_int(_heads(k, "k")),
                                c_int(_heads(v, "v")), _gate(gate, q)[1], c_int(max_len), c_int(window or 0), c_float(scale),
-                               _bf(q.dtype), _stream()), "attn_rows", 2 if need else 1)
+                               _p(cu_seqlens), c_int(n_seq), c_int(max_q), _bf(q.dtype), _stream()), "attn_rows",
+           2 if need else 1)
     return out
 
 

@@ -188,11 +188,13 @@ def kv_append(kcache, vcache, k, v, meta):
     vcache.view(-1, *vcache.shape[2:])[rows] = v
 
 
-def attention_rows(q, k, v, kv_base, kv_len, max_len, scale, sink=None, alibi_slopes=None, window=None, gate=None):
+def attention_rows(q, k, v, kv_base, kv_len, max_len, scale, sink=None, alibi_slopes=None, window=None, gate=None,
+                   cu_seqlens=None, max_q=None):
     """Causal attention of query rows over key/value rows (a cache, or the packed batch itself), see
-    ``reference_infer.attention_rows``.  ``max_len`` bounds ``kv_len``."""
+    ``reference_infer.attention_rows``.  ``max_len`` bounds ``kv_len``.  ``cu_seqlens`` (with ``max_q``, a bound of their
+    lengths): the query rows between two borders are consecutive tokens of one sequence, so they can share its keys."""
     if _kern(q):
-        return _cu().attention_rows(q, k, v, kv_base, kv_len, max_len, scale, sink, alibi_slopes, window, gate)
+        return _cu().attention_rows(q, k, v, kv_base, kv_len, max_len, scale, sink, alibi_slopes, window, gate, cu_seqlens, max_q)
     return ref.attention_rows(q, k, v, kv_base, kv_len, scale, sink, alibi_slopes, window, gate)
 
 

@@ -194,3 +194,52 @@ def test_attention_dropout_is_rejected_with_the_fused_kernels_and_applied_on_the
         update_model_cfg(dict(base, transformer_layer_params={"attention_dropout": 0.1}))
     args = update_model_cfg(dict(base, transformer_layer_params={"attention_dropout": 0.1, "use_flash_attn": False}))
     assert args.attention_dropout == 0.1 and not args.use_flash_attn
+
+
+def _rows_exact(q, k, v, base, length, scale, sink, slopes, window, gate):
+    """``attention_rows`` in 64 bits, row by row."""
+    T, H, _ = q.shape
+    G = k.shape[1]
+    out = []
+    for t in range(T):
+        lo = max(0, length[t] - window) if window else 0
+        rows = slice(base[t] + lo, base[t] + length[t])
+        kt, vt = (x[rows].double().repeat_interleave(H // G, 1) for x in (k, v))
+        s = torch.einsum("hd,khd->hk", q[t].double(), kt) * scale
+        if slopes is not None:
+            s = s + slopes.double()[:, None] * torch.arange(lo - length[t] + 1, 1, device=q.device)
+        if sink is not None:
+            s = torch.cat((s, sink.double()[:, None]), 1)
+        o = torch.einsum("hk,khd->hd", torch.softmax(s, -1)[:, :kt.shape[0]], vt)
+        out.append(o if gate is None else o * torch.sigmoid(gate[t].double())[:, None])
+    return torch.stack(out)
+
+
+@pytest.mark.parametrize("extras", ["plain", "sink", "slopes", "window", "window gate"])
+@pytest.mark.parametrize("H,G,d,dv", [(8, 2, 128, 128), (4, 4, 64, 96), (24, 1, 96, 48), (10, 2, 16, 128), (32, 2, 128, 64)])
+@pytest.mark.parametrize("steps,past", [([1, 1, 1], [0, 700, 63]), ([3, 1], [5, 130]), ([65, 17, 200], [300, 0, 64]),
+                                        ([1, 129], [1023, 1])])
+def test_attention_over_cached_rows(steps, past, H, G, d, dv, extras):
+    """Decoding and continued prompts: rows at the edges of units, tiles and ranges of keys, groups of query heads that do not
+    fill a tile or need two.  The result is a 64-bit one rounded to bf16 (2^-9 / sqrt(3) relative, 1.65e-3 over many values):
+    weights of 8 bits would add as much again."""
+    from easyllm_b200.ops import infer as iops
+    torch.manual_seed(sum(steps) + H * d)
+    dev, cap = "cuda", 1280
+    k, v = (torch.randn(len(steps) * cap, G, n, device=dev).bfloat16() for n in (d, dv))
+    T = sum(steps)
+    q = torch.randn(T, H, d + 8, device=dev).bfloat16().flatten(1)[:, :H * d].unflatten(1, (H, d))
+    base = [i * cap for i, n in enumerate(steps) for _ in range(n)]
+    length = [p + j + 1 for n, p in zip(steps, past) for j in range(n)]
+    cu = torch.tensor([0] + steps, device=dev).cumsum(0).int()
+    sink = torch.randn(H, device=dev) if "sink" in extras else None
+    slopes = torch.rand(H, device=dev) * 0.2 if "slopes" in extras else None
+    window = 77 if "window" in extras else None
+    gate = torch.randn(T, H, device=dev).bfloat16() if "gate" in extras else None
+    b, n = (torch.tensor(x, dtype=torch.int32, device=dev) for x in (base, length))
+    want = _rows_exact(q, k, v, base, length, d ** -0.5, sink, slopes, window, gate)
+    for kw in ({"cu_seqlens": cu, "max_q": max(steps)}, {"cu_seqlens": cu, "max_q": max(steps) + 70}, {}):
+        for bound in (max(length), cap):
+            o = iops.attention_rows(q, k, v, b, n, bound, d ** -0.5, sink, slopes, window, gate, **kw)
+            assert (o.double() - want).norm() <= 1.9e-3 * want.norm()
+            assert (o.double() - want).abs().max() <= 2.0 ** -8 * want.abs().max()
