@@ -70,6 +70,7 @@ __host__ __device__ inline ArLayout ar_layout(int d, int dv, int esz, int KT, in
 
 template <typename T, int KT, int REP, bool VEC>
 __global__ void __launch_bounds__(kArThreads) attn_rows_kernel(const AttnRowsArgs a) {
+  chain_enter();
   extern __shared__ __align__(16) float sm[];
   const ArLayout L = ar_layout(a.d, a.dv, sizeof(T), KT, REP);
   const int t = blockIdx.x, rep = a.H / a.G, groups = (rep + REP - 1) / REP;
@@ -278,6 +279,7 @@ __global__ void __launch_bounds__(kArThreads) attn_rows_kernel(const AttnRowsArg
 constexpr int kArMaxSplits = 64;
 template <typename T>
 __global__ void __launch_bounds__(kArThreads) attn_rows_merge_kernel(const AttnRowsArgs a) {
+  chain_enter();
   __shared__ float weight[kArMaxSplits];
   const int t = blockIdx.x, h = blockIdx.y, step = a.dv + 2;
   const float* pt = a.part + ((size_t)t * a.H + h) * a.splits * step;
@@ -359,6 +361,7 @@ __device__ __forceinline__ void mma_bf16(float* c, const uint32_t* a, uint32_t b
 template <int MT>
 __global__ void __launch_bounds__(kAlWarps * 32)
 attn_latent_kernel(const __grid_constant__ CUtensorMap tmK, const AttnRowsArgs a) {
+  chain_enter();
   extern __shared__ uint8_t alsm_raw[];
   uint8_t* kv = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(alsm_raw) + 1023) & ~(uintptr_t)1023);
   constexpr int HM = 16 * MT;
@@ -789,6 +792,7 @@ __device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
 // NB: groups of 8 rows.
 template <int NB>
 __global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const AttnRowsArgs a, const int* __restrict__ cu, int tiles, int tt) {
+  chain_enter(cu);
   extern __shared__ __align__(128) uint8_t atsm[];
   AtTile T;
   if (!T.init(a, cu, tiles, tt)) return;
@@ -976,6 +980,7 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const AttnRowsA
 }
 
 __global__ void __launch_bounds__(kAtThreads, 2) attn_tile_kernel(const AttnRowsArgs a, const int* __restrict__ cu, int tiles, int tt) {
+  chain_enter(cu);
   extern __shared__ __align__(128) uint8_t atsm[];
   AtTile T;
   if (!T.init(a, cu, tiles, tt)) return;
@@ -1086,8 +1091,8 @@ static int launch_at(Kernel kern, int smem, bool& configured, const AttnRowsArgs
   const bool one = p.tt == 1;
   dim3 grid(one ? a.n : n_seq * p.tiles, a.G * groups, p.splits);
   if (grid.y > 65535) return -2;
-  kern<<<grid, kAtThreads, smem, stream>>>(a, one ? nullptr : cu, p.tiles, p.tt);
-  if (a.splits > 1) attn_rows_merge_kernel<__nv_bfloat16><<<dim3(a.n, a.H), kArThreads, 0, stream>>>(a);
+  launch_chained(kern, grid, kAtThreads, smem, stream, a, one ? nullptr : cu, p.tiles, p.tt);
+  if (a.splits > 1) launch_chained(attn_rows_merge_kernel<__nv_bfloat16>, dim3(a.n, a.H), kArThreads, 0, stream, a);
   return launch_status();
 }
 static int launch_attn_tile(const AttnRowsArgs& a, const AtPlan& p, const int* cu, int n_seq, cudaStream_t stream) {
@@ -1125,8 +1130,8 @@ static int launch_attn_latent(const AttnRowsArgs& a, long long rows, cudaStream_
     if (e != cudaSuccess) return (int)e;
     configured = bytes;
   }
-  attn_latent_kernel<MT><<<dim3(a.n, (a.H + 16 * MT - 1) / (16 * MT), a.splits), kAlWarps * 32, bytes, stream>>>(tk, a);
-  if (a.splits > 1) attn_rows_merge_kernel<__nv_bfloat16><<<dim3(a.n, a.H), kArThreads, 0, stream>>>(a);
+  launch_chained(attn_latent_kernel<MT>, dim3(a.n, (a.H + 16 * MT - 1) / (16 * MT), a.splits), kAlWarps * 32, bytes, stream, tk, a);
+  if (a.splits > 1) launch_chained(attn_rows_merge_kernel<__nv_bfloat16>, dim3(a.n, a.H), kArThreads, 0, stream, a);
   return launch_status();
 }
 
@@ -1160,8 +1165,8 @@ static int launch_attn_rows_kt(const AttnRowsArgs& a, dim3 grid, cudaStream_t st
     if (e != cudaSuccess) return (int)e;
     configured = bytes;
   }
-  kern<<<grid, kArThreads, bytes, stream>>>(a);
-  if (a.splits > 1) attn_rows_merge_kernel<T><<<dim3(a.n, a.H), kArThreads, 0, stream>>>(a);
+  launch_chained(kern, grid, kArThreads, bytes, stream, a);
+  if (a.splits > 1) launch_chained(attn_rows_merge_kernel<T>, dim3(a.n, a.H), kArThreads, 0, stream, a);
   return launch_status();
 }
 

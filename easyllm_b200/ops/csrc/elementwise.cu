@@ -18,6 +18,7 @@ namespace ell {
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __restrict__ cos_t,
                             const float* __restrict__ sin_t, const int* __restrict__ pos, int T, int row_stride,
                             int n_rot_heads, int D, float sin_sign, int table_rows, int* __restrict__ err) {
+  chain_enter(cos_t, sin_t, pos);
   const int half = D / 2, vec_per_head = half / 8;
   const long long total = (long long)T * n_rot_heads * vec_per_head;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -52,6 +53,7 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __rest
 }
 
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, int T, int F) {
+  chain_enter(gu);
   const int fv = F / 8;
   const long long total = (long long)T * fv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -124,7 +126,7 @@ ELL_API int ell_rope(void* qkv, const float* cos_t, const float* sin_t, const in
   if (D % 16) return -1;
   long long total = (long long)T * n_rot_heads * (D / 16);
   if (total == 0) return 0;
-  rope_kernel<<<ew_grid(total, 256), 256, 0, stream>>>((__nv_bfloat16*)qkv, cos_t, sin_t, pos, T, row_stride,
+  launch_chained(rope_kernel, ew_grid(total, 256), 256, 0, stream, (__nv_bfloat16*)qkv, cos_t, sin_t, pos, T, row_stride,
                                                        n_rot_heads, D, backward ? -1.f : 1.f, table_rows, err);
   return launch_status();
 }
@@ -133,7 +135,7 @@ ELL_API int ell_swiglu_fwd(const void* gu, void* out, int T, int F, cudaStream_t
   if (F % 8) return -1;
   long long total = (long long)T * (F / 8);
   if (total == 0) return 0;
-  swiglu_fwd_kernel<<<ew_grid(total, 256), 256, 0, stream>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)out, T, F);
+  launch_chained(swiglu_fwd_kernel, ew_grid(total, 256), 256, 0, stream, (const __nv_bfloat16*)gu, (__nv_bfloat16*)out, T, F);
   return launch_status();
 }
 

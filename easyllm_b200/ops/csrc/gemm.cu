@@ -92,6 +92,9 @@ struct GemmCfg {
   static constexpr int kSmemBytes = kStages * kStageBytes + 2 * kEpiBufBytes + 1024 /*align slack*/ + 256;
 };
 
+// Up to one row tile of A: the first kAheadBlocks k-blocks of B go into L2 ahead of the wait (39 MB over the SMs).
+constexpr int kAheadRows = 128, kAheadBlocks = 8;
+
 struct GemmShared {
   uint64_t full[8];
   uint64_t empty[8];
@@ -117,17 +120,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   GemmShared* sh = reinterpret_cast<GemmShared*>(sC + 2 * kEpiBufBytes);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_m = FUSE == kFuseGroup ? min(*fuse.n_row_tiles, (M + kBM - 1) / kBM) : (M + kBM - 1) / kBM;
   const int tiles_n = (N + BN - 1) / BN;
-  const int num_tiles = tiles_m * tiles_n;
   const int num_kb = (K + kBK - 1) / kBK;
   const int n_comm = FUSE == kFuseNone ? 0 : fuse.n_comm;
   const int cta0 = (int)blockIdx.x - n_comm;            // index among the GEMM CTAs
   const int cta_stride = (int)gridDim.x - n_comm;
-  const int n_split = split_tail_tiles(num_tiles, cta_stride, FUSE == kFuseNone && BN == 256 && OUT != kOutBf16CE &&
-                                                               !fuse.no_tail_split);
-  const int num_full = num_tiles - n_split;
-  const int num_units = num_tiles + n_split;
 
   if (FUSE != kFuseNone && (int)blockIdx.x < n_comm) {
     if (FUSE == kFuseAG) ag_comm_role(fuse, K, err, smem, 0, n_comm);
@@ -157,6 +154,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
   volatile int* abort_flag = &sh->abort_flag;
+  chain_next();
+  if (FUSE == kFuseNone && !B_MN && M <= kAheadRows && threadIdx.x == 0 && cta0 < tiles_n)
+    // few rows: the launch is bound by the bytes of B, whose first tile comes into L2 while the kernel before this one ends
+    for (int kb = 0; kb < min(num_kb, kAheadBlocks); ++kb) tma_prefetch_l2_2d(&tmB, kb * kBK, cta0 * BN);
+  chain_wait(bias);
+  const int tiles_m = FUSE == kFuseGroup ? min(*fuse.n_row_tiles, (M + kBM - 1) / kBM) : (M + kBM - 1) / kBM;
+  const int num_tiles = tiles_m * tiles_n;
+  const int n_split = split_tail_tiles(num_tiles, cta_stride, FUSE == kFuseNone && BN == 256 && OUT != kOutBf16CE &&
+                                                               !fuse.no_tail_split);
+  const int num_full = num_tiles - n_split;
+  const int num_units = num_tiles + n_split;
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -599,8 +607,11 @@ static int launch_gemm(const CUtensorMap& tA, const CUtensorMap& tB, const CUten
   }
   const int tiles = ((M + kBM - 1) / kBM) * ((N + BN - 1) / BN);
   int grid = (FUSE != kFuseNone || tiles >= max_ctas) ? max_ctas : tiles;   // fused launches keep a fixed grid
-  kern<<<grid, kGemmThreads, GemmCfg<BN>::kSmemBytes, stream>>>(tA, tB, tC, tA2 ? *tA2 : tA, fuse, bias, M, N, K, ldc,
-                                                                err);
+  if (FUSE == kFuseNone || FUSE == kFuseGroup)
+    launch_chained(kern, grid, kGemmThreads, GemmCfg<BN>::kSmemBytes, stream, tA, tB, tC, tA2 ? *tA2 : tA, fuse, bias, M, N, K,
+                   ldc, err);
+  else
+    kern<<<grid, kGemmThreads, GemmCfg<BN>::kSmemBytes, stream>>>(tA, tB, tC, tA2 ? *tA2 : tA, fuse, bias, M, N, K, ldc, err);
   return launch_status();
 }
 

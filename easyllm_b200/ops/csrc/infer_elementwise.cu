@@ -12,6 +12,7 @@ template <typename T, int V>
 __global__ void embed_scaled_kernel(const long long* __restrict__ ids, const T* __restrict__ table,
                                     float* __restrict__ out, int n, int W, long long rows, float scale,
                                     int* __restrict__ err) {
+  chain_enter(ids, table);
   const int wv = W / V;
   const long long total = (long long)n * wv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -35,6 +36,7 @@ __global__ void embed_scaled_kernel(const long long* __restrict__ ids, const T* 
 template <typename T, int V>
 __global__ void dynamic_tanh_kernel(float* __restrict__ x, const float* __restrict__ alpha, const float* __restrict__ w,
                                     const float* __restrict__ b, const T* __restrict__ add, T* __restrict__ y, int n, int W) {
+  chain_enter(alpha, w, b, add);
   const int wv = W / V;
   const long long total = (long long)n * wv;
   const float al = *alpha;
@@ -60,6 +62,7 @@ enum Act { kActSilu = 0, kActGeluTanh = 1 };
 
 template <typename T, int V>
 __global__ void glu_kernel(const T* __restrict__ gu, T* __restrict__ out, int n, int F, int ld, int act) {
+  chain_enter(gu);
   const int fv = F / V;
   const long long total = (long long)n * fv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -77,6 +80,7 @@ __global__ void glu_kernel(const T* __restrict__ gu, T* __restrict__ out, int n,
 template <typename T, int V>
 __global__ void relu2_scaled_kernel(const T* __restrict__ x, const float* __restrict__ z, T* __restrict__ out, int n,
                                     int F, int ld, int ldz) {
+  chain_enter(x, z);
   const int fv = F / V;
   const long long total = (long long)n * fv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -95,6 +99,7 @@ __global__ void relu2_scaled_kernel(const T* __restrict__ x, const float* __rest
 
 template <typename T>
 __global__ void tanh_cast_kernel(const float* __restrict__ x, T* __restrict__ y, int n, int N, int ldx) {
+  chain_enter(x);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)n * N;
        i += (long long)gridDim.x * blockDim.x)
     y[i] = from_f<T>(tanhf(x[(i / N) * ldx + i % N]));
@@ -102,6 +107,7 @@ __global__ void tanh_cast_kernel(const float* __restrict__ x, T* __restrict__ y,
 
 // z = exp(-exp(z + w0[column]))
 __global__ void wkv_decay_kernel(float* __restrict__ z, const float* __restrict__ w0, long long total, int C) {
+  chain_enter(w0);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
     z[i] = expf(-expf(z[i] + w0[i % C]));
 }
@@ -113,6 +119,7 @@ template <typename T, int V>
 __global__ void token_mix_kernel(const T* __restrict__ h, const float* __restrict__ mu, T* __restrict__ out,
                                  const int* __restrict__ cu, const int* __restrict__ slots, const int* __restrict__ pos0,
                                  T* __restrict__ last, int W, int nmix, int n, int chunk) {
+  chain_enter(h, mu, cu, slots, pos0);
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * V;
   if (c >= W) return;
   const int s = blockIdx.z, a = cu[s], b = cu[s + 1];
@@ -208,6 +215,7 @@ template <typename T, int V>
 __global__ void head_norm_gate_kernel(const float* __restrict__ o, const float* __restrict__ w, const T* __restrict__ gate,
                                       T* __restrict__ y, int n, int H, int dv, int w_per_head, int ldg, int silu_gate,
                                       float eps) {
+  chain_enter(o, w, gate);
   const int warps = blockDim.x >> 5, lane = threadIdx.x & 31;
   for (long long i = blockIdx.x * (long long)warps + (threadIdx.x >> 5); i < (long long)n * H; i += (long long)gridDim.x * warps) {
     const int t = (int)(i / H), hd = (int)(i % H);
@@ -226,6 +234,7 @@ template <typename T, int V>
 __global__ void kv_append_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ kc, T* __restrict__ vc,
                                  const int* __restrict__ base, const int* __restrict__ len, int n, int dk, int dv, int ldk,
                                  int ldv) {
+  chain_enter(k, v, base, len);
   const int per = (dk + dv) / V;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)n * per;
        i += (long long)gridDim.x * blockDim.x) {
@@ -252,6 +261,7 @@ __global__ void embed_pairs_kernel(const long long* __restrict__ ids, const T* _
                                    const int* __restrict__ base, const int* __restrict__ len, int* __restrict__ hist, int W,
                                    long long rows, long long buckets, long long mul_prev, long long mul_cur, float scale,
                                    int* __restrict__ err) {
+  chain_enter(ids, table, pairs, row_start, base, len);
   const int t = blockIdx.x;
   const long long id = ids[t];
   const bool first_row = row_start[t] == t;
@@ -294,6 +304,7 @@ template <typename T, int IT>
 __global__ void __launch_bounds__(kLnPairThreads)
 layer_norms_kernel(const float* __restrict__ x, const float* __restrict__ w1, const float* __restrict__ w2,
                    T* __restrict__ y1, T* __restrict__ y2, int W, float eps) {
+  chain_enter(x, w1, w2);
   __shared__ float red[2][kLnPairThreads / 32];
   const float* row = x + (size_t)blockIdx.x * W;
   T* o1 = y1 + (size_t)blockIdx.x * W;
@@ -366,6 +377,7 @@ latent_inputs_kernel(T* __restrict__ z, T* __restrict__ q_dst, T* __restrict__ c
                      const float* __restrict__ cosT, const float* __restrict__ sinT, const int* __restrict__ pos,
                      const int* __restrict__ base, const int* __restrict__ len, int H, int dim, int rot, int rank, int pairs,
                      int ldz, int q_stride, int ldc, float eps) {
+  chain_enter(norm_w, cosT, sinT, pos, base, len);
   __shared__ float red[kLatThreads / 32];
   const int t = blockIdx.x;
   constexpr int VL = V == 8 ? 8 : 1;                    // pieces of the latent (any rank)
@@ -454,12 +466,12 @@ using namespace ell;
   do {                                                                                                 \
     if (is_bf16) {                                                                                     \
       using T = __nv_bfloat16;                                                                         \
-      if (cond_vec) KERNEL<T, 4><<<GRID, BLOCK, 0, stream>>>(__VA_ARGS__);                             \
-      else KERNEL<T, 1><<<GRID, BLOCK, 0, stream>>>(__VA_ARGS__);                                      \
+      if (cond_vec) launch_chained(KERNEL<T, 4>, GRID, BLOCK, 0, stream, __VA_ARGS__);                 \
+      else launch_chained(KERNEL<T, 1>, GRID, BLOCK, 0, stream, __VA_ARGS__);                          \
     } else {                                                                                           \
       using T = float;                                                                                 \
-      if (cond_vec) KERNEL<T, 4><<<GRID, BLOCK, 0, stream>>>(__VA_ARGS__);                             \
-      else KERNEL<T, 1><<<GRID, BLOCK, 0, stream>>>(__VA_ARGS__);                                      \
+      if (cond_vec) launch_chained(KERNEL<T, 4>, GRID, BLOCK, 0, stream, __VA_ARGS__);                 \
+      else launch_chained(KERNEL<T, 1>, GRID, BLOCK, 0, stream, __VA_ARGS__);                          \
     }                                                                                                  \
   } while (0)
 
@@ -503,14 +515,14 @@ ELL_API int ell_relu2_scaled(const void* x, const float* z, void* out, int n, in
 ELL_API int ell_tanh_cast(const float* x, void* y, int n, int N, int ldx, int is_bf16, cudaStream_t stream) {
   if (n <= 0) return 0;
   const int g = grid_for((long long)n * N, 256);
-  if (is_bf16) tanh_cast_kernel<__nv_bfloat16><<<g, 256, 0, stream>>>(x, (__nv_bfloat16*)y, n, N, ldx);
-  else tanh_cast_kernel<float><<<g, 256, 0, stream>>>(x, (float*)y, n, N, ldx);
+  if (is_bf16) launch_chained(tanh_cast_kernel<__nv_bfloat16>, g, 256, 0, stream, x, (__nv_bfloat16*)y, n, N, ldx);
+  else launch_chained(tanh_cast_kernel<float>, g, 256, 0, stream, x, (float*)y, n, N, ldx);
   return launch_status();
 }
 
 ELL_API int ell_wkv_decay(float* z, const float* w0, int n, int C, cudaStream_t stream) {
   if (n <= 0) return 0;
-  wkv_decay_kernel<<<grid_for((long long)n * C, 256), 256, 0, stream>>>(z, w0, (long long)n * C, C);
+  launch_chained(wkv_decay_kernel, grid_for((long long)n * C, 256), 256, 0, stream, z, w0, (long long)n * C, C);
   return launch_status();
 }
 
@@ -571,10 +583,10 @@ ELL_API int ell_layer_norms(const float* x, const float* w1, const float* w2, vo
 #define ELL_LN(IT)                                                                                                     \
   do {                                                                                                                 \
     if (is_bf16)                                                                                                       \
-      layer_norms_kernel<__nv_bfloat16, IT><<<n, kLnPairThreads, 0, stream>>>(x, w1, w2, (__nv_bfloat16*)y1,           \
+      launch_chained(layer_norms_kernel<__nv_bfloat16, IT>, n, kLnPairThreads, 0, stream, x, w1, w2, (__nv_bfloat16*)y1, \
                                                                              (__nv_bfloat16*)y2, W, eps);             \
     else                                                                                                               \
-      layer_norms_kernel<float, IT><<<n, kLnPairThreads, 0, stream>>>(x, w1, w2, (float*)y1, (float*)y2, W, eps);      \
+      launch_chained(layer_norms_kernel<float, IT>, n, kLnPairThreads, 0, stream, x, w1, w2, (float*)y1, (float*)y2, W, eps); \
   } while (0)
   if (it == 0) ELL_LN(0);
   else if (it == 1) ELL_LN(1);
@@ -594,7 +606,7 @@ ELL_API int ell_latent_inputs(void* z, void* q_dst, void* cache, const float* no
   const bool v = dim % 8 == 0 && rot % 8 == 0 && rank % 8 == 0 && pairs % 4 == 0 && aligned_to(cosT, 16) && aligned_to(sinT, 16) && ldz % 8 == 0 && q_stride % 8 == 0 && ldc % 8 == 0 &&
                  aligned_to(z, 16) && aligned_to(q_dst, 16) && aligned_to(cache, 16) && aligned_to(norm_w, 16);
 #define ELL_LAT(T, V)                                                                                                   \
-  latent_inputs_kernel<T, V><<<n, kLatThreads, 0, stream>>>((T*)z, (T*)q_dst, (T*)cache, norm_w, cosT, sinT, pos, base, \
+  launch_chained(latent_inputs_kernel<T, V>, n, kLatThreads, 0, stream, (T*)z, (T*)q_dst, (T*)cache, norm_w, cosT, sinT, pos, base, \
                                                             len, H, dim, rot, rank, pairs, ldz, q_stride, ldc, eps)
   if (is_bf16) {
     if (v) ELL_LAT(__nv_bfloat16, 8);

@@ -22,6 +22,7 @@ struct MatvecArgs {
 
 template <typename T, int MR, int NW, bool VEC>
 __global__ void __launch_bounds__(kMvWarps * 32) matvec_kernel(const MatvecArgs a) {
+  chain_enter();
   __shared__ float red[kMvWarps][NW * MR];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ks = a.ks, part = warp % ks, n0 = (blockIdx.x * (kMvWarps / ks) + warp / ks) * NW, m0 = blockIdx.y * MR;
@@ -103,6 +104,15 @@ __global__ void __launch_bounds__(kMvWarps * 32) matvec_mma_kernel(const MatvecA
   const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(a.w) + blockIdx.z * a.wb;
   const __nv_bfloat16* w0 = w + (size_t)min(n0 + g, a.N - 1) * a.K;
   const __nv_bfloat16* w1 = w + (size_t)min(n0 + g + 8, a.N - 1) * a.K;
+  chain_next();
+  {
+    // the CTA's rows of W come into L2 while the kernel before this one ends, a row (16-byte pieces) a thread
+    const int first = blockIdx.x * (kMvWarps / ks) * 16, rows = min(kMvWarps / ks * 16, a.N - first);
+    if (threadIdx.x < rows && blockIdx.y == 0)
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(w + (size_t)(first + threadIdx.x) * a.K), "r"(a.K * 2)
+                   : "memory");
+  }
+  chain_wait();
   const __nv_bfloat16* xr[MT];
 #pragma unroll
   for (int m = 0; m < MT; ++m) xr[m] = x + (size_t)min(m * 8 + g, M - 1) * a.ldx;
@@ -166,8 +176,8 @@ static int launch_matvec_mma(MatvecArgs a, int batch, cudaStream_t stream) {
   const int per = kMvWarps / a.ks;
   dim3 grid((tiles + per - 1) / per, (a.M + 15) / 16, batch);
   if (grid.y > 65535) return -2;
-  if (a.M <= 8) matvec_mma_kernel<1><<<grid, kMvWarps * 32, 0, stream>>>(a);
-  else matvec_mma_kernel<2><<<grid, kMvWarps * 32, 0, stream>>>(a);
+  if (a.M <= 8) launch_chained(matvec_mma_kernel<1>, grid, kMvWarps * 32, 0, stream, a);
+  else launch_chained(matvec_mma_kernel<2>, grid, kMvWarps * 32, 0, stream, a);
   return launch_status();
 }
 
@@ -179,8 +189,8 @@ int launch_matvec(MatvecArgs a, int batch, bool vec, cudaStream_t stream) {
   const int per = kMvWarps / a.ks;
   dim3 grid(((a.N + NW - 1) / NW + per - 1) / per, (a.M + MR - 1) / MR, batch);
   if (grid.y > 65535) return -2;
-  if (vec) matvec_kernel<T, MR, NW, true><<<grid, kMvWarps * 32, 0, stream>>>(a);
-  else matvec_kernel<T, MR, NW, false><<<grid, kMvWarps * 32, 0, stream>>>(a);
+  if (vec) launch_chained(matvec_kernel<T, MR, NW, true>, grid, kMvWarps * 32, 0, stream, a);
+  else launch_chained(matvec_kernel<T, MR, NW, false>, grid, kMvWarps * 32, 0, stream, a);
   return launch_status();
 }
 
@@ -197,6 +207,7 @@ int dispatch_matvec(const MatvecArgs& a, int batch, bool vec, cudaStream_t strea
 // chosen logits.  bias [E] (or null) is added to the logits first.
 __global__ void moe_route_kernel(const float* __restrict__ z, const float* __restrict__ bias, int* __restrict__ idx,
                                  float* __restrict__ w, int n, int E, int top, int ldz, int softmax) {
+  chain_enter(z, bias);
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (t >= n) return;
   const float* row = z + (size_t)t * ldz;
@@ -243,6 +254,7 @@ template <typename T, bool VEC, bool GLU>
 __global__ void __launch_bounds__(256) moe_up_kernel(const T* __restrict__ h, const T* __restrict__ up,
                                                      const int* __restrict__ idx, const float* __restrict__ wgt,
                                                      T* __restrict__ hid, int top, int F, int W, int block) {
+  chain_enter(h, up, idx, wgt);
   const int slot = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int f0 = (blockIdx.x * 8 + warp) * (GLU ? 1 : 2);
   if (f0 >= F) return;
@@ -294,6 +306,7 @@ template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) moe_down_kernel(const T* __restrict__ hid, const T* __restrict__ down,
                                                        const int* __restrict__ idx, float* __restrict__ acc, int top, int F,
                                                        int W) {
+  chain_enter(hid, down, idx);
   const int t = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = (blockIdx.x * 8 + warp) * 2;
   if (n0 >= W) return;
@@ -340,6 +353,7 @@ __global__ void __launch_bounds__(256) moe_down_kernel(const T* __restrict__ hid
 __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ idx, const float* __restrict__ wgt, int slots,
                                                         int E, int* __restrict__ pos, float* __restrict__ row_scale,
                                                         int* __restrict__ tile_expert, int* __restrict__ n_tiles) {
+  chain_enter(idx, wgt);
   __shared__ int count[1024], first[1024], scan[1024];
   const int e = threadIdx.x;
   count[e] = 0;
@@ -373,6 +387,7 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
 // xs[pos[slot]] = h[token], 16 bytes a thread.
 __global__ void moe_gather_kernel(const uint4* __restrict__ h, uint4* __restrict__ xs, const int* __restrict__ pos, int slots,
                                   int top, int wv) {
+  chain_enter(h, pos);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)slots * wv;
        i += (long long)gridDim.x * blockDim.x) {
     const int slot = (int)(i / wv), c = (int)(i % wv);
@@ -383,6 +398,7 @@ __global__ void moe_gather_kernel(const uint4* __restrict__ h, uint4* __restrict
 // acc[token] += sum over its slots of ys[pos[slot]]
 __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ ys, const int* __restrict__ pos, float* __restrict__ acc,
                                    int n, int top, int W) {
+  chain_enter(ys, pos);
   const int wv = W / 4;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)n * wv;
        i += (long long)gridDim.x * blockDim.x) {
@@ -422,7 +438,7 @@ ELL_API int ell_moe_route(const float* z, const float* bias, int* idx, float* w,
                           cudaStream_t stream) {
   if (n <= 0) return 0;
   if (E > 1024 || top > E || top < 1) return -2;
-  moe_route_kernel<<<(n + 7) / 8, 256, 0, stream>>>(z, bias, idx, w, n, E, top, ldz, softmax);
+  launch_chained(moe_route_kernel, (n + 7) / 8, 256, 0, stream, z, bias, idx, w, n, E, top, ldz, softmax);
   return launch_status();
 }
 
@@ -436,9 +452,9 @@ ELL_API int ell_moe_rows(const void* h, const void* up, const void* down, const 
   if (glu_block < 0 || (glu_block > 0 && F % glu_block)) return -2;
   dim3 gu(glu_block ? (F + 7) / 8 : (F + 15) / 16, n * top), gd((W + 15) / 16, n);
 #define ELL_MOE_ROWS(T, V)                                                                                          \
-  if (glu_block) moe_up_kernel<T, V, true><<<gu, 256, 0, stream>>>((const T*)h, (const T*)up, idx, w, (T*)hid, top, F, W, glu_block); \
-  else moe_up_kernel<T, V, false><<<gu, 256, 0, stream>>>((const T*)h, (const T*)up, idx, w, (T*)hid, top, F, W, 1); \
-  moe_down_kernel<T, V><<<gd, 256, 0, stream>>>((const T*)hid, (const T*)down, idx, acc, top, F, W);
+  if (glu_block) launch_chained(moe_up_kernel<T, V, true>, gu, 256, 0, stream, (const T*)h, (const T*)up, idx, w, (T*)hid, top, F, W, glu_block); \
+  else launch_chained(moe_up_kernel<T, V, false>, gu, 256, 0, stream, (const T*)h, (const T*)up, idx, w, (T*)hid, top, F, W, 1); \
+  launch_chained(moe_down_kernel<T, V>, gd, 256, 0, stream, (const T*)hid, (const T*)down, idx, acc, top, F, W);
   if (is_bf16) {
     if (v) { ELL_MOE_ROWS(__nv_bfloat16, true) } else { ELL_MOE_ROWS(__nv_bfloat16, false) }
   } else {
@@ -453,8 +469,8 @@ ELL_API int ell_moe_gather(const void* h, void* xs, const int* idx, const float*
                            int* tile_expert, int* n_tiles, int n, int top, int E, int W, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (E > 1024 || W % 8) return -2;
-  moe_plan_kernel<<<1, 1024, 0, stream>>>(idx, w, n * top, E, pos, row_scale, tile_expert, n_tiles);
-  moe_gather_kernel<<<grid_for((long long)n * top * (W / 8), 256), 256, 0, stream>>>((const uint4*)h, (uint4*)xs, pos,
+  launch_chained(moe_plan_kernel, 1, 1024, 0, stream, idx, w, n * top, E, pos, row_scale, tile_expert, n_tiles);
+  launch_chained(moe_gather_kernel, grid_for((long long)n * top * (W / 8), 256), 256, 0, stream, (const uint4*)h, (uint4*)xs, pos,
                                                                                     n * top, top, W / 8);
   return launch_status();
 }
@@ -462,6 +478,6 @@ ELL_API int ell_moe_gather(const void* h, void* xs, const int* idx, const float*
 ELL_API int ell_moe_combine(const void* ys, const int* pos, float* acc, int n, int top, int W, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (W % 4) return -2;
-  moe_combine_kernel<<<grid_for((long long)n * (W / 4), 256), 256, 0, stream>>>((const __nv_bfloat16*)ys, pos, acc, n, top, W);
+  launch_chained(moe_combine_kernel, grid_for((long long)n * (W / 4), 256), 256, 0, stream, (const __nv_bfloat16*)ys, pos, acc, n, top, W);
   return launch_status();
 }

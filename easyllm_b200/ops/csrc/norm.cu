@@ -76,6 +76,7 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   __shared__ float s_red[2][kNormWarps][kNormRowsMax];
   constexpr int kNormRows = norm_rows(kVpt);
   const int nvec = cols / 8;
+  chain_enter(x, res, w);
   bf16x8 wv[kVpt];
 #pragma unroll
   for (int i = 0; i < kVpt; ++i) {
@@ -267,10 +268,10 @@ void launch_norm_fwd(int vpt, dim3 grid, cudaStream_t stream, const __nv_bfloat1
                      float eps) {
   dim3 block(kNormThreads);
   switch (vpt) {
-    case 1: rmsnorm_fwd_kernel<1, kHasRes><<<grid, block, 0, stream>>>(x, res, w, y, h_out, rstd, rows, cols, eps); break;
-    case 2: rmsnorm_fwd_kernel<2, kHasRes><<<grid, block, 0, stream>>>(x, res, w, y, h_out, rstd, rows, cols, eps); break;
-    case 3: rmsnorm_fwd_kernel<3, kHasRes><<<grid, block, 0, stream>>>(x, res, w, y, h_out, rstd, rows, cols, eps); break;
-    default: rmsnorm_fwd_kernel<4, kHasRes><<<grid, block, 0, stream>>>(x, res, w, y, h_out, rstd, rows, cols, eps); break;
+    case 1: launch_chained(rmsnorm_fwd_kernel<1, kHasRes>, grid, block, 0, stream, x, res, w, y, h_out, rstd, rows, cols, eps); break;
+    case 2: launch_chained(rmsnorm_fwd_kernel<2, kHasRes>, grid, block, 0, stream, x, res, w, y, h_out, rstd, rows, cols, eps); break;
+    case 3: launch_chained(rmsnorm_fwd_kernel<3, kHasRes>, grid, block, 0, stream, x, res, w, y, h_out, rstd, rows, cols, eps); break;
+    default: launch_chained(rmsnorm_fwd_kernel<4, kHasRes>, grid, block, 0, stream, x, res, w, y, h_out, rstd, rows, cols, eps); break;
   }
 }
 

@@ -363,6 +363,8 @@ int launch_scan(const ScanArgs& a, int n_seq, int vec, cudaStream_t stream) {
     configured = true;
   }
   dim3 grid((a.dv + kScanCols - 1) / kScanCols, a.H, n_seq);
+  // Not chained: CTAs that come in while the kernel before ends are packed where there is room first, and with two CTAs on an SM
+  // a scan of 4096 tokens took 1.5 times as long.
   kern<<<grid, ScanTok<DP>::kThreads, bytes, stream>>>(a, vec);
   return launch_status();
 }
@@ -419,6 +421,7 @@ __device__ __forceinline__ float warp_sum16(float* v) {
 // it replaces it by the sequence's last inputs afterwards (each thread its own channel).  NT: taps (0: any number).
 template <typename T, int NT>
 __global__ void delta_inputs_kernel(const DeltaInArgs p) {
+  chain_enter();
   __shared__ float red[kConvTok][33];
   const int s = blockIdx.z, sa = p.cu[s], sb = p.cu[s + 1];
   const int t0 = sa + blockIdx.y * kConvTok, t1 = min(t0 + kConvTok, sb);
@@ -521,11 +524,11 @@ __global__ void delta_inputs_kernel(const DeltaInArgs p) {
 template <typename T>
 static void launch_delta_inputs(const DeltaInArgs& p, dim3 grid, int threads, cudaStream_t stream) {
   switch (p.n_taps) {
-    case 1: delta_inputs_kernel<T, 1><<<grid, threads, 0, stream>>>(p); break;
-    case 2: delta_inputs_kernel<T, 2><<<grid, threads, 0, stream>>>(p); break;
-    case 3: delta_inputs_kernel<T, 3><<<grid, threads, 0, stream>>>(p); break;
-    case 4: delta_inputs_kernel<T, 4><<<grid, threads, 0, stream>>>(p); break;
-    default: delta_inputs_kernel<T, 0><<<grid, threads, 0, stream>>>(p);
+    case 1: launch_chained(delta_inputs_kernel<T, 1>, grid, threads, 0, stream, p); break;
+    case 2: launch_chained(delta_inputs_kernel<T, 2>, grid, threads, 0, stream, p); break;
+    case 3: launch_chained(delta_inputs_kernel<T, 3>, grid, threads, 0, stream, p); break;
+    case 4: launch_chained(delta_inputs_kernel<T, 4>, grid, threads, 0, stream, p); break;
+    default: launch_chained(delta_inputs_kernel<T, 0>, grid, threads, 0, stream, p);
   }
 }
 

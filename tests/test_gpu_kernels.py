@@ -240,3 +240,57 @@ def test_out_of_range_indices_are_reported_not_dereferenced(cu):
         cu.check_err_flag()
     assert torch.equal(out[2], torch.zeros_like(out[2])) and torch.equal(out[1], w[2])
     cu.check_err_flag()                                              # cleared
+
+
+@pytest.mark.parametrize("rows", [1, 20, 100])
+@pytest.mark.parametrize("capture", [False, True])
+def test_chained_launches_keep_their_order(cu, rows, capture):
+    """A run of dependent launches over three buffers that every launch reuses (matrix-vector, thin and tiled products, norm,
+    GLU, accumulation), torch kernels, a copy and a forked stream in between: the result is that of the same launches with the
+    GPU waited for after each."""
+    import easyllm_b200.ops.cuda_infer as ci
+    torch.manual_seed(rows)
+    W, F = 1024, 2816
+    w = [(torch.randn(n, k, device="cuda") * k ** -0.5).to(torch.bfloat16) for n, k in ((2 * F, W), (W, F), (W, W))]
+    nw = torch.ones(W, device="cuda", dtype=torch.bfloat16)
+    x0 = torch.randn(rows, W, device="cuda", dtype=torch.bfloat16)
+    x, acc = torch.empty_like(x0), torch.empty(rows, W, device="cuda")
+    side = torch.cuda.Stream()
+
+    def chain(wait):
+        x.copy_(x0)
+        acc.zero_()
+        for i in range(12):
+            y = cu.rmsnorm_fwd(x, None, nw, 1e-5)[0]
+            wait()
+            h = ci.glu(ci.linear(y, w[0]), "silu")
+            wait()
+            ci.linear_add_(acc, h, w[1])
+            wait()
+            if i % 4 == 3:
+                side.wait_stream(torch.cuda.current_stream())
+                with torch.cuda.stream(side):
+                    z = ci.linear(y, w[2])
+                torch.cuda.current_stream().wait_stream(side)
+                z.record_stream(torch.cuda.current_stream())
+            else:
+                z = ci.linear(y, w[2])
+            wait()
+            x.copy_(z)
+            wait()
+            x.add_(acc)
+            wait()
+        return x.clone(), acc.clone()
+
+    want = chain(torch.cuda.synchronize)
+    if capture:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = chain(lambda: None)
+        for _ in range(3):
+            graph.replay()
+    else:
+        got = chain(lambda: None)
+    torch.cuda.synchronize()
+    cu.check_err_flag()
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
