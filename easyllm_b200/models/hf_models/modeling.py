@@ -212,6 +212,15 @@ class RMSNorm(nn.Module):
         return ops.add_rmsnorm(x, residual, self.weight, self.eps)
 
 
+class TokenEmbedding(nn.Embedding):
+    """The token table; its gradient goes straight into the weight's ``main_grad``."""
+
+    def forward(self, ids):
+        if self.padding_idx is None and self.max_norm is None and not self.sparse and not self.scale_grad_by_freq:
+            return ops.token_embedding(ids, self.weight)
+        return super().forward(ids)
+
+
 class Attention(nn.Module):
     """Causal attention: GQA, RoPE / ALiBi / no positions, value heads of another size than the keys', a given score
     scale, and a learned sink per head in the softmax denominator.  ``m``: sizes of this layer (None: the arch's)."""
@@ -435,7 +444,7 @@ class ParallelLayer(nn.Module):
 class Decoder(nn.Module):
     def __init__(self, a: HFArch, dtype):
         super().__init__()
-        self.embed_tokens = nn.Embedding(a.vocab_size, a.hidden_size, dtype=dtype)
+        self.embed_tokens = TokenEmbedding(a.vocab_size, a.hidden_size, dtype=dtype)
         self.embedding_scale, self.hybrid, self.bigram = a.embedding_scale, a.layers is not None, a.bigram
         self.keeps_tokens = a.bigram is not None          # the state holds token ids: the embedding looks one back
         if self.bigram is not None:

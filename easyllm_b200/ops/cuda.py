@@ -127,11 +127,15 @@ def scratch(nelem, dtype=torch.float32, tag="default"):
     return b
 
 
+def transforms_active():
+    """Whether a function transform or forward-mode differentiation is under way."""
+    return torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0
+
+
 def nothing_to_record():
     """Whether a call may skip its autograd function (25 us of host time): no gradients are recorded, and neither a function
     transform nor forward-mode differentiation is active, which the functions refuse."""
-    return not torch.is_grad_enabled() and not torch._C._are_functorch_transforms_active() and \
-        torch.autograd.forward_ad._current_level < 0
+    return not torch.is_grad_enabled() and not transforms_active()
 
 
 # ---- norm ------------------------------------------------------------------------------------

@@ -294,3 +294,34 @@ def test_chained_launches_keep_their_order(cu, rows, capture):
     torch.cuda.synchronize()
     cu.check_err_flag()
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("tokens,rows,cols,dtype", [(1, 8, 8, torch.int64), (37, 5, 264, torch.int32), (3001, 32000, 1024, torch.int64)])
+@pytest.mark.parametrize("deterministic", [False, True])
+def test_embedding_gradient_goes_to_main_grad(cu, tokens, rows, cols, dtype, deterministic):
+    """Rows that come often, and a main_grad that already holds something; fp32 sums of n bf16 rows are within n 2^-24 of the
+    sum of magnitudes.  Deterministic programs get F.embedding's own dense gradient."""
+    from easyllm_b200.models.hf_models.modeling import TokenEmbedding
+    torch.manual_seed(1)
+    emb = TokenEmbedding(rows, cols, device="cuda", dtype=torch.bfloat16)
+    ids = torch.randint(0, rows, (tokens,), device="cuda", dtype=dtype)
+    before = torch.randn(rows, cols, device="cuda")
+    emb.weight.main_grad = before.clone()
+    dy = torch.randn(tokens, cols, device="cuda", dtype=torch.bfloat16)
+    torch.use_deterministic_algorithms(deterministic)
+    try:
+        y = emb(ids)
+        y.backward(dy)
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert torch.equal(y, emb.weight[ids.long()])
+    if deterministic:
+        other = emb.weight.detach().clone().requires_grad_()
+        torch.nn.functional.embedding(ids, other).backward(dy)
+        assert torch.equal(emb.weight.grad, other.grad) and torch.equal(emb.weight.main_grad, before)
+        return
+    assert emb.weight.grad is None
+    want, size = before.double(), before.double().abs()
+    want.index_add_(0, ids.long(), dy.double())
+    size.index_add_(0, ids.long(), dy.double().abs())
+    assert ((emb.weight.main_grad.double() - want).abs() <= size * (tokens + 1) * 2.0 ** -24).all()
