@@ -23,9 +23,9 @@ LIB_PATH = os.path.join(HERE, "libeasyllm_b200.so")
 # the kernels that serving a model loads and launches; `ensure_serving` builds these alone
 SERVE_LIB_PATH = os.path.join(HERE, "libeasyllm_b200_serve.so")
 SERVE_SOURCES = ("attn_rows", "elementwise", "flash_attn", "gemm", "gemm_pair", "gemm_thin", "infer_elementwise", "matvec", "norm",
-                 "optim", "recurrent")
+                 "optim", "recurrent", "scan_chunks")
 # sources whose fp32 results must keep full accuracy (no approximate exp / tanh / division)
-ACCURATE_SOURCES = ("attn_rows", "gemm_thin", "infer_elementwise", "matvec", "recurrent")
+ACCURATE_SOURCES = ("attn_rows", "gemm_thin", "infer_elementwise", "matvec", "recurrent", "scan_chunks")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "--use_fast_math", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]

@@ -39,7 +39,8 @@ def lib():
             raise KernelError(f"{_LIB_PATH} is missing: run `python -m easyllm_b200.ops.build` "
                               "(or __graft_entry__.build()) before using the CUDA ops")
         _lib = ctypes.CDLL(_LIB_PATH if os.path.exists(_LIB_PATH) else _SERVE_LIB_PATH)
-        for name in ("ell_rmsnorm_bwd_scratch_elems", "ell_attn_rows_scratch", "ell_attn_latent_scratch"):
+        for name in ("ell_rmsnorm_bwd_scratch_elems", "ell_attn_rows_scratch", "ell_attn_latent_scratch",
+                     "ell_scan_chunks_work"):
             getattr(_lib, name).restype = c_longlong
     return _lib
 
@@ -99,6 +100,7 @@ def check_err_flag():
         raise KernelError(f"a kernel gave up a bounded wait (code {v}: 1 producer, 2 mma, 3 epilogue, 4 communication "
                           "role, 5 peer flag; 11-15 the same roles of the CTA-pair GEMM; 21 cross-entropy exchange; "
                           "31 a token id outside the embedding table; 32 a position outside the rotary tables; "
+                          "41 a scan over chunks; "
                           "6 / 16 a tile index outside a fused kernel's buffers)")
 
 

@@ -323,10 +323,30 @@ def wkv_decay_(z, w0):
     return z
 
 
+def _scan_chunks(mode, q, k, v, decay, beta, u, o, meta, state):
+    """A scan 16 tokens at a time (``csrc/scan_chunks.cu``); False where it has to go token by token."""
+    (T, G, d), (H, dv) = k.shape, v.shape[1:]
+    c, sl, p0, n = _seq(meta, state)
+    ldv, size = _heads(v, "v"), v.element_size()
+    if v.data_ptr() % 16 or ldv * size % 16 or dv * size % 16:
+        return False
+    need = lib().ell_scan_chunks_work(c_int(mode), c_int(T), c_int(n), c_int(meta["max_seqlen"]), c_int(H), c_int(d), c_int(dv))
+    if not need:
+        return False
+    work = torch.empty(need, dtype=torch.float32, device=v.device)
+    _check(lib().ell_scan_chunks(c_int(mode), _p(q), _p(k), _p(v), _p(_f32(decay, "decay")), _p(beta), _p(u), _p(o), _p(state), c, sl,
+                                 p0, c_int(T), c_int(n), c_int(meta["max_seqlen"]), c_int(H), c_int(G), c_int(d), c_int(dv),
+                                 c_int(_heads(q, "q")), c_int(_heads(k, "k")), c_int(ldv), _bf(v.dtype), _p(work),
+                                 _p(err_flag(v.device)), _stream()), "scan_chunks", 2)
+    return True
+
+
 def wkv_scan(r, k, v, decay, u, meta, state):
     T, H, d = k.shape
     dv = v.shape[2]
     o = torch.empty(T, H, dv, dtype=torch.float32, device=k.device)
+    if _scan_chunks(0, r, k, v, decay, None, _f32(u, "u"), o, meta, state):
+        return o
     c, sl, p0, n = _seq(meta, state)
     _check(lib().ell_wkv_scan(_p(r), _p(k), _p(v), _p(_f32(decay, "decay")), _p(_f32(u, "u")), _p(o), _p(state), c, sl, p0,
                               c_int(n), c_int(H), c_int(d), c_int(dv), c_int(_heads(r, "r")), c_int(_heads(k, "k")),
@@ -358,6 +378,8 @@ def delta_scan(q, k, v, g, beta, meta, state):
     c, sl, p0, n = _seq(meta, state)
     for t, name in ((q, "q"), (k, "k"), (v, "v"), (g, "g"), (beta, "beta")):
         _f32(t, name)
+    if _scan_chunks(1, q, k, v, g, beta, None, o, meta, state):
+        return o
     _check(lib().ell_delta_scan(_p(q), _p(k), _p(v), _p(g), _p(beta), _p(o), _p(state), c, sl, p0, c_int(n), c_int(H),
                                 c_int(q.shape[1]), c_int(q.shape[2]), c_int(dv), _stream()), "delta_scan")
     return o

@@ -276,6 +276,77 @@ def test_scans(device, kind, dtype, H, G, d, dv):
         at += c
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,dtype", [("wkv", F32), ("wkv", BF16), ("delta", F32)])
+@pytest.mark.parametrize("H,G,d,dv,counts", [(2, 2, 64, 64, [256]), (4, 2, 20, 48, [300, 1, 37]), (2, 1, 128, 128, [257, 16]),
+                                             (1, 1, 100, 8, [15, 270, 273])])
+def test_scans_in_chunks(kind, dtype, H, G, d, dv, counts):
+    """Sequences long enough for chunks of 16 tokens, beside short ones and going on from a slot's state; decays between 0 and 1 with
+    both ends among them.  Sums of up to 273 tokens in fp32: the tolerance of the other scans."""
+    dev = _device("cuda")
+    if kind == "wkv":
+        G = H
+    T = sum(counts)
+    ins = list(_scan_inputs(kind, H, G, d, dv, 2 * T, dtype))
+    ins[3][::7, :, ::3], ins[3][::5, :, 1::3] = 0.0, 1.0
+    which = [h // (H // G) for h in range(H)]
+    qd, kd, vd, gd, ud = (x.double() for x in ins)
+    state = torch.full((5, H, dv, iops.padded_rows(d)), 5.0, device=dev)
+    slots = [3, 0, 1][:len(counts)]
+    done = [0] * len(counts)
+    S = [None] * len(counts)
+    for go in range(2):
+        m = meta_of(counts, dev, slots, done)
+        got = _scan(kind, ins, slice(go * T, (go + 1) * T), m, state, dev)
+        at = go * T
+        for i, c in enumerate(counts):
+            p = slice(at, at + c)
+            o, S[i] = (plain.wkv_recurrence(qd[p], kd[p], vd[p], gd[p], ud, S[i]) if kind == "wkv"
+                       else plain.delta_recurrence(qd[p][:, which], kd[p][:, which], vd[p], gd[p], ud[p], S[i]))
+            close(got[at - go * T:at - go * T + c], o, 4e-6)
+            close(state[slots[i]][..., :d], S[i].transpose(1, 2), 4e-6)
+            assert d % 32 == 0 or bool((state[slots[i]][..., d:] == 0).all())
+            at, done[i] = at + c, done[i] + c
+    assert bool((state[[2, 4]] == 5).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["wkv", "delta"])
+def test_a_chunk_does_not_look_ahead(kind):
+    """A value that is not a number shows in its own column from its token on, not before it nor beside it."""
+    dev = _device("cuda")
+    T, t, j = 300, 133, 5
+    ins = list(_scan_inputs(kind, 2, 2, 64, 32, T, F32))
+    clean = _scan(kind, ins, slice(0, T), meta_of([T], dev), None, dev)
+    ins[2] = ins[2].clone()
+    ins[2][t, 1, j] = math.nan
+    got = _scan(kind, ins, slice(0, T), meta_of([T], dev), None, dev)
+    hit = torch.zeros_like(got, dtype=torch.bool)
+    hit[t:, 1, j] = True
+    assert torch.equal(got[~hit], clean[~hit]) and bool(got[t + 1:, 1, j].isnan().all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["wkv", "delta"])
+def test_scans_in_rounds_of_chunks(kind, monkeypatch):
+    """More tokens than the records of one round hold, against the kernels that go token by token."""
+    from easyllm_b200.ops import cuda, cuda_infer
+    dev = _device("cuda")
+    H, T = 64, 5000 if kind == "delta" else 7500
+    ins = _scan_inputs(kind, H, H, 128, 8, T, F32)
+    need = cuda.lib().ell_scan_chunks_work(int(kind == "delta"), T, 2, T - 40, H, 128, 8)
+    assert need * 4 < 520 << 20                        # the records of all chunks would take 550 MiB and more
+    got = []
+    for chunks in (True, False):
+        if not chunks:
+            monkeypatch.setattr(cuda_infer, "_scan_chunks", lambda *a: False)
+        state = torch.zeros(2, H, 8, 128, device=dev)
+        got.append((_scan(kind, ins, slice(0, T), meta_of([T - 40, 40], dev, [1, 0], [0, 0]), state, dev), state))
+    cuda.check_err_flag()
+    close(got[0][0], got[1][0].cpu(), 1e-5)
+    close(got[0][1], got[1][1].cpu(), 1e-5)
+
+
 @pytest.mark.parametrize("device", DEVICES)
 @pytest.mark.parametrize("kind", ["wkv", "delta"])
 def test_state_is_carried_far(device, kind):
