@@ -257,13 +257,13 @@ class Attention(nn.Module):
         return (qkv[:, :nq].view(T, self.hq, self.d), qkv[:, nq:nq + nk].view(T, self.hk, self.d),
                 qkv[:, nq + nk:].view(T, self.hk, self.dv))
 
-    def _attend(self, q, k, v, meta, cache):
+    def _attend(self, q, k, v, meta, cache, appended=False):
         """Serving attention: prompts that start here on the prefill kernel, everything else over the cached rows.
-        ``cache``: the layer's ``KVRows``, or None for packed sequences that keep nothing."""
+        ``cache``: the layer's ``KVRows``, or None for packed sequences that keep nothing.  ``appended``: it has the step's keys."""
         T = q.shape[0]
         sl = self.slopes.to(q.device) if self.slopes is not None else None
         sink = self.sink.detach() if self.sink is not None else None
-        if cache is not None:
+        if cache is not None and not appended:
             iops.kv_append(cache.k, cache.v, k, v, meta)
         fresh = cache is None or (meta["fresh"] and not meta["one_token"])
         if fresh and iops.prefill_kernel_ok(q, v):
@@ -307,14 +307,16 @@ class Attention(nn.Module):
             o = ops.flash_attention_packed(qkv, hq, hk, d, meta["cu_seqlens"], meta["max_seqlen"], alibi_slopes=sl,
                                            rope=rope, row_start=meta.get("row_start"))
             return ops.linear(o, self.o_proj.weight, self.o_proj.bias)
-        if rope is not None:
+        appended = rope is not None and isinstance(cache, KVRows) and \
+            ops.rope_append(qkv, cos, sin, pos, hq, hk, d, cache.k, cache.v, meta["kv_base"], meta["kv_len"])
+        if rope is not None and not appended:
             qkv = ops.rope_packed(qkv, cos, sin, pos, hq, hk, d)
         q, k, v = self._split(qkv)
         if a.use_logn_attn and not self.training:
             logn = torch.clamp(torch.log(pos.float() + 1) / math.log(a.seq_length), min=1.0)
             q = (q.float() * logn.view(T, 1, 1)).to(q.dtype)
         if isinstance(cache, KVRows):
-            o = self._attend(q, k, v, meta, cache)
+            o = self._attend(q, k, v, meta, cache, appended)
         elif cache is not None:               # dense batch of equal length in a dict: 8-bit cache, draft trees, prefixes
             B = meta["batch"]
             S = T // B

@@ -505,6 +505,17 @@ def rope_packed(qkv, cos, sin, pos, n_q_heads, n_kv_heads, head_dim):
     return torch.cat((q.reshape(T, nq), k.reshape(T, nk), qkv[:, nq + nk:]), dim=1)
 
 
+def rope_append(qkv, cos, sin, pos, n_q_heads, n_kv_heads, head_dim, kcache, vcache, kv_base, kv_len):
+    """``rope_packed`` in place, and the rotated keys and the values to their rows of a cache ``[.., kv_heads, head_dim]``, in one
+    launch where nothing is recorded; False (and nothing done) where that cannot be."""
+    if not (_kern(qkv) and head_dim % 16 == 0 and _cu().nothing_to_record() and qkv.is_contiguous()) or \
+            any(c.dtype != qkv.dtype or not c.is_contiguous() or c.shape[-2:] != (n_kv_heads, head_dim) or c.data_ptr() % 16
+                for c in (kcache, vcache)) or qkv.data_ptr() % 16 or any(t.dtype != torch.int32 for t in (pos, kv_base, kv_len)):
+        return False
+    _cu().rope_append_(qkv, cos, sin, pos, n_q_heads, n_kv_heads, head_dim, kcache, vcache, kv_base, kv_len)
+    return True
+
+
 class _SwiGLU(torch.autograd.Function):
     @staticmethod
     def forward(ctx, gu):

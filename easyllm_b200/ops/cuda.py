@@ -218,6 +218,18 @@ def rope_(qkv, cos, sin, pos, n_rot_heads, head_dim, backward=False):
     return qkv
 
 
+def rope_append_(qkv, cos, sin, pos, n_q, n_kv, head_dim, kcache, vcache, base, length):
+    """``rotate_`` of the q and k heads, with keys and values also written to cache rows ``base + length - 1``."""
+    _bf16c(qkv, "qkv"), _bf16c(kcache, "kcache"), _bf16c(vcache, "vcache")
+    if any(t.dtype != torch.int32 for t in (pos, base, length)) or qkv.shape[1] != (n_q + 2 * n_kv) * head_dim:
+        raise ValueError("rope_append_: int32 positions and places, rows of q, k and v heads")
+    rc = lib().ell_rope_append(_p(qkv), _p(cos), _p(sin), _p(pos), _p(kcache), _p(vcache), _p(base), _p(length), c_int(qkv.shape[0]),
+                               c_int(n_q), c_int(n_kv), c_int(head_dim), c_int(cos.shape[0]), _p(err_flag(qkv.device)), _stream())
+    _check(rc, "rope_append")
+    torch.autograd.graph.increment_version(qkv)
+    return qkv
+
+
 def rotate_(qkv, cos, sin, pos, n_rot_heads, head_dim):
     """``rope_`` as an in-place operation that autograd's version check sees."""
     rope_(qkv, cos, sin, pos, n_rot_heads, head_dim)

@@ -325,3 +325,24 @@ def test_embedding_gradient_goes_to_main_grad(cu, tokens, rows, cols, dtype, det
     want.index_add_(0, ids.long(), dy.double())
     size.index_add_(0, ids.long(), dy.double().abs())
     assert ((emb.weight.main_grad.double() - want).abs() <= size * (tokens + 1) * 2.0 ** -24).all()
+
+
+@pytest.mark.parametrize("T,hq,hk,D", [(1, 1, 1, 16), (7, 8, 2, 128), (301, 5, 5, 80)])
+def test_rope_append_is_rope_and_append(cu, T, hq, hk, D):
+    """Bit for bit the two launches it stands for: rotated rows, and the cache rows of scattered places; other rows stay."""
+    import easyllm_b200.ops.cuda_infer as ci
+    from easyllm_b200.ops import reference as ref
+    torch.manual_seed(T)
+    cos, sin = ref.rope_tables(D, 512, device="cuda")
+    qkv = torch.randn(T, (hq + 2 * hk) * D, device="cuda", dtype=torch.bfloat16)
+    pos = torch.randint(0, 512, (T,), device="cuda", dtype=torch.int32)
+    rows = torch.randperm(3 * T, device="cuda")[:T].to(torch.int32)
+    length = torch.randint(1, 4, (T,), device="cuda", dtype=torch.int32)
+    base = rows - length + 1 + 4
+    caches = [[torch.full((3 * T + 4, hk, D), 7.0, device="cuda", dtype=torch.bfloat16) for _ in "kv"] for _ in range(2)]
+    want = cu.rope_(qkv.clone(), cos, sin, pos, hq + hk, D)
+    k, v = want[:, hq * D:(hq + hk) * D].view(T, hk, D), want[:, (hq + hk) * D:].view(T, hk, D)
+    ci.kv_append(*caches[0], k, v, base, length)
+    got = cu.rope_append_(qkv, cos, sin, pos, hq, hk, D, *caches[1], base, length)
+    cu.check_err_flag()
+    assert torch.equal(got, want) and all(torch.equal(a, b) for a, b in zip(*caches))
