@@ -30,9 +30,9 @@ class DenseGLU(nn.Module):
             ([[self.gate_proj.bias, self.up_proj.bias]] if self.bias else [])
 
     def forward(self, h, residual):
-        gu = iops.linear_cat(h, [self.gate_proj.weight, self.up_proj.weight],
-                             [self.gate_proj.bias, self.up_proj.bias] if self.bias else None)
-        return iops.linear_add_(residual, iops.glu(gu, self.act), self.down_proj.weight)
+        a = iops.glu_linear(h, [self.gate_proj.weight, self.up_proj.weight],
+                            [self.gate_proj.bias, self.up_proj.bias] if self.bias else None, self.act)
+        return iops.linear_add_(residual, a, self.down_proj.weight)
 
 
 class _UpDown(nn.Module):

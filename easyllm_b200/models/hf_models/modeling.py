@@ -381,8 +381,7 @@ class MLP(nn.Module):
         return [[self.gate_proj.weight, self.up_proj.weight]]
 
     def forward(self, x):
-        gu = ops.linear_parts(x, (self.gate_proj.weight, self.up_proj.weight))
-        return ops.linear(ops.glu(gu, "silu"), self.down_proj.weight)
+        return ops.linear(ops.glu_linear(x, self.gate_proj.weight, self.up_proj.weight), self.down_proj.weight)
 
 
 class DecoderLayer(nn.Module):

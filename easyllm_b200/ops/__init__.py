@@ -540,6 +540,18 @@ def glu(gate_up, activation="silu"):
     return ref.GLU_ACTIVATIONS[activation](gate_up[..., :F_], gate_up[..., F_:])
 
 
+def glu_linear(x, gate, up):
+    """``silu(x Wgᵀ) * (x Wuᵀ)``: one launch where nothing is recorded, the weights lie next to each other and the rows fill CTA
+    pairs; otherwise ``glu`` of ``linear_parts``."""
+    if _kern(x) and x.dim() == 2 and _GEMM == "tcgen05" and gate.shape == up.shape and _cu().nothing_to_record() and \
+            _cu().glu_route(x.shape[0], gate.shape[0]):
+        w = _adjacent_alias([gate.detach(), up.detach()])
+        y = None if w is None else _cu().gemm_glu(x, w, None, "silu")
+        if y is not None:
+            return y
+    return glu(linear_parts(x, (gate, up)), "silu")
+
+
 # ---------------------------------------------------------------------------------------------
 # Attention
 # ---------------------------------------------------------------------------------------------

@@ -43,7 +43,7 @@ constexpr int kEpiBufBytes = 128 * 64 * 2; // one 128x64 bf16 store box
 
 // kOutBf16CE: bf16 C plus, per row and column slot, the cross-entropy statistics (max, sum-exp, target logit)
 // of the rounded logits, computed in the epilogue while the tile is in registers.
-enum GemmOut { kOutBf16 = 0, kOutF32Accum = 1, kOutF32 = 2, kOutBf16CE = 3 };
+enum GemmOut { kOutBf16 = 0, kOutF32Accum = 1, kOutF32 = 2, kOutBf16CE = 3, kOutGlu = 4 };
 enum GemmErr { kErrProducer = 1, kErrMma = 2, kErrEpilogue = 3, kErrComm = 4, kErrFlagWait = 5, kErrBounds = 6 };
 enum GemmFuse { kFuseNone = 0, kFuseAG = 1, kFuseRS = 2, kFuseAR = 3, kFuseAGK = 4, kFuseGroup = 5 };
 constexpr int kMaxTp = 8;
@@ -74,7 +74,7 @@ struct FuseArgs {
   const int* tile_expert;                // Group: expert of every row tile
   const int* n_row_tiles;                // Group: number of row tiles in use
   const float* row_scale;                // Group: per-row scale of the activation in the epilogue, or null
-  int group_glu;                         // Group: the activation is silu(gate) * up over interleaved columns
+  int group_glu;                         // Group: the activation is silu(gate) * up over interleaved columns; kOutGlu: the gate's (GluAct)
   int rs_lag_q;                          // CTA-pair reduce-scatter: own tiles trail the peers' by this many quarter waves (0: default)
 };
 

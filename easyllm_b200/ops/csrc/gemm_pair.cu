@@ -31,7 +31,13 @@
 // the peers' partial sums from the LOCAL staging buffer into the two epilogue buffers, and the epilogue adds them
 // to the fp32 accumulator in a fixed source order before the one rounding to bf16 (deterministic; the own partial
 // is never rounded).  GEMM -> all-reduce keeps the staged two-phase reduction of gemm_fuse.cuh.
+//
+// The gated form (kOutGlu) is the first product of a feed-forward layer that serves: W holds F gate rows, then F up rows, and a unit
+// of 256 columns is 128 of each.  The even CTA stages the gate rows and the odd one the up rows, so an accumulator row holds both
+// halves of its hidden units, and the epilogue writes act(gate + b) * (up + b) only: 2 F columns are neither written nor read again,
+// nor rounded in between.  4096 rows of 4096, F 11008: the pass over the 2 F columns took 46 us beside a product of 530.
 #include "gemm_fuse.cuh"
+#include "vec.cuh"
 
 namespace ell {
 namespace pair {
@@ -48,6 +54,7 @@ constexpr int kStageBytes = kABytes + kBBytes;
 constexpr int kTmemCols = 2 * kTileN;       // two accumulator buffers
 constexpr int kSmemBytes = kStages * kStageBytes + 2 * kEpiBufBytes + 1024 + 512;
 constexpr int kGroupM = 8;                  // rasterisation: 8 M-tiles x all N-tiles per group
+enum GluAct { kGluSilu = 1, kGluGelu = 2 };
 enum Err { kErrPairProducer = 11, kErrPairMma = 12, kErrPairEpilogue = 13, kErrPairFlagWait = 15 };
 
 struct Shared {
@@ -358,7 +365,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const Unit u = decode_unit(unit, tiles_m, tiles_n, num_full, FUSE, fuse.rank, fuse.tp, n_clusters, fuse.rs_lag_q);
         const int b_rows = u.bn / 2;                                // B rows staged by one CTA (128, or 64 in a half unit)
         const int m0 = u.mt * kTileM + (int)cta_rank * kHalfM;     // A rows of this CTA
-        const int nb0 = u.n0 + (int)cta_rank * b_rows;             // B rows of this CTA
+        // B rows of this CTA (gated: gate rows in the even CTA, the same up rows in the odd one)
+        const int nb0 = OUT == kOutGlu ? u.n0 / 2 + (int)cta_rank * (N / 2) : u.n0 + (int)cta_rank * b_rows;
         const CUtensorMap* b_map = (u.bn == kTileN) ? &tmB : &tmBh; // half units: box of 64 B rows
         const uint32_t stage_tx = 2u * (kABytes + (uint32_t)b_rows * kBK * 2);
         const CUtensorMap* a_map = &tmA;
@@ -678,6 +686,45 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               mbar_arrive(&sh->part_empty[slot]);
             }
           }
+        }
+      } else if (OUT == kOutGlu) {
+        const int F = N / 2, f0 = n0 / 2;
+#pragma unroll 1
+        for (int j = 0; j < u.bn / 128; ++j) {
+          uint8_t* buf = sC + (store_count & 1) * kEpiBufBytes;
+          if (store_thread) tma_store_wait_read<1>();
+          named_bar_sync(1, kEpiThreads);
+          uint8_t* row_ptr = buf + row_in_tile * 128;
+#pragma unroll 1
+          for (int p = 0; p < 2; ++p) {
+            const int col = f0 + j * 64 + p * 32;
+            uint32_t r[64];
+            tmem_ld_32x32(t_row + j * 64 + p * 32, r);
+            tmem_ld_32x32(t_row + u.bn / 2 + j * 64 + p * 32, r + 32);
+            tmem_ld_wait();
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              float v[8];
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                float gate = __uint_as_float(r[c * 8 + e]), up = __uint_as_float(r[32 + c * 8 + e]);
+                if (HAS_BIAS) {
+                  const int at = col + c * 8 + e;
+                  gate += at < F ? __bfloat162float(bias[at]) : 0.f;
+                  up += at < F ? __bfloat162float(bias[F + at]) : 0.f;
+                }
+                v[e] = up * (fuse.group_glu == kGluGelu ? gelu_tanh_f(gate) : silu_f(gate));
+              }
+              *reinterpret_cast<bf16x8*>(row_ptr + (((p * 4 + c) ^ (row_in_tile & 7)) << 4)) = pack8(v);  // 128B swizzle
+            }
+          }
+          fence_proxy_async_smem();
+          named_bar_sync(1, kEpiThreads);
+          if (store_thread) {
+            if (f0 + j * 64 < F && m0 < M) tma_store_2d(&tmC, buf, f0 + j * 64, m0);
+            tma_store_commit();
+          }
+          ++store_count;
         }
       } else if (OUT == kOutBf16 || OUT == kOutBf16CE) {
         // reduce-scatter, a tile another rank owns: the blocks go to warp 7 instead of being stored from here
@@ -1114,6 +1161,27 @@ ELL_API int ell_gemm_bf16_pair(const void* A, const void* B, void* C, const void
   ELL_PAIR_CASE(false, true, kOutF32, false)
 #undef ELL_PAIR_CASE
   return -3;
+}
+
+// out [M, F] (rows of ldo) = act(x Wg^T + bg) * (x Wu^T + bu); W [2 F, K] and bias [2 F] (or null) hold the gate's part first.
+// act: 1 silu, 2 gelu (tanh form).
+ELL_API int ell_gemm_glu_pair(const void* x, const void* W, void* out, const void* bias, int M, int F, int K, int ldx, int ldo,
+                              int act, int* err, cudaStream_t stream) {
+  using namespace ell::pair;
+  if (M <= 0 || F <= 0 || K <= 0) return 0;
+  if (act != kGluSilu && act != kGluGelu) return -2;
+  CUtensorMap tA, tB, tC, tBh;
+  int rc = make_tmap_bf16_2d(&tA, x, (uint64_t)K, (uint64_t)M, (uint64_t)ldx * 2, kBK, kHalfM);
+  if (!rc) rc = make_tmap_bf16_2d(&tB, W, (uint64_t)K, (uint64_t)2 * F, (uint64_t)K * 2, kBK, kHalfN);
+  if (!rc) rc = make_tmap_bf16_2d(&tBh, W, (uint64_t)K, (uint64_t)2 * F, (uint64_t)K * 2, kBK, kHalfN / 2);
+  if (!rc) rc = make_tmap_bf16_2d(&tC, out, (uint64_t)F, (uint64_t)M, (uint64_t)ldo * 2, 64, 128);
+  if (rc) return rc;
+  FuseArgs f{};
+  f.no_tail_split = g_no_tail_split;
+  f.group_glu = act;
+  const __nv_bfloat16* bp = reinterpret_cast<const __nv_bfloat16*>(bias);
+  if (bias) return launch<false, false, kOutGlu, true>(tA, tB, tC, tBh, tA, f, bp, M, 2 * F, K, err, stream);
+  return launch<false, false, kOutGlu, false>(tA, tB, tC, tBh, tA, f, bp, M, 2 * F, K, err, stream);
 }
 
 // Slots of cross-entropy partials the CTA-pair epilogue fills (one per 128 columns).

@@ -431,6 +431,29 @@ def gemm(a, b, out=None, bias=None, a_mn=False, b_mn=False, out_mode=0, bn=0, pa
     return out
 
 
+def glu_route(M, F):
+    """Whether the gated form of the CTA-pair GEMM takes ``M`` rows: where the plain product would run on CTA pairs too."""
+    return _use_pair(M, 2 * F, 0)
+
+
+def gemm_glu(x, w, bias, act):
+    """``act(x Wgᵀ + bg) * (x Wuᵀ + bu)`` in one product; ``w [2F, K]`` and ``bias [2F]`` (or None) hold the gate's part first, x has
+    rows of contiguous elements.  None where the launch is refused or the operands don't fit."""
+    (M, K), F = x.shape, w.shape[0] // 2
+    ldx = x.stride(0) if M > 1 else K
+    if x.dtype != torch.bfloat16 or w.dtype != x.dtype or (bias is not None and bias.dtype != x.dtype) or x.stride(1) != 1 or \
+            not w.is_contiguous() or (bias is not None and not bias.is_contiguous()) or w.shape != (2 * F, K) or \
+            F % 8 or K % 8 or ldx % 8 or (x.data_ptr() | w.data_ptr()) & 15:
+        return None
+    out = torch.empty(M, F, dtype=x.dtype, device=x.device)
+    rc = lib().ell_gemm_glu_pair(_p(x), _p(w), _p(out), _p(bias), c_int(M), c_int(F), c_int(K), c_int(ldx), c_int(F),
+                                 c_int({"silu": 1, "gelu_tanh": 2}[act]), _p(err_flag(x.device)), _stream())
+    if rc in _PAIR_LAUNCH_REFUSED:
+        return None
+    _check(rc, "gemm_glu_pair")
+    return out
+
+
 def flash_fwd_plan(row_start):
     """Host-only: per (tile pair, tile) of the attention forward the first key row, the number of 128-key tiles it
     walks and which of them are masked element-wise, from the kernel's own arithmetic (``row_start``: a list or CPU

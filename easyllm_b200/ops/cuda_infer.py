@@ -88,6 +88,11 @@ def linear(x, w, bias=None, out_f32=False, act=None):
     return cu.matvec(x, ldx, w, bias, y, ld, out_f32=out_f32, act_tanh=act == "tanh")[:, :N]
 
 
+def glu_linear(x, w, bias, act):
+    """The gated product in one launch, or None (``cuda.gemm_glu``)."""
+    return cu.gemm_glu(x, w, bias, act) if cu.glu_route(x.shape[0], w.shape[0] // 2) else None
+
+
 def linear_batch(xs, w):
     """xs ``[n, T, K]``, w ``[n, N, K]`` contiguous → ``[n, T, N]``."""
     n, M, K = xs.shape

@@ -97,6 +97,18 @@ def linear_cat_f32(x, weights):
     return linear_f32(x, fused(weights))
 
 
+def glu_linear(x, weights, biases, act):
+    """``act(x Wgᵀ + bg) * (x Wuᵀ + bu)`` for ``weights`` and ``biases`` (or None) of gate and up: one launch for bf16 rows that fill
+    CTA pairs, once the weights are adjacent."""
+    if x.is_cuda and x.dtype == torch.bfloat16 and weights[0].shape == weights[1].shape:
+        w, b = fused_alias(weights), None if biases is None else fused_alias(biases)
+        if w is not None and (b is not None or biases is None):
+            y = _cu().glu_linear(x, w, b, act)
+            if y is not None:
+                return y
+    return glu(linear_cat(x, weights, biases), act)
+
+
 def linear_batch(xs, weights):
     """``xs[i] W_iᵀ`` for equally shaped weights → ``[n, T, N]``."""
     if _kern(xs):

@@ -245,3 +245,24 @@ def test_gemm_routes_agree(cu, T, N, K):
     want = cu.gemm(a, w, out=acc.clone(), out_mode=1, pair=False)
     _check(cu.gemm(a, w, out=acc, out_mode=1), want, K)
     cu.check_err_flag()
+
+
+@pytest.mark.parametrize("M,F,K", [(256, 128, 64), (256, 1000, 72), (2049, 200, 520), (2304, 2824, 1024)])
+@pytest.mark.parametrize("act,bias", [("silu", False), ("gelu_tanh", True)])
+def test_gated_product(cu, M, F, K, act, bias):
+    """One launch against the two it stands for in 64 bits: the result is rounded to bf16 once (2^-9 of itself), sums of K products
+    in fp32 are off by at most K 2^-23 of the sum of magnitudes, which the activation (slope up to 1.13) passes on."""
+    g = torch.Generator(device="cuda").manual_seed(M + F)
+    x = torch.randn(M, 2 * K, device="cuda", generator=g).to(torch.bfloat16)[:, K:]          # rows of a wider tensor
+    w = (torch.randn(2 * F, K, device="cuda", generator=g) * K ** -0.5).to(torch.bfloat16)
+    b = torch.randn(2 * F, device="cuda", generator=g).to(torch.bfloat16) if bias else None
+    y = cu.gemm_glu(x, w, b, act)
+    cu.check_err_flag()
+    z = x.double() @ w.double().t()
+    size = x.double().abs() @ w.double().abs().t() * K * 2.0 ** -23
+    if bias:
+        z, size = z + b.double(), size + b.double().abs() * 2.0 ** -22
+    a = torch.nn.functional.silu(z[:, :F]) if act == "silu" else torch.nn.functional.gelu(z[:, :F], approximate="tanh")
+    want = a * z[:, F:]
+    bound = want.abs() * 2.0 ** -8 + 1.2 * (size[:, :F] * z[:, F:].abs() + size[:, F:] * a.abs()) + 1e-6
+    assert ((y.double() - want).abs() <= bound).all()
