@@ -94,6 +94,9 @@ struct GemmCfg {
 
 // Up to one row tile of A: the first kAheadBlocks k-blocks of B go into L2 ahead of the wait (39 MB over the SMs).
 constexpr int kAheadRows = 128, kAheadBlocks = 8;
+// Rows up to which a launch starts while the kernel before it ends.  With many, nothing is gained, and the CTAs come in where the
+// kernel before left room first: 16 experts of 4096 x 2752, rows of 4096 tokens, 593 us chained and 562 not; of 128 tokens 217 and 221.
+constexpr int kChainedRows = 4096;
 
 struct GemmShared {
   uint64_t full[8];
@@ -607,7 +610,7 @@ static int launch_gemm(const CUtensorMap& tA, const CUtensorMap& tB, const CUten
   }
   const int tiles = ((M + kBM - 1) / kBM) * ((N + BN - 1) / BN);
   int grid = (FUSE != kFuseNone || tiles >= max_ctas) ? max_ctas : tiles;   // fused launches keep a fixed grid
-  if (FUSE == kFuseNone || FUSE == kFuseGroup)
+  if ((FUSE == kFuseNone || FUSE == kFuseGroup) && M <= kChainedRows)
     launch_chained(kern, grid, kGemmThreads, GemmCfg<BN>::kSmemBytes, stream, tA, tB, tC, tA2 ? *tA2 : tA, fuse, bias, M, N, K,
                    ldc, err);
   else
