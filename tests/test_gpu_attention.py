@@ -243,3 +243,20 @@ def test_attention_over_cached_rows(steps, past, H, G, d, dv, extras):
             o = iops.attention_rows(q, k, v, b, n, bound, d ** -0.5, sink, slopes, window, gate, **kw)
             assert (o.double() - want).norm() <= 1.9e-3 * want.norm()
             assert (o.double() - want).abs().max() <= 2.0 ** -8 * want.abs().max()
+
+
+@pytest.mark.parametrize("hq,hk", [(5, 5), (6, 2)])
+def test_heads_in_several_groups(cu, hq, hk):
+    """So many tokens that the heads' CTAs come in several groups, the last one smaller: documents of 512 tokens alone (the same
+    tiles, in one group) give the same bits."""
+    torch.manual_seed(0)
+    T, D, doc = (40960 if hq == hk else 81920), 128, 512
+    q, k, v = (torch.randn(T, h, D, device="cuda", dtype=torch.bfloat16) for h in (hq, hk, hk))
+    start = torch.arange(T, device="cuda", dtype=torch.int32) // doc * doc
+    out, lse = cu.flash_attn_fwd(q, k, v, start, D ** -0.5)[:2]
+    cu.check_err_flag()
+    for a in (0, T // 2, T - 4 * doc):
+        part = slice(a, a + 4 * doc)
+        o, l = cu.flash_attn_fwd(q[part].contiguous(), k[part].contiguous(), v[part].contiguous(), start[:4 * doc].contiguous(),
+                                 D ** -0.5)[:2]
+        assert torch.equal(out[part], o) and torch.equal(lse[:, part], l)
