@@ -342,11 +342,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
       float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
 #pragma unroll
-      for (int i = 0; i < KN; i += 4) {
-        mx0 = fmaxf(mx0, __uint_as_float(s[i]));
-        mx1 = fmaxf(mx1, __uint_as_float(s[i + 1]));
-        mx2 = fmaxf(mx2, __uint_as_float(s[i + 2]));
-        mx3 = fmaxf(mx3, __uint_as_float(s[i + 3]));
+      for (int i = 0; i < KN; i += 8) {
+        mx0 = fmax3(mx0, __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
+        mx1 = fmax3(mx1, __uint_as_float(s[i + 2]), __uint_as_float(s[i + 3]));
+        mx2 = fmax3(mx2, __uint_as_float(s[i + 4]), __uint_as_float(s[i + 5]));
+        mx3 = fmax3(mx3, __uint_as_float(s[i + 6]), __uint_as_float(s[i + 7]));
       }
       const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * scale_log2;
       const float m_new = fmaxf(m_used, mx);
@@ -376,18 +376,26 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         tmem_st_wait();
         tc_fence_before();
       }
-      // P = exp2(s*scale - m_used) -> bf16 -> swizzled smem, 8 columns (one 16-byte chunk) at a time
-      float ps0 = 0.f, ps1 = 0.f, ps2 = 0.f, ps3 = 0.f;
-      const float neg_m = -m_used;
+      // P = exp2(s*scale - m_used) -> bf16 -> swizzled smem, 8 columns (one 16-byte chunk) at a time.  The softmax warps are bound
+      // by the instructions they issue, so everything but ex2 and the conversion works on pairs (or takes three operands): 4096
+      // tokens, 32 heads 198 -> 187 us, 8192 tokens 612 -> 574.  (Exponentials on the FMA pipe, exact to fp32, cost more
+      // instructions than they take off the special-function pipe: a quarter of them 198, half 208, three quarters 238.)
+      float2 ps0 = make_float2(0.f, 0.f), ps1 = ps0;
+      const float2 scale2 = make_float2(scale_log2, scale_log2), neg_m = make_float2(-m_used, -m_used);
 #pragma unroll
       for (int c = 0; c < KN / 8; ++c) {
         float p[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) p[i] = exp2f(fmaf(__uint_as_float(s[c * 8 + i]), scale_log2, neg_m));
-        ps0 += p[0] + p[4]; ps1 += p[1] + p[5]; ps2 += p[2] + p[6]; ps3 += p[3] + p[7];
+        for (int i = 0; i < 8; i += 2) {
+          const float2 x = ffma2(make_float2(__uint_as_float(s[c * 8 + i]), __uint_as_float(s[c * 8 + i + 1])), scale2, neg_m);
+          p[i] = ex2_approx(x.x);
+          p[i + 1] = ex2_approx(x.y);
+          if (i & 2) ps1 = fadd2(ps1, make_float2(p[i], p[i + 1]));
+          else ps0 = fadd2(ps0, make_float2(p[i], p[i + 1]));
+        }
         *reinterpret_cast<bf16x8*>(p_row + (c >> 3) * Cfg::kQChunk + (((c & 7) ^ sw) << 4)) = pack8(p);
       }
-      l += (ps0 + ps1) + (ps2 + ps3);
+      l += (ps0.x + ps0.y) + (ps1.x + ps1.y);
       fence_proxy_async_smem();
       mbar_arrive(&sh->p_full[t]);
       if (threadIdx.x == 64) FA_TRACE(1, j, 5);
