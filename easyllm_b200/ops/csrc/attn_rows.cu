@@ -1056,6 +1056,27 @@ struct AtPlan {
   bool fits, few;
   int tt, tiles, splits, range;
 };
+// Ranges of decoding rows: the CTAs come in rounds of two an SM, and the last round takes as long as a full one, so the number of
+// ranges decides how much of it is idle.  A round reads its keys at 5 TB/s and costs 3 us besides, a merge 3.  Measured (us; 32 query
+// heads on 8 key heads, ranges 1 / 2 / 3 / 4): 48 sequences of 2048 keys 130 / 104 / 100 / 105, 64 of them 132 / 138 / 137 / 134, 24 of
+// 3000 95 / 91 / 78 / 79; 10 sequences with 32 key heads 128 / 99 / 91 / 88.  A CTA an SM and fewer go in about one round: the last
+// range, which ends before the bound of the lengths, may be a few CTAs over it (4 sequences of 3000, 16 key heads: 4 ranges 33, 5 ranges
+// 29; 8 of 4096, 8 key heads: 41 and 41).
+static int at_ranges(long long ctas, long long most, double bytes_of_cta) {
+  if (ctas <= kNumSMs) return (int)((2LL * kNumSMs + ctas / 2) / ctas < most ? (2LL * kNumSMs + ctas / 2) / ctas : most);
+  const double whole = bytes_of_cta * 2 * kNumSMs / 5e6;
+  int best = 1;
+  double least = 1e30;
+  for (int s = 1; s <= most; ++s) {
+    const long long rounds = (ctas * s + 2 * kNumSMs - 1) / (2 * kNumSMs);
+    const double us = rounds * (whole / s + 3.0) + (s > 1 ? 3.0 : 0.0);
+    if (us < least) {
+      least = us;
+      best = s;
+    }
+  }
+  return best;
+}
 static AtPlan at_plan(int n, int n_seq, int max_q, int H, int G, int d, int dv, int max_len, int window, bool is_bf16) {
   AtPlan p{};
   p.fits = is_bf16 && d % 16 == 0 && dv % 16 == 0 && d <= 128 && dv <= 128 && d > 0 && dv > 0;
@@ -1068,10 +1089,10 @@ static AtPlan at_plan(int n, int n_seq, int max_q, int H, int G, int d, int dv, 
   const long long ctas = (long long)(one ? n : n_seq * p.tiles) * G * groups;
   if (window > 0 && max_len > window) max_len = window;
   max_len += p.tt - 1;                                  // a tile's rows see windows that start apart
-  // the two CTAs that fit an SM: one round of long ranges (8 x 4096 keys x 8 heads: 41.5 us at 5 ranges, 55 at 3, 50 at 28);
-  // the tiles of continued prompts differ in length, so they are dealt finer
-  long long s = p.few ? (2LL * kNumSMs + ctas / 2) / ctas : (4LL * kNumSMs + ctas - 1) / ctas;
+  // the tiles of continued prompts differ in length, so they are dealt finer than the two CTAs that fit an SM
   const long long most = (max_len + 127) / 128;
+  long long s = p.few ? at_ranges(ctas, most < kArMaxSplits ? most : kArMaxSplits, (double)max_len * (d + dv) * 2)
+                      : (4LL * kNumSMs + ctas - 1) / ctas;
   if (s > most) s = most;
   if (s > kArMaxSplits) s = kArMaxSplits;
   p.splits = s < 1 ? 1 : (int)s;

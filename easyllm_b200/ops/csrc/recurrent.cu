@@ -1,6 +1,6 @@
 // Recurrent token mixers (inference): the short convolutions and gates of the gated delta rule, and the scans of the
-// delta rule and of RWKV-style time mixing over packed sequences.  One source for prompts (long sequences) and decoding
-// (one token); the recurrent state is fp32 throughout and so is everything that enters it.
+// delta rule and of RWKV-style time mixing over packed sequences, token by token: decoding, short prompts and the head sizes
+// that scan_chunks.cu does not take; the recurrent state is fp32 throughout and so is everything that enters it.
 //
 // A state matrix S [d key rows x dv value columns] of one head evolves column by column without mixing columns:
 //   time mixing   o_j = sum_i r_i (S_ij + u_i k_i v_j),          S_ij <- w_i S_ij + k_i v_j

@@ -260,3 +260,24 @@ def test_heads_in_several_groups(cu, hq, hk):
         o, l = cu.flash_attn_fwd(q[part].contiguous(), k[part].contiguous(), v[part].contiguous(), start[:4 * doc].contiguous(),
                                  D ** -0.5)[:2]
         assert torch.equal(out[part], o) and torch.equal(lse[:, part], l)
+
+
+@pytest.mark.parametrize("n,H,G,bound", [(1, 8, 2, 4000), (3, 4, 4, 100), (40, 8, 4, 4352), (148, 1, 1, 3000), (149, 1, 1, 3000)])
+def test_ranges_of_decoding_rows(cu, n, H, G, bound):
+    """Both sides of the rule for the number of key ranges, lengths from one key to the bound, against the softmax in 64 bits: weights
+    enter in two bf16 parts (2^-16), the result is rounded to bf16 (2^-9 of values below 5)."""
+    import easyllm_b200.ops.cuda_infer as ci
+    d = 64
+    g = torch.Generator(device="cuda").manual_seed(n)
+    cap = bound + 8
+    k, v = (torch.randn(n * cap, G, d, device="cuda", generator=g).to(torch.bfloat16) for _ in "kv")
+    q = torch.randn(n, H, d, device="cuda", generator=g).to(torch.bfloat16)
+    length = torch.randint(1, bound + 1, (n,), device="cuda", generator=g, dtype=torch.int32)
+    length[0], length[-1] = 1, bound
+    base = torch.arange(n, device="cuda", dtype=torch.int32) * cap
+    out = ci.attention_rows(q, k, v, base, length, bound, d ** -0.5)
+    for i in {0, n // 2, n - 1}:
+        keys = slice(int(base[i]), int(base[i] + length[i]))
+        kk, vv = (t[keys].double().repeat_interleave(H // G, 1) for t in (k, v))
+        p = torch.softmax(torch.einsum("hd,khd->hk", q[i].double(), kk) * d ** -0.5, -1)
+        assert (out[i].double() - torch.einsum("hk,khd->hd", p, vv)).abs().max() <= 5 * (2.0 ** -9 + 2.0 ** -15)
