@@ -57,7 +57,8 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
 }
 // As mbar_wait, for a barrier that other CTAs of the cluster arrive on.
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                                  unsigned long long limit_ns) {
   const unsigned long long t0 = globaltimer_ns();
   uint32_t spins = 0;
   while (true) {
@@ -68,8 +69,12 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     if (ok) return true;
-    if ((++spins & 255u) == 0 && (*abort_flag || globaltimer_ns() - t0 > kWaitTimeoutNs)) return false;
+    if ((++spins & 255u) == 0 && (*abort_flag || globaltimer_ns() - t0 > limit_ns)) return false;
   }
+}
+
+__device__ __forceinline__ void set_in_peer(uint32_t addr, int v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
 // Barrier of the epilogue that tells every thread whether any of them failed.
@@ -100,6 +105,8 @@ struct ThinArgs {
   void* out;
   const __nv_bfloat16* bias;
   int T, N, K, ldo, out_mode, split, split_log2;
+  unsigned long long limit_ns;   // of a wait for a peer
+  int mute;                      // CTA of a cluster that sends nothing (a test of the waits), or -1
   int* err;
 };
 
@@ -265,11 +272,13 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     const uint32_t block = (uint32_t)cols * kThRows * 4;
     int it = 0, ex = 0;
     bool failed = false;
-    for (int tile = first; tile < tiles && !failed; tile += step, ++it) {
+    // A wait that runs out is one thread's own finding.  It stays set until the next vote, where all threads of the epilogue leave
+    // together: one that left alone would strand the others at their barrier.
+    for (int tile = first; tile < tiles; tile += step, ++it) {
       const int n0 = tile / tiles_t * kThRows, t0 = tile % tiles_t * BN, n = n0 + row;
       const int acc = it & 1;
-      failed = epi_any(!mbar_wait(&sh->tmem_full[acc], (it >> 1) & 1, abort_flag));
-      if (failed) break;                             // uniform across the epilogue
+      failed = epi_any(failed || !mbar_wait(&sh->tmem_full[acc], (it >> 1) & 1, abort_flag));
+      if (failed) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       const float bias = a.bias != nullptr && n < a.N ? __bfloat162float(a.bias[n]) : 0.f;
@@ -301,7 +310,7 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       }
       for (int c0 = 0; c0 < BN; c0 += EX, ++ex) {
         // the peers are done with the exchange before: its bytes have left `send`, and their `recv` may be written
-        if (ex > 0) failed = !mbar_wait_cluster(&sh->recv_free, (ex - 1) & 1, abort_flag);
+        if (ex > 0 && !mbar_wait_cluster(&sh->recv_free, (ex - 1) & 1, abort_flag, a.limit_ns)) failed = true;
 #pragma unroll 1
         for (int c = 0; c < EX; c += 16) {
           uint32_t v[16];
@@ -319,14 +328,16 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         if (failed) break;
         if (threadIdx.x == 64) {
           mbar_expect_tx(&sh->recv_full, (split - 1) * block);
-          for (int d = 1; d < split; ++d) {          // slot of this CTA at peer p: its rank among the others
+          for (int d = 1; d < split && rank != a.mute; ++d) {          // slot of this CTA at peer p: its rank among the others
             const int p = (rank + d) & (split - 1);
             bulk_copy_to_peer(map_to_rank(smem_u32(recv), p) + (rank - (rank > p)) * block, send + (size_t)p * cols * kThRows,
                               block, map_to_rank(smem_u32(&sh->recv_full), p));
           }
         }
-        failed = !mbar_wait_cluster(&sh->recv_full, ex & 1, abort_flag);
-        if (!failed && n < a.N) {
+        if (!mbar_wait_cluster(&sh->recv_full, ex & 1, abort_flag, a.limit_ns)) {
+          failed = true;
+          sh->abort_flag = 1;
+        } else if (n < a.N) {
           const int tc = t0 + c0 + rank * cols;
           const float *mine = send + (size_t)rank * cols * kThRows + row, *theirs = recv + row;
           if (cols >= 8) sum_columns<8>(mine, theirs, cols, rank, split, tc, a.T, old, put);
@@ -346,6 +357,11 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 
   tc_fence_before();
   __syncthreads();
+  if (split > 1) {
+    // a CTA that gave up may still be sent to, and its copies may still be on their way: all of the cluster wait for them
+    if (*abort_flag && threadIdx.x < split) set_in_peer(map_to_rank(smem_u32(&sh->abort_flag), threadIdx.x), 1);
+    cluster_sync_all();                              // no CTA starts a copy any more
+  }
   if (*abort_flag && threadIdx.x == 0) {
     // error path: give copies and MMAs in flight time to land before shared memory and TMEM go away
     const unsigned long long t0 = globaltimer_ns();
@@ -353,7 +369,6 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     }
   }
   __syncthreads();
-  if (split > 1) cluster_sync_all();                 // no peer writes here any more
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc<Cfg::kTmemCols>(tmem_base);
@@ -461,9 +476,10 @@ ELL_API int ell_gemm_thin_route(int T, int N, int K) {
 
 // out [T, N] rows of ldo = x [T, K] rows of ldx · W^T (+ bias [N], bf16 output only); W [N, K] (w_mn 0) or [K, N] (w_mn 1),
 // rows of ldw.  out_mode: 0 bf16, 1 fp32 +=, 2 fp32 =.  K, ldx, ldw multiples of 8, x and W on 16-byte boundaries.
-// split: CTAs per reduction, 0 for the rule above.
+// split: CTAs per reduction, 0 for the rule above.  wait_us: limit of the wait for another CTA's sums (0: 2 s), after which the error
+// word is set; mute: CTA of a cluster that withholds its sums, so that a test can let that wait run out (-1: none).
 ELL_API int ell_gemm_thin(const void* x, const void* W, void* out, const void* bias, int T, int N, int K, int ldx, int ldw,
-                          int ldo, int w_mn, int out_mode, int split, int* err, cudaStream_t stream) {
+                          int ldo, int w_mn, int out_mode, int split, int wait_us, int mute, int* err, cudaStream_t stream) {
   if (T <= 0 || N <= 0 || K <= 0) return 0;
   if (out_mode < kOutBf16 || out_mode > kOutF32 || (bias && out_mode != kOutBf16)) return -2;
   if (split != 0 && split != 1 && split != 2 && split != 4 && split != 8) return -2;
@@ -474,7 +490,8 @@ ELL_API int ell_gemm_thin(const void* x, const void* W, void* out, const void* b
   if (!rc) rc = make_tmap_bf16_2d(&tx, x, (uint64_t)K, (uint64_t)T, (uint64_t)ldx * 2, kBK, BN);
   if (rc) return rc;
   if (split > (K + kBK - 1) / kBK) return -2;
-  const ThinArgs a{out, (const __nv_bfloat16*)bias, T, N, K, ldo, out_mode, split, 0, err};
+  const unsigned long long limit = wait_us > 0 ? wait_us * 1000ull : kWaitTimeoutNs;
+  const ThinArgs a{out, (const __nv_bfloat16*)bias, T, N, K, ldo, out_mode, split, 0, limit, mute, err};
 #define ELL_THIN(BN_)                                                                     \
   if (BN == BN_) return w_mn ? launch_thin<BN_, true>(tw, tx, a, stream) : launch_thin<BN_, false>(tw, tx, a, stream);
   ELL_THIN(16)

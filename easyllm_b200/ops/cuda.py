@@ -378,7 +378,7 @@ def gemm_thin(x, w, out, bias=None, ldx=None, ldw=None, ldo=None, w_mn=False, ou
     N = w.shape[1] if w_mn else w.shape[0]
     rc = lib().ell_gemm_thin(_p(x), _p(w), _p(out), _p(bias), c_int(T), c_int(N), c_int(K), c_int(ldx or x.shape[1]),
                              c_int(ldw or w.shape[1]), c_int(ldo or N), c_int(w_mn), c_int(out_mode), c_int(split),
-                             _p(err_flag(x.device)), _stream())
+                             c_int(0), c_int(-1), _p(err_flag(x.device)), _stream())
     _check(rc, "gemm_thin")
     return out
 

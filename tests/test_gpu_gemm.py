@@ -266,3 +266,22 @@ def test_gated_product(cu, M, F, K, act, bias):
     want = a * z[:, F:]
     bound = want.abs() * 2.0 ** -8 + 1.2 * (size[:, :F] * z[:, F:].abs() + size[:, F:] * a.abs()) + 1e-6
     assert ((y.double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("T,N,K,split", [(16, 1024, 1024, 2), (128, 20000, 512, 4), (256, 4096, 1024, 8)])
+def test_sums_that_never_arrive_end_in_an_error(cu, T, N, K, split):
+    """One CTA of every cluster withholds its sums: the others' waits (2 ms here) run out, in the first exchange of a tile and in
+    the second (128 rows and more have two), with tiles left to do and without.  The launch ends, reports it, and the next one is
+    as ever."""
+    from ctypes import c_int
+    x, w = (torch.randn(*s, device="cuda", dtype=torch.bfloat16) for s in ((T, K), (N, K)))
+    out = torch.empty(T, N, device="cuda")
+    for mute in (0, split - 1):
+        rc = cu.lib().ell_gemm_thin(cu._p(x), cu._p(w), cu._p(out), cu._p(None), *(c_int(i) for i in (T, N, K, K, K, N, 0, 2, split)),
+                                    c_int(2000), c_int(mute), cu._p(cu.err_flag(x.device)), cu._stream())
+        assert rc == 0
+        with pytest.raises(cu.KernelError, match="gave up"):
+            cu.check_err_flag()
+        cu.gemm_thin(x, w, out, out_mode=2, split=split)
+        cu.check_err_flag()
+        _check(out, (x.double() @ w.double().t()).float(), K)
