@@ -296,13 +296,15 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           uint32_t v[16];
           tmem_ld_32x16(t_row + c, v);
           tmem_ld_wait();
-          if (n >= a.N) continue;
-          float before[16];
+          if (n < a.N) {
+            float before[16];
 #pragma unroll
-          for (int i = 0; i < 16; ++i) before[i] = t0 + c + i < a.T ? old(t0 + c + i) : 0.f;
+            for (int i = 0; i < 16; ++i) before[i] = t0 + c + i < a.T ? old(t0 + c + i) : 0.f;
 #pragma unroll
-          for (int i = 0; i < 16; ++i)
-            if (t0 + c + i < a.T) put(t0 + c + i, before[i] + __uint_as_float(v[i]));
+            for (int i = 0; i < 16; ++i)
+              if (t0 + c + i < a.T) put(t0 + c + i, before[i] + __uint_as_float(v[i]));
+          }
+          __syncwarp();                              // lanes past N skip the stores; the next load takes the whole warp
         }
         tc_fence_before();
         mbar_arrive(&sh->tmem_empty[acc]);

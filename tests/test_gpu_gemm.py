@@ -285,3 +285,17 @@ def test_sums_that_never_arrive_end_in_an_error(cu, T, N, K, split):
         cu.gemm_thin(x, w, out, out_mode=2, split=split)
         cu.check_err_flag()
         _check(out, (x.double() @ w.double().t()).float(), K)
+
+
+@pytest.mark.parametrize("N", [1, 33, 127, 1000, 18999])
+def test_few_rows_of_a_weight_that_ends_within_a_warp(cu, N):
+    """Unsplit reductions of 64 and 128 rows: the lanes past the last row of the weight store nothing, and the warp goes on to the
+    next 16 columns, and to the next tile, together.  Sums of 64 products in fp32, rounded to bf16 once."""
+    for T in (64, 100, 256):
+        torch.manual_seed(N + T)
+        x, w = (torch.randn(*s, device="cuda", dtype=torch.bfloat16) for s in ((T, 64), (N, 64)))
+        out = torch.full((T, N + 8), 3.0, device="cuda", dtype=torch.bfloat16)
+        cu.gemm_thin(x, w, out, ldo=N + 8, split=1)
+        cu.check_err_flag()
+        want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+        assert ((out[:, :N].double() - want).abs() <= want.abs() * 2.0 ** -8 + size * 2.0 ** -17).all() and (out[:, N:] == 3.0).all()
