@@ -64,6 +64,7 @@ struct ChunkArgs {
   float* carry;                 // [n_seq, H, dv, DP]: the state between two launches over one sequence, or null
   int H, G, d, dv, ldq, ldk, ldv;
   int c0, c1, per_seq;          // chunks of this launch; records per sequence (0: counted by tokens)
+  int final;                    // no chunks come after this launch
   int* err;
 };
 
@@ -310,6 +311,53 @@ __device__ __forceinline__ RawValues<T> load_values(const ChunkArgs& a, int star
   return x;
 }
 
+// Tokens t0 .. t1 - 1 of a sequence one by one, as scan_kernel computes them, for a warp's NC columns from `col` on.  Lane l holds
+// key rows l, l + 32, ... of them.  What chunks cannot do comes here: it is slow (0.5 us a token) and rare.
+template <int MODE, typename T, int DP, int NC>
+__device__ __noinline__ void walk_tokens(const ChunkArgs& a, int start, int t0, int t1, int h, int col, float (&S)[NC][DP / 32]) {
+  constexpr int J = DP / 32;
+  const int lane = threadIdx.x & 31, hk = h / (a.H / a.G);
+  float u[J];
+#pragma unroll
+  for (int j = 0; j < J; ++j) u[j] = MODE == kWkv && lane + 32 * j < a.d ? a.u[(size_t)h * a.d + lane + 32 * j] : 0.f;
+  for (int t = t0; t < t1; ++t) {
+    const size_t at = (size_t)start + t;
+    float q[J], k[J], g[J], dot = 0.f;
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const int r = lane + 32 * j;
+      const bool in = r < a.d;
+      q[j] = in ? to_f<T>(reinterpret_cast<const T*>(a.q)[at * a.ldq + (size_t)hk * a.d + r]) : 0.f;
+      k[j] = in ? to_f<T>(reinterpret_cast<const T*>(a.k)[at * a.ldk + (size_t)hk * a.d + r]) : 0.f;
+      g[j] = in ? a.g[(at * a.H + h) * a.d + r] : 0.f;
+      dot = MODE == kWkv ? fmaf(q[j] * k[j], u[j], dot) : fmaf(q[j], k[j], dot);
+    }
+    dot = warp_sum(dot);
+    const float beta = MODE == kDelta ? a.beta[at * a.H + h] : 0.f;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      if (col + c >= a.dv) break;                      // the same in all lanes
+      const float v = to_f<T>(reinterpret_cast<const T*>(a.v)[at * a.ldv + (size_t)h * a.dv + col + c]);
+      float ks = 0.f, qs = 0.f;
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        if (MODE == kDelta) {
+          S[c][j] *= g[j];
+          ks = fmaf(k[j], S[c][j], ks);
+        }
+        qs = fmaf(q[j], S[c][j], qs);
+      }
+      if (MODE == kDelta) ks = warp_sum(ks);
+      qs = warp_sum(qs);
+      const float e = MODE == kDelta ? beta * (v - ks) : v;
+#pragma unroll
+      for (int j = 0; j < J; ++j)
+        if (lane + 32 * j < a.d) S[c][j] = MODE == kDelta ? fmaf(k[j], e, S[c][j]) : fmaf(g[j], S[c][j], k[j] * e);
+      if (lane == 0) a.o[(at * a.H + h) * a.dv + col + c] = fmaf(dot, e, qs);
+    }
+  }
+}
+
 template <int MODE, typename T, int DP>
 __global__ void __launch_bounds__(ScanSmem<MODE, DP>::kThreads) chunk_scan_kernel(const ChunkArgs a) {
   using R = Rec<MODE, DP>;
@@ -501,19 +549,40 @@ __global__ void __launch_bounds__(ScanSmem<MODE, DP>::kThreads) chunk_scan_kerne
       for (int u = 0; u < CW; u += 2)
         if (col0 + fin + u < a.dv && (a.c0 + c) * kCk + tok < n_tok) o[u] = y[u / 2];
     }
+    // where the state of column c goes: to the next launch, or the slot
+    auto kept_at = [&](int c, int r) -> float* {
+      if (c >= a.dv) return nullptr;
+      if (last < chunks && !a.final) return carry_at(c, r);
+      return a.state != nullptr && r < sp ? state_at(c, r) : nullptr;
+    };
     if (failed) {
       *stop = 1;
       if (lane == 0) atomicCAS(a.err, 0, kErrScan);
+    } else if (last < chunks && a.final) {
+      // a sequence longer than the bound that the launches were sized by: its other tokens
+      constexpr int J = DP / 32;
+      float* fin = part;                               // [column][row]: the state, by columns
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          *reinterpret_cast<float2*>(fin + (g + 8 * u) * DP + row0 + 8 * j + t2) = make_float2(S[j][2 * u], S[j][2 * u + 1]);
+      state_barrier<kWarps * 32>();
+      const int mine = warp * CW;
+      float W[CW][J];
+      for (int x = 0; x < CW; ++x)
+        for (int j = 0; j < J; ++j) W[x][j] = fin[(mine + x) * DP + lane + 32 * j];
+      walk_tokens<MODE, T, DP, CW>(a, start, last * kCk, n_tok, h, col0 + mine, W);
+      for (int x = 0; x < CW; ++x)
+        for (int j = 0; j < J; ++j)
+          if (float* to = kept_at(col0 + mine + x, lane + 32 * j)) *to = W[x][j];
     } else {
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int c = col0 + g + 8 * u, r = row0 + 8 * j + t2;
-          float* to = nullptr;
-          if (c < a.dv) to = last < chunks ? carry_at(c, r) : (a.state != nullptr && r < sp ? state_at(c, r) : nullptr);
-          if (to != nullptr) *reinterpret_cast<float2*>(to) = make_float2(S[j][2 * u], S[j][2 * u + 1]);
-        }
+        for (int u = 0; u < 2; ++u)
+          if (float* to = kept_at(col0 + g + 8 * u, row0 + 8 * j + t2))
+            *reinterpret_cast<float2*>(to) = make_float2(S[j][2 * u], S[j][2 * u + 1]);
     }
   }
   __syncthreads();
@@ -579,6 +648,7 @@ static int launch_chunks(ChunkArgs a, const ChunkPlan& p, int n_seq, cudaStream_
   for (int c0 = 0; c0 < p.chunks; c0 += p.round) {
     a.c0 = c0;
     a.c1 = c0 + p.round;
+    a.final = a.c1 >= p.chunks;
     const int now = p.chunks - c0 < p.round ? p.chunks - c0 : p.round;
     chunk_prepare_kernel<MODE, T, DP><<<dim3(now, a.H, n_seq), DP, 0, stream>>>(a);
     scan<<<dim3((a.dv + kCkCols - 1) / kCkCols, a.H, n_seq), ScanSmem<MODE, DP>::kThreads, bytes, stream>>>(a);
@@ -603,7 +673,7 @@ ELL_API long long ell_scan_chunks_work(int mode, int n, int n_seq, int max_len, 
 }
 
 // Arguments as those of ell_wkv_scan (mode 0; beta null) and ell_delta_scan (mode 1; u null, fp32, ldq = ldk = G d, ldv = H dv); n
-// tokens, no sequence longer than max_len, work of ell_scan_chunks_work floats on a 16-byte boundary.  v: rows of 16-byte pieces.
+// tokens in all; max_len sizes the launches: a longer sequence goes token by token from there on.  work: ell_scan_chunks_work floats on a 16-byte boundary.  v: rows of 16-byte pieces.
 ELL_API int ell_scan_chunks(int mode, const void* q, const void* k, const void* v, const float* decay, const float* beta,
                             const float* u, float* o, float* state, const int* cu, const int* slots, const int* pos0, int n,
                             int n_seq, int max_len, int H, int G, int d, int dv, int ldq, int ldk, int ldv, int is_bf16, float* work,
@@ -614,7 +684,7 @@ ELL_API int ell_scan_chunks(int mode, const void* q, const void* k, const void* 
   if (!p.fits || H % G || n_seq > 65535 || H > 65535 || (mode == kDelta && is_bf16)) return -2;
   if (work == nullptr || !aligned_to(work, 16) || !aligned_to(v, 16) || ldv * esz % 16 || dv * esz % 16) return -2;
   ChunkArgs a{q, k, v, decay, beta, u, o, state, cu, slots, pos0, work, p.carry_floats ? work + p.rec_floats : nullptr,
-              H, G, d, dv, ldq, ldk, ldv, 0, 0, 0, err};
+              H, G, d, dv, ldq, ldk, ldv, 0, 0, 0, 1, err};
   if (mode == kDelta) return run_chunks<kDelta, float>(a, p, n_seq, stream);
   return is_bf16 ? run_chunks<kWkv, __nv_bfloat16>(a, p, n_seq, stream) : run_chunks<kWkv, float>(a, p, n_seq, stream);
 }

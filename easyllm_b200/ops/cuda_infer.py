@@ -333,14 +333,15 @@ def _scan_chunks(mode, q, k, v, decay, beta, u, o, meta, state):
     (T, G, d), (H, dv) = k.shape, v.shape[1:]
     c, sl, p0, n = _seq(meta, state)
     ldv, size = _heads(v, "v"), v.element_size()
-    if v.data_ptr() % 16 or ldv * size % 16 or dv * size % 16:
+    longest = meta.get("max_seqlen")
+    if longest is None or v.data_ptr() % 16 or ldv * size % 16 or dv * size % 16:
         return False
-    need = lib().ell_scan_chunks_work(c_int(mode), c_int(T), c_int(n), c_int(meta["max_seqlen"]), c_int(H), c_int(d), c_int(dv))
+    need = lib().ell_scan_chunks_work(c_int(mode), c_int(T), c_int(n), c_int(longest), c_int(H), c_int(d), c_int(dv))
     if not need:
         return False
     work = torch.empty(need, dtype=torch.float32, device=v.device)
     _check(lib().ell_scan_chunks(c_int(mode), _p(q), _p(k), _p(v), _p(_f32(decay, "decay")), _p(beta), _p(u), _p(o), _p(state), c, sl,
-                                 p0, c_int(T), c_int(n), c_int(meta["max_seqlen"]), c_int(H), c_int(G), c_int(d), c_int(dv),
+                                 p0, c_int(T), c_int(n), c_int(longest), c_int(H), c_int(G), c_int(d), c_int(dv),
                                  c_int(_heads(q, "q")), c_int(_heads(k, "k")), c_int(ldv), _bf(v.dtype), _p(work),
                                  _p(err_flag(v.device)), _stream()), "scan_chunks", 2)
     return True

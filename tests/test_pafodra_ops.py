@@ -347,6 +347,36 @@ def test_scans_in_rounds_of_chunks(kind, monkeypatch):
     close(got[0][1], got[1][1].cpu(), 1e-5)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,dtype,H,d,dv", [("wkv", BF16, 2, 64, 64), ("wkv", F32, 1, 100, 24), ("delta", F32, 2, 128, 40), ("delta", F32, 2, 36, 64)])
+@pytest.mark.parametrize("bound", [None, 256, 257])
+def test_scans_of_sequences_longer_than_their_bound(kind, dtype, H, d, dv, bound):
+    """The scans need no bound of the sequences' lengths: one that is missing or too small (by whole chunks and by a few tokens)
+    gives what the right one gives, going on from a slot's state."""
+    dev = _device("cuda")
+    counts = [300, 5, 260]
+    T = sum(counts)
+    ins = _scan_inputs(kind, H, H, d, dv, T, dtype)
+    qd, kd, vd, gd, ud = (x.double() for x in ins)
+    state = torch.zeros(3, H, dv, iops.padded_rows(d), device=dev)
+    state[..., :d].normal_(generator=torch.Generator(dev).manual_seed(1))
+    S0 = state.double().cpu()[..., :d].transpose(2, 3)
+    m = meta_of(counts, dev, [2, 0, 1], [9, 9, 0])
+    m["max_seqlen"] = bound
+    if bound is None:
+        del m["max_seqlen"]
+    got = _scan(kind, ins, slice(0, T), m, state, dev)
+    at = 0
+    for i, c in enumerate(counts):
+        p = slice(at, at + c)
+        S = S0[[2, 0, 1][i]] if i < 2 else None
+        o, S = (plain.wkv_recurrence if kind == "wkv" else plain.delta_recurrence)(qd[p], kd[p], vd[p], gd[p], ud if kind == "wkv" else ud[p], S)
+        close(got[p], o, 4e-6)
+        close(state[[2, 0, 1][i]][..., :d], S.transpose(1, 2), 4e-6)
+        at += c
+    assert bool((state[..., d:] == 0).all())
+
+
 @pytest.mark.parametrize("device", DEVICES)
 @pytest.mark.parametrize("kind", ["wkv", "delta"])
 def test_state_is_carried_far(device, kind):
