@@ -312,9 +312,12 @@ __device__ __forceinline__ RawValues<T> load_values(const ChunkArgs& a, int star
 }
 
 // Tokens t0 .. t1 - 1 of a sequence one by one, as scan_kernel computes them, for a warp's NC columns from `col` on.  Lane l holds
-// key rows l, l + 32, ... of them.  What chunks cannot do comes here: it is slow (0.5 us a token) and rare.
+// key rows l, l + 32, ... of them.  What chunks cannot do comes here: it is slow (0.5 us a token) and rare.  mend: only outputs
+// that are not finite are written.
+__device__ __forceinline__ bool is_finite(float x) { return x * 0.f == 0.f; }
 template <int MODE, typename T, int DP, int NC>
-__device__ __noinline__ void walk_tokens(const ChunkArgs& a, int start, int t0, int t1, int h, int col, float (&S)[NC][DP / 32]) {
+__device__ __noinline__ void walk_tokens(const ChunkArgs& a, int start, int t0, int t1, int h, int col, float (&S)[NC][DP / 32],
+                                         bool mend) {
   constexpr int J = DP / 32;
   const int lane = threadIdx.x & 31, hk = h / (a.H / a.G);
   float u[J];
@@ -353,7 +356,8 @@ __device__ __noinline__ void walk_tokens(const ChunkArgs& a, int start, int t0, 
 #pragma unroll
       for (int j = 0; j < J; ++j)
         if (lane + 32 * j < a.d) S[c][j] = MODE == kDelta ? fmaf(k[j], e, S[c][j]) : fmaf(g[j], S[c][j], k[j] * e);
-      if (lane == 0) a.o[(at * a.H + h) * a.dv + col + c] = fmaf(dot, e, qs);
+      float* o = a.o + (at * a.H + h) * a.dv + col + c;
+      if (lane == 0 && !(mend && is_finite(*o))) *o = fmaf(dot, e, qs);
     }
   }
 }
@@ -366,6 +370,7 @@ __global__ void __launch_bounds__(ScanSmem<MODE, DP>::kThreads) chunk_scan_kerne
   extern __shared__ __align__(128) float sm[];
   __shared__ uint64_t full[kCkStages], empty[kCkStages];
   __shared__ int gave_up;
+  __shared__ uint32_t odd_columns;                     // those with values that are not finite
   const int s = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * kCkCols;
   const int start = a.cu[s], n_tok = a.cu[s + 1] - start;
   const int chunks = (n_tok + kCk - 1) / kCk, last = min(a.c1, chunks), n = last - a.c0;
@@ -377,6 +382,7 @@ __global__ void __launch_bounds__(ScanSmem<MODE, DP>::kThreads) chunk_scan_kerne
       mbar_init(&empty[i], kWarps);
     }
     gave_up = 0;
+    odd_columns = 0;
     fence_barrier_init();
   }
   __syncthreads();
@@ -443,6 +449,9 @@ __global__ void __launch_bounds__(ScanSmem<MODE, DP>::kThreads) chunk_scan_kerne
       }
     float* o = a.o + ((size_t)(start + a.c0 * kCk + tok) * a.H + h) * a.dv + col0 + fin;
     const size_t o_chunk = (size_t)kCk * a.H * a.dv;
+    float probe[CW / 2];                               // becomes NaN with the first output that is not finite
+#pragma unroll
+    for (int u = 0; u < CW / 2; ++u) probe[u] = 0.f;
     bool failed = false;
     for (int c = 0; c < n; ++c, o += o_chunk) {
       const int i = c % kCkStages;
@@ -546,8 +555,10 @@ __global__ void __launch_bounds__(ScanSmem<MODE, DP>::kThreads) chunk_scan_kerne
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[i]);
 #pragma unroll
-      for (int u = 0; u < CW; u += 2)
+      for (int u = 0; u < CW; u += 2) {
+        probe[u / 2] = fmaf(y[u / 2], 0.f, probe[u / 2]);
         if (col0 + fin + u < a.dv && (a.c0 + c) * kCk + tok < n_tok) o[u] = y[u / 2];
+      }
     }
     // where the state of column c goes: to the next launch, or the slot
     auto kept_at = [&](int c, int r) -> float* {
@@ -555,11 +566,22 @@ __global__ void __launch_bounds__(ScanSmem<MODE, DP>::kThreads) chunk_scan_kerne
       if (last < chunks && !a.final) return carry_at(c, r);
       return a.state != nullptr && r < sp ? state_at(c, r) : nullptr;
     };
+#pragma unroll
+    for (int u = 0; u < CW; u += 2)
+      if (!is_finite(probe[u / 2])) atomicOr(&odd_columns, 1u << (fin + u));
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (!is_finite(fmaf(S[0][2 * u], 0.f, S[0][2 * u + 1] * 0.f) + fmaf(S[1][2 * u], 0.f, S[1][2 * u + 1] * 0.f)))
+        atomicOr(&odd_columns, 1u << (g + 8 * u));
+    state_barrier<kWarps * 32>();
+    const uint32_t odd = odd_columns;
     if (failed) {
       *stop = 1;
       if (lane == 0) atomicCAS(a.err, 0, kErrScan);
-    } else if (last < chunks && a.final) {
-      // a sequence longer than the bound that the launches were sized by: its other tokens
+    } else if (odd != 0 || (last < chunks && a.final)) {
+      // The parts of an infinity are not a number, and sums over a chunk may overflow where those over a token do not: what came out
+      // not finite is computed again, token by token.  And the other tokens of a sequence longer than the bound that the launches
+      // were sized by.
       constexpr int J = DP / 32;
       float* fin = part;                               // [column][row]: the state, by columns
 #pragma unroll
@@ -570,9 +592,21 @@ __global__ void __launch_bounds__(ScanSmem<MODE, DP>::kThreads) chunk_scan_kerne
       state_barrier<kWarps * 32>();
       const int mine = warp * CW;
       float W[CW][J];
+      if (odd >> mine & ((1u << CW) - 1)) {
+        for (int x = 0; x < CW; ++x)
+          for (int j = 0; j < J; ++j) {
+            const int c = col0 + mine + x, r = lane + 32 * j;
+            W[x][j] = c >= a.dv ? 0.f : (a.c0 > 0 ? *carry_at(c, r) : (kept && r < sp ? *state_at(c, r) : 0.f));
+          }
+        __syncwarp();                                  // the outputs of this warp's other lanes
+        walk_tokens<MODE, T, DP, CW>(a, start, a.c0 * kCk, min(last * kCk, n_tok), h, col0 + mine, W, true);
+      }
       for (int x = 0; x < CW; ++x)
-        for (int j = 0; j < J; ++j) W[x][j] = fin[(mine + x) * DP + lane + 32 * j];
-      walk_tokens<MODE, T, DP, CW>(a, start, last * kCk, n_tok, h, col0 + mine, W);
+        for (int j = 0; j < J; ++j) {
+          const float y = fin[(mine + x) * DP + lane + 32 * j];
+          if (!(odd >> (mine + x) & 1) || is_finite(y)) W[x][j] = y;
+        }
+      if (last < chunks && a.final) walk_tokens<MODE, T, DP, CW>(a, start, last * kCk, n_tok, h, col0 + mine, W, false);
       for (int x = 0; x < CW; ++x)
         for (int j = 0; j < J; ++j)
           if (float* to = kept_at(col0 + mine + x, lane + 32 * j)) *to = W[x][j];

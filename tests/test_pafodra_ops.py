@@ -377,6 +377,46 @@ def test_scans_of_sequences_longer_than_their_bound(kind, dtype, H, d, dv, bound
     assert bool((state[..., d:] == 0).all())
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,dtype,d", [("wkv", BF16, 64), ("wkv", F32, 128), ("delta", F32, 64), ("delta", F32, 128)])
+@pytest.mark.parametrize("where", ["value", "state", "large", "key", "none"])
+def test_infinities_in_a_scan_in_chunks(kind, dtype, d, where, monkeypatch):
+    """An infinite value, state entry or key, and a finite value whose bf16 part is infinite, end where the scan token by token has
+    them, with their sign; what is finite there is finite here."""
+    from easyllm_b200.ops import cuda_infer
+    dev = _device("cuda")
+    H, dv, T, t = 2, 24, 300, 133
+    ins = [x.clone() for x in _scan_inputs(kind, H, H, d, dv, T, dtype)]
+    ins[0], ins[1] = ins[0].abs(), ins[1].abs()            # no infinities of both signs in a sum, which would be NaN anyway
+    if kind == "wkv":
+        ins[4] = ins[4].abs()
+    first = torch.rand(1, H, dv, iops.padded_rows(d), device=dev)
+    if where == "value":
+        ins[2][t, 1, 5], ins[2][t + 60, 0, 17] = math.inf, -math.inf
+    elif where == "large":
+        ins[2][t, 1, 5] = torch.finfo(dtype).max
+    elif where == "state":
+        first[0, 1, 7, 3] = math.inf
+    elif where == "key":
+        ins[1][t, 1, 9] = math.inf
+    got, kept = [], []
+    for chunks in (True, False):
+        if not chunks:
+            monkeypatch.setattr(cuda_infer, "_scan_chunks", lambda *a: False)
+        state = first.clone()
+        got.append(_scan(kind, ins, slice(0, T), meta_of([T], dev, [0], [1]), state, dev))
+        kept.append(state)
+    assert where in ("none", "large") or not bool(got[1].isfinite().all())
+    for a, b in (got, kept):
+        fine = b.isfinite()
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf()) and bool((a[b.isinf()] == b[b.isinf()]).all())
+        rest = fine.clone()
+        if where == "large":                               # a column of its own size
+            rest[(slice(None), 1, 5) if b is got[1] else (0, 1, 5)] = False
+        close(a[rest], b[rest].cpu(), 1e-5)
+        assert bool(((a - b).abs()[fine & ~rest] <= 1e-5 * b.abs()[fine & ~rest].max()).all()) if bool((fine & ~rest).any()) else True
+
+
 @pytest.mark.parametrize("device", DEVICES)
 @pytest.mark.parametrize("kind", ["wkv", "delta"])
 def test_state_is_carried_far(device, kind):
