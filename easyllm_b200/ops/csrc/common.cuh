@@ -86,8 +86,9 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 //     writes there is not missed.
 // Measured, decode steps: 79 launches of a latent-attention model (64 sequences) 751 -> 690 us, 70 of a hybrid (8 sequences)
 // 514 -> 479, 48 to 52 of a Llama 480 -> 469 (one sequence) and 1056 -> 1042 (64).
-// Without the launch attribute both instructions do nothing.  Pointers that are `const __restrict__` go through chain_wait:
-// their loads could be taken for loads of constants and be moved in front of the wait.
+// Without the launch attribute both instructions do nothing.  Every pointer that is `__restrict__`, to constants or not, goes
+// through chain_wait: the compiler may take it that a statement which does not get the pointer leaves alone what it points to, and
+// move loads, or stores, in front of the wait.
 template <typename T>
 __device__ __forceinline__ void unknown_pointer(T& p) { asm volatile("" : "+l"(p)::"memory"); }
 template <typename... T>

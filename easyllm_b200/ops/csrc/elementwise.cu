@@ -18,7 +18,7 @@ namespace ell {
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __restrict__ cos_t,
                             const float* __restrict__ sin_t, const int* __restrict__ pos, int T, int row_stride,
                             int n_rot_heads, int D, float sin_sign, int table_rows, int* __restrict__ err) {
-  chain_enter(cos_t, sin_t, pos);
+  chain_enter(qkv, cos_t, sin_t, pos, err);
   const int half = D / 2, vec_per_head = half / 8;
   const long long total = (long long)T * n_rot_heads * vec_per_head;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -60,7 +60,7 @@ __global__ void rope_append_kernel(__nv_bfloat16* __restrict__ qkv, const float*
                                    const int* __restrict__ pos, __nv_bfloat16* __restrict__ kc, __nv_bfloat16* __restrict__ vc,
                                    const int* __restrict__ base, const int* __restrict__ len, int T, int Hq, int Hk, int D,
                                    int table_rows, int* __restrict__ err) {
-  chain_enter(cos_t, sin_t, pos, base, len);
+  chain_enter(qkv, cos_t, sin_t, pos, kc, vc, base, len, err);
   const int half = D / 2, rot = (Hq + Hk) * (half / 8), per = rot + Hk * (D / 8), W = (Hq + 2 * Hk) * D;
   const long long total = (long long)T * per;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -106,7 +106,7 @@ __global__ void rope_append_kernel(__nv_bfloat16* __restrict__ qkv, const float*
 }
 
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, int T, int F) {
-  chain_enter(gu);
+  chain_enter(gu, out);
   const int fv = F / 8;
   const long long total = (long long)T * fv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;

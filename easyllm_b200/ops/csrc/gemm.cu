@@ -161,7 +161,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (FUSE == kFuseNone && !B_MN && M <= kAheadRows && threadIdx.x == 0 && cta0 < tiles_n)
     // few rows: the launch is bound by the bytes of B, whose first tile comes into L2 while the kernel before this one ends
     for (int kb = 0; kb < min(num_kb, kAheadBlocks); ++kb) tma_prefetch_l2_2d(&tmB, kb * kBK, cta0 * BN);
-  chain_wait(bias);
+  chain_wait(bias, err);
   const int tiles_m = FUSE == kFuseGroup ? min(*fuse.n_row_tiles, (M + kBM - 1) / kBM) : (M + kBM - 1) / kBM;
   const int num_tiles = tiles_m * tiles_n;
   const int n_split = split_tail_tiles(num_tiles, cta_stride, FUSE == kFuseNone && BN == 256 && OUT != kOutBf16CE &&

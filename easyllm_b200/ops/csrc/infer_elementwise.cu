@@ -12,7 +12,7 @@ template <typename T, int V>
 __global__ void embed_scaled_kernel(const long long* __restrict__ ids, const T* __restrict__ table,
                                     float* __restrict__ out, int n, int W, long long rows, float scale,
                                     int* __restrict__ err) {
-  chain_enter(ids, table);
+  chain_enter(ids, table, out, err);
   const int wv = W / V;
   const long long total = (long long)n * wv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -36,7 +36,7 @@ __global__ void embed_scaled_kernel(const long long* __restrict__ ids, const T* 
 template <typename T, int V>
 __global__ void dynamic_tanh_kernel(float* __restrict__ x, const float* __restrict__ alpha, const float* __restrict__ w,
                                     const float* __restrict__ b, const T* __restrict__ add, T* __restrict__ y, int n, int W) {
-  chain_enter(alpha, w, b, add);
+  chain_enter(x, alpha, w, b, add, y);
   const int wv = W / V;
   const long long total = (long long)n * wv;
   const float al = *alpha;
@@ -62,7 +62,7 @@ enum Act { kActSilu = 0, kActGeluTanh = 1 };
 
 template <typename T, int V>
 __global__ void glu_kernel(const T* __restrict__ gu, T* __restrict__ out, int n, int F, int ld, int act) {
-  chain_enter(gu);
+  chain_enter(gu, out);
   const int fv = F / V;
   const long long total = (long long)n * fv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -80,7 +80,7 @@ __global__ void glu_kernel(const T* __restrict__ gu, T* __restrict__ out, int n,
 template <typename T, int V>
 __global__ void relu2_scaled_kernel(const T* __restrict__ x, const float* __restrict__ z, T* __restrict__ out, int n,
                                     int F, int ld, int ldz) {
-  chain_enter(x, z);
+  chain_enter(x, z, out);
   const int fv = F / V;
   const long long total = (long long)n * fv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -99,7 +99,7 @@ __global__ void relu2_scaled_kernel(const T* __restrict__ x, const float* __rest
 
 template <typename T>
 __global__ void tanh_cast_kernel(const float* __restrict__ x, T* __restrict__ y, int n, int N, int ldx) {
-  chain_enter(x);
+  chain_enter(x, y);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)n * N;
        i += (long long)gridDim.x * blockDim.x)
     y[i] = from_f<T>(tanhf(x[(i / N) * ldx + i % N]));
@@ -107,7 +107,7 @@ __global__ void tanh_cast_kernel(const float* __restrict__ x, T* __restrict__ y,
 
 // z = exp(-exp(z + w0[column]))
 __global__ void wkv_decay_kernel(float* __restrict__ z, const float* __restrict__ w0, long long total, int C) {
-  chain_enter(w0);
+  chain_enter(z, w0);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
     z[i] = expf(-expf(z[i] + w0[i % C]));
 }
@@ -119,7 +119,7 @@ template <typename T, int V>
 __global__ void token_mix_kernel(const T* __restrict__ h, const float* __restrict__ mu, T* __restrict__ out,
                                  const int* __restrict__ cu, const int* __restrict__ slots, const int* __restrict__ pos0,
                                  T* __restrict__ last, int W, int nmix, int n, int chunk) {
-  chain_enter(h, mu, cu, slots, pos0);
+  chain_enter(h, mu, out, cu, slots, pos0, last);
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * V;
   if (c >= W) return;
   const int s = blockIdx.z, a = cu[s], b = cu[s + 1];
@@ -215,7 +215,7 @@ template <typename T, int V>
 __global__ void head_norm_gate_kernel(const float* __restrict__ o, const float* __restrict__ w, const T* __restrict__ gate,
                                       T* __restrict__ y, int n, int H, int dv, int w_per_head, int ldg, int silu_gate,
                                       float eps) {
-  chain_enter(o, w, gate);
+  chain_enter(o, w, gate, y);
   const int warps = blockDim.x >> 5, lane = threadIdx.x & 31;
   for (long long i = blockIdx.x * (long long)warps + (threadIdx.x >> 5); i < (long long)n * H; i += (long long)gridDim.x * warps) {
     const int t = (int)(i / H), hd = (int)(i % H);
@@ -234,7 +234,7 @@ template <typename T, int V>
 __global__ void kv_append_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ kc, T* __restrict__ vc,
                                  const int* __restrict__ base, const int* __restrict__ len, int n, int dk, int dv, int ldk,
                                  int ldv) {
-  chain_enter(k, v, base, len);
+  chain_enter(k, v, kc, vc, base, len);
   const int per = (dk + dv) / V;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)n * per;
        i += (long long)gridDim.x * blockDim.x) {
@@ -261,7 +261,7 @@ __global__ void embed_pairs_kernel(const long long* __restrict__ ids, const T* _
                                    const int* __restrict__ base, const int* __restrict__ len, int* __restrict__ hist, int W,
                                    long long rows, long long buckets, long long mul_prev, long long mul_cur, float scale,
                                    int* __restrict__ err) {
-  chain_enter(ids, table, pairs, row_start, base, len);
+  chain_enter(ids, table, pairs, out, row_start, base, len, hist, err);
   const int t = blockIdx.x;
   const long long id = ids[t];
   const bool first_row = row_start[t] == t;
@@ -304,7 +304,7 @@ template <typename T, int IT>
 __global__ void __launch_bounds__(kLnPairThreads)
 layer_norms_kernel(const float* __restrict__ x, const float* __restrict__ w1, const float* __restrict__ w2,
                    T* __restrict__ y1, T* __restrict__ y2, int W, float eps) {
-  chain_enter(x, w1, w2);
+  chain_enter(x, w1, w2, y1, y2);
   __shared__ float red[2][kLnPairThreads / 32];
   const float* row = x + (size_t)blockIdx.x * W;
   T* o1 = y1 + (size_t)blockIdx.x * W;
@@ -377,7 +377,7 @@ latent_inputs_kernel(T* __restrict__ z, T* __restrict__ q_dst, T* __restrict__ c
                      const float* __restrict__ cosT, const float* __restrict__ sinT, const int* __restrict__ pos,
                      const int* __restrict__ base, const int* __restrict__ len, int H, int dim, int rot, int rank, int pairs,
                      int ldz, int q_stride, int ldc, float eps) {
-  chain_enter(norm_w, cosT, sinT, pos, base, len);
+  chain_enter(z, q_dst, cache, norm_w, cosT, sinT, pos, base, len);
   __shared__ float red[kLatThreads / 32];
   const int t = blockIdx.x;
   constexpr int VL = V == 8 ? 8 : 1;                    // pieces of the latent (any rank)

@@ -207,7 +207,7 @@ int dispatch_matvec(const MatvecArgs& a, int batch, bool vec, cudaStream_t strea
 // chosen logits.  bias [E] (or null) is added to the logits first.
 __global__ void moe_route_kernel(const float* __restrict__ z, const float* __restrict__ bias, int* __restrict__ idx,
                                  float* __restrict__ w, int n, int E, int top, int ldz, int softmax) {
-  chain_enter(z, bias);
+  chain_enter(z, bias, idx, w);
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (t >= n) return;
   const float* row = z + (size_t)t * ldz;
@@ -254,7 +254,7 @@ template <typename T, bool VEC, bool GLU>
 __global__ void __launch_bounds__(256) moe_up_kernel(const T* __restrict__ h, const T* __restrict__ up,
                                                      const int* __restrict__ idx, const float* __restrict__ wgt,
                                                      T* __restrict__ hid, int top, int F, int W, int block) {
-  chain_enter(h, up, idx, wgt);
+  chain_enter(h, up, idx, wgt, hid);
   const int slot = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int f0 = (blockIdx.x * 8 + warp) * (GLU ? 1 : 2);
   if (f0 >= F) return;
@@ -306,7 +306,7 @@ template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) moe_down_kernel(const T* __restrict__ hid, const T* __restrict__ down,
                                                        const int* __restrict__ idx, float* __restrict__ acc, int top, int F,
                                                        int W) {
-  chain_enter(hid, down, idx);
+  chain_enter(hid, down, idx, acc);
   const int t = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = (blockIdx.x * 8 + warp) * 2;
   if (n0 >= W) return;
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(256) moe_down_kernel(const T* __restrict__ hid
 __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ idx, const float* __restrict__ wgt, int slots,
                                                         int E, int* __restrict__ pos, float* __restrict__ row_scale,
                                                         int* __restrict__ tile_expert, int* __restrict__ n_tiles) {
-  chain_enter(idx, wgt);
+  chain_enter(idx, wgt, pos, row_scale, tile_expert, n_tiles);
   __shared__ int count[1024], first[1024], scan[1024];
   const int e = threadIdx.x;
   count[e] = 0;
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
 // xs[pos[slot]] = h[token], 16 bytes a thread.
 __global__ void moe_gather_kernel(const uint4* __restrict__ h, uint4* __restrict__ xs, const int* __restrict__ pos, int slots,
                                   int top, int wv) {
-  chain_enter(h, pos);
+  chain_enter(h, xs, pos);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)slots * wv;
        i += (long long)gridDim.x * blockDim.x) {
     const int slot = (int)(i / wv), c = (int)(i % wv);
@@ -398,7 +398,7 @@ __global__ void moe_gather_kernel(const uint4* __restrict__ h, uint4* __restrict
 // acc[token] += sum over its slots of ys[pos[slot]]
 __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ ys, const int* __restrict__ pos, float* __restrict__ acc,
                                    int n, int top, int W) {
-  chain_enter(ys, pos);
+  chain_enter(ys, pos, acc);
   const int wv = W / 4;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)n * wv;
        i += (long long)gridDim.x * blockDim.x) {

@@ -76,7 +76,7 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   __shared__ float s_red[2][kNormWarps][kNormRowsMax];
   constexpr int kNormRows = norm_rows(kVpt);
   const int nvec = cols / 8;
-  chain_enter(x, res, w);
+  chain_enter(x, res, w, y, h_out, rstd_out);
   bf16x8 wv[kVpt];
 #pragma unroll
   for (int i = 0; i < kVpt; ++i) {
