@@ -783,6 +783,51 @@ struct AtTile {
   }
 };
 
+__device__ __forceinline__ bool not_finite(float x) { return !(x * 0.f == 0.f); }
+
+// Row m of the tile key by key, by one warp, with the keys that the row sees and no others.  In the tiles a key that a row does not
+// see has the weight 0, and 0 times an infinity or NaN of a later token (or of one that left the window) is NaN; the bf16 parts of a
+// weight times an infinity are of either sign.  A row that came out not finite is therefore computed again here (1 us a few keys).
+__device__ __noinline__ void at_row_alone(const AttnRowsArgs& a, const AtTile& T, int m) {
+  const int lane = threadIdx.x & 31, tok = T.token(m), head = T.head(m), end = a.len[tok];
+  const __nv_bfloat16* q = reinterpret_cast<const __nv_bfloat16*>(a.q) + (size_t)tok * a.ldq + (size_t)head * a.d;
+  const float slope = a.slopes != nullptr ? a.slopes[head] : 0.f;
+  float qv[4], acc[4], mx = -INFINITY, l = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    qv[i] = lane + 32 * i < a.d ? __bfloat162float(q[lane + 32 * i]) : 0.f;
+    acc[i] = 0.f;
+  }
+  for (int key = max(T.k0, end - a.window); key < min(T.k1, end); ++key) {
+    const __nv_bfloat16* k = reinterpret_cast<const __nv_bfloat16*>(a.k) + (T.base + key) * a.ldk + (size_t)T.g * a.d;
+    const __nv_bfloat16* v = reinterpret_cast<const __nv_bfloat16*>(a.v) + (T.base + key) * a.ldv + (size_t)T.g * a.dv;
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (lane + 32 * i < a.d) s = fmaf(qv[i], __bfloat162float(k[lane + 32 * i]), s);
+    s = warp_sum(s) * a.scale;
+    if (a.slopes != nullptr) s += slope * (float)(key - (end - 1));
+    const float now = fmaxf(mx, s), al = mx == now ? 1.f : expf(mx - now), w = s == -INFINITY ? 0.f : expf(s - now);
+    mx = now;
+    l = l * al + w;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (lane + 32 * i < a.dv) acc[i] = fmaf(w, __bfloat162float(v[lane + 32 * i]), acc[i] * al);
+  }
+  float f, *part;
+  __nv_bfloat16* out = T.place(a, m, mx, l, f, part);
+  if (part != nullptr && lane == 0) {
+    part[0] = mx;
+    part[1] = l;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (lane + 32 * i < a.dv) {
+      if (part != nullptr) part[2 + lane + 32 * i] = acc[i];
+      else out[lane + 32 * i] = __float2bfloat16_rn(acc[i] * f);
+    }
+}
+
 __device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
   uint32_t y;
   asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
@@ -965,6 +1010,7 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const AttnRowsA
       part[0] = mx;
       part[1] = sum;
     }
+    bool odd = not_finite(sum);
     for (int c = lane * 2; c < a.dv; c += 64) {
       float2 o = make_float2(0.f, 0.f);
 #pragma unroll
@@ -973,9 +1019,13 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const AttnRowsA
         o.x = fmaf(w[x], v.x, o.x);
         o.y = fmaf(w[x], v.y, o.y);
       }
+      odd |= not_finite(o.x) || not_finite(o.y);
       if (part != nullptr) *reinterpret_cast<float2*>(part + 2 + c) = o;
       else *reinterpret_cast<__nv_bfloat162*>(out + c) = __floats2bfloat162_rn(o.x * f, o.y * f);
     }
+    odd = __any_sync(0xffffffffu, odd);
+    __syncwarp();
+    if (odd) at_row_alone(a, T, r);
   }
 }
 
@@ -1027,10 +1077,18 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_tile_kernel(const AttnRows
       }
     }
   }
+  uint32_t odd_rows = 0;                             // of the warp's sixteen
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     r.l[h] += __shfl_xor_sync(0xffffffffu, r.l[h], 1);
     r.l[h] += __shfl_xor_sync(0xffffffffu, r.l[h], 2);
+    float probe = r.l[h] * 0.f;                      // NaN once a value is not finite
+#pragma unroll
+    for (int n = 0; n < 16; ++n) probe = fmaf(acc[n][2 * h], 0.f, fmaf(acc[n][2 * h + 1], 0.f, probe));
+    const uint32_t lanes = __ballot_sync(0xffffffffu, not_finite(probe));
+#pragma unroll
+    for (int x = 0; x < 8; ++x)
+      if (lanes >> 4 * x & 15) odd_rows |= 1u << (8 * h + x);
     const int m = row0 + gr + 8 * h;
     if (m >= T.rows) continue;
     float f, *part;
@@ -1048,6 +1106,9 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_tile_kernel(const AttnRows
       }
     }
   }
+  __syncwarp();
+  for (int x = 0; x < 16; ++x)
+    if (odd_rows >> x & 1 && row0 + x < T.rows) at_row_alone(a, T, row0 + x);
 }
 
 // How a call runs on these kernels: tokens and CTAs of a tile, ranges of keys.  One sequence per `cu` entry, or one token

@@ -245,6 +245,35 @@ def test_attention_over_cached_rows(steps, past, H, G, d, dv, extras):
             assert (o.double() - want).abs().max() <= 2.0 ** -8 * want.abs().max()
 
 
+@pytest.mark.parametrize("window", [None, 77])
+@pytest.mark.parametrize("steps,past,H,G", [([1, 1], [700, 63], 8, 2), ([3, 4], [130, 20], 8, 2), ([65, 40], [300, 25], 8, 2), ([2, 20], [2500, 30], 4, 4)])
+def test_values_that_are_not_finite_reach_the_rows_that_see_them(steps, past, H, G, window):
+    """Infinities of both signs and NaN among the values and keys of cached and of later tokens: rows that do not see them (earlier
+    tokens, windows that have moved on) have the finite result, rows that see an infinity have it with its sign."""
+    from easyllm_b200.ops import infer as iops
+    torch.manual_seed(sum(steps))
+    dev, d, cap = "cuda", 64, 2560
+    q = torch.randn(sum(steps), H, d, device=dev).bfloat16()
+    k, v = (torch.randn(len(steps) * cap, G, d, device=dev).bfloat16() for _ in "kv")
+    base = [i * cap for i, n in enumerate(steps) for _ in range(n)]
+    length = [p + j + 1 for n, p in zip(steps, past) for j in range(n)]
+    for i, (n, p) in enumerate(zip(steps, past)):
+        last, mid, old = i * cap + p + n - 1, i * cap + p + n // 2, i * cap + p - 15
+        v[last, 0, 0], v[last, G - 1, 3], v[last, 0, 5] = float("inf"), float("nan"), float("-inf")
+        v[mid, 0, 9], v[old, G - 1, 7], v[i * cap + 2, 0, 11] = float("-inf"), float("inf"), float("inf")
+    k[cap + past[1] + steps[1] - 1, G - 1, 4] = float("nan")
+    b, n = (torch.tensor(x, dtype=torch.int32, device=dev) for x in (base, length))
+    cu = torch.tensor([0] + steps, device=dev).cumsum(0).int()
+    want = _rows_exact(q, k, v, base, length, d ** -0.5, None, None, window, None)
+    fine = want.isfinite()
+    assert 0 < int(fine.sum()) < fine.numel()
+    for kw in ({"cu_seqlens": cu, "max_q": max(steps)}, {}):
+        o = iops.attention_rows(q, k, v, b, n, max(length), d ** -0.5, window=window, **kw)
+        assert torch.equal(o.isnan(), want.isnan()) and torch.equal(o.isinf(), want.isinf())
+        assert bool((o[want.isinf()].double() == want[want.isinf()]).all())
+        assert (o[fine].double() - want[fine]).norm() <= 1.9e-3 * want[fine].norm()
+
+
 @pytest.mark.parametrize("hq,hk", [(5, 5), (6, 2)])
 def test_heads_in_several_groups(cu, hq, hk):
     """So many tokens that the heads' CTAs come in several groups, the last one smaller: documents of 512 tokens alone (the same
