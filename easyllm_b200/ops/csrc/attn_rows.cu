@@ -788,7 +788,7 @@ __device__ __forceinline__ bool not_finite(float x) { return !(x * 0.f == 0.f); 
 // Row m of the tile key by key, by one warp, with the keys that the row sees and no others.  In the tiles a key that a row does not
 // see has the weight 0, and 0 times an infinity or NaN of a later token (or of one that left the window) is NaN; the bf16 parts of a
 // weight times an infinity are of either sign.  A row that came out not finite is therefore computed again here (1 us a few keys).
-__device__ __noinline__ void at_row_alone(const AttnRowsArgs& a, const AtTile& T, int m) {
+__device__ __noinline__ void at_row_alone(const AttnRowsArgs& a, const AtTile T, int m) {
   const int lane = threadIdx.x & 31, tok = T.token(m), head = T.head(m), end = a.len[tok];
   const __nv_bfloat16* q = reinterpret_cast<const __nv_bfloat16*>(a.q) + (size_t)tok * a.ldq + (size_t)head * a.d;
   const float slope = a.slopes != nullptr ? a.slopes[head] : 0.f;
@@ -836,7 +836,7 @@ __device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
 
 // NB: groups of 8 rows.
 template <int NB>
-__global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const AttnRowsArgs a, const int* __restrict__ cu, int tiles, int tt) {
+__global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const __grid_constant__ AttnRowsArgs a, const int* __restrict__ cu, int tiles, int tt) {
   chain_enter(cu);
   extern __shared__ __align__(128) uint8_t atsm[];
   AtTile T;
@@ -1029,7 +1029,7 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const AttnRowsA
   }
 }
 
-__global__ void __launch_bounds__(kAtThreads, 2) attn_tile_kernel(const AttnRowsArgs a, const int* __restrict__ cu, int tiles, int tt) {
+__global__ void __launch_bounds__(kAtThreads, 2) attn_tile_kernel(const __grid_constant__ AttnRowsArgs a, const int* __restrict__ cu, int tiles, int tt) {
   chain_enter(cu);
   extern __shared__ __align__(128) uint8_t atsm[];
   AtTile T;

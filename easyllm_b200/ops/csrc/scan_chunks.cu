@@ -363,7 +363,7 @@ __device__ __noinline__ void walk_tokens(const ChunkArgs& a, int start, int t0, 
 }
 
 template <int MODE, typename T, int DP>
-__global__ void __launch_bounds__(ScanSmem<MODE, DP>::kThreads) chunk_scan_kernel(const ChunkArgs a) {
+__global__ void __launch_bounds__(ScanSmem<MODE, DP>::kThreads) chunk_scan_kernel(const __grid_constant__ ChunkArgs a) {
   using R = Rec<MODE, DP>;
   using Sm = ScanSmem<MODE, DP>;
   constexpr int kWarps = Sm::kWarps, CW = Sm::kColsOfWarp, kTiles = R::kRows / 8;
