@@ -575,7 +575,8 @@ attn_latent_kernel(const __grid_constant__ CUtensorMap tmK, const AttnRowsArgs a
 // context once per token (1060 us for 301 tokens over 3000, 50 here).  Here a tile of 16 rows is the consecutive tokens of one
 // sequence times the query heads of one key head, and m16n8k16 does the products:
 //   scores  exact bf16 products, fp32 sums, scale and bias applied in fp32
-//   values  the fp32 weights go in as two bf16 parts (value and remainder), so they keep 16 bits of mantissa
+//   values  the fp32 weights go in as three bf16 parts, so they keep their 24 bits.  With two parts, in turn for one accumulator at
+//           a time, 64 rows x 2048 keys took 136 us; with three, several accumulators taking turns, 125
 //   attn_few_kernel   up to 16 rows (decoding).  Keys are the M side of both products and rows the N side, so 8 rows cost
 //                     half of 16: S^T = K q^T, O^T = V^T P^T.  The four warps take units of 16 keys in turn, each with a
 //                     softmax, accumulators and a ring of cp.async stages of its own; no barrier until their results meet.
@@ -601,11 +602,14 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&v);
 }
-// x as a bf16 pair and the pair of what is left
-__device__ __forceinline__ void split_bf16(float x, float y, uint32_t& part, uint32_t& rest) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
-  part = *reinterpret_cast<const uint32_t*>(&v);
-  rest = pack_bf16(x - __low2float(v), y - __high2float(v));
+// x and y as three bf16 parts each: 24 bits, nothing is lost
+__device__ __forceinline__ void split_bf16(float x, float y, uint32_t (&p)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    p[i] = pack_bf16(x, y);
+    x -= __uint_as_float(p[i] << 16);
+    y -= __uint_as_float(p[i] & 0xffff0000u);
+  }
 }
 
 // What a thread keeps of its rows g and g + 8 (g = lane / 4).
@@ -679,21 +683,28 @@ __device__ __forceinline__ void at_unit(const uint8_t* ks, const uint8_t* vs, in
     }
 #pragma unroll
   for (int k = 0; k < UK / 16; ++k) {
-    uint32_t hi[4], lo[4];
-    split_bf16(s[2 * k][0], s[2 * k][1], hi[0], lo[0]);
-    split_bf16(s[2 * k][2], s[2 * k][3], hi[1], lo[1]);
-    split_bf16(s[2 * k + 1][0], s[2 * k + 1][1], hi[2], lo[2]);
-    split_bf16(s[2 * k + 1][2], s[2 * k + 1][3], hi[3], lo[3]);
+    uint32_t w[3][4];
 #pragma unroll
-    for (int n = 0; n < 8; ++n) {
-      if (n < vtiles) {
-        uint32_t b[4];
-        ldsm4_t(b, vs + at_place(k * 16 + (quad & 1) * 8 + l8, n * 2 + (quad >> 1)));
-        mma_bf16(acc[2 * n], hi, b[0], b[1]);
-        mma_bf16(acc[2 * n + 1], hi, b[2], b[3]);
-        mma_bf16(acc[2 * n], lo, b[0], b[1]);
-        mma_bf16(acc[2 * n + 1], lo, b[2], b[3]);
-      }
+    for (int i = 0; i < 4; ++i) {
+      uint32_t p[3];
+      split_bf16(s[2 * k + (i >> 1)][2 * (i & 1)], s[2 * k + (i >> 1)][2 * (i & 1) + 1], p);
+#pragma unroll
+      for (int x = 0; x < 3; ++x) w[x][i] = p[x];
+    }
+#pragma unroll
+    for (int n = 0; n < 8; n += 2) {
+      uint32_t b[2][4];
+#pragma unroll
+      for (int y = 0; y < 2; ++y)
+        if (n + y < vtiles) ldsm4_t(b[y], vs + at_place(k * 16 + (quad & 1) * 8 + l8, (n + y) * 2 + (quad >> 1)));
+#pragma unroll
+      for (int x = 0; x < 3; ++x)                      // products of one accumulator wait for one another: four take turns
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+          if (n + y < vtiles) {
+            mma_bf16(acc[2 * (n + y)], w[x], b[y][0], b[y][1]);
+            mma_bf16(acc[2 * (n + y) + 1], w[x], b[y][2], b[y][3]);
+          }
     }
   }
 }
@@ -878,6 +889,7 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const __grid_co
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[n][b][i] = 0.f;
 
+  constexpr int kTogether = 4 / NB;
   const uint32_t k_row = (quad & 1) * 8 + l8, v_row = (quad >> 1) * 8 + l8;          // & 7 = l8
   int stage = 0;
   for (int u = warp; u < n_units; u += 4) {
@@ -940,26 +952,30 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const __grid_co
 #pragma unroll
           for (int i = 0; i < 4; ++i) acc[n][b][i] *= al[b][i & 1];
     }
-    uint32_t hi[NB][2], lo[NB][2];                   // weights as the B operand: keys 2 t .. of row gr
+    uint32_t w[NB][2][3];                            // weights as the B operand: keys 2 t .. of row gr
 #pragma unroll
     for (int b = 0; b < NB; ++b)
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
-        split_bf16(s[b][2 * c], s[b][2 * c + 1], hi[b][c], lo[b][c]);
-        hi[b][c] = transpose_8x8(hi[b][c]);
-        lo[b][c] = transpose_8x8(lo[b][c]);
+        split_bf16(s[b][2 * c], s[b][2 * c + 1], w[b][c]);
+#pragma unroll
+        for (int x = 0; x < 3; ++x) w[b][c][x] = transpose_8x8(w[b][c][x]);
       }
 #pragma unroll
-    for (int n = 0; n < 8; ++n) {
-      if (n < vtiles) {
-        uint32_t x[4];
-        ldsm4_t(x, vs + (((n * 2 + (quad & 1)) ^ l8) << 4));
+    for (int n = 0; n < 8; n += kTogether) {
+      // the parts' products of one accumulator wait for one another, so several accumulators take turns
+      uint32_t x[kTogether][4];
 #pragma unroll
-        for (int b = 0; b < NB; ++b) {
-          mma_bf16(acc[n][b], x, hi[b][0], hi[b][1]);
-          mma_bf16(acc[n][b], x, lo[b][0], lo[b][1]);
-        }
-      }
+      for (int y = 0; y < kTogether; ++y)
+        if (n + y < vtiles) ldsm4_t(x[y], vs + ((((n + y) * 2 + (quad & 1)) ^ l8) << 4));
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int y = 0; y < kTogether; ++y)
+          if (n + y < vtiles) {
+#pragma unroll
+            for (int b = 0; b < NB; ++b) mma_bf16(acc[n + y][b], x[y], w[b][0][i], w[b][1][i]);
+          }
     }
   }
 #pragma unroll

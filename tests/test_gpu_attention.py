@@ -245,6 +245,32 @@ def test_attention_over_cached_rows(steps, past, H, G, d, dv, extras):
             assert (o.double() - want).abs().max() <= 2.0 ** -8 * want.abs().max()
 
 
+@pytest.mark.parametrize("steps,past,H,G", [([1] * 40, [63] * 40, 8, 1), ([1] * 40, [63] * 40, 8, 8), ([60, 60], [5, 130], 4, 2)])
+def test_weights_of_cached_rows_keep_32_bits(steps, past, H, G):
+    """Values +1 and -1 under pairs of keys that differ by a bf16 step in one place: the result is a sum of differences, some 2^-12, of
+    weights.  Rounding the result to bf16 is 1.65e-3 over many values, the fp32 exponentials (1e-7 of a weight each) add 0.6e-3;
+    weights of 16 bits, 2^-18 off at random, would add 1e-2."""
+    from easyllm_b200.ops import infer as iops
+    torch.manual_seed(H + G)
+    dev, d, cap = "cuda", 64, 256
+    q = torch.randn(sum(steps), H, d, device=dev).bfloat16()
+    q[..., 0] *= 0.25
+    k = torch.randn(len(steps) * cap, G, d, device=dev).bfloat16()
+    k[1::2] = k[0::2]
+    k[1::2, :, 0] *= 1 + 2.0 ** -7
+    v = torch.ones(len(steps) * cap, G, d, device=dev).bfloat16()
+    v[1::2] = -1
+    base = [i * cap for i, n in enumerate(steps) for _ in range(n)]
+    length = [p + j + 1 for n, p in zip(steps, past) for j in range(n)]
+    b, n = (torch.tensor(x, dtype=torch.int32, device=dev) for x in (base, length))
+    kw = {"cu_seqlens": torch.tensor([0] + steps, device=dev).cumsum(0).int(), "max_q": max(steps)} if max(steps) > 1 else {}
+    pairs = n % 2 == 0                                   # rows that see whole pairs
+    o = iops.attention_rows(q, k, v, b, n, max(length), d ** -0.5, **kw)[pairs].double()
+    want = _rows_exact(q, k, v, base, length, d ** -0.5, None, None, None, None)[pairs]
+    assert want.numel() > 0 and want.abs().mean() < 2.0 ** -9
+    assert (o - want).norm() <= 2.4e-3 * want.norm()
+
+
 @pytest.mark.parametrize("window", [None, 77])
 @pytest.mark.parametrize("steps,past,H,G", [([1, 1], [700, 63], 8, 2), ([3, 4], [130, 20], 8, 2), ([65, 40], [300, 25], 8, 2), ([2, 20], [2500, 30], 4, 4)])
 def test_values_that_are_not_finite_reach_the_rows_that_see_them(steps, past, H, G, window):
