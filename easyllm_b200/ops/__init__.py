@@ -247,9 +247,10 @@ def _gemm_ok(op, a, *dims):
     return True
 
 
-def matmul_nt(a, b, bias=None, few_rows=True):
-    """a [M,K] · b [N,K]ᵀ → [M,N] (bf16).  ``few_rows`` False keeps a short ``a`` on the tiled kernels too: the recorded
-    forward pass does, so that a loss does not change in its last bits with the number of tokens in the batch."""
+def matmul_nt(a, b, bias=None, few_rows=False):
+    """a [M,K] · b [N,K]ᵀ → [M,N] (bf16).  ``few_rows``: a short ``a`` may take the kernels for few rows.  Recorded forward
+    passes, tensor-parallel ones too, stay on the tiled kernels, so that a loss does not change in its last bits with the number
+    of tokens in the batch."""
     if _gemm_ok("matmul_nt", a, a.shape[-1], b.shape[-1], b.shape[0]):
         return _cu().gemm(a, b, bias=bias, few_rows=few_rows)
     return F.linear(a, b, bias)
@@ -296,7 +297,7 @@ class _Linear(torch.autograd.Function):
     def forward(ctx, x, w, bias):
         ctx.save_for_backward(x, w)
         ctx.wref, ctx.bref = w, bias
-        return matmul_nt(x, w, bias, few_rows=False)
+        return matmul_nt(x, w, bias)
 
     @staticmethod
     def backward(ctx, dy):
@@ -319,7 +320,7 @@ class _Linear(torch.autograd.Function):
 def linear(x, w, bias=None):
     if _kern(x):
         x2 = x.reshape(-1, x.shape[-1]).contiguous()
-        y = matmul_nt(x2, w, bias) if _cu().nothing_to_record() else _Linear.apply(x2, w, bias)
+        y = matmul_nt(x2, w, bias, few_rows=True) if _cu().nothing_to_record() else _Linear.apply(x2, w, bias)
         return y if x.dim() == 2 else y.view(*x.shape[:-1], w.shape[0])
     return F.linear(x, w, bias)
 
@@ -356,7 +357,7 @@ class _LinearParts(torch.autograd.Function):
         ctx.save_for_backward(x, W)
         ctx.wrefs = weights
         ctx.has_bias = bias is not None
-        return matmul_nt(x, W, bias, few_rows=False)
+        return matmul_nt(x, W, bias)
 
     @staticmethod
     def backward(ctx, dy):
@@ -389,7 +390,7 @@ def linear_parts(x, weights, biases=None):
         bias = torch.cat(list(biases), 0)
     if _kern(x):
         x2 = x.reshape(-1, x.shape[-1]).contiguous()
-        y = matmul_nt(x2, _LinearParts.fused(weights), bias) if _cu().nothing_to_record() else \
+        y = matmul_nt(x2, _LinearParts.fused(weights), bias, few_rows=True) if _cu().nothing_to_record() else \
             _LinearParts.apply(x2, bias, *weights)
         return y if x.dim() == 2 else y.view(*x.shape[:-1], y.shape[-1])
     return F.linear(x, torch.cat(list(weights), 0), bias)

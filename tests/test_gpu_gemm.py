@@ -299,3 +299,17 @@ def test_few_rows_of_a_weight_that_ends_within_a_warp(cu, N):
         cu.check_err_flag()
         want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
         assert ((out[:, :N].double() - want).abs() <= want.abs() * 2.0 ** -8 + size * 2.0 ** -17).all() and (out[:, N:] == 3.0).all()
+
+
+@pytest.mark.parametrize("rows", [1, 16, 100, 256])
+@pytest.mark.parametrize("N,K", [(2816, 1024), (1024, 2816)])
+def test_forward_products_do_not_depend_on_the_other_rows(cu, rows, N, K):
+    """The products that the tensor-parallel and the plain forward passes record: the bits of a row are those it has among 300."""
+    from easyllm_b200 import ops
+    torch.manual_seed(rows)
+    x = torch.randn(300, K, device="cuda", dtype=torch.bfloat16)
+    w = torch.randn(N, K, device="cuda", dtype=torch.bfloat16).requires_grad_()
+    many = ops.matmul_nt(x, w.detach())
+    assert torch.equal(ops.matmul_nt(x[:rows].contiguous(), w.detach()), many[:rows])
+    assert torch.equal(ops.linear(x[:rows], w).detach(), many[:rows])
+    cu.check_err_flag()
