@@ -132,7 +132,8 @@ class MedusaModel(nn.Module):
 
     def _hidden(self, input_ids, attention_mask=None, position_ids=None, caches=None, meta=None):
         meta = meta or build_meta(input_ids, attention_mask, position_ids)
-        return self.base_model.hidden_states(input_ids, meta, caches)
+        with ops.serving(caches is not None):
+            return self.base_model.hidden_states(input_ids, meta, caches)
 
     def forward(self, input_ids=None, attention_mask=None, labels=None, output_orig=False, position_ids=None,
                 return_dict=None, **_):
@@ -169,8 +170,9 @@ class MedusaModel(nn.Module):
                 for _ in range(a.num_hidden_layers)]
 
     def _step_logits(self, h):
-        med = torch.stack([head(h) for head in self.medusa_head], 0).float()     # [heads, n, V]
-        base = ops.linear(h, self.base_model.head_weight()).float()               # [n, V]
+        with ops.serving():
+            med = torch.stack([head(h) for head in self.medusa_head], 0).float()     # [heads, n, V]
+            base = ops.linear(h, self.base_model.head_weight()).float()               # [n, V]
         return med, base
 
     @torch.no_grad()
@@ -210,7 +212,8 @@ class MedusaModel(nn.Module):
                 pos = (tree.position_ids + n0).view(1, -1)
                 meta = build_meta(tree_tokens.view(1, -1), None, pos)
                 meta["tree_mask"] = tree.attn_mask
-                h = self.base_model.hidden_states(tree_tokens.view(1, -1), meta, caches)
+                with ops.serving():
+                    h = self.base_model.hidden_states(tree_tokens.view(1, -1), meta, caches)
                 med_t, base_t = self._step_logits(h)                                   # [heads, n_tree, V], [n_tree, V]
                 ri = tree.retrieve_indices
                 valid = ri >= 0

@@ -628,14 +628,16 @@ class CausalLM(nn.Module):
             parts = [torch.as_tensor(t, dtype=torch.long).reshape(-1) for t in tokens]
             counts, ids = [p.numel() for p in parts], torch.cat(parts).to(dev, non_blocking=True)
         meta = state.step_meta(slots, counts)
-        return self.hidden_states(ids, meta, state.layers, inputs_embeds=inputs_embeds, tokens=state.tokens), meta
+        with ops.serving():
+            return self.hidden_states(ids, meta, state.layers, inputs_embeds=inputs_embeds, tokens=state.tokens), meta
 
     @torch.no_grad()
     def logits(self, h):
         """fp32 logits of hidden rows."""
         if self.model.hybrid:
             return iops.linear_f32(h, self.lm_head.weight)
-        return ops.linear(h, self.head_weight()).float()
+        with ops.serving():
+            return ops.linear(h, self.head_weight()).float()
 
     @torch.no_grad()
     def _decode_steps(self, input_ids, max_new_tokens=64, do_sample=False, temperature=1.0, top_k=0, top_p=0.0,

@@ -18,6 +18,8 @@ from __future__ import annotations
 
 import torch
 
+from ... import ops
+
 BLOCK = 256          # positions a key/value cache grows by
 
 
@@ -161,7 +163,8 @@ class DecodeGraph:
         self.graph = torch.cuda.CUDAGraph()
         torch.cuda.synchronize()
         with torch.no_grad(), torch.cuda.graph(self.graph):
-            self.logits = model.logits(model.hidden_states(self.ids, self.meta, state.layers, tokens=state.tokens))
+            with ops.serving():
+                self.logits = model.logits(model.hidden_states(self.ids, self.meta, state.layers, tokens=state.tokens))
             for name in ("seq_pos0", "position_ids", "kv_len"):
                 self.meta[name].add_(1)
 

@@ -238,6 +238,10 @@ class LlamaModelPipe(nn.Module):
     def forward_stage(self, io: StageIO, labels=None, return_logits=False):
         """Runs this stage.  Returns a StageIO (intermediate stage), a scalar loss (last stage
         with ``labels``) or logits ``[b, s, V(/tp)]`` (last stage, ``return_logits``)."""
+        with ops.serving(self.kv_caches is not None):
+            return self._forward_stage(io, labels, return_logits)
+
+    def _forward_stage(self, io, labels, return_logits):
         g = get_grid()
         a = self.args
         if self.has_embedding:

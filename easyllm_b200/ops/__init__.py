@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import math
 import os
+import threading
 
 import torch
 import torch.distributed as dist
@@ -40,6 +41,29 @@ def set_strict(flag):
 def fallbacks():
     """``{(op, reason): count}`` of the calls that left the kernel path since the process started."""
     return dict(_FALLBACKS)
+
+
+_TLS = threading.local()
+
+
+class serving:
+    """Context of a step that decodes or continues sequences (of this thread; autograd's do not see it).  In it products may take
+    the kernels for few rows and the gated one, whose results differ in their last bits from those of the forward pass that
+    training records.  Outside of it a pass without gradients, an evaluation, gives the bits of the recorded one."""
+
+    def __init__(self, on=True):
+        self.on = bool(on)
+
+    def __enter__(self):
+        self.before = is_serving()
+        _TLS.serving = self.before or self.on
+
+    def __exit__(self, *_):
+        _TLS.serving = self.before
+
+
+def is_serving():
+    return getattr(_TLS, "serving", False)
 
 
 def note_fallback(op, t, reason):
@@ -248,9 +272,9 @@ def _gemm_ok(op, a, *dims):
 
 
 def matmul_nt(a, b, bias=None, few_rows=False):
-    """a [M,K] · b [N,K]ᵀ → [M,N] (bf16).  ``few_rows``: a short ``a`` may take the kernels for few rows.  Recorded forward
-    passes, tensor-parallel ones too, stay on the tiled kernels, so that a loss does not change in its last bits with the number
-    of tokens in the batch."""
+    """a [M,K] · b [N,K]ᵀ → [M,N] (bf16).  ``few_rows``: a short ``a`` may take the kernels for few rows (``serving``).  Forward
+    passes of training and evaluation, tensor-parallel ones too, stay on the tiled kernels, so that a loss does not change in its
+    last bits with the number of tokens in the batch, nor with whether gradients are recorded."""
     if _gemm_ok("matmul_nt", a, a.shape[-1], b.shape[-1], b.shape[0]):
         return _cu().gemm(a, b, bias=bias, few_rows=few_rows)
     return F.linear(a, b, bias)
@@ -320,7 +344,7 @@ class _Linear(torch.autograd.Function):
 def linear(x, w, bias=None):
     if _kern(x):
         x2 = x.reshape(-1, x.shape[-1]).contiguous()
-        y = matmul_nt(x2, w, bias, few_rows=True) if _cu().nothing_to_record() else _Linear.apply(x2, w, bias)
+        y = matmul_nt(x2, w, bias, few_rows=is_serving()) if _cu().nothing_to_record() else _Linear.apply(x2, w, bias)
         return y if x.dim() == 2 else y.view(*x.shape[:-1], w.shape[0])
     return F.linear(x, w, bias)
 
@@ -390,7 +414,7 @@ def linear_parts(x, weights, biases=None):
         bias = torch.cat(list(biases), 0)
     if _kern(x):
         x2 = x.reshape(-1, x.shape[-1]).contiguous()
-        y = matmul_nt(x2, _LinearParts.fused(weights), bias, few_rows=True) if _cu().nothing_to_record() else \
+        y = matmul_nt(x2, _LinearParts.fused(weights), bias, few_rows=is_serving()) if _cu().nothing_to_record() else \
             _LinearParts.apply(x2, bias, *weights)
         return y if x.dim() == 2 else y.view(*x.shape[:-1], y.shape[-1])
     return F.linear(x, torch.cat(list(weights), 0), bias)
@@ -542,9 +566,9 @@ def glu(gate_up, activation="silu"):
 
 
 def glu_linear(x, gate, up):
-    """``silu(x Wgᵀ) * (x Wuᵀ)``: one launch where nothing is recorded, the weights lie next to each other and the rows fill CTA
-    pairs; otherwise ``glu`` of ``linear_parts``."""
-    if _kern(x) and x.dim() == 2 and _GEMM == "tcgen05" and gate.shape == up.shape and _cu().nothing_to_record() and \
+    """``silu(x Wgᵀ) * (x Wuᵀ)``: one launch in a ``serving`` step whose rows fill CTA pairs, if the weights lie next to each other;
+    otherwise ``glu`` of ``linear_parts``, which rounds the 2 F columns in between."""
+    if is_serving() and _kern(x) and x.dim() == 2 and _GEMM == "tcgen05" and gate.shape == up.shape and _cu().nothing_to_record() and \
             _cu().glu_route(x.shape[0], gate.shape[0]):
         w = _adjacent_alias([gate.detach(), up.detach()])
         y = None if w is None else _cu().gemm_glu(x, w, None, "silu")

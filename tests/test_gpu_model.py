@@ -162,3 +162,47 @@ def test_synchronizing_reads_do_not_grow_with_the_number_of_micro_batches():
             torch.cuda.set_sync_debug_mode("default")
         counts.append(sum("synchroniz" in str(w.message).lower() for w in seen))
     assert counts[0] == counts[1], counts
+
+
+@pytest.mark.parametrize("tokens", [5, 40, 256, 512])
+@pytest.mark.parametrize("width,ff,kv", [(256, 704, 2), (1024, 2816, 8)])
+def test_an_evaluation_gives_the_bits_of_the_recorded_pass(tokens, width, ff, kv):
+    """One batch with gradients and without, before the model has served and after (which puts gate and up weights next to each
+    other): the same logits and the same loss, bit for bit, at row counts of all the kernels that serving chooses between.  A step
+    that serves the same tokens is near them."""
+    from easyllm_b200.models.hf_models import CausalLM, arch_from_hf_config
+    torch.manual_seed(tokens)
+    cfg = {"model_type": "llama", "vocab_size": 512, "hidden_size": width, "intermediate_size": ff, "num_hidden_layers": 2,
+           "num_attention_heads": width // 128, "num_key_value_heads": min(kv, width // 128), "rms_norm_eps": 1e-6,
+           "max_position_embeddings": 1024}
+    with torch.device("cuda"):
+        model = CausalLM(arch_from_hf_config(cfg), dtype=torch.bfloat16)
+    ids = torch.randint(0, 512, (1, tokens), device="cuda")
+    for served in (False, True):
+        if served:
+            state = model.new_state(1, tokens)
+            h, _ = model.step(state, [state.open()], [ids[0]])
+            step = model.logits(h)
+        recorded = model(ids)["logits"]
+        assert recorded.requires_grad
+        loss = model(ids, labels=ids)["loss"]
+        with torch.no_grad():
+            assert torch.equal(model(ids)["logits"], recorded) and torch.equal(model(ids, labels=ids)["loss"], loss)
+    want = recorded.detach().float()[0]
+    assert (step - want).norm() <= 2e-2 * want.norm()
+
+
+def test_what_the_recorded_functions_refuse_is_refused_without_gradients():
+    """vmap and forward-mode differentiation of an op, with gradients recorded and without: the functions refuse both, and so do the
+    launches that skip them."""
+    from easyllm_b200 import ops
+    x = torch.randn(3, 16, 64, device="cuda", dtype=torch.bfloat16)
+    w, nw = torch.randn(64, 64, device="cuda", dtype=torch.bfloat16), torch.ones(64, device="cuda", dtype=torch.bfloat16)
+    for f in (lambda a: ops.linear(a, w), lambda a: ops.rmsnorm(a, nw), lambda a: ops.glu(a), lambda a: ops.linear_parts(a, (w, w))):
+        for grad in (True, False):
+            with torch.set_grad_enabled(grad):
+                f(x[0])
+                with pytest.raises(RuntimeError):
+                    torch.func.vmap(f)(x)
+                with pytest.raises(RuntimeError), torch.autograd.forward_ad.dual_level():
+                    f(torch.autograd.forward_ad.make_dual(x[0], torch.ones_like(x[0])))
