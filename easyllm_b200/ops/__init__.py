@@ -470,14 +470,25 @@ class _EmbeddingToMain(torch.autograd.Function):
         (ids,) = ctx.saved_tensors
         w = ctx.wref
         dout = dout.contiguous()
-        if not _embedding_main_grad(w) or dout.data_ptr() % 16:
+        if not _embedding_main_grad(w) or dout.data_ptr() % 16 or _gradient_is_seen(w):
             return None, torch.ops.aten.embedding_dense_backward(dout, ids, w.shape[0], -1, False)
-        _cu().embedding_bwd_(ids, dout, w.main_grad, 0)
+        _cu().embedding_bwd_ordered_(ids, dout, w.main_grad)
         return None, None
 
 
+def _gradient_is_seen(w):
+    """In a backward pass: whether somebody else gets the gradient of the leaf ``w`` that autograd is handed: hooks on it,
+    ``torch.autograd.grad`` for it, a pass that is itself recorded."""
+    if w._backward_hooks or getattr(w, "_post_accumulate_grad_hooks", None) or torch.is_grad_enabled():
+        return True
+    try:
+        return not torch._C._will_engine_execute_node(torch.autograd.graph.get_gradient_edge(w).node)
+    except RuntimeError:                       # a leaf whose gradient torch.autograd.grad returns
+        return True
+
+
 def _embedding_main_grad(w):
-    """Whether rows of the gradient can be added to ``w.main_grad`` by 16-byte vector atomics."""
+    """Whether rows of the gradient can be added to ``w.main_grad`` in 16-byte pieces."""
     mg = getattr(w, "main_grad", None)
     return mg is not None and mg.dtype == torch.float32 and mg.shape == w.shape and mg.is_contiguous() and \
         mg.data_ptr() % 16 == 0 and w.shape[1] % 8 == 0
@@ -486,8 +497,10 @@ def _embedding_main_grad(w):
 def token_embedding(ids, weight):
     """``F.embedding(ids, weight)``.  With an fp32 ``main_grad`` the gradient rows are added to it as they are: autograd's dense
     bf16 gradient costs a pass over the whole table to clear, one to fill and one to add, 700 us for 32000 x 4096 where the
-    4096 rows of a batch take 30.  The order of the sums is not fixed, so a program that asks for deterministic algorithms keeps
-    the dense gradient."""
+    4096 rows of a batch take 60.  The rows of one id are added up in the order of the tokens, so a step repeats itself bit for bit.
+    ``weight.grad`` stays None then, as for the other weights with a ``main_grad``; where hooks on the weight or
+    ``torch.autograd.grad`` look at its gradient, and in programs that ask for deterministic algorithms, it is autograd's dense
+    one."""
     if _kern(weight) and weight.requires_grad and torch.is_grad_enabled() and ids.is_cuda and _embedding_main_grad(weight) and \
             not torch.are_deterministic_algorithms_enabled() and not _cu().transforms_active():
         return _EmbeddingToMain.apply(ids, weight)

@@ -263,6 +263,46 @@ __global__ void embedding_bwd_kernel(const long long* __restrict__ ids, const __
   }
 }
 
+// The same with a fixed order of the sums: `sorted` are the ids in ascending order, `order` the tokens they come from (a stable
+// sort), and the CTA at the first of a run of equal ids adds the rows of the run up, in the order of the tokens, before it adds
+// them to the table's row, which no other CTA writes.  A thread owns eight columns and has kRunAhead rows in flight.
+constexpr int kRunAhead = 16;
+__global__ void __launch_bounds__(128) embedding_bwd_runs_kernel(const long long* __restrict__ sorted, const long long* __restrict__ order,
+                                                                 const __nv_bfloat16* __restrict__ dout, float* __restrict__ grad32,
+                                                                 int T, int cols, long long rows) {
+  const int p = blockIdx.x, c = (blockIdx.y * 128 + threadIdx.x) * 8;
+  const long long id = sorted[p];
+  if ((p > 0 && sorted[p - 1] == id) || id < 0 || id >= rows || c >= cols) return;
+  float acc[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+  for (int i = p;; i += kRunAhead) {
+    int n = 0;                                       // rows of the run from i on
+#pragma unroll
+    for (int j = 0; j < kRunAhead; ++j) n += i + j < T && sorted[i + j] == id;
+    bf16x8 x[kRunAhead];
+#pragma unroll
+    for (int j = 0; j < kRunAhead; ++j)
+      if (j < n) x[j] = *reinterpret_cast<const bf16x8*>(dout + (size_t)order[i + j] * cols + c);
+#pragma unroll
+    for (int j = 0; j < kRunAhead; ++j) {
+      if (j < n) {
+        float f[8];
+        unpack8(x[j], f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += f[e];
+      }
+    }
+    if (n < kRunAhead) break;
+  }
+  float4* dst = reinterpret_cast<float4*>(grad32 + id * cols + c);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const float4 g = dst[h];
+    dst[h] = make_float4(g.x + acc[4 * h], g.y + acc[4 * h + 1], g.z + acc[4 * h + 2], g.w + acc[4 * h + 3]);
+  }
+}
+
 }  // namespace ell
 
 // vocab_total > 0 with err != nullptr: ids outside [0, vocab_total) set *err to 31.
@@ -284,6 +324,16 @@ ELL_API int ell_embedding_bwd(const long long* ids, const void* dout, float* gra
   const int grid = T < ell::kNumSMs * 16 ? T : ell::kNumSMs * 16;
   ell::embedding_bwd_kernel<<<grid, 128, 0, stream>>>(ids, (const __nv_bfloat16*)dout, grad32, T, cols, vocab_start,
                                                        rows);
+  return ell::launch_status();
+}
+
+ELL_API int ell_embedding_bwd_runs(const long long* sorted, const long long* order, const void* dout, float* grad32, int T, int cols,
+                                   long long rows, cudaStream_t stream) {
+  if (T == 0) return 0;
+  if (cols % 8) return -1;
+  if (cols > 65535 * 1024) return -2;
+  ell::embedding_bwd_runs_kernel<<<dim3(T, (cols + 1023) / 1024), 128, 0, stream>>>(sorted, order, (const __nv_bfloat16*)dout, grad32, T,
+                                                                                   cols, rows);
   return ell::launch_status();
 }
 

@@ -309,6 +309,16 @@ def embedding_bwd_(ids, dout, grad32, vocab_start):
     _check(rc, "embedding_bwd")
 
 
+def embedding_bwd_ordered_(ids, dout, grad32):
+    """``grad32[id] += `` the sum of the rows ``dout[t]`` of every id, in the order of the tokens."""
+    ids, order = torch.sort(ids.reshape(-1).to(torch.int64), stable=True)
+    d = dout.reshape(ids.numel(), -1)
+    _bf16c(d, "dout")
+    rc = lib().ell_embedding_bwd_runs(_p(ids), _p(order), _p(d), _p(grad32), c_int(ids.numel()), c_int(d.shape[1]),
+                                      c_longlong(grad32.shape[0]), _stream())
+    _check(rc, "embedding_bwd_runs")
+
+
 # ---- cross entropy ----------------------------------------------------------------------------
 def ce_fwd(logits, target, vocab_start, valid_cols):
     _bf16c(logits, "logits")

@@ -327,6 +327,54 @@ def test_embedding_gradient_goes_to_main_grad(cu, tokens, rows, cols, dtype, det
     assert ((emb.weight.main_grad.double() - want).abs() <= size * (tokens + 1) * 2.0 ** -24).all()
 
 
+@pytest.mark.parametrize("tokens,rows,cols", [(1, 3, 8), (2000, 7, 1032), (4096, 300, 2048)])
+def test_embedding_gradient_repeats_itself(cu, tokens, rows, cols):
+    """Ids that come hundreds of times: the same bits every time, those of the sum in the order of the tokens in fp32."""
+    from easyllm_b200 import ops
+    torch.manual_seed(tokens)
+    w = torch.nn.Parameter(torch.randn(rows, cols, device="cuda", dtype=torch.bfloat16))
+    ids = torch.randint(0, rows, (tokens,), device="cuda")
+    ids[tokens // 2:] = ids[0]
+    dy = torch.randn(tokens, cols, device="cuda", dtype=torch.bfloat16)
+    before = torch.randn(rows, cols, device="cuda")
+    got = []
+    for _ in range(4):
+        w.main_grad = before.clone()
+        ops.token_embedding(ids, w).backward(dy)
+        got.append(w.main_grad)
+    assert w.grad is None and all(torch.equal(got[0], g) for g in got[1:])
+    for i in {int(ids[0]), int(ids[tokens // 3])}:
+        want = torch.zeros(cols, device="cuda")
+        for t in (ids == i).nonzero().flatten().tolist():
+            want += dy[t].float()
+        assert torch.equal(got[0][i], before[i] + want)
+
+
+def test_embedding_gradient_that_somebody_looks_at(cu):
+    """torch.autograd.grad for the table, hooks on it and a recorded backward pass get the dense gradient; a gradient asked for
+    another leaf alone changes nothing."""
+    from easyllm_b200 import ops
+    torch.manual_seed(0)
+    w = torch.nn.Parameter(torch.randn(50, 64, device="cuda", dtype=torch.bfloat16))
+    scale = torch.nn.Parameter(torch.ones(64, device="cuda", dtype=torch.bfloat16))
+    ids, dy = torch.randint(0, 50, (30,), device="cuda"), torch.randn(30, 64, device="cuda", dtype=torch.bfloat16)
+    want = torch.autograd.grad(torch.nn.functional.embedding(ids, w), w, dy)[0]
+    w.main_grad = torch.zeros(50, 64, device="cuda")
+    assert torch.equal(torch.autograd.grad(ops.token_embedding(ids, w), w, dy)[0], want)
+    assert torch.equal(torch.autograd.grad(ops.token_embedding(ids, w), w, dy, create_graph=True)[0], want)
+    torch.autograd.grad(ops.token_embedding(ids, w) * scale, scale, dy)
+    assert not w.main_grad.any()
+    for register in (w.register_hook, w.register_post_accumulate_grad_hook):
+        seen = []
+        handle = register(lambda g: seen.append(g.grad.clone() if g is w else g.clone()))
+        ops.token_embedding(ids, w).backward(dy)
+        handle.remove()
+        assert torch.equal(seen[0], want) and not w.main_grad.any()
+        w.grad = None
+    ops.token_embedding(ids, w).backward(dy)
+    assert w.grad is None and torch.allclose(w.main_grad, want.float(), atol=0.02, rtol=0.02)
+
+
 @pytest.mark.parametrize("T,hq,hk,D", [(1, 1, 1, 16), (7, 8, 2, 128), (301, 5, 5, 80)])
 def test_rope_append_is_rope_and_append(cu, T, hq, hk, D):
     """Bit for bit the two launches it stands for: rotated rows, and the cache rows of scattered places; other rows stay."""
