@@ -37,7 +37,6 @@
 // halves of its hidden units, and the epilogue writes act(gate + b) * (up + b) only: 2 F columns are neither written nor read again,
 // nor rounded in between.  4096 rows of 4096, F 11008: the pass over the 2 F columns took 46 us beside a product of 530.
 #include "gemm_fuse.cuh"
-#include "vec.cuh"
 
 namespace ell {
 namespace pair {
@@ -55,6 +54,18 @@ constexpr int kTmemCols = 2 * kTileN;       // two accumulator buffers
 constexpr int kSmemBytes = kStages * kStageBytes + 2 * kEpiBufBytes + 1024 + 512;
 constexpr int kGroupM = 8;                  // rasterisation: 8 M-tiles x all N-tiles per group
 enum GluAct { kGluSilu = 1, kGluGelu = 2 };
+// e^x to some 2^-22 of itself for every x.  This file is built with --use_fast_math, whose expf rounds x log2(e) to one float, an
+// error that grows with x (2^-18 at 60); here the product keeps its remainder.
+__device__ __forceinline__ float exp_whole(float x) {
+  x = fminf(fmaxf(x, -200.f), 200.f);                // 0 and infinity, before the remainder is not a number
+  const float t = __fmul_rn(x, 1.44269502f);         // log2(e) = 1.44269502 + 1.9259630e-8
+  const float rest = fmaf(x, 1.9259630e-8f, fmaf(x, 1.44269502f, -t));
+  return ex2_approx(t) * fmaf(0.69314718f, rest, 1.f);
+}
+// The forms of vec.cuh: z sigmoid(z), and 0.5 (1 + tanh(u)) = sigmoid(2 u)
+__device__ __forceinline__ float glu_act(float z, int act) {
+  return __fdividef(z, 1.f + exp_whole(act == kGluGelu ? -1.5957691216057308f * (z + 0.044715f * z * z * z) : -z));
+}
 enum Err { kErrPairProducer = 11, kErrPairMma = 12, kErrPairEpilogue = 13, kErrPairFlagWait = 15 };
 
 struct Shared {
@@ -713,7 +724,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                   gate += at < F ? __bfloat162float(bias[at]) : 0.f;
                   up += at < F ? __bfloat162float(bias[F + at]) : 0.f;
                 }
-                v[e] = up * (fuse.group_glu == kGluGelu ? gelu_tanh_f(gate) : silu_f(gate));
+                v[e] = up * glu_act(gate, fuse.group_glu);
               }
               *reinterpret_cast<bf16x8*>(row_ptr + (((p * 4 + c) ^ (row_in_tile & 7)) << 4)) = pack8(v);  // 128B swizzle
             }

@@ -73,7 +73,7 @@ __device__ __forceinline__ void store_v(__nv_bfloat16* p, const float* f) {
   }
 }
 
-// Accurate expf, and a division of at most 2 ulp (0 for a denominator above 2^126, which is the limit here).
+// For the sources that are built without --use_fast_math: accurate expf, and a division of at most 2 ulp (0 for a denominator above 2^126, which is the limit here).
 __device__ __forceinline__ float sigmoid_f(float z) { return __fdividef(1.f, 1.f + expf(-z)); }
 __device__ __forceinline__ float silu_f(float z) { return __fdividef(z, 1.f + expf(-z)); }
 // 0.5 (1 + tanh(x)) = sigmoid(2 x)

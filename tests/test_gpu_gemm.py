@@ -313,3 +313,22 @@ def test_forward_products_do_not_depend_on_the_other_rows(cu, rows, N, K):
     assert torch.equal(ops.matmul_nt(x[:rows].contiguous(), w.detach()), many[:rows])
     assert torch.equal(ops.linear(x[:rows], w).detach(), many[:rows])
     cu.check_err_flag()
+
+
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh"])
+def test_gated_product_of_extreme_gates(cu, act):
+    """Gates from -inf to inf, where the exponential over- and underflows: one product of a single term, so that gate and up are what
+    is written here, against the activation in 64 bits (one rounding to bf16; results below 2^-126 may be 0)."""
+    gates = [0.0, 1e-3, -1e-3, 1.0, -1.0, 5.0, -5.0, 20.0, -20.0, -60.0, 80.0, -80.0, 3e4, -3e4, 1e38, -1e38, float("inf"), float("-inf"), float("nan")]
+    M, F, K = 256, 256, 64
+    x, w = (torch.zeros(n, K, device="cuda", dtype=torch.bfloat16) for n in (M, 2 * F))
+    g = torch.tensor(gates, device="cuda", dtype=torch.bfloat16)
+    x[:, 0] = 1.0
+    w[:len(gates), 0], w[F:, 0] = g, 2.0
+    y = cu.gemm_glu(x, w, None, act)[:, :len(gates)].double()
+    cu.check_err_flag()
+    z = g.double()
+    want = 2 * (torch.nn.functional.silu(z) if act == "silu" else torch.nn.functional.gelu(z, approximate="tanh"))
+    ok = want.isfinite() & z.isfinite()
+    assert ((y[:, ok] - want[ok]).abs() <= want[ok].abs() * 2.0 ** -8 + 2.0 ** -100).all()
+    assert y[:, gates.index(float("inf"))].isinf().all() and y[:, -1].isnan().all()

@@ -1,4 +1,5 @@
-"""Kernels that start while the one before ends: what they may touch, and when."""
+"""Rules that the kernel sources keep: what a kernel that starts while the one before ends may touch, and when; what is built
+without approximate math."""
 import glob
 import os
 import re
@@ -31,6 +32,16 @@ def test_every_restricted_pointer_goes_through_the_wait():
     assert len(waits) > 25
     for path, kernel, pointers, passed in waits:
         assert set(pointers) <= set(passed), (path, kernel, set(pointers) - set(passed))
+
+
+def test_fast_math_sources_do_not_use_the_accurate_activations():
+    """vec.cuh's activations are as accurate as the expf that the compiler's flags give them."""
+    from easyllm_b200.ops import build
+    for path in build.sources():
+        base = os.path.splitext(os.path.basename(path))[0]
+        if base not in build.ACCURATE_SOURCES:
+            text = open(path).read()
+            assert not any(f + "(" in text for f in ("silu_f", "sigmoid_f", "gelu_tanh_f")), base
 
 
 @pytest.mark.gpu
