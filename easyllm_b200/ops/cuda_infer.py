@@ -227,8 +227,8 @@ def attention_rows(q, k, v, base, length, max_len, scale, sink=None, alibi_slope
                    max_q=None):
     T, H, d = q.shape
     G, dv = k.shape[1], v.shape[2]
-    if cu_seqlens is not None and (cu_seqlens.dtype != torch.int32 or not cu_seqlens.is_contiguous()):
-        raise ValueError("attention_rows: int32 sequence borders")
+    if cu_seqlens is not None:
+        cu_seqlens = cu_seqlens.to(torch.int32).contiguous()
     n_seq, max_q = (0, 1) if cu_seqlens is None else (cu_seqlens.numel() - 1, max_q)
     out = torch.empty(T, H, dv, dtype=q.dtype, device=q.device)
     need = lib().ell_attn_rows_scratch(c_int(T), c_int(H), c_int(G), c_int(d), c_int(dv), c_int(max_len), c_int(window or 0),

@@ -336,3 +336,15 @@ def test_ranges_of_decoding_rows(cu, n, H, G, bound):
         kk, vv = (t[keys].double().repeat_interleave(H // G, 1) for t in (k, v))
         p = torch.softmax(torch.einsum("hd,khd->hk", q[i].double(), kk) * d ** -0.5, -1)
         assert (out[i].double() - torch.einsum("hk,khd->hd", p, vv)).abs().max() <= 5 * (2.0 ** -9 + 2.0 ** -15)
+
+
+def test_sequence_borders_of_any_integer_type(cu):
+    """Borders in 64 bits, and every other element of a tensor, are the borders they hold."""
+    import easyllm_b200.ops.cuda_infer as ci
+    torch.manual_seed(0)
+    q, k, v = (torch.randn(n, 4, 64, device="cuda", dtype=torch.bfloat16) for n in (20, 40, 40))
+    base, length = torch.zeros(20, dtype=torch.int32, device="cuda"), torch.arange(21, 41, dtype=torch.int32, device="cuda")
+    borders = torch.tensor([0, 20], device="cuda")
+    got = [ci.attention_rows(q, k, v, base, length, 40, 0.125, cu_seqlens=c, max_q=20)
+           for c in (borders.int(), borders, torch.tensor([0, 7, 20, 7], device="cuda", dtype=torch.int32)[::2])]
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
