@@ -453,7 +453,7 @@ def gemm_glu(x, w, bias, act):
     ldx = x.stride(0) if M > 1 else K
     if x.dtype != torch.bfloat16 or w.dtype != x.dtype or (bias is not None and bias.dtype != x.dtype) or x.stride(1) != 1 or \
             not w.is_contiguous() or (bias is not None and not bias.is_contiguous()) or w.shape != (2 * F, K) or \
-            F % 8 or K % 8 or ldx % 8 or (x.data_ptr() | w.data_ptr()) & 15:
+            F % 8 or K % 8 or ldx % 8 or ldx < K or (x.data_ptr() | w.data_ptr()) & 15:
         return None
     out = torch.empty(M, F, dtype=x.dtype, device=x.device)
     rc = lib().ell_gemm_glu_pair(_p(x), _p(w), _p(out), _p(bias), c_int(M), c_int(F), c_int(K), c_int(ldx), c_int(F),

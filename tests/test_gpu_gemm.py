@@ -332,3 +332,16 @@ def test_gated_product_of_extreme_gates(cu, act):
     ok = want.isfinite() & z.isfinite()
     assert ((y[:, ok] - want[ok]).abs() <= want[ok].abs() * 2.0 ** -8 + 2.0 ** -100).all()
     assert y[:, gates.index(float("inf"))].isinf().all() and y[:, -1].isnan().all()
+
+
+def test_gated_product_of_rows_that_share_memory(cu):
+    """An expanded row has no row stride that TMA takes: the two launches, which copy it first, give the result."""
+    from easyllm_b200 import ops
+    torch.manual_seed(0)
+    w = torch.randn(1024, 128, device="cuda", dtype=torch.bfloat16)
+    x = torch.randn(1, 128, device="cuda", dtype=torch.bfloat16)
+    with torch.no_grad(), ops.serving():
+        want = ops.glu_linear(x.repeat(256, 1), w[:512], w[512:])
+        got = ops.glu_linear(x.expand(256, 128), w[:512], w[512:])
+    cu.check_err_flag()
+    assert (got - want).float().norm() <= 1e-2 * want.float().norm()
