@@ -15,15 +15,17 @@
 // brings records (one bulk copy each) and the values into a ring; the other warps hold 16 key rows of the state each, in the layout of
 // mma.sync's accumulators, which is also that of its left operand.
 //
-// Precision: fp32 throughout.  The products with the state take both operands as three bf16 parts (24 bits) and sum six of the nine
-// partial products in fp32; the state itself is updated by fused multiply-adds.  Against 64 bits, relative errors of 700 tokens of
-// 128 x 128 heads are 1.2e-7 (time mixing; token by token 1.0e-7) and 1.4e-7 (delta rule; 1.2e-7), of 2500 tokens with decays near 1
-// 2.3e-7 (2.8e-7) and 2.1e-7 (3.1e-7): fewer steps are rounded.  (With fp32 multiply-adds in place of the parts: the same errors
-// and 450 us where the delta rule takes 370, since the sums over key rows then cross the lanes of a warp.)
+// Precision: fp32 or better throughout.  Products of decays are pairs of floats, sums over the channels are added up in 64 bits.  The
+// products with the state take both operands as three bf16 parts (24 bits) and sum six of the nine partial products in fp32; the
+// state itself is updated by fused multiply-adds.  Against 64 bits, relative errors of 700 tokens of 128 x 128 heads are 0.94e-7 (time
+// mixing; token by token 1.00e-7) and 1.04e-7 (delta rule; 1.22e-7), of 2500 tokens with decays near 1 1.5e-7 (2.8e-7) and 1.5e-7
+// (3.1e-7): fewer steps are rounded.  With products and sums in one float they were 1.21e-7 and 1.42e-7 for 700 tokens, larger than
+// token by token.  (With fp32 multiply-adds in place of the bf16 parts: the same errors and 450 us where the delta rule takes 370,
+// since the sums over key rows then cross the lanes of a warp.)
 //
 // Bound by the issue of some 550 instructions a warp and chunk (delta rule; half of the slots are used, the rest waits on the chain
-// from the state to the next one).  One sequence of 4096 tokens, both launches: 16 heads of 128 x 128, delta rule, 1044 -> 422 us; 32
-// heads of 64 x 64, time mixing, 516 -> 293.  8 sequences of 512: 530 -> 390 and 207 -> 182.
+// from the state to the next one).  One sequence of 4096 tokens, both launches: 16 heads of 128 x 128, delta rule, 1044 -> 430 us; 32
+// heads of 64 x 64, time mixing, 516 -> 265.  8 sequences of 512: 530 -> 397 and 207 -> 168.
 #include "sm100.cuh"
 #include "vec.cuh"
 
@@ -73,6 +75,23 @@ __device__ __forceinline__ size_t first_record(const ChunkArgs& a, int s, int st
   return a.per_seq > 0 ? (size_t)s * a.per_seq : (size_t)(start / kCk + s);
 }
 
+// Product of up to 16 decays as an unevaluated sum of two floats: in one float its rounding errors, one a factor, were most of the
+// error of a chunk.
+struct DecayProduct {
+  float hi = 1.f, lo = 0.f;
+  __device__ __forceinline__ void times(float g) {
+    const float h = __fmul_rn(hi, g);
+    lo = fmaf(lo, g, fmaf(hi, g, -h));
+    hi = h;
+  }
+  __device__ __forceinline__ float of(float x) const { return fmaf(x, hi, __fmul_rn(x, lo)); }
+};
+
+__device__ __forceinline__ double dot4(const float* x, const float* y) {
+  const float4 a = *reinterpret_cast<const float4*>(x), b = *reinterpret_cast<const float4*>(y);
+  return (double)fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x)));
+}
+
 // Dot products of one level: token i of a right half with token j of the left half before it, for halves of HS tokens.  A thread
 // takes a share of the channels of one pair; neighbours add theirs.
 template <int MODE, int HS, int DP>
@@ -86,19 +105,12 @@ __device__ __forceinline__ void level_products(const float* rows, const float* k
     const bool kk = MODE == kDelta && dot >= kPairs;
     const float* x = (kk ? keys : rows) + i * kStride;
     const float* y = keys + j * kStride;
-    float s0 = 0.f, s1 = 0.f;
-#pragma unroll 4
-    for (int c = share * 4; c < DP; c += kShares * 4) {
-      const float4 a = *reinterpret_cast<const float4*>(x + c), b = *reinterpret_cast<const float4*>(y + c);
-      s0 = fmaf(a.x, b.x, s0);
-      s1 = fmaf(a.y, b.y, s1);
-      s0 = fmaf(a.z, b.z, s0);
-      s1 = fmaf(a.w, b.w, s1);
-    }
-    s0 += s1;
+    double sum = 0.;
+#pragma unroll 8
+    for (int c = share * 4; c < DP; c += kShares * 4) sum += dot4(x + c, y + c);
 #pragma unroll
-    for (int o = kShares / 2; o >= 1; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-    if (share == 0) (kk ? akk : aqk)[i * kCkMat + j] = s0;
+    for (int o = kShares / 2; o >= 1; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (share == 0) (kk ? akk : aqk)[i * kCkMat + j] = (float)sum;
   }
 }
 
@@ -110,19 +122,18 @@ __device__ __forceinline__ void level(const float (&q)[kCk], const float (&k)[kC
   const int c = threadIdx.x;
 #pragma unroll
   for (int mid = HS; mid < kCk; mid += 2 * HS) {
-    float p = 1.f;
+    DecayProduct p, back;
 #pragma unroll
     for (int i = mid; i < mid + HS; ++i) {
-      if (MODE == kDelta) p *= g[i];
-      rows[i * kStride + c] = q[i] * p;
-      if (MODE == kDelta) keys[i * kStride + c] = k[i] * p;
-      if (MODE == kWkv) p *= g[i];
+      if (MODE == kDelta) p.times(g[i]);
+      rows[i * kStride + c] = p.of(q[i]);
+      if (MODE == kDelta) keys[i * kStride + c] = p.of(k[i]);
+      if (MODE == kWkv) p.times(g[i]);
     }
-    p = 1.f;
 #pragma unroll
     for (int j = mid - 1; j >= mid - HS; --j) {
-      keys[j * kStride + c] = k[j] * p;
-      p *= g[j];
+      keys[j * kStride + c] = back.of(k[j]);
+      back.times(g[j]);
     }
   }
   __syncthreads();
@@ -163,20 +174,19 @@ __global__ void __launch_bounds__(DP) chunk_prepare_kernel(const ChunkArgs a) {
   if (MODE == kDelta && threadIdx.x < kCk)
     beta[threadIdx.x] = threadIdx.x < cnt ? a.beta[(first + threadIdx.x) * a.H + h] : 0.f;
   {
-    float p = 1.f;
+    DecayProduct p, back;
 #pragma unroll
     for (int i = 0; i < kCk; ++i) {
-      if (MODE == kDelta) p *= g[i];
-      rec[R::kQ + i * R::kStride + c] = q[i] * p;
-      if (MODE == kDelta) rec[R::kK + i * R::kStride + c] = k[i] * p;
-      if (MODE == kWkv) p *= g[i];
+      if (MODE == kDelta) p.times(g[i]);
+      rec[R::kQ + i * R::kStride + c] = p.of(q[i]);
+      if (MODE == kDelta) rec[R::kK + i * R::kStride + c] = p.of(k[i]);
+      if (MODE == kWkv) p.times(g[i]);
     }
-    rec[R::kP + c] = p;
-    p = 1.f;
+    rec[R::kP + c] = p.hi + p.lo;
 #pragma unroll
     for (int i = kCk - 1; i >= 0; --i) {
-      rec[R::kS + i * R::kStride + c] = k[i] * p;
-      p *= g[i];
+      rec[R::kS + i * R::kStride + c] = back.of(k[i]);
+      back.times(g[i]);
     }
     // the diagonal of A: q . k, or the bonus of the token itself
     const float u = MODE == kWkv && in ? a.u[(size_t)h * a.d + c] : 1.f;
@@ -190,18 +200,12 @@ __global__ void __launch_bounds__(DP) chunk_prepare_kernel(const ChunkArgs a) {
   {
     constexpr int kShares = DP / kCk;
     const int i = threadIdx.x / kShares, share = threadIdx.x % kShares;
-    float sum = 0.f;
+    double sum = 0.;
 #pragma unroll
-    for (int x = share * 4; x < DP; x += kShares * 4) {
-      const float4 y = *reinterpret_cast<const float4*>(rows + i * kStride + x), z = *reinterpret_cast<const float4*>(keys + i * kStride + x);
-      sum = fmaf(y.x, z.x, sum);
-      sum = fmaf(y.y, z.y, sum);
-      sum = fmaf(y.z, z.z, sum);
-      sum = fmaf(y.w, z.w, sum);
-    }
+    for (int x = share * 4; x < DP; x += kShares * 4) sum += dot4(rows + i * kStride + x, keys + i * kStride + x);
 #pragma unroll
     for (int o = kShares / 2; o >= 1; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (share == 0) aqk[i * kCkMat + i] = sum;
+    if (share == 0) aqk[i * kCkMat + i] = (float)sum;
   }
   __syncthreads();
   level<MODE, 8, DP>(q, k, g, rows, keys, aqk, akk);

@@ -348,6 +348,48 @@ def test_scans_in_rounds_of_chunks(kind, monkeypatch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["wkv", "delta"])
+@pytest.mark.parametrize("d,T", [(64, 260), (128, 260), (128, 900)])
+@pytest.mark.parametrize("decay", ["served", -3.0, 0.0])
+def test_chunks_are_as_precise_as_tokens(kind, d, T, decay, monkeypatch):
+    """The error of a scan in chunks against 64 bits is no larger than that of the scan token by token, from decays as a trained model
+    has them to decays that forget in a few tokens: of the outputs always, of the state where it spans more than a few tokens (one
+    rounding of a product is all of it otherwise)."""
+    from easyllm_b200.ops import cuda_infer
+    dev = _device("cuda")
+    H = 4
+    g = torch.Generator(dev).manual_seed(T + d)
+    q, k, v, x = (torch.randn(T, H, d, device=dev, generator=g) for _ in range(4))
+    rate = torch.rand(1, H, d, device=dev, generator=g) * 5 - 6 + 0.1 * x if decay == "served" else x + decay
+    dec = torch.exp(-torch.exp(rate))
+    if kind == "wkv":
+        ins = [q.to(BF16), (k * d ** -0.5).to(BF16), v.to(BF16), dec, torch.randn(H, d, device=dev, generator=g)]
+    else:
+        ins = [plain.unit(q) * d ** -0.5, plain.unit(k), v, dec, torch.sigmoid(torch.randn(T, H, device=dev, generator=g))]
+    qd, kd, vd, gd, ud = (t.double() for t in ins)
+    S, want = torch.zeros(H, d, d, dtype=torch.float64, device=dev), torch.empty(T, H, d, dtype=torch.float64, device=dev)
+    for t in range(T):                                      # [H, value column, key row]
+        if kind == "wkv":
+            kv = vd[t].unsqueeze(-1) * kd[t].unsqueeze(-2)
+            want[t] = ((S + kv * ud.unsqueeze(-2)) * qd[t].unsqueeze(-2)).sum(-1)
+            S = S * gd[t].unsqueeze(-2) + kv
+        else:
+            S = S * gd[t].unsqueeze(-2)
+            e = ud[t].unsqueeze(-1) * (vd[t] - (S * kd[t].unsqueeze(-2)).sum(-1))
+            S = S + e.unsqueeze(-1) * kd[t].unsqueeze(-2)
+            want[t] = (S * qd[t].unsqueeze(-2)).sum(-1)
+    off = []
+    for chunks in (True, False):
+        if not chunks:
+            monkeypatch.setattr(cuda_infer, "_scan_chunks", lambda *a: False)
+        state = torch.zeros(1, H, d, d, device=dev)
+        o = _scan(kind, ins, slice(0, T), meta_of([T], dev, [0], [0]), state, dev)
+        off.append(((o.double() - want).norm() / want.norm(), (state[0].double() - S).norm() / S.norm()))
+    (o, s), (o_tokens, s_tokens) = off
+    assert o <= 1.02 * o_tokens and (decay == 0.0 or s <= 1.02 * s_tokens), off
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("kind,dtype,H,d,dv", [("wkv", BF16, 2, 64, 64), ("wkv", F32, 1, 100, 24), ("delta", F32, 2, 128, 40), ("delta", F32, 2, 36, 64)])
 @pytest.mark.parametrize("bound", [None, 256, 257])
 def test_scans_of_sequences_longer_than_their_bound(kind, dtype, H, d, dv, bound):
