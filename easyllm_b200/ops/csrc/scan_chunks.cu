@@ -635,10 +635,12 @@ __global__ void __launch_bounds__(ScanSmem<MODE, DP>::kThreads) chunk_scan_kerne
 // ---- plan of a call ----
 // Shorter sequences stay token by token: two launches and their records cost what that many tokens take there (one sequence, us, in
 // chunks | by token: time mixing, 128 tokens 30 | 22, 256 tokens 32 | 39; delta rule, 64 tokens 25 | 22, 128 tokens 27 | 39).  The
-// records of a call may take kCkMaxBytes; longer ones go in several rounds over as many chunks as fit, with the state carried
-// between them.
+// records of a call and what is carried between rounds may take kCkMaxBytes; calls that need more go in several rounds over as many
+// chunks as fit, with the state carried between them, or token by token where a round would be under kCkMinRound chunks (many
+// sequences, which fill the GPU that way too).
 constexpr int kCkMinTokens[2] = {256, 128};
 constexpr long long kCkMaxBytes = 512ll << 20;
+constexpr int kCkMinRound = 4;
 
 struct ChunkPlan {
   bool fits;
@@ -664,10 +666,11 @@ static ChunkPlan chunk_plan(int mode, int n, int n_seq, int max_len, int H, int 
     p.round = p.chunks;
     p.rec_floats = all;
   } else {
-    long long r = kCkMaxBytes / 4 / (per * n_seq);
-    p.round = (int)(r < 4 ? 4 : (r > p.chunks ? p.chunks : r));
-    p.rec_floats = (long long)n_seq * p.round * per;
     p.carry_floats = (long long)n_seq * H * dv * p.dp;
+    const long long r = (kCkMaxBytes / 4 - p.carry_floats) / (per * n_seq);
+    p.fits = r >= kCkMinRound;
+    p.round = (int)(r > p.chunks ? p.chunks : r);
+    p.rec_floats = (long long)n_seq * p.round * per;
   }
   return p;
 }

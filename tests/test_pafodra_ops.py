@@ -459,6 +459,19 @@ def test_infinities_in_a_scan_in_chunks(kind, dtype, d, where, monkeypatch):
         assert bool(((a - b).abs()[fine & ~rest] <= 1e-5 * b.abs()[fine & ~rest].max()).all()) if bool((fine & ~rest).any()) else True
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("n_seq", [1, 7, 61, 256, 1024, 5000])
+@pytest.mark.parametrize("longest", [128, 300, 4096, 32768])
+def test_records_of_a_scan_stay_within_their_limit(mode, n_seq, longest):
+    """Host only: whatever the number and the lengths of the sequences, a scan's work space is 512 MiB at most, or it goes token by
+    token and needs none; a single sequence of any length goes in chunks."""
+    from easyllm_b200.ops import cuda
+    for H, d, dv in ((16, 128, 128), (64, 128, 128), (64, 64, 64)):
+        need = cuda.lib().ell_scan_chunks_work(mode, n_seq * longest, n_seq, longest, H, d, dv)
+        assert 0 <= need * 4 <= 512 << 20
+        assert n_seq > 1 or longest < 256 or need > 0
+
+
 @pytest.mark.parametrize("device", DEVICES)
 @pytest.mark.parametrize("kind", ["wkv", "delta"])
 def test_state_is_carried_far(device, kind):
