@@ -64,7 +64,7 @@ struct ChunkArgs {
   const int *cu, *slots, *pos0;
   float* rec;
   float* carry;                 // [n_seq, H, dv, DP]: the state between two launches over one sequence, or null
-  int H, G, d, dv, ldq, ldk, ldv;
+  int H, G, d, dv, ldq, ldk, ldv, n_seq;
   int c0, c1, per_seq;          // chunks of this launch; records per sequence (0: counted by tokens)
   int final;                    // no chunks come after this launch
   int* err;
@@ -149,9 +149,20 @@ __global__ void __launch_bounds__(DP) chunk_prepare_kernel(const ChunkArgs a) {
   __shared__ float4 rows4[kCk * kStride / 4], keys4[kCk * kStride / 4];
   __shared__ float aqk[kCk * kCkMat], akk[kCk * kCkMat], beta[kCk];
   float *rows = reinterpret_cast<float*>(rows4), *keys = reinterpret_cast<float*>(keys4);
-  const int s = blockIdx.z, h = blockIdx.y, chunk = a.c0 + blockIdx.x;
+  // one CTA a record: chunks of this round by sequence, or, counted by tokens, the sequence whose records these are
+  int s = blockIdx.z, chunk = a.c0 + blockIdx.x;
+  const int h = blockIdx.y;
+  if (a.per_seq == 0) {
+    int past = a.n_seq;
+    while (past - s > 1) {
+      const int mid = (s + past) / 2;
+      if (first_record(a, mid, a.cu[mid]) <= blockIdx.x) s = mid;
+      else past = mid;
+    }
+    chunk = blockIdx.x - (int)first_record(a, s, a.cu[s]);
+  }
   const int start = a.cu[s], n_tok = a.cu[s + 1] - start, t0 = chunk * kCk;
-  if (t0 >= n_tok) return;
+  if (chunk < 0 || t0 >= n_tok) return;
   const int cnt = min(kCk, n_tok - t0), c = threadIdx.x, hk = h / (a.H / a.G);
   float* rec = a.rec + ((first_record(a, s, start) + (a.per_seq > 0 ? blockIdx.x : chunk)) * a.H + h) * R::kFloats;
   float q[kCk], k[kCk], g[kCk];
@@ -638,7 +649,16 @@ __global__ void __launch_bounds__(ScanSmem<MODE, DP>::kThreads) chunk_scan_kerne
 // records of a call and what is carried between rounds may take kCkMaxBytes; calls that need more go in several rounds over as many
 // chunks as fit, with the state carried between them, or token by token where a round would be under kCkMinRound chunks (many
 // sequences, which fill the GPU that way too).
+//
+// Many short sequences beside a long one: the start of a CTA costs more here than token by token, a chunk costs less than 16 tokens.
+// Fitted to both scans of 8 to 61 sequences of 16 to 2048 tokens, in units of 16 tokens of 16 columns token by token (kCkUnitNs a key
+// row: 1.9 us on the GPU for 16 heads of 128 x 128, delta rule): 0.77 a chunk and 1.03 a sequence here, 1 and 0.41 there, within 10 %.
+// So the mean length should be 48, unless the chain of the longest sequence outlasts the work.  Us in chunks | by token, delta rule, 16
+// heads, 60 sequences beside one: 32 tokens, 256: 330 | 305; 32, 1024: 398 | 389; 32, 2048: 490 | 526; 100, 256: 761 | 759; time mixing,
+// 32 heads of 64: 123 | 118, 148 | 168, 201 | 296, 274 | 293.
 constexpr int kCkMinTokens[2] = {256, 128};
+constexpr int kCkMinMean = 48;
+constexpr float kCkUnitNs[2] = {0.091f, 0.118f}, kCkTokenUs[2] = {0.13f, 0.26f};
 constexpr long long kCkMaxBytes = 512ll << 20;
 constexpr int kCkMinRound = 4;
 
@@ -646,6 +666,7 @@ struct ChunkPlan {
   bool fits;
   int dp, chunks, round;        // padded key rows; chunks of the longest sequence; chunks of a round
   bool by_tokens;
+  int records;                  // of a head, counted by tokens
   long long rec_floats, carry_floats;
 };
 
@@ -656,11 +677,15 @@ static int rec_floats(int mode, int dp) {
 
 static ChunkPlan chunk_plan(int mode, int n, int n_seq, int max_len, int H, int d, int dv) {
   ChunkPlan p{};
-  p.fits = max_len >= kCkMinTokens[mode] && d <= 128 && dv % 8 == 0;
-  if (!p.fits) return p;
   p.dp = d <= 64 ? 64 : 128;
+  const float units = 0.77f * (n / kCk + n_seq / 2) + 1.03f * n_seq;
+  const float work_us = units * H * ((dv + kCkCols - 1) / kCkCols) * kCkUnitNs[mode] * p.dp * 1e-3f;
+  p.fits = max_len >= kCkMinTokens[mode] && d <= 128 && dv % 8 == 0 &&
+           (n >= (long long)kCkMinMean * n_seq || max_len * kCkTokenUs[mode] > work_us);
+  if (!p.fits) return p;
   p.chunks = (max_len + kCk - 1) / kCk;
-  const long long per = (long long)H * rec_floats(mode, p.dp), all = (long long)(n / kCk + n_seq) * per;
+  p.records = n / kCk + n_seq;
+  const long long per = (long long)H * rec_floats(mode, p.dp), all = p.records * per;
   p.by_tokens = all * 4 <= kCkMaxBytes;
   if (p.by_tokens) {
     p.round = p.chunks;
@@ -691,7 +716,8 @@ static int launch_chunks(ChunkArgs a, const ChunkPlan& p, int n_seq, cudaStream_
     a.c1 = c0 + p.round;
     a.final = a.c1 >= p.chunks;
     const int now = p.chunks - c0 < p.round ? p.chunks - c0 : p.round;
-    chunk_prepare_kernel<MODE, T, DP><<<dim3(now, a.H, n_seq), DP, 0, stream>>>(a);
+    const dim3 records = p.by_tokens ? dim3(p.records, a.H) : dim3(now, a.H, n_seq);
+    chunk_prepare_kernel<MODE, T, DP><<<records, DP, 0, stream>>>(a);
     scan<<<dim3((a.dv + kCkCols - 1) / kCkCols, a.H, n_seq), ScanSmem<MODE, DP>::kThreads, bytes, stream>>>(a);
   }
   return launch_status();
@@ -725,7 +751,7 @@ ELL_API int ell_scan_chunks(int mode, const void* q, const void* k, const void* 
   if (!p.fits || H % G || n_seq > 65535 || H > 65535 || (mode == kDelta && is_bf16)) return -2;
   if (work == nullptr || !aligned_to(work, 16) || !aligned_to(v, 16) || ldv * esz % 16 || dv * esz % 16) return -2;
   ChunkArgs a{q, k, v, decay, beta, u, o, state, cu, slots, pos0, work, p.carry_floats ? work + p.rec_floats : nullptr,
-              H, G, d, dv, ldq, ldk, ldv, 0, 0, 0, 1, err};
+              H, G, d, dv, ldq, ldk, ldv, n_seq, 0, 0, 0, 1, err};
   if (mode == kDelta) return run_chunks<kDelta, float>(a, p, n_seq, stream);
   return is_bf16 ? run_chunks<kWkv, __nv_bfloat16>(a, p, n_seq, stream) : run_chunks<kWkv, float>(a, p, n_seq, stream);
 }

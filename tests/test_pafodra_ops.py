@@ -472,6 +472,40 @@ def test_records_of_a_scan_stay_within_their_limit(mode, n_seq, longest):
         assert n_seq > 1 or longest < 256 or need > 0
 
 
+@pytest.mark.parametrize("counts,chunks", [([4096], True), ([512] * 8, True), ([128] + [16] * 60, False), ([256] + [32] * 60, False),
+                                           ([300] * 20, True), ([2048] + [100] * 60, True), ([1024] + [16] * 30, True),
+                                           ([260] + [1] * 63, False)])
+def test_one_long_sequence_does_not_send_many_short_ones_through_chunks(counts, chunks):
+    """Host only: which way a scan of the delta rule goes, 16 heads of 128 x 128."""
+    from easyllm_b200.ops import cuda
+    assert (cuda.lib().ell_scan_chunks_work(1, sum(counts), len(counts), max(counts), 16, 128, 128) > 0) == chunks
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,dtype", [("wkv", BF16), ("delta", F32)])
+def test_records_of_every_sequence_are_found(kind, dtype):
+    """Sequences of no token, of one and of many, in an order where the borders of records and of sequences fall apart: each has the
+    result that it has alone."""
+    dev = _device("cuda")
+    counts = [1, 0, 257, 16, 15, 0, 0, 300, 33, 1, 1, 640, 17]
+    T, H = sum(counts), 2
+    ins = _scan_inputs(kind, H, H, 64, 32, T, dtype)
+    state = torch.full((len(counts) + 1, H, 32, 64), 5.0, device=dev)
+    slots = [(5 * i + 3) % len(counts) for i in range(len(counts))]
+    got = _scan(kind, ins, slice(0, T), meta_of(counts, dev, slots, [0] * len(counts)), state, dev)
+    at = 0
+    for c, slot in zip(counts, slots):
+        if c:
+            one = torch.zeros(1, H, 32, 64, device=dev)
+            part = [x[at:at + c] for x in ins[:4]] + [ins[4] if kind == "wkv" else ins[4][at:at + c]]
+            want = _scan(kind, part, slice(0, c), meta_of([c], dev, [0], [0]), one, dev)
+            close(got[at:at + c], want.cpu(), 4e-6)
+            close(state[slot], one[0].cpu(), 4e-6)
+        else:
+            assert bool((state[slot] == 5).all())
+        at += c
+
+
 @pytest.mark.parametrize("device", DEVICES)
 @pytest.mark.parametrize("kind", ["wkv", "delta"])
 def test_state_is_carried_far(device, kind):
