@@ -106,7 +106,7 @@ struct FaArgs {
 };
 
 // Query heads whose CTAs come together, in the order of their work.  Head by head, the last head's long walks started last and left
-// SMs idle: 30 % of them for 32 heads over 4096 tokens, 260 us where this order takes 190.  As many heads as have their keys and values
+// SMs idle: 30 % of them for 32 heads over 4096 tokens, 233 us where this order took 198.  As many heads as have their keys and values
 // in kFaGroupBytes, so that the walks of a group still meet them in L2.
 constexpr long long kFaGroupBytes = 64ll << 20;
 static int fa_head_group(int T, int Hq, int Hk, int d, int dv) {
@@ -378,8 +378,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
       // P = exp2(s*scale - m_used) -> bf16 -> swizzled smem, 8 columns (one 16-byte chunk) at a time.  The softmax warps are bound
       // by the instructions they issue, so everything but ex2 and the conversion works on pairs (or takes three operands): 4096
-      // tokens, 32 heads 198 -> 187 us, 8192 tokens 612 -> 574.  (Exponentials on the FMA pipe, exact to fp32, cost more
-      // instructions than they take off the special-function pipe: a quarter of them 198, half 208, three quarters 238.)
+      // tokens, 32 heads 198 -> 189 us, 8192 tokens 612 -> 580.  (Exponentials on the FMA pipe, exact to fp32, cost more
+      // instructions than they take off the special-function pipe: with a quarter of them there 187 -> 198, half 208, three
+      // quarters 238.)
       float2 ps0 = make_float2(0.f, 0.f), ps1 = ps0;
       const float2 scale2 = make_float2(scale_log2, scale_log2), neg_m = make_float2(-m_used, -m_used);
 #pragma unroll
