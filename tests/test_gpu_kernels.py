@@ -334,7 +334,7 @@ def test_embedding_gradient_repeats_itself(cu, tokens, rows, cols):
     torch.manual_seed(tokens)
     w = torch.nn.Parameter(torch.randn(rows, cols, device="cuda", dtype=torch.bfloat16))
     ids = torch.randint(0, rows, (tokens,), device="cuda")
-    ids[tokens // 2:] = ids[0]
+    ids[tokens // 2:] = int(ids[0])
     dy = torch.randn(tokens, cols, device="cuda", dtype=torch.bfloat16)
     before = torch.randn(rows, cols, device="cuda")
     got = []
