@@ -571,8 +571,8 @@ attn_latent_kernel(const __grid_constant__ CUtensorMap tmK, const AttnRowsArgs a
 
 // ---- bf16 rows over cached keys on mma.sync ------------------------------------------------------------
 // Decoding reads every cached key and value once for a few query rows: bound by those bytes, if the arithmetic keeps up.
-// On the FMA pipe it did not (230 us for 64 rows x 2048 keys x 8 key heads, 537 MB, which take 81; 134 here); and a continued prompt read its whole
-// context once per token (1060 us for 301 tokens over 3000, 50 here).  Here a tile of 16 rows is the consecutive tokens of one
+// On the FMA pipe it did not (230 us for 64 rows x 2048 keys x 8 key heads, 537 MB, which take 83; 115 here); and a continued prompt
+// read its whole context once per token (1060 us for 301 tokens of two sequences over 3000, 115 here).  Here a tile of 16 rows is the consecutive tokens of one
 // sequence times the query heads of one key head, and m16n8k16 does the products:
 //   scores  exact bf16 products, fp32 sums, scale and bias applied in fp32
 //   values  the fp32 weights go in as three bf16 parts, so they keep their 24 bits.  With two parts, in turn for one accumulator at
@@ -1135,10 +1135,10 @@ struct AtPlan {
 };
 // Ranges of decoding rows: the CTAs come in rounds of two an SM, and the last round takes as long as a full one, so the number of
 // ranges decides how much of it is idle.  A round reads its keys at 5 TB/s and costs 3 us besides, a merge 3.  Measured (us; 32 query
-// heads on 8 key heads, ranges 1 / 2 / 3 / 4): 48 sequences of 2048 keys 130 / 104 / 100 / 105, 64 of them 132 / 138 / 137 / 134, 24 of
-// 3000 95 / 91 / 78 / 79; 10 sequences with 32 key heads 128 / 99 / 91 / 88.  A CTA an SM and fewer go in about one round: the last
-// range, which ends before the bound of the lengths, may be a few CTAs over it (4 sequences of 3000, 16 key heads: 4 ranges 33, 5 ranges
-// 29; 8 of 4096, 8 key heads: 41 and 41).
+// heads on 8 key heads, ranges 1 / 2 / 3 / 4): 48 sequences of 2048 keys 111 / 94 / 90 / 99, 64 of them 114 / 122 / 125 / 122, 24 of
+// 3000 82 / 88 / 66 / 74; 10 sequences of 2048 with 32 key heads 105 / 88 / 83 / 83.  A CTA an SM and fewer go in about one round: the
+// last range, which ends before the bound of the lengths, may be a few CTAs over it.  (That pays where the lengths stay below the
+// bound; with all rows at it, 4 sequences of 3000 with 16 key heads take 28 in 4 ranges and 33 in 5, 8 of 4096 with 8 take 37 and 51.)
 static int at_ranges(long long ctas, long long most, double bytes_of_cta) {
   if (ctas <= kNumSMs) return (int)((2LL * kNumSMs + ctas / 2) / ctas < most ? (2LL * kNumSMs + ctas / 2) / ctas : most);
   const double whole = bytes_of_cta * 2 * kNumSMs / 5e6;

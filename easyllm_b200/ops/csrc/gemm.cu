@@ -95,7 +95,10 @@ struct GemmCfg {
 // Up to one row tile of A: the first kAheadBlocks k-blocks of B go into L2 ahead of the wait (39 MB over the SMs).
 constexpr int kAheadRows = 128, kAheadBlocks = 8;
 // Rows up to which a launch starts while the kernel before it ends.  With many, nothing is gained, and the CTAs come in where the
-// kernel before left room first: 16 experts of 4096 x 2752, rows of 4096 tokens, 593 us chained and 562 not; of 128 tokens 217 and 221.
+// kernel before left room first.  Us chained | not, feed-forward layers of 16 experts, two a token (a grouped product has the rows of
+// its slots and of up to 128 more an expert): 4096 x 2752, 64 tokens 218 | 221, 1024 256 | 262, 2048 361 | 368, 3072 496 | 480, 4096
+// 593 | 570; 2048 x 1408, 64 tokens 77 | 81, 1024 87 | 92, 2048 114 | 120, 3072 150 | 157, 4096 177 | 177.  A norm and a product, 300
+// to 2000 rows of 2048 x 2048 22 | 23, of 4096 x 11264 41 to 142 | 40 to 143.
 constexpr int kChainedRows = 4096;
 
 struct GemmShared {

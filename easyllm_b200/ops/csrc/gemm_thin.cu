@@ -76,6 +76,11 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 __device__ __forceinline__ void set_in_peer(uint32_t addr, int v) {
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
+// The whole cluster stops waiting: a CTA that gave up may still be sent to, and its copies may still be on their way.
+__device__ __forceinline__ void give_up(ThinShared* sh, int split) {
+  sh->abort_flag = 1;
+  for (int r = 0; r < split && split > 1; ++r) set_in_peer(map_to_rank(smem_u32(&sh->abort_flag), r), 1);
+}
 
 // Barrier of the epilogue that tells every thread whether any of them failed.
 __device__ __forceinline__ bool epi_any(bool failed) {
@@ -223,7 +228,7 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         }
       }
       if (!ok) {
-        sh->abort_flag = 1;
+        give_up(sh, split);
         atomicCAS(a.err, 0, kErrProducer);
       }
     }
@@ -261,7 +266,7 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         if (ok) umma_commit(&sh->tmem_full[acc]);
       }
       if (!ok) {
-        sh->abort_flag = 1;
+        give_up(sh, split);
         atomicCAS(a.err, 0, kErrMma);
       }
     }
@@ -338,7 +343,7 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         }
         if (!mbar_wait_cluster(&sh->recv_full, ex & 1, abort_flag, a.limit_ns)) {
           failed = true;
-          sh->abort_flag = 1;
+          give_up(sh, split);
         } else if (n < a.N) {
           const int tc = t0 + c0 + rank * cols;
           const float *mine = send + (size_t)rank * cols * kThRows + row, *theirs = recv + row;
@@ -352,25 +357,21 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       }
     }
     if (failed) {
-      sh->abort_flag = 1;
+      give_up(sh, split);
       atomicCAS(a.err, 0, kErrEpilogue);
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  if (split > 1) {
-    // a CTA that gave up may still be sent to, and its copies may still be on their way: all of the cluster wait for them
-    if (*abort_flag && threadIdx.x < split) set_in_peer(map_to_rank(smem_u32(&sh->abort_flag), threadIdx.x), 1);
-    cluster_sync_all();                              // no CTA starts a copy any more
-  }
-  if (*abort_flag && threadIdx.x == 0) {
+  if (split > 1) cluster_sync_all();                 // no CTA starts a copy any more
+  if (*abort_flag) {                                 // the same in the whole CTA behind either barrier
     // error path: give copies and MMAs in flight time to land before shared memory and TMEM go away
     const unsigned long long t0 = globaltimer_ns();
-    while (globaltimer_ns() - t0 < 200000ull) {
+    while (threadIdx.x == 0 && globaltimer_ns() - t0 < 200000ull) {
     }
+    __syncthreads();
   }
-  __syncthreads();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc<Cfg::kTmemCols>(tmem_base);

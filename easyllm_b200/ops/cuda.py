@@ -309,14 +309,23 @@ def embedding_bwd_(ids, dout, grad32, vocab_start):
     _check(rc, "embedding_bwd")
 
 
+ORDERED_TOKENS = 1 << 17    # whose ids are marked at a time (4 MB of marks for 32000 rows); longer batches go in pieces, in order
+
+
 def embedding_bwd_ordered_(ids, dout, grad32):
     """``grad32[id] += `` the sum of the rows ``dout[t]`` of every id, in the order of the tokens."""
-    ids, order = torch.sort(ids.reshape(-1).to(torch.int64), stable=True)
+    ids = ids.reshape(-1).to(torch.int64).contiguous()
     d = dout.reshape(ids.numel(), -1)
     _bf16c(d, "dout")
-    rc = lib().ell_embedding_bwd_runs(_p(ids), _p(order), _p(d), _p(grad32), c_int(ids.numel()), c_int(d.shape[1]),
-                                      c_longlong(grad32.shape[0]), _stream())
-    _check(rc, "embedding_bwd_runs")
+    global LAUNCHES
+    for a in range(0, ids.numel(), ORDERED_TOKENS):
+        part, rows = ids[a:a + ORDERED_TOKENS], d[a:a + ORDERED_TOKENS]
+        words = lib().ell_embedding_bwd_words(c_int(part.numel()))
+        seen = torch.empty(grad32.shape[0] * words, dtype=torch.int32, device=ids.device)
+        rc = lib().ell_embedding_bwd_ordered(_p(part), _p(seen), _p(rows), _p(grad32), c_int(part.numel()), c_int(d.shape[1]),
+                                             c_longlong(grad32.shape[0]), _stream())
+        _check(rc, "embedding_bwd_ordered")
+        LAUNCHES += 1                          # marking the ids is a launch of its own
 
 
 # ---- cross entropy ----------------------------------------------------------------------------

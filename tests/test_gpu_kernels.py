@@ -327,10 +327,13 @@ def test_embedding_gradient_goes_to_main_grad(cu, tokens, rows, cols, dtype, det
     assert ((emb.weight.main_grad.double() - want).abs() <= size * (tokens + 1) * 2.0 ** -24).all()
 
 
-@pytest.mark.parametrize("tokens,rows,cols", [(1, 3, 8), (2000, 7, 1032), (4096, 300, 2048)])
-def test_embedding_gradient_repeats_itself(cu, tokens, rows, cols):
-    """Ids that come hundreds of times: the same bits every time, those of the sum in the order of the tokens in fp32."""
+@pytest.mark.parametrize("tokens,rows,cols", [(1, 3, 8), (128, 200, 64), (129, 2, 64), (2000, 7, 1032), (4096, 300, 2048), (9000, 40, 64), (9000, 3000, 64)])
+def test_embedding_gradient_repeats_itself(cu, tokens, rows, cols, monkeypatch):
+    """Ids that come once and hundreds of times, within a block of tokens and over many, in one piece (up to 9000 tokens, three
+    words of marks) and in several: the same bits every time, those of the sum in the order of the tokens in fp32."""
     from easyllm_b200 import ops
+    if rows == 40:
+        monkeypatch.setattr(cu, "ORDERED_TOKENS", 4200)
     torch.manual_seed(tokens)
     w = torch.nn.Parameter(torch.randn(rows, cols, device="cuda", dtype=torch.bfloat16))
     ids = torch.randint(0, rows, (tokens,), device="cuda")
@@ -344,10 +347,14 @@ def test_embedding_gradient_repeats_itself(cu, tokens, rows, cols):
         got.append(w.main_grad)
     assert w.grad is None and all(torch.equal(got[0], g) for g in got[1:])
     for i in {int(ids[0]), int(ids[tokens // 3])}:
-        want = torch.zeros(cols, device="cuda")
-        for t in (ids == i).nonzero().flatten().tolist():
-            want += dy[t].float()
-        assert torch.equal(got[0][i], before[i] + want)
+        want = before[i].clone()
+        for first in range(0, tokens, cu.ORDERED_TOKENS):
+            rows_of = (ids[first:first + cu.ORDERED_TOKENS] == i).nonzero().flatten() + first
+            total = torch.zeros(cols, device="cuda")
+            for t in rows_of.tolist():
+                total += dy[t].float()
+            want += total
+        assert torch.equal(got[0][i], want)
 
 
 def test_embedding_gradient_that_somebody_looks_at(cu):
