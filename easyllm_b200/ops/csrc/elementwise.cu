@@ -264,7 +264,8 @@ __global__ void embedding_bwd_kernel(const long long* __restrict__ ids, const __
 }
 
 // The same with a fixed order of the sums.  Tokens come in blocks of kIdBlock; seen[id] has a bit for every block that holds the id.
-constexpr int kIdBlock = 128, kIdWarps = kIdBlock / 32;
+// Up to kUnmarkedIds tokens are looked through whole instead: a small batch is bound by the host, and marking is two launches more.
+constexpr int kIdBlock = 128, kIdWarps = kIdBlock / 32, kUnmarkedIds = 1024;
 __global__ void embedding_mark_kernel(const long long* __restrict__ ids, uint32_t* __restrict__ seen, int T, int words, long long rows) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= T || ids[t] < 0 || ids[t] >= rows) return;
@@ -283,14 +284,22 @@ __global__ void __launch_bounds__(kIdBlock) embedding_bwd_ordered_kernel(const l
   const int t = blockIdx.x, own = t / kIdBlock, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long id = ids[t];
   if (id < 0 || id >= rows) return;
-  const uint32_t* blocks = seen + id * words;
+  const uint32_t* blocks = seen != nullptr ? seen + id * words : nullptr;
   int word = own / 32;
-  uint32_t left = blocks[word];                        // blocks still to look through
-  for (int w = 0; w < word; ++w)
-    if (blocks[w] != 0) return;
-  if (left & ((1u << (own & 31)) - 1)) return;
-  const int at = own * kIdBlock + threadIdx.x;
-  if (__syncthreads_or(at < t && ids[at] == id)) return;
+  uint32_t left;                                       // blocks still to look through
+  bool earlier = false;
+  if (blocks != nullptr) {
+    left = blocks[word];
+    for (int w = 0; w < word; ++w)
+      if (blocks[w] != 0) return;
+    if (left & ((1u << (own & 31)) - 1)) return;
+    const int at = own * kIdBlock + threadIdx.x;
+    earlier = at < t && ids[at] == id;
+  } else {
+    left = (1u << (T + kIdBlock - 1) / kIdBlock) - (1u << own);
+    for (int i = threadIdx.x; i < t; i += kIdBlock) earlier |= ids[i] == id;
+  }
+  if (__syncthreads_or(earlier)) return;
   const int c = (blockIdx.y * kIdBlock + threadIdx.x) * 8;
   const __nv_bfloat16* src = dout + c;
   float acc[8];
@@ -379,8 +388,10 @@ ELL_API int ell_embedding_bwd(const long long* ids, const void* dout, float* gra
   return ell::launch_status();
 }
 
-// 32-bit words of work space a table row takes.
-ELL_API int ell_embedding_bwd_words(int T) { return (T + 32 * ell::kIdBlock - 1) / (32 * ell::kIdBlock); }
+// 32-bit words of work space a table row takes (0: none is needed).
+ELL_API int ell_embedding_bwd_words(int T) {
+  return T <= ell::kUnmarkedIds ? 0 : (T + 32 * ell::kIdBlock - 1) / (32 * ell::kIdBlock);
+}
 
 // seen: rows * ell_embedding_bwd_words(T) words of work space.
 ELL_API int ell_embedding_bwd_ordered(const long long* ids, void* seen, const void* dout, float* grad32, int T, int cols, long long rows,
@@ -389,11 +400,13 @@ ELL_API int ell_embedding_bwd_ordered(const long long* ids, void* seen, const vo
   if (cols % 8) return -1;
   const int per = 8 * ell::kIdBlock, words = ell_embedding_bwd_words(T);
   if (cols > 65535 * per) return -2;
-  const cudaError_t e = cudaMemsetAsync(seen, 0, (size_t)rows * words * 4, stream);
-  if (e != cudaSuccess) return (int)e;
-  ell::embedding_mark_kernel<<<(T + 255) / 256, 256, 0, stream>>>(ids, (uint32_t*)seen, T, words, rows);
+  if (words > 0) {
+    const cudaError_t e = cudaMemsetAsync(seen, 0, (size_t)rows * words * 4, stream);
+    if (e != cudaSuccess) return (int)e;
+    ell::embedding_mark_kernel<<<(T + 255) / 256, 256, 0, stream>>>(ids, (uint32_t*)seen, T, words, rows);
+  }
   ell::embedding_bwd_ordered_kernel<<<dim3(T, (cols + per - 1) / per), ell::kIdBlock, 0, stream>>>(
-      ids, (const uint32_t*)seen, (const __nv_bfloat16*)dout, grad32, T, words, cols, rows);
+      ids, words > 0 ? (const uint32_t*)seen : nullptr, (const __nv_bfloat16*)dout, grad32, T, words, cols, rows);
   return ell::launch_status();
 }
 

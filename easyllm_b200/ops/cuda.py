@@ -318,14 +318,15 @@ def embedding_bwd_ordered_(ids, dout, grad32):
     d = dout.reshape(ids.numel(), -1)
     _bf16c(d, "dout")
     global LAUNCHES
+    whole = ids.numel() <= ORDERED_TOKENS
     for a in range(0, ids.numel(), ORDERED_TOKENS):
-        part, rows = ids[a:a + ORDERED_TOKENS], d[a:a + ORDERED_TOKENS]
+        part, rows = (ids, d) if whole else (ids[a:a + ORDERED_TOKENS], d[a:a + ORDERED_TOKENS])
         words = lib().ell_embedding_bwd_words(c_int(part.numel()))
-        seen = torch.empty(grad32.shape[0] * words, dtype=torch.int32, device=ids.device)
+        seen = torch.empty(grad32.shape[0] * words, dtype=torch.int32, device=ids.device) if words else None
         rc = lib().ell_embedding_bwd_ordered(_p(part), _p(seen), _p(rows), _p(grad32), c_int(part.numel()), c_int(d.shape[1]),
                                              c_longlong(grad32.shape[0]), _stream())
         _check(rc, "embedding_bwd_ordered")
-        LAUNCHES += 1                          # marking the ids is a launch of its own
+        LAUNCHES += bool(words)                # marking the ids is a launch of its own
 
 
 # ---- cross entropy ----------------------------------------------------------------------------

@@ -327,7 +327,7 @@ def test_embedding_gradient_goes_to_main_grad(cu, tokens, rows, cols, dtype, det
     assert ((emb.weight.main_grad.double() - want).abs() <= size * (tokens + 1) * 2.0 ** -24).all()
 
 
-@pytest.mark.parametrize("tokens,rows,cols", [(1, 3, 8), (128, 200, 64), (129, 2, 64), (2000, 7, 1032), (4096, 300, 2048), (9000, 40, 64), (9000, 3000, 64)])
+@pytest.mark.parametrize("tokens,rows,cols", [(1, 3, 8), (128, 200, 64), (129, 2, 64), (1024, 9, 64), (1025, 9, 64), (2000, 7, 1032), (4096, 300, 2048), (9000, 40, 64), (9000, 3000, 64)])
 def test_embedding_gradient_repeats_itself(cu, tokens, rows, cols, monkeypatch):
     """Ids that come once and hundreds of times, within a block of tokens and over many, in one piece (up to 9000 tokens, three
     words of marks) and in several: the same bits every time, those of the sum in the order of the tokens in fp32."""
