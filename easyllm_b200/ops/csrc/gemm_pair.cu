@@ -54,17 +54,23 @@ constexpr int kTmemCols = 2 * kTileN;       // two accumulator buffers
 constexpr int kSmemBytes = kStages * kStageBytes + 2 * kEpiBufBytes + 1024 + 512;
 constexpr int kGroupM = 8;                  // rasterisation: 8 M-tiles x all N-tiles per group
 enum GluAct { kGluSilu = 1, kGluGelu = 2 };
-// e^x to some 2^-22 of itself for every x.  This file is built with --use_fast_math, whose expf rounds x log2(e) to one float, an
-// error that grows with x (2^-18 at 60); here the product keeps its remainder.
-__device__ __forceinline__ float exp_whole(float x) {
-  x = fminf(fmaxf(x, -200.f), 200.f);                // 0 and infinity, before the remainder is not a number
-  const float t = __fmul_rn(x, 1.44269502f);         // log2(e) = 1.44269502 + 1.9259630e-8
-  const float rest = fmaf(x, 1.9259630e-8f, fmaf(x, 1.44269502f, -t));
-  return ex2_approx(t) * fmaf(0.69314718f, rest, 1.f);
+// e^x to some 2^-22 of itself for every x, of a pair at a time.  This file is built with --use_fast_math, whose expf rounds x log2(e)
+// to one float, an error that grows with x (2^-18 at 60); here the product keeps its remainder.
+__device__ __forceinline__ float2 exp_whole(float2 x) {
+  x.x = fminf(fmaxf(x.x, -200.f), 200.f);            // 0 and infinity, before the remainder is not a number
+  x.y = fminf(fmaxf(x.y, -200.f), 200.f);
+  const float2 log2e = make_float2(1.44269502f, 1.44269502f), log2e_rest = make_float2(1.9259630e-8f, 1.9259630e-8f);
+  const float2 t = ffma2(x, log2e, make_float2(-0.f, -0.f));
+  const float2 rest = ffma2(x, log2e_rest, ffma2(x, log2e, make_float2(-t.x, -t.y)));
+  const float2 f = ffma2(rest, make_float2(0.69314718f, 0.69314718f), make_float2(1.f, 1.f));
+  return make_float2(ex2_approx(t.x) * f.x, ex2_approx(t.y) * f.y);
 }
 // The forms of vec.cuh: z sigmoid(z), and 0.5 (1 + tanh(u)) = sigmoid(2 u)
-__device__ __forceinline__ float glu_act(float z, int act) {
-  return __fdividef(z, 1.f + exp_whole(act == kGluGelu ? -1.5957691216057308f * (z + 0.044715f * z * z * z) : -z));
+__device__ __forceinline__ float2 glu_act(float2 z, int act) {
+  const float2 e = exp_whole(act == kGluGelu ? make_float2(-1.5957691216057308f * (z.x + 0.044715f * z.x * z.x * z.x),
+                                                           -1.5957691216057308f * (z.y + 0.044715f * z.y * z.y * z.y))
+                                             : make_float2(-z.x, -z.y));
+  return make_float2(__fdividef(z.x, 1.f + e.x), __fdividef(z.y, 1.f + e.y));
 }
 enum Err { kErrPairProducer = 11, kErrPairMma = 12, kErrPairEpilogue = 13, kErrPairFlagWait = 15 };
 
@@ -715,16 +721,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             tmem_ld_wait();
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-              float v[8];
+              float v[8], gate[8];
 #pragma unroll
               for (int e = 0; e < 8; ++e) {
-                float gate = __uint_as_float(r[c * 8 + e]), up = __uint_as_float(r[32 + c * 8 + e]);
+                gate[e] = __uint_as_float(r[c * 8 + e]);
+                v[e] = __uint_as_float(r[32 + c * 8 + e]);
                 if (HAS_BIAS) {
                   const int at = col + c * 8 + e;
-                  gate += at < F ? __bfloat162float(bias[at]) : 0.f;
-                  up += at < F ? __bfloat162float(bias[F + at]) : 0.f;
+                  gate[e] += at < F ? __bfloat162float(bias[at]) : 0.f;
+                  v[e] += at < F ? __bfloat162float(bias[F + at]) : 0.f;
                 }
-                v[e] = up * glu_act(gate, fuse.group_glu);
+              }
+#pragma unroll
+              for (int e = 0; e < 8; e += 2) {
+                const float2 a = glu_act(make_float2(gate[e], gate[e + 1]), fuse.group_glu);
+                v[e] *= a.x;
+                v[e + 1] *= a.y;
               }
               *reinterpret_cast<bf16x8*>(row_ptr + (((p * 4 + c) ^ (row_in_tile & 7)) << 4)) = pack8(v);  // 128B swizzle
             }
