@@ -43,7 +43,11 @@ def fallbacks():
     return dict(_FALLBACKS)
 
 
-_TLS = threading.local()
+class _PerThread(threading.local):
+    serving = False
+
+
+_TLS = _PerThread()
 
 
 class serving:
@@ -55,7 +59,7 @@ class serving:
         self.on = bool(on)
 
     def __enter__(self):
-        self.before = is_serving()
+        self.before = _TLS.serving
         _TLS.serving = self.before or self.on
 
     def __exit__(self, *_):
@@ -63,7 +67,7 @@ class serving:
 
 
 def is_serving():
-    return getattr(_TLS, "serving", False)
+    return _TLS.serving
 
 
 def note_fallback(op, t, reason):
@@ -344,7 +348,7 @@ class _Linear(torch.autograd.Function):
 def linear(x, w, bias=None):
     if _kern(x):
         x2 = x.reshape(-1, x.shape[-1]).contiguous()
-        y = matmul_nt(x2, w, bias, few_rows=is_serving()) if _cu().nothing_to_record() else _Linear.apply(x2, w, bias)
+        y = matmul_nt(x2, w, bias, few_rows=_TLS.serving) if _cu().nothing_to_record() else _Linear.apply(x2, w, bias)
         return y if x.dim() == 2 else y.view(*x.shape[:-1], w.shape[0])
     return F.linear(x, w, bias)
 
@@ -414,7 +418,7 @@ def linear_parts(x, weights, biases=None):
         bias = torch.cat(list(biases), 0)
     if _kern(x):
         x2 = x.reshape(-1, x.shape[-1]).contiguous()
-        y = matmul_nt(x2, _LinearParts.fused(weights), bias, few_rows=is_serving()) if _cu().nothing_to_record() else \
+        y = matmul_nt(x2, _LinearParts.fused(weights), bias, few_rows=_TLS.serving) if _cu().nothing_to_record() else \
             _LinearParts.apply(x2, bias, *weights)
         return y if x.dim() == 2 else y.view(*x.shape[:-1], y.shape[-1])
     return F.linear(x, torch.cat(list(weights), 0), bias)
@@ -581,7 +585,7 @@ def glu(gate_up, activation="silu"):
 def glu_linear(x, gate, up):
     """``silu(x Wgᵀ) * (x Wuᵀ)``: one launch in a ``serving`` step whose rows fill CTA pairs, if the weights lie next to each other;
     otherwise ``glu`` of ``linear_parts``, which rounds the 2 F columns in between."""
-    if is_serving() and _kern(x) and x.dim() == 2 and _GEMM == "tcgen05" and gate.shape == up.shape and _cu().nothing_to_record() and \
+    if _TLS.serving and _kern(x) and x.dim() == 2 and _GEMM == "tcgen05" and gate.shape == up.shape and _cu().nothing_to_record() and \
             _cu().glu_route(x.shape[0], gate.shape[0]):
         w = _adjacent_alias([gate.detach(), up.detach()])
         y = None if w is None else _cu().gemm_glu(x, w, None, "silu")

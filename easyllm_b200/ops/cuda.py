@@ -391,6 +391,9 @@ def matvec(x, ldx, w, bias, out, ldo, out_f32=False, accumulate=False, act_tanh=
     return out
 
 
+_NO_TEST_OF_WAITS = (c_int(0), c_int(-1))     # the usual limit of the waits, no CTA that withholds its sums
+
+
 def gemm_thin(x, w, out, bias=None, ldx=None, ldw=None, ldo=None, w_mn=False, out_mode=0, split=0):
     """``out [T, N] (+)= x [T, K] Wᵀ (+ bias)`` for few rows of ``x``; ``w [N, K]``, or ``[K, N]`` with ``w_mn``.  ``split``:
     CTAs that share a reduction (0: chosen from the sizes)."""
@@ -398,7 +401,7 @@ def gemm_thin(x, w, out, bias=None, ldx=None, ldw=None, ldo=None, w_mn=False, ou
     N = w.shape[1] if w_mn else w.shape[0]
     rc = lib().ell_gemm_thin(_p(x), _p(w), _p(out), _p(bias), c_int(T), c_int(N), c_int(K), c_int(ldx or x.shape[1]),
                              c_int(ldw or w.shape[1]), c_int(ldo or N), c_int(w_mn), c_int(out_mode), c_int(split),
-                             c_int(0), c_int(-1), _p(err_flag(x.device)), _stream())
+                             *_NO_TEST_OF_WAITS, _p(err_flag(x.device)), _stream())
     _check(rc, "gemm_thin")
     return out
 

@@ -227,7 +227,7 @@ def attention_rows(q, k, v, base, length, max_len, scale, sink=None, alibi_slope
                    max_q=None):
     T, H, d = q.shape
     G, dv = k.shape[1], v.shape[2]
-    if cu_seqlens is not None:
+    if cu_seqlens is not None and (cu_seqlens.dtype != torch.int32 or not cu_seqlens.is_contiguous()):
         cu_seqlens = cu_seqlens.to(torch.int32).contiguous()
     n_seq, max_q = (0, 1) if cu_seqlens is None else (cu_seqlens.numel() - 1, max_q)
     out = torch.empty(T, H, dv, dtype=q.dtype, device=q.device)
