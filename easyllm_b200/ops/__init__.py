@@ -501,7 +501,7 @@ def _embedding_main_grad(w):
 def token_embedding(ids, weight):
     """``F.embedding(ids, weight)``.  With an fp32 ``main_grad`` the gradient rows are added to it as they are: autograd's dense
     bf16 gradient costs a pass over the whole table to clear, one to fill and one to add, 700 us for 32000 x 4096 where the
-    4096 rows of a batch take 60.  The rows of one id are added up in the order of the tokens, so a step repeats itself bit for bit.
+    4096 rows of a batch take 75 to 100.  The rows of one id are added up in the order of the tokens, so a step repeats itself bit for bit.
     ``weight.grad`` stays None then, as for the other weights with a ``main_grad``; where hooks on the weight or
     ``torch.autograd.grad`` look at its gradient, and in programs that ask for deterministic algorithms, it is autograd's dense
     one."""
