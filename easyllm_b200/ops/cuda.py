@@ -490,6 +490,14 @@ def flash_fwd_plan(row_start):
     return [tuple(out[3 * i:3 * i + 3]) for i in range(2 * n_pairs)]
 
 
+def flash_fwd_skipped(row_start, window=None, kn=128):
+    """Host-only: per tile pair, the key tiles of ``kn`` keys that the second query tile leaves out at the start of its walk."""
+    rs = [int(x) for x in row_start]
+    out = (c_int * ((len(rs) + 255) // 256))()
+    lib().ell_flash_fwd_skipped((c_int * len(rs))(*rs), c_int(len(rs)), c_int(window or 0), c_int(kn), out)
+    return list(out)
+
+
 def gemm_work_units(M, N, bn=256, fuse=0, tp=1, rank=0, ctas=148, allow_split=True):
     """Host-only: the (row tile, column tile, first column, width) work units of a single-CTA GEMM launch in the
     order the kernel walks them, produced by the kernel's own tile-order code (no GPU is touched).

@@ -103,6 +103,38 @@ def test_flash_bwd_packed(cu, T, Hq, Hk, cu_list):
         assert err < tol, (name, err, tol)
 
 
+def _exact(q, k, v, rs, scale, window, sink):
+    T, H, i = q.shape[0], q.shape[1], torch.arange(q.shape[0], device=q.device)
+    k, v = (t.repeat_interleave(H // k.shape[1], 1) for t in (k, v))
+    seen = (i.view(1, -1) <= i.view(-1, 1)) & (i.view(1, -1) >= rs.view(-1, 1)) & (i.view(1, -1) > i.view(-1, 1) - (window or T))
+    s = (torch.einsum("qhd,khd->hqk", q, k) * scale).masked_fill(~seen, float("-inf"))
+    if sink is not None:
+        s = torch.cat((s, sink.double().view(-1, 1, 1).expand(-1, T, 1)), 2)
+    return torch.einsum("hqk,khd->qhd", torch.softmax(s, -1)[..., :T], v)
+
+
+@pytest.mark.parametrize("lens,Hq,Hk,d,dv,window", [
+    ([1], 1, 1, 128, 128, None), ([129], 3, 1, 128, 128, None), ([256, 1], 2, 2, 64, 128, None), ([90, 38, 500], 2, 1, 128, 72, None),
+    ([300, 212, 1, 255], 150, 75, 64, 64, None), ([5] * 200, 3, 3, 40, 128, None), ([900], 2, 2, 128, 128, 70), ([1200, 30], 40, 8, 128, 128, 300)])
+def test_attention_items_and_tiles(cu, lens, Hq, Hk, d, dv, window):
+    """Borders of query tiles, second tiles without rows or with documents of their own, more items than CTAs, head sizes that
+    fill no chunk.  Against 64 bits: scores are exact to fp32, P (2^-9) and the result (2^-9) are rounded to bf16 once each, so
+    the relative error stays below 2 * 2^-9 / sqrt(3) where the roundings are independent, and below 2^-8 in any case."""
+    torch.manual_seed(len(lens) + Hq)
+    T = sum(lens)
+    qkv = torch.randn(T, Hq * d + Hk * (d + dv), device="cuda", dtype=torch.bfloat16)
+    q, k, v = qkv[:, :Hq * d].view(T, Hq, d), qkv[:, Hq * d:(Hq + Hk) * d].view(T, Hk, d), qkv[:, (Hq + Hk) * d:].view(T, Hk, dv)
+    if qkv.stride(0) % 8:
+        pytest.skip("rows of the packed buffer are not 16-byte aligned")
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    rs = torch.tensor([s for s, n in zip(starts, lens) for _ in range(n)], dtype=torch.int32, device="cuda")
+    sink = torch.randn(Hq, device="cuda")
+    out = cu.flash_attn_fwd(q, k, v, rs, d ** -0.5, sink=sink, window=window)[0]
+    cu.check_err_flag()
+    want = _exact(q.double(), k.double(), v.double(), rs, d ** -0.5, window, sink)
+    assert ((out.double() - want).norm() / want.norm()).item() < 2.0 ** -8
+
+
 def test_flash_packed_autograd_matches_library(cu):
     from easyllm_b200 import ops
     torch.manual_seed(3)

@@ -205,6 +205,22 @@ def test_attention_forward_plan_covers_visible_keys_and_skips_masks_only_when_sa
             assert all(rs[i] <= k0 and k0 + 127 <= i for i in rows), (idx, j)
 
 
+@pytest.mark.parametrize("kn", [64, 128])
+@pytest.mark.parametrize("T,docs,window", [(512, [512], None), (700, [100, 28, 572], 130), (777, [255, 2, 520], None), (640, [300, 340], 60),
+                                           (2048, [5] * 409 + [3], None), (1536, [100, 1436], 1), (129, [129], None), (100, [100], 7)])
+def test_attention_forward_leaves_out_only_key_tiles_that_the_second_query_tile_does_not_see(cu, T, docs, window, kn):
+    rs = _row_starts(T, docs)
+    first_key = [max(s, i - (window or T) + 1) for i, s in enumerate(rs)]
+    skipped = cu.flash_fwd_skipped(rs, window, kn)
+    assert len(skipped) == (T + 255) // 256
+    for p, skip in enumerate(skipped):
+        kv_lo, rows = first_key[256 * p], range(256 * p + 128, min(256 * p + 256, T))
+        seen = [i for i in rows if first_key[i] < kv_lo + skip * kn]
+        assert not seen and skip >= 0
+        if rows:                                    # no whole tile that could be left out is walked, and one at least is
+            assert first_key[rows[0]] < kv_lo + (skip + 1) * kn and kv_lo + skip * kn <= rows[-1]
+
+
 @pytest.mark.parametrize("tp", [2, 4, 8])
 @pytest.mark.parametrize("M,N,resident", [(4096, 4096, 74), (2048, 1024, 74), (8192, 2048, 70), (4096, 8192, 37)])
 def test_reduce_scatter_schedule_cannot_deadlock_across_ranks(cu, tp, M, N, resident):
