@@ -666,16 +666,15 @@ def flash_attn_bwd(do, q, k, v, out, lse, row_start, scale, dq=None, dk=None, dv
         dv = torch.empty(T, Hk, D, dtype=torch.bfloat16, device=q.device)
     if dk.stride(0) != dv.stride(0):
         raise ValueError("flash_attn_bwd: dk and dv must share a row stride")
-    acc = scratch(T * Hq * D, tag="fa_bwd_dq")
     delta = scratch(T * Hq, tag="fa_bwd_delta")
     kv_acc = scratch(2 * T * Hk * D, tag="fa_bwd_dkv") if Hq > Hk else None
     rc = lib().ell_flash_attn_bwd(_p(q), _p(k), _p(v), _p(out), _p(do), _p(lse), _p(row_start), _p(dq), _p(dk), _p(dv),
-                                  _p(acc), _p(delta), _p(kv_acc), c_int(T), c_int(Hq), c_int(Hk), c_int(q.stride(0)),
+                                  _p(delta), _p(kv_acc), c_int(T), c_int(Hq), c_int(Hk), c_int(q.stride(0)),
                                   c_int(k.stride(0)), c_int(dq.stride(0)), c_int(dk.stride(0)), c_float(scale),
                                   _p(_slopes(alibi_slopes, Hq, q.device)), _p(err_flag(q.device)), _stream())
     _check(rc, "flash_attn_bwd")
     global LAUNCHES
-    LAUNCHES += 3  # memset, delta and dq-convert launches beside the main kernel
+    LAUNCHES += 2  # row sums, keys, queries
     return dq, dk, dv
 
 

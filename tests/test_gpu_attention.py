@@ -135,6 +135,29 @@ def test_attention_items_and_tiles(cu, lens, Hq, Hk, d, dv, window):
     assert ((out.double() - want).norm() / want.norm()).item() < 2.0 ** -8
 
 
+@pytest.mark.parametrize("lens,Hq,Hk", [([1], 1, 1), ([127, 2], 2, 1), ([128, 128], 2, 2), ([33] * 20, 4, 2), ([300, 1, 84], 30, 30),
+                                        ([500, 700], 16, 1)])
+def test_attention_backward_against_64_bits(cu, lens, Hq, Hk):
+    """Keys that end their document inside a query tile, items beyond the CTAs, query heads split over CTAs.  Each of dq, dk, dv takes
+    two values rounded to bf16 into every product (P or dS, after P was rounded) and is rounded itself: at most 4 * 2^-9 / sqrt(3),
+    with twice that for sums that cancel."""
+    torch.manual_seed(len(lens) + Hq)
+    T, scale = sum(lens), 128 ** -0.5
+    qkv = torch.randn(T, (Hq + 2 * Hk) * 128, device="cuda", dtype=torch.bfloat16)
+    q, k, v = cu._split_packed(qkv, Hq, Hk, 128)
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    rs = torch.tensor([s for s, n in zip(starts, lens) for _ in range(n)], dtype=torch.int32, device="cuda")
+    out, lse = cu.flash_attn_fwd(q, k, v, rs, scale)
+    do = torch.randn_like(out)
+    grads = cu.flash_attn_bwd(do, q, k, v, out, lse, rs, scale)
+    cu.check_err_flag()
+    wide = [t.double().requires_grad_() for t in (q, k, v)]
+    _exact(*wide, rs, scale, None, None).backward(do.double())
+    for name, a, b in zip(("dq", "dk", "dv"), grads, wide):
+        bound = 8 * 2.0 ** -9 / 3 ** 0.5 * max(b.grad.norm().item(), 1e-2 * do.double().norm().item())
+        assert (a.double() - b.grad).norm().item() < bound, name
+
+
 def test_flash_packed_autograd_matches_library(cu):
     from easyllm_b200 import ops
     torch.manual_seed(3)
