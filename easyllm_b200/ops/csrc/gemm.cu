@@ -125,7 +125,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint8_t* sC = smem + Cfg::kStages * Cfg::kStageBytes;
   GemmShared* sh = reinterpret_cast<GemmShared*>(sC + 2 * kEpiBufBytes);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int tiles_n = (N + BN - 1) / BN;
   const int num_kb = (K + kBK - 1) / kBK;
   const int n_comm = FUSE == kFuseNone ? 0 : fuse.n_comm;
@@ -240,8 +240,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0) {
+    // ------------------------------ MMA issuer (the whole warp, see sm100.cuh) --------
+    {
+      const uint32_t e = elect_one(), tm = __reduce_or_sync(0xffffffffu, tmem_base);
       constexpr uint32_t idesc_full = make_idesc_bf16(kBM, BN, A_MN, B_MN);
       constexpr uint32_t idesc_half = make_idesc_bf16(kBM, BN / 2, A_MN, B_MN);
       // K-major: 8-row groups 1024 B apart; one K=16 step is 32 B inside the swizzle row.
@@ -249,43 +250,40 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       // one K=16 step is two such groups (2 KiB).
       constexpr uint32_t a_lbo = A_MN ? 64 * kBK * 2 : 16, a_sbo = 1024, a_kstep = A_MN ? 2048 : 32;
       constexpr uint32_t b_lbo = B_MN ? 64 * kBK * 2 : 16, b_sbo = 1024, b_kstep = B_MN ? 2048 : 32;
+      const uint64_t a_desc = make_smem_desc(smem_u32(sA), a_lbo, a_sbo), b_desc = make_smem_desc(smem_u32(sB), b_lbo, b_sbo);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       int it = 0;
-      for (int tile = cta0; tile < num_units && ok; tile += cta_stride, ++it) {
-        const uint32_t idesc = (FUSE == kFuseNone && tile >= num_full) ? idesc_half : idesc_full;
+      for (int tile = cta0; warp_uniform(tile < num_units) && ok; tile += cta_stride, ++it) {
+        const uint32_t idesc = (FUSE == kFuseNone && warp_uniform(tile >= num_full)) ? idesc_half : idesc_full;
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&sh->tmem_empty[acc], acc_phase ^ 1, abort_flag)) {
+        if (!mbar_wait_warp(&sh->tmem_empty[acc], acc_phase ^ 1, abort_flag)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
+        const uint32_t d_tmem = tm + acc * BN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&sh->full[stage], phase, abort_flag)) {
+          if (!mbar_wait_warp(&sh->full[stage], phase, abort_flag)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(sA + stage * kABytes);
-          const uint32_t b_addr = smem_u32(sB + stage * Cfg::kBBytes);
+          const uint64_t da = a_desc + stage * (kABytes >> 4), db = b_desc + stage * (Cfg::kBBytes >> 4);
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k) {
-            const uint64_t da = make_smem_desc(a_addr + k * a_kstep, a_lbo, a_sbo);
-            const uint64_t db = make_smem_desc(b_addr + k * b_kstep, b_lbo, b_sbo);
-            umma_bf16(d_tmem, da, db, idesc, (kb | k) != 0);
-          }
-          umma_commit(&sh->empty[stage]);
+          for (int k = 0; k < kBK / 16; ++k)
+            umma_bf16_warp(e, d_tmem, da + ((k * a_kstep) >> 4), db + ((k * b_kstep) >> 4), idesc, kb | k);
+          umma_commit_warp(e, &sh->empty[stage]);
           if (++stage == Cfg::kStages) {
             stage = 0;
             phase ^= 1;
           }
         }
-        if (ok) umma_commit(&sh->tmem_full[acc]);
+        if (ok) umma_commit_warp(e, &sh->tmem_full[acc]);
       }
-      if (!ok) {
+      if (!ok && e) {
         sh->abort_flag = 1;
         atomicCAS(err, 0, kErrMma);
       }

@@ -135,23 +135,26 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "n"(kTmemCols) : "memory");
 }
 
-__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+__device__ __forceinline__ void umma_bf16_pair(uint32_t elected, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                                                uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(elected)
       : "memory");
 }
 
 // Arrive on the barrier at this shared-memory offset in BOTH CTAs once every tcgen05.mma issued so far is done.
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+__device__ __forceinline__ void umma_commit_pair(uint32_t elected, uint64_t* bar) {
   const uint16_t both = 3;
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-                   smem_u32(bar)),
-               "h"(both)
-               : "memory");
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %2, 0;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+      ::"r"(smem_u32(bar)), "h"(both), "r"(elected)
+      : "memory");
 }
 
 // __host__ __device__ so that the enumerate functions below can run the same code for a CPU coverage test
@@ -298,7 +301,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint8_t* sC = smem + kStages * kStageBytes;
   Shared* sh = reinterpret_cast<Shared*>(sC + 2 * kEpiBufBytes);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t cta_rank = cluster_cta_rank();       // 0: leader, 1: peer
   const bool is_leader = cta_rank == 0;
   const int cluster_id = ((int)blockIdx.x - n_comm) >> 1, n_clusters = ((int)gridDim.x - n_comm) >> 1;
@@ -458,54 +461,52 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    // ------------------------------ MMA issuer (leader CTA only) --------------------------
-    if (lane == 0 && is_leader) {
+    // ------------------------------ MMA issuer (leader CTA only; the whole warp, see sm100.cuh) ------
+    if (is_leader) {
+      const uint32_t e = elect_one(), tm = __reduce_or_sync(0xffffffffu, tmem_base);
       constexpr uint32_t idesc_full = make_idesc_bf16(kTileM, kTileN, A_MN, B_MN);
       constexpr uint32_t idesc_half = make_idesc_bf16(kTileM, kTileN / 2, A_MN, B_MN);
       constexpr uint32_t a_lbo = A_MN ? 64 * kBK * 2 : 16, a_sbo = 1024, a_kstep = A_MN ? 2048 : 32;
       constexpr uint32_t b_lbo = B_MN ? 64 * kBK * 2 : 16, b_sbo = 1024, b_kstep = B_MN ? 2048 : 32;
+      const uint64_t a_desc = make_smem_desc(smem_u32(sA), a_lbo, a_sbo), b_desc = make_smem_desc(smem_u32(sB), b_lbo, b_sbo);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       int it = 0;
-      for (int unit = cluster_id; unit < num_units && ok; unit += n_clusters, ++it) {
-        const uint32_t idesc = unit >= num_full ? idesc_half : idesc_full;
+      for (int unit = cluster_id; warp_uniform(unit < num_units) && ok; unit += n_clusters, ++it) {
+        const uint32_t idesc = warp_uniform(unit >= num_full) ? idesc_half : idesc_full;
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&sh->tmem_empty[acc], acc_phase ^ 1, abort_flag)) {
+        if (!mbar_wait_warp(&sh->tmem_empty[acc], acc_phase ^ 1, abort_flag)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * kTileN;
+        const uint32_t d_tmem = tm + acc * kTileN;
         int n_kb = num_kb;
         if (k_passes == 2) {
           const int kphase = (unit >= num_full ? num_full + ((unit - num_full) >> 1) : unit) / (tiles_m * tiles_n);
           n_kb = kphase == 0 ? num_kb / 2 : num_kb - num_kb / 2;
         }
-        for (int kb = 0; kb < n_kb; ++kb) {
-          if (!mbar_wait(&sh->full[stage], phase, abort_flag)) {
+        for (int kb = 0; warp_uniform(kb < n_kb); ++kb) {
+          if (!mbar_wait_warp(&sh->full[stage], phase, abort_flag)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(sA + stage * kABytes);
-          const uint32_t b_addr = smem_u32(sB + stage * kBBytes);
+          const uint64_t da = a_desc + stage * (kABytes >> 4), db = b_desc + stage * (kBBytes >> 4);
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k) {
-            const uint64_t da = make_smem_desc(a_addr + k * a_kstep, a_lbo, a_sbo);
-            const uint64_t db = make_smem_desc(b_addr + k * b_kstep, b_lbo, b_sbo);
-            umma_bf16_pair(d_tmem, da, db, idesc, (kb | k) != 0);
-          }
-          umma_commit_pair(&sh->empty[stage]);
+          for (int k = 0; k < kBK / 16; ++k)
+            umma_bf16_pair(e, d_tmem, da + ((k * a_kstep) >> 4), db + ((k * b_kstep) >> 4), idesc, kb | k);
+          umma_commit_pair(e, &sh->empty[stage]);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1;
           }
         }
-        if (ok) umma_commit_pair(&sh->tmem_full[acc]);
+        if (ok) umma_commit_pair(e, &sh->tmem_full[acc]);
       }
-      if (!ok) {
+      if (!ok && e) {
         sh->abort_flag = 1;
         atomicCAS(err, 0, kErrPairMma);
       }

@@ -155,7 +155,7 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   float* send = reinterpret_cast<float*>(smem + Cfg::kStages * Cfg::kStageBytes);   // [column][row]
   float* recv = send + Cfg::kExBytes / 4;                                            // [peer][column][row]
   ThinShared* sh = reinterpret_cast<ThinShared*>(recv + Cfg::kExBytes / 4);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int split = a.split, rank = split > 1 ? (int)cluster_rank() : 0;
   const int tiles_t = (a.T + BN - 1) / BN, tiles = tiles_t * ((a.N + kThRows - 1) / kThRows);
   const int blocks = (a.K + kBK - 1) / kBK;
@@ -233,39 +233,41 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {                                                // the whole warp, see sm100.cuh
+      const uint32_t e = elect_one(), tm = __reduce_or_sync(0xffffffffu, tmem_base);
       constexpr uint32_t idesc = make_idesc_bf16(kThRows, BN, W_MN, false);
       constexpr uint32_t w_lbo = W_MN ? 64 * kBK * 2 : 16, w_kstep = W_MN ? 2048 : 32;
+      const uint64_t w_desc = make_smem_desc(smem_u32(sW), w_lbo, 1024), x_desc = make_smem_desc(smem_u32(sX), 16, 1024);
       int stage = 0, it = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = first; tile < tiles && ok; tile += step, ++it) {
+      for (int tile = first; warp_uniform(tile < tiles) && ok; tile += step, ++it) {
         const int acc = it & 1;
-        if (!mbar_wait(&sh->tmem_empty[acc], ((it >> 1) & 1) ^ 1, abort_flag)) {
+        if (!mbar_wait_warp(&sh->tmem_empty[acc], ((it >> 1) & 1) ^ 1, abort_flag)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&sh->full[stage], phase, abort_flag)) {
+        for (int kb = kb0; warp_uniform(kb < kb1); ++kb) {
+          if (!mbar_wait_warp(&sh->full[stage], phase, abort_flag)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t w = smem_u32(sW + stage * kThWBytes), x = smem_u32(sX + stage * (BN * kBK * 2));
+          const uint64_t dw = w_desc + stage * (kThWBytes >> 4), dx = x_desc + stage * ((BN * kBK * 2) >> 4);
+          const uint32_t add = warp_uniform(kb > kb0);
 #pragma unroll
           for (int k = 0; k < kBK / 16; ++k)
-            umma_bf16(tmem_base + acc * BN, make_smem_desc(w + k * w_kstep, w_lbo, 1024), make_smem_desc(x + k * 32, 16, 1024),
-                      idesc, kb > kb0 || k > 0);
-          umma_commit(&sh->empty[stage]);
+            umma_bf16_warp(e, tm + acc * BN, dw + ((k * w_kstep) >> 4), dx + ((k * 32) >> 4), idesc, add | k);
+          umma_commit_warp(e, &sh->empty[stage]);
           if (++stage == Cfg::kStages) {
             stage = 0;
             phase ^= 1;
           }
         }
-        if (ok) umma_commit(&sh->tmem_full[acc]);
+        if (ok) umma_commit_warp(e, &sh->tmem_full[acc]);
       }
-      if (!ok) {
+      if (!ok && e) {
         give_up(sh, split);
         atomicCAS(a.err, 0, kErrMma);
       }
