@@ -69,11 +69,11 @@ class SparseMoE(nn.Module):
 
     def forward(self, h, residual):
         E = self.router.weight.shape[0]
-        z = iops.linear_cat_f32(h, [self.router.weight] + ([self.shared_gate.weight] if self.shared is not None else []))
+        z, routed = iops.moe_router(h, [self.router.weight] + ([self.shared_gate.weight] if self.shared is not None else []), E, self.top)
         if self.shared is not None:
             a = iops.relu2_scaled(iops.linear(h, self.shared.up_proj.weight), z[:, E])
             iops.linear_add_(residual, a, self.shared.down_proj.weight)
-        return iops.moe_relu2_add_(residual, h, z[:, :E], self.top, self.experts_up, self.experts_down)
+        return iops.moe_relu2_add_(residual, h, z[:, :E], self.top, self.experts_up, self.experts_down, routed)
 
 
 class SparseGLU(nn.Module):
@@ -114,8 +114,8 @@ class SparseGLU(nn.Module):
         return v[:, 0].reshape(F, W), v[:, 1].reshape(F, W)
 
     def forward(self, h, residual):
-        z = iops.linear_f32(h, self.router.weight)
+        z, routed = iops.moe_router(h, [self.router.weight], self.router.weight.shape[0], self.top, self.router_bias, softmax=True)
         if self.shared is not None:
             self.shared(h, residual)
         return iops.moe_glu_add_(residual, h, z, self.router_bias, self.top, self.experts_gate_up, self.block,
-                                 self.experts_down)
+                                 self.experts_down, routed)

@@ -12,7 +12,7 @@
 //
 // Structure (one persistent CTA per SM, 192 threads):
 //   warp 0      TMA producer: cp.async.bulk.tensor 2-D tiles (128B swizzle) into a 4–6 stage ring
-//   warp 1      allocates TMEM, one thread issues tcgen05.mma (128 x BN x 16 per instruction),
+//   warp 1      allocates TMEM, issues tcgen05.mma (128 x BN x 16 per instruction),
 //               tcgen05.commit releases smem stages and publishes finished accumulators
 //   warps 2-5   epilogue: tcgen05.ld TMEM -> registers -> (bias) -> bf16 -> swizzled smem ->
 //               TMA store, or fp32 read-modify-write to global for gradient accumulation

@@ -7,7 +7,7 @@
 // columns that a peer finishes to that peer (distributed shared memory, an mbarrier per direction), and each sums its
 // columns in the order of the cluster's ranks, so results do not depend on timing and no workspace exists.
 //   warp 0     TMA producer: a [128 x 64] box of W and a [BN x 64] box of x per stage
-//   warp 1     one thread issues tcgen05.mma (128 x BN x 16); two accumulators in TMEM
+//   warp 1     issues tcgen05.mma (128 x BN x 16); two accumulators in TMEM
 //   warps 2-5  TMEM -> peers' shared memory -> sum -> bias -> global; a warp stores 32 consecutive columns of a row
 // W_MN: W is stored [K, N] (the input gradient of a linear layer reads its weight in place).
 #include "gemm_fuse.cuh"

@@ -246,6 +246,114 @@ __global__ void moe_route_kernel(const float* __restrict__ z, const float* __res
     for (int k = 0; k < top; ++k) w[t * top + k] /= sum;
 }
 
+// Router product and routing in one launch, bf16, up to 16 choices and 64 rows of W (experts first, then what else is wanted of the logits): 16 tokens
+// a CTA, its warps split K as in matvec_mma_kernel.  The tiled product pads N to 128 and so filled 30 SMs with 3777 tokens of 2048:
+// 14 us and 5.5 more for the routing, now 7; 64 tokens 8 and 3, now 5.5.
+// The routing of moe_route_kernel for half a warp and up to 64 experts and 16 choices: lane k keeps choice k.
+__device__ __forceinline__ void route_half(const float* row, const float* __restrict__ bias, int* __restrict__ idx, float* __restrict__ w,
+                                           int E, int top, int softmax, int lane, uint32_t lanes) {
+  float v[4], chosen = 0.f, largest = 0.f, sum = 0.f;
+  int expert = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = i * 16 + lane < E ? row[i * 16 + lane] + (bias != nullptr ? bias[i * 16 + lane] : 0.f) : 0.f;
+  uint32_t taken = 0;                                  // bit i: expert 16 i + lane
+  for (int k = 0; k < top; ++k) {
+    float best = -INFINITY;
+    int be = 0x7fffffff;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (i * 16 + lane < E && !(taken >> i & 1) && (v[i] > best || be == 0x7fffffff)) {
+        best = v[i];
+        be = i * 16 + lane;
+      }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      const float ov = __shfl_xor_sync(lanes, best, o);
+      const int oe = __shfl_xor_sync(lanes, be, o);
+      if (oe != 0x7fffffff && (be == 0x7fffffff || ov > best || (ov == best && oe < be))) {
+        best = ov;
+        be = oe;
+      }
+    }
+    if ((be & 15) == lane) taken |= 1u << (be >> 4);
+    if (k == 0) largest = best;
+    if (k == lane) {
+      chosen = best;
+      expert = be;
+    }
+  }
+  float e = softmax ? expf(chosen - largest) : sigmoid_f(chosen);
+  if (softmax) {
+    for (int k = 0; k < top; ++k) sum += __shfl_sync(lanes, e, k, 16);
+    e /= sum;
+  }
+  if (lane < top) {
+    idx[lane] = expert;
+    w[lane] = e;
+  }
+}
+
+template <int NT>
+__global__ void __launch_bounds__(kMvWarps * 32) moe_router_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                                                    const float* __restrict__ bias, float* __restrict__ z,
+                                                                    int* __restrict__ idx, float* __restrict__ score, int n, int N, int K,
+                                                                    int ldx, int ldz, int E, int top, int softmax) {
+  __shared__ float red[kMvWarps][16][8 * NT + 1];
+  __shared__ float logits[16][8 * NT];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, t0 = blockIdx.x * 16;
+  chain_next();
+  if (blockIdx.x == 0 && threadIdx.x < N)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(w + (size_t)threadIdx.x * K), "r"(K * 2) : "memory");
+  chain_wait(x, w, bias, z, idx, score);
+  const __nv_bfloat16 *x0 = x + (size_t)min(t0 + g, n - 1) * ldx, *x1 = x + (size_t)min(t0 + g + 8, n - 1) * ldx;
+  float c[NT][4];
+#pragma unroll
+  for (int i = 0; i < NT; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) c[i][j] = 0.f;
+  constexpr int U = NT > 4 ? 2 : 4;
+  for (int kb = warp; kb * 32 < K; kb += kMvWarps * U) {
+    uint4 xa[U], xb[U], wv[U][NT];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = (kb + u * kMvWarps) * 32 + t * 8, kc = k < K ? k : 0;
+      xa[u] = *reinterpret_cast<const uint4*>(x0 + kc);
+      xb[u] = *reinterpret_cast<const uint4*>(x1 + kc);
+      if (k >= K) xa[u] = xb[u] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int i = 0; i < NT; ++i) wv[u][i] = *reinterpret_cast<const uint4*>(w + (size_t)min(i * 8 + g, N - 1) * K + kc);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int i = 0; i < NT; ++i) {
+        mma_16816(c[i], xa[u].x, xb[u].x, xa[u].y, xb[u].y, wv[u][i].x, wv[u][i].y);
+        mma_16816(c[i], xa[u].z, xb[u].z, xa[u].w, xb[u].w, wv[u][i].z, wv[u][i].w);
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < NT; ++i) {
+    red[warp][g][i * 8 + 2 * t] = c[i][0];
+    red[warp][g][i * 8 + 2 * t + 1] = c[i][1];
+    red[warp][g + 8][i * 8 + 2 * t] = c[i][2];
+    red[warp][g + 8][i * 8 + 2 * t + 1] = c[i][3];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < 16 * 8 * NT; e += kMvWarps * 32) {
+    const int m = e / (8 * NT), i = e % (8 * NT);
+    float v = 0.f;
+#pragma unroll
+    for (int p = 0; p < kMvWarps; ++p) v += red[p][m][i];
+    logits[m][i] = v;
+    if (i < N && t0 + m < n) z[(size_t)(t0 + m) * ldz + i] = v;
+  }
+  __syncthreads();
+  const int m = warp * 2 + (lane >> 4);
+  if (t0 + m < n)
+    route_half(logits[m], bias, idx + (size_t)(t0 + m) * top, score + (size_t)(t0 + m) * top, E, top, softmax, lane & 15,
+               lane < 16 ? 0xffffu : 0xffff0000u);
+}
+
 // For slot = token * top + k, a warp multiplies two weight rows of expert e = idx[slot] with the token:
 //   GLU false  hidden units f0, f0 + 1 of up [E, F, W]:  hid[slot][f] = (w_slot relu(up_e[f] . h))^2
 //   GLU true   the gate and up rows of one hidden unit of [E, 2 F, W], which alternate in blocks of `block` rows:
@@ -348,70 +456,106 @@ __global__ void __launch_bounds__(256) moe_down_kernel(const T* __restrict__ hid
 }
 
 // ---- mixture of experts: rows sorted by expert for the grouped GEMM ---------------------------------
-// One CTA.  Every expert's rows start at a multiple of 128; tile_expert[i] is the expert of row tile i, *n_tiles their
-// number, pos[slot] the row of slot = token * top + k, row_scale[row] its score (rows of the padding: 0).
-__global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ idx, const float* __restrict__ wgt, int slots,
-                                                        int E, int* __restrict__ pos, float* __restrict__ row_scale,
-                                                        int* __restrict__ tile_expert, int* __restrict__ n_tiles) {
-  chain_enter(idx, wgt, pos, row_scale, tile_expert, n_tiles);
-  __shared__ int count[1024], first[1024], scan[1024];
-  const int e = threadIdx.x;
-  count[e] = 0;
+// Row plan and gathered rows in one launch.  Every expert's rows start at a multiple of 128, in the order of their slots (slot = token *
+// top + k); tile_expert[i] is the expert of row tile i, *n_tiles their number, pos[slot] the row of a slot, row_scale[row] its score
+// (rows of the padding: 0), xs[pos[slot]] = h[token].
+// A CTA takes a range of slots and counts for itself, over all slots, the rows of every expert and those before its range: reading the
+// indexes 148 times (30 kB for 3777 tokens, top 2) costs less than a plan made by one CTA and a launch that waits for it.  3777
+// tokens of 2048: 20 us in two launches -> 12; 64 tokens 6.6 -> 4.
+constexpr int kGatherThreads = 512;
+__global__ void __launch_bounds__(kGatherThreads) moe_gather_kernel(const uint4* __restrict__ h, uint4* __restrict__ xs,
+                                                                     const int* __restrict__ idx, const float* __restrict__ wgt,
+                                                                     int* __restrict__ pos, float* __restrict__ row_scale,
+                                                                     int* __restrict__ tile_expert, int* __restrict__ n_tiles, int slots,
+                                                                     int top, int E, int wv) {
+  __shared__ int total[1024], next[1024], first[1024], row[kGatherThreads];
+  chain_enter(h, xs, idx, wgt, pos, row_scale, tile_expert, n_tiles);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int s0 = (int)((long long)slots * blockIdx.x / gridDim.x), s1 = (int)((long long)slots * (blockIdx.x + 1) / gridDim.x);
+  for (int e = threadIdx.x; e < E; e += kGatherThreads) total[e] = next[e] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < slots; i += 1024) atomicAdd(&count[idx[i]], 1);
-  __syncthreads();
-  const int mine = e < E ? (count[e] + 127) / 128 : 0;
-  scan[e] = mine;
-  __syncthreads();
-  for (int o = 1; o < 1024; o <<= 1) {
-    const int v = e >= o ? scan[e - o] : 0;
-    __syncthreads();
-    scan[e] += v;
-    __syncthreads();
+  // the range's own first slots, for later
+  const int own = s0 + lane < s1 ? idx[s0 + lane] : -1;
+  const float own_w = s0 + lane < s1 ? wgt[s0 + lane] : 0.f;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < slots; i += kGatherThreads) {
+    const int e = idx[i];
+    atomicAdd(&total[e], 1);
+    if (i < s0) atomicAdd(&next[e], 1);
   }
-  const int t0 = scan[e] - mine;
-  first[e] = t0 * 128;
-  for (int i = 0; i < mine; ++i) tile_expert[t0 + i] = e;
-  for (int i = count[e]; i < mine * 128; ++i) row_scale[t0 * 128 + i] = 0.f;
-  if (e == 1023) *n_tiles = scan[1023];
   __syncthreads();
-  count[e] = 0;
-  __syncthreads();
-  for (int i = threadIdx.x; i < slots; i += 1024) {
-    const int x = idx[i], r = first[x] + atomicAdd(&count[x], 1);
-    pos[i] = r;
-    row_scale[r] = wgt[i];
-  }
-}
-
-// xs[pos[slot]] = h[token], 16 bytes a thread.
-__global__ void moe_gather_kernel(const uint4* __restrict__ h, uint4* __restrict__ xs, const int* __restrict__ pos, int slots,
-                                  int top, int wv) {
-  chain_enter(h, xs, pos);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)slots * wv;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int slot = (int)(i / wv), c = (int)(i % wv);
-    xs[(size_t)pos[slot] * wv + c] = h[(size_t)(slot / top) * wv + c];
-  }
-}
-
-// acc[token] += sum over its slots of ys[pos[slot]]
-__global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ ys, const int* __restrict__ pos, float* __restrict__ acc,
-                                   int n, int top, int W) {
-  chain_enter(ys, pos, acc);
-  const int wv = W / 4;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)n * wv;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int t = (int)(i / wv), c = (int)(i % wv) * 4;
-    float s[4];
-    load_v<4>(acc + (size_t)t * W + c, s);
-    for (int k = 0; k < top; ++k) {
-      float f[4];
-      load_v<4>(ys + (size_t)pos[t * top + k] * W + c, f);
+  if (warp == 0) {                                    // first row tile of every expert; next[e]: the row of the range's first slot for e
+    int tiles = 0;
+    for (int b = 0; b < E; b += 32) {
+      const int e = b + lane, n = e < E ? total[e] : 0, mine = (n + 127) / 128;
+      int upto = mine;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) s[j] += f[j];
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+      }
+      const int t0 = tiles + upto - mine;
+      if (e < E) {
+        next[e] += t0 * 128;
+        if (blockIdx.x == 0) {
+          for (int i = 0; i < mine; ++i) tile_expert[t0 + i] = e;
+          first[e] = t0 * 128;
+        }
+      }
+      tiles += __shfl_sync(0xffffffffu, upto, 31);
     }
-    store_v<4>(acc + (size_t)t * W + c, s);
+    if (blockIdx.x == 0 && lane == 0) *n_tiles = tiles;
+  }
+  if (blockIdx.x == 0) {                              // a warp per expert: the padding of its last tile
+    __syncthreads();
+    for (int e = warp; e < E; e += kGatherThreads / 32)
+      for (int i = total[e] + lane; i < (total[e] + 127) / 128 * 128; i += 32) row_scale[first[e] + i] = 0.f;
+  }
+  for (int c0 = s0; c0 < s1; c0 += kGatherThreads) {
+    const int c1 = min(c0 + kGatherThreads, s1);
+    __syncthreads();
+    if (warp == 0) {                                  // rows of the slots, in order
+      for (int b = c0; b < c1; b += 32) {
+        const int i = b + lane, e = b == s0 ? own : i < c1 ? idx[i] : -1;
+        const uint32_t same = __match_any_sync(0xffffffffu, e);
+        const int r = e >= 0 ? next[e] + __popc(same & ((1u << lane) - 1)) : 0;
+        __syncwarp();
+        if (e >= 0) {
+          if (__ffs(same) == lane + 1) next[e] += __popc(same);
+          row[i - c0] = r;
+          pos[i] = r;
+          row_scale[r] = b == s0 ? own_w : wgt[i];
+        }
+        __syncwarp();
+      }
+    }
+    __syncthreads();
+    for (int i = c0 + warp; i < c1; i += kGatherThreads / 32) {
+      const uint4* src = h + (size_t)(i / top) * wv;
+      uint4* dst = xs + (size_t)row[i - c0] * wv;
+#pragma unroll 4
+      for (int c = lane; c < wv; c += 32) dst[c] = src[c];
+    }
+  }
+}
+
+// acc[token] += sum over its slots of ys[pos[slot]]; a CTA per token, 8 columns a thread (W a multiple of 8).  Indexed through 64-bit
+// divisions, four columns a thread, 3777 tokens of 2048 took 20 us where this takes 15.
+__global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ ys, const int* __restrict__ pos, float* __restrict__ acc, int top,
+                                   int W) {
+  chain_enter(ys, pos, acc);
+  const int* p = pos + (size_t)blockIdx.x * top;
+  float* a = acc + (size_t)blockIdx.x * W;
+  for (int c = threadIdx.x * 8; c < W; c += blockDim.x * 8) {
+    float s[8];
+    load_v<8>(a + c, s);
+    for (int k = 0; k < top; ++k) {
+      float f[8];
+      load_v<8>(ys + (size_t)p[k] * W + c, f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s[j] += f[j];
+    }
+    store_v<8>(a + c, s);
   }
 }
 
@@ -442,6 +586,18 @@ ELL_API int ell_moe_route(const float* z, const float* bias, int* idx, float* w,
   return launch_status();
 }
 
+// z [n, N] = x w^T (rows of ldz), and the routing of its first E columns: bf16 x [n, K] (rows of ldx) and w [N, K], N up to 64, K a
+// multiple of 8, 16-byte rows.
+ELL_API int ell_moe_router(const void* x, const void* w, const float* bias, float* z, int* idx, float* score, int n, int N, int K,
+                           int ldx, int ldz, int E, int top, int softmax, cudaStream_t stream) {
+  if (n <= 0) return 0;
+  if (N < 1 || N > 64 || E > N || top > E || top < 1 || top > 16 || K % 8 || ldx % 8 || !aligned_to(x, 16) || !aligned_to(w, 16)) return -2;
+  auto kern = N <= 8 ? moe_router_kernel<1> : N <= 16 ? moe_router_kernel<2> : N <= 32 ? moe_router_kernel<4> : moe_router_kernel<8>;
+  launch_chained(kern, (n + 15) / 16, kMvWarps * 32, 0, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, bias, z, idx, score, n, N,
+                 K, ldx, ldz, E, top, softmax);
+  return launch_status();
+}
+
 // acc [n, W] fp32 += experts; up [E, F, W], down [E, W, F]; hid: scratch [n * top, F] of the activation type.
 // glu_block > 0: gated experts, up [E, 2 F, W] with gate and up rows in alternating blocks of glu_block (a divisor of F).
 ELL_API int ell_moe_rows(const void* h, const void* up, const void* down, const int* idx, const float* w, void* hid,
@@ -469,15 +625,15 @@ ELL_API int ell_moe_gather(const void* h, void* xs, const int* idx, const float*
                            int* tile_expert, int* n_tiles, int n, int top, int E, int W, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (E > 1024 || W % 8) return -2;
-  launch_chained(moe_plan_kernel, 1, 1024, 0, stream, idx, w, n * top, E, pos, row_scale, tile_expert, n_tiles);
-  launch_chained(moe_gather_kernel, grid_for((long long)n * top * (W / 8), 256), 256, 0, stream, (const uint4*)h, (uint4*)xs, pos,
-                                                                                    n * top, top, W / 8);
+  const int slots = n * top, grid = slots < 8 * kNumSMs ? (slots + 7) / 8 : 2 * kNumSMs;   // 8 slots a CTA until two CTAs fill an SM
+  launch_chained(moe_gather_kernel, grid, kGatherThreads, 0, stream, (const uint4*)h, (uint4*)xs, idx, w, pos, row_scale, tile_expert,
+                 n_tiles, slots, top, E, W / 8);
   return launch_status();
 }
 
 ELL_API int ell_moe_combine(const void* ys, const int* pos, float* acc, int n, int top, int W, cudaStream_t stream) {
   if (n <= 0) return 0;
-  if (W % 4) return -2;
-  launch_chained(moe_combine_kernel, grid_for((long long)n * (W / 4), 256), 256, 0, stream, (const __nv_bfloat16*)ys, pos, acc, n, top, W);
+  if (W % 8) return -2;
+  launch_chained(moe_combine_kernel, n, W >= 2048 ? 256 : (W / 8 + 31) / 32 * 32, 0, stream, (const __nv_bfloat16*)ys, pos, acc, top, W);
   return launch_status();
 }

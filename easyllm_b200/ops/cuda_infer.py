@@ -417,12 +417,29 @@ def moe_route(z, top, bias=None, softmax=False):
     return idx, w
 
 
-def moe_relu2_add_(acc, h, z, top, up, down):
-    return _moe_add_(acc, h, *moe_route(z, top), up, down)
+def moe_router(h, w, experts, top, bias=None, softmax=False):
+    """fp32 ``h wᵀ`` and the routing of its first ``experts`` columns in one launch: ``(z, (idx, scores))``; None where the kernel does
+    not take the operands."""
+    (T, W), N = h.shape, w.shape[0]
+    if h.dtype != torch.bfloat16 or w.dtype != h.dtype or N > 64 or top > 16 or W % 8 or not w.is_contiguous() or T == 0:
+        return None
+    ldx = _rows(h, "h")
+    if ldx % 8 or (h.data_ptr() | w.data_ptr()) & 15:
+        return None
+    z = torch.empty(T, N, dtype=torch.float32, device=h.device)
+    idx = torch.empty(T, top, dtype=torch.int32, device=h.device)
+    score = torch.empty(T, top, dtype=torch.float32, device=h.device)
+    _check(lib().ell_moe_router(_p(h), _p(w), _p(None if bias is None else _f32(bias, "bias")), _p(z), _p(idx), _p(score), c_int(T), c_int(N),
+                                c_int(W), c_int(ldx), c_int(N), c_int(experts), c_int(top), c_int(softmax), _stream()), "moe_router")
+    return z, (idx, score)
 
 
-def moe_glu_add_(acc, h, z, bias, top, gate_up, block, down):
-    return _moe_add_(acc, h, *moe_route(z, top, bias, softmax=True), gate_up, down, block)
+def moe_relu2_add_(acc, h, z, top, up, down, routed=None):
+    return _moe_add_(acc, h, *(routed or moe_route(z, top)), up, down)
+
+
+def moe_glu_add_(acc, h, z, bias, top, gate_up, block, down, routed=None):
+    return _moe_add_(acc, h, *(routed or moe_route(z, top, bias, softmax=True)), gate_up, down, block)
 
 
 def _moe_add_(acc, h, idx, w, up, down, block=0):
@@ -456,7 +473,7 @@ def _moe_grouped(acc, h, idx, w, up, down, block=0):
     scale = torch.empty(rows, dtype=torch.float32, device=dev)
     xs = torch.empty(rows, W, dtype=h.dtype, device=dev)
     _check(lib().ell_moe_gather(_p(h), _p(xs), _p(idx), _p(w), _p(pos), _p(scale), _p(tile_expert), _p(n_tiles), c_int(T),
-                                c_int(top), c_int(E), c_int(W), _stream()), "moe_gather", 2)
+                                c_int(top), c_int(E), c_int(W), _stream()), "moe_gather")
     hid = torch.empty(rows, F, dtype=h.dtype, device=dev)
     ys = torch.empty(rows, W, dtype=h.dtype, device=dev)
     for x, wt, out, n, k, sc in ((xs, up, hid, up.shape[1], W, scale), (hid, down, ys, W, F, None)):

@@ -299,21 +299,34 @@ def head_norm_gate(o, w, gate, gate_act, eps, out_dtype):
 
 
 # ---- mixture of experts ------------------------------------------------------------------------------
-def moe_relu2_add_(acc, h, z, top, up, down):
-    """``acc += sum over the top experts of down_e relu(up_e (s_e h))^2`` with scores ``s = sigmoid(z)``."""
+def moe_router(h, weights, experts, top, bias=None, softmax=False):
+    """Router logits ``z = h [W_1; W_2; ...]ᵀ`` in fp32, and the routing of the first ``experts`` of them (for the ``routed`` of the
+    expert ops) where one kernel does both, else None."""
+    no_grad_check(h, *weights)
+    if _kern(h):
+        both = _cu().moe_router(h, fused(weights), experts, top, None if bias is None else bias.detach(), softmax)
+        if both is not None:
+            return both
+    return linear_cat_f32(h, weights), None
+
+
+def moe_relu2_add_(acc, h, z, top, up, down, routed=None):
+    """``acc += sum over the top experts of down_e relu(up_e (s_e h))^2`` with scores ``s = sigmoid(z)``.  ``routed``: experts and
+    scores, if they are known."""
     no_grad_check(h, up)
     if _kern(h):
-        return _cu().moe_relu2_add_(acc, h, z, top, up.detach(), down.detach())
+        return _cu().moe_relu2_add_(acc, h, z, top, up.detach(), down.detach(), routed)
     idx, w = ref.route(z, top)
     return acc.add_(ref.moe_relu2(h, idx, w, up, down))
 
 
-def moe_glu_add_(acc, h, z, bias, top, gate_up, block, down):
+def moe_glu_add_(acc, h, z, bias, top, gate_up, block, down, routed=None):
     """``acc += sum over the top experts of w_e down_e (silu(gate_e h) * up_e h)``, ``w`` the softmax over the chosen logits
-    of ``z + bias``; gate_up ``[E, 2 F, W]`` holds gate and up rows in alternating blocks of ``block``."""
+    of ``z + bias``; gate_up ``[E, 2 F, W]`` holds gate and up rows in alternating blocks of ``block``.  ``routed``: experts and
+    weights, if they are known."""
     no_grad_check(h, gate_up)
     bias = None if bias is None else bias.detach()
     if _kern(h):
-        return _cu().moe_glu_add_(acc, h, z, bias, top, gate_up.detach(), block, down.detach())
+        return _cu().moe_glu_add_(acc, h, z, bias, top, gate_up.detach(), block, down.detach(), routed)
     idx, w = ref.route_softmax(z, bias, top)
     return acc.add_(ref.moe_glu(h, idx, w, gate_up, block, down))

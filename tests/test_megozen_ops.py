@@ -273,3 +273,57 @@ def test_router_weights_and_ties():
     assert idx.tolist() == [[3, 1, 2], [0, 2, 4]]
     close(w[0], torch.softmax(torch.tensor([8.0, 5.0, 5.0]), -1), 1e-6)
     close(w[1], torch.softmax(torch.tensor([80.0, 79.0, 78.0]), -1), 1e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,K,E,extra,top", [(1, 40, 8, 0, 1), (16, 2048, 16, 0, 2), (17, 64, 16, 1, 2), (100, 328, 33, 0, 5), (64, 4096, 60, 4, 16),
+                                             (3777, 256, 7, 1, 7)])
+@pytest.mark.parametrize("softmax", [False, True])
+def test_router_product_and_routing_in_one_launch(T, K, E, extra, top, softmax):
+    """Tiles of 16 tokens and 8 logits with remainders.  Logits are sums of K products of bf16 numbers in fp32: off by at most K * 2^-24
+    of the sum of the products' sizes.  The routing of these logits is that of the kernel that takes logits, to the bit."""
+    from easyllm_b200.ops import cuda_infer as ci
+    gen = torch.Generator().manual_seed(T + K)
+    h = torch.randn(T, K, generator=gen).bfloat16().cuda()
+    w = torch.randn(E + extra, K, generator=gen).bfloat16().cuda()
+    bias = torch.randn(E, generator=gen).cuda() if softmax else None
+    z, (idx, score) = ci.moe_router(h, w, E, top, bias, softmax)
+    exact, sizes = h.double() @ w.double().t(), h.double().abs() @ w.double().abs().t()
+    assert ((z.double() - exact).abs() <= K * 2.0 ** -24 * sizes).all()
+    want_idx, want_score = ci.moe_route(z[:, :E], top, bias, softmax)
+    assert torch.equal(idx, want_idx) and torch.equal(score, want_score)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,top,E", [(1, 1, 1), (33, 2, 16), (700, 3, 5), (64, 2, 1024), (5000, 2, 40)])
+def test_row_plan_of_the_grouped_product(T, top, E):
+    """Fewer slots than a warp, ranges of several CTAs, experts without rows and with several row tiles, more slots a CTA than it
+    takes at once: every token's row lies in its slot's place, experts in order, rows of an expert in the order of their slots."""
+    from ctypes import c_int
+    from easyllm_b200.ops import cuda as cu
+    gen, W = torch.Generator().manual_seed(T), 8
+    idx = torch.randint(0, E, (T, top), generator=gen, dtype=torch.int32)
+    idx[:T // 3] = E - 1
+    w = torch.rand(T, top, generator=gen)
+    h = torch.randn(T, W, generator=gen).bfloat16().cuda()
+    used = min(E, T * top)
+    tiles = (T * top - used) // 128 + used
+    pos, tile_expert, n_tiles = (torch.full((n,), -1, dtype=torch.int32, device="cuda") for n in (T * top, tiles, 1))
+    scale, xs = torch.full((tiles * 128,), -1.0, device="cuda"), torch.zeros(tiles * 128, W, dtype=torch.bfloat16, device="cuda")
+    di, dw = idx.cuda(), w.cuda()
+    cu._check(cu.lib().ell_moe_gather(*(cu._p(t) for t in (h, xs, di, dw, pos, scale, tile_expert, n_tiles)), c_int(T), c_int(top), c_int(E),
+                                      c_int(W), cu._stream()), "moe_gather")
+    counts = torch.bincount(idx.flatten().long(), minlength=E)
+    per = (counts + 127) // 128
+    first = (per.cumsum(0) - per) * 128
+    want, seen = torch.empty(T * top, dtype=torch.int32), [0] * E
+    for i, e in enumerate(idx.flatten().tolist()):
+        want[i] = first[e] + seen[e]
+        seen[e] += 1
+    assert torch.equal(pos.cpu(), want) and int(n_tiles) == int(per.sum())
+    assert torch.equal(tile_expert[:int(n_tiles)].cpu(), torch.repeat_interleave(torch.arange(E), per).int())
+    rows = want.long()
+    assert torch.equal(xs.cpu()[rows], h.cpu().repeat_interleave(top, 0))
+    want_scale = torch.zeros(int(n_tiles) * 128)
+    want_scale[rows] = w.flatten()
+    assert torch.equal(scale[:int(n_tiles) * 128].cpu(), want_scale)
