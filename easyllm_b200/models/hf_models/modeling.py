@@ -33,6 +33,8 @@ from .latent import LatentAttention
 from .mixers import ChannelDelta, DynamicTanh, LayerNorm, TimeMix
 from .state import DecodeGraph, DecodeState, KVRows
 
+_global_hooks = nn.modules.module._has_any_global_hook
+
 
 @dataclass
 class LayerSpec:
@@ -384,6 +386,35 @@ class MLP(nn.Module):
         return ops.linear(ops.glu_linear(x, self.gate_proj.weight, self.up_proj.weight), self.down_proj.weight)
 
 
+def _plain(m, cls):
+    """Whether ``m`` is a ``cls`` itself whose call is its class's ``forward`` and nothing besides."""
+    return type(m) is cls and "forward" not in m.__dict__ and \
+        not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+
+
+def _adjacent_rows(cols, *parts):
+    """Address of bf16 weights ``[rows, cols]`` (pairs of a Linear without bias and its rows) that lie back to back, or None."""
+    at = base = None
+    for lin, rows in parts:
+        w = lin._parameters.get("weight")
+        if not _plain(lin, nn.Linear) or w is None or lin._parameters["bias"] is not None or w.dtype != torch.bfloat16 or \
+                not w.is_cuda or tuple(w.shape) != (rows, cols) or not w.is_contiguous():
+            return None
+        if at is None:
+            at = first = w.data_ptr()
+            base = w.untyped_storage().data_ptr()
+        elif w.data_ptr() != at or w.untyped_storage().data_ptr() != base:
+            return None
+        at += 2 * rows * cols
+    return None if first & 15 else first
+
+
+def _norm_weight(norm, cols, eps):
+    w = norm._parameters.get("weight") if _plain(norm, RMSNorm) and norm.eps == eps else None
+    return w if w is not None and w.dtype == torch.bfloat16 and w.is_cuda and w.shape[0] == cols and w.is_contiguous() and \
+        not w.data_ptr() & 15 else None
+
+
 class DecoderLayer(nn.Module):
     def __init__(self, a: HFArch, dtype):
         super().__init__()
@@ -403,6 +434,26 @@ class DecoderLayer(nn.Module):
             n1, h = self.input_layernorm(delta, residual)
         n2, h = self.post_attention_layernorm(self.self_attn(n1, meta, cache), h)
         return self.mlp(n2), h
+
+    def addresses(self, width, meta, cache, eps):
+        """What ``ops.infer.decoder_step`` needs to know of this layer, or None where it does not stand for ``forward``."""
+        at, mlp = self._modules["self_attn"], self._modules["mlp"]
+        if not (_plain(self, DecoderLayer) and _plain(at, Attention) and _plain(mlp, MLP) and type(cache) is KVRows):
+            return None
+        hq, hk, d, ff = at.hq, at.hk, at.d, at.a.intermediate_size
+        part, k, v = at._modules, cache.k, cache.v
+        if any(c.dtype != torch.bfloat16 or not c.is_cuda or not c.is_contiguous() or c.shape[2:] != (hk, d) or c.data_ptr() & 15
+               for c in (k, v)):
+            return None
+        n1, n2 = (_norm_weight(self._modules[n], width, eps) for n in ("input_layernorm", "post_attention_layernorm"))
+        mats = (_adjacent_rows(width, (part["q_proj"], hq * d), (part["k_proj"], hk * d), (part["v_proj"], hk * d)),
+                _adjacent_rows(hq * d, (part["o_proj"], width)),
+                _adjacent_rows(width, (mlp._modules["gate_proj"], ff), (mlp._modules["up_proj"], ff)),
+                _adjacent_rows(ff, (mlp._modules["down_proj"], width)))
+        if n1 is None or n2 is None or None in mats:
+            return None
+        cos, sin = at.rotary.get(int(meta["max_position"]), k.device)
+        return (*mats, n1.data_ptr(), n2.data_ptr(), k.data_ptr(), v.data_ptr(), cos.data_ptr(), sin.data_ptr(), cos.shape[0])
 
 
 def _block_norm(a: HFArch, dtype):
@@ -559,6 +610,10 @@ class CausalLM(nn.Module):
         if self.model.hybrid:
             iops.no_grad_check(x, self.lm_head.weight)
             x = x.float() if inputs_embeds is None else x.to(torch.float32, copy=True)     # the layers write into it
+        if caches is not None and ops.is_serving():
+            y = self._step_natively(x, meta, caches)
+            if y is not None:
+                return y
         delta, residual = x, None
         for i, layer in enumerate(self.model.layers):
             cache = caches[i] if caches is not None else None
@@ -570,6 +625,28 @@ class CausalLM(nn.Module):
         if residual is None:
             return self.model.norm(delta)
         return self.model.norm(delta, residual)[0]
+
+    def _step_natively(self, x, meta, caches):
+        """All layers of a serving step and the norm behind them in one call (``ops.infer.decoder_step``), which launches what the
+        modules' own ``forward`` would; None where a module is not as it was built here (replaced, adapted, hooked), or the operands
+        are not those of that call."""
+        a, layers, norm = self.arch, self.model.layers, self.model.norm
+        d = a.head_dim
+        if a.position != "rope" or self.model.hybrid or a.use_logn_attn or a.qkv_bias or a.o_bias or d % 16 or d > 128 or len(layers) == 0 or \
+                len(caches) != len(layers) or _global_hooks() or not iops.decoder_step_ok(x, meta) or a.hidden_size != x.shape[1]:
+            return None
+        w = _norm_weight(norm, x.shape[1], a.rms_norm_eps)
+        if w is None or not _plain(layers, nn.ModuleList):
+            return None
+        table = []
+        for layer, cache in zip(layers, caches):
+            t = layer.addresses(x.shape[1], meta, cache, a.rms_norm_eps) if type(layer) is DecoderLayer else None
+            if t is None:
+                return None
+            table.append(t)
+        fresh = bool(meta["fresh"]) and not meta["one_token"]
+        return iops.decoder_step(x, table, w, (a.num_attention_heads, a.kv_heads, d, a.intermediate_size), meta, fresh,
+                                 int(meta.get("kv_bound", meta["max_position"])), a.rms_norm_eps, layers[0].self_attn.scale)
 
     def forward(self, input_ids=None, attention_mask=None, labels=None, position_ids=None, cu_seqlens=None,
                 inputs_embeds=None, return_dict=True, **_):

@@ -22,8 +22,8 @@ OBJ_DIR = os.path.join(HERE, "_build")
 LIB_PATH = os.path.join(HERE, "libeasyllm_b200.so")
 # the kernels that serving a model loads and launches; `ensure_serving` builds these alone
 SERVE_LIB_PATH = os.path.join(HERE, "libeasyllm_b200_serve.so")
-SERVE_SOURCES = ("attn_rows", "elementwise", "flash_attn", "gemm", "gemm_pair", "gemm_thin", "infer_elementwise", "matvec", "norm",
-                 "optim", "recurrent", "scan_chunks")
+SERVE_SOURCES = ("attn_rows", "decoder_step", "elementwise", "flash_attn", "gemm", "gemm_pair", "gemm_thin", "infer_elementwise",
+                 "matvec", "norm", "optim", "recurrent", "scan_chunks")
 # sources whose fp32 results must keep full accuracy (no approximate exp / tanh / division)
 ACCURATE_SOURCES = ("attn_rows", "gemm_thin", "infer_elementwise", "matvec", "recurrent", "scan_chunks")
 

@@ -40,7 +40,7 @@ def lib():
                               "(or __graft_entry__.build()) before using the CUDA ops")
         _lib = ctypes.CDLL(_LIB_PATH if os.path.exists(_LIB_PATH) else _SERVE_LIB_PATH)
         for name in ("ell_rmsnorm_bwd_scratch_elems", "ell_attn_rows_scratch", "ell_attn_latent_scratch",
-                     "ell_scan_chunks_work"):
+                     "ell_scan_chunks_work", "ell_decoder_step_work"):
             getattr(_lib, name).restype = c_longlong
     return _lib
 
@@ -370,6 +370,14 @@ def set_gemm_pair(enabled):
 _PAIR_LAUNCH_REFUSED = (-20, 9, 701, 912)
 
 
+def pairs_refused(rc):
+    """The launch itself was refused (no device work was issued): this device cannot co-schedule the two-CTA cluster with the kernel's
+    shared memory.  The single-CTA kernel is used from here on."""
+    import warnings
+    warnings.warn(f"CTA-pair GEMM launch refused (code {rc}); using the single-CTA tcgen05 kernel")
+    set_gemm_pair(False)
+
+
 def _use_pair(M, N, bn):
     return _GEMM_PAIR and bn == 0 and M >= 256 and N >= 256 and (M % 256 == 0 or M >= 2048)
 
@@ -442,11 +450,7 @@ def gemm(a, b, out=None, bias=None, a_mn=False, b_mn=False, out_mode=0, bn=0, pa
         if rc not in _PAIR_LAUNCH_REFUSED:
             _check(rc, "gemm_bf16_pair")
             return out
-        # the launch itself was refused (no device work was issued): this device cannot co-schedule the two-CTA
-        # cluster with the kernel's shared memory.  Use the single-CTA kernel from here on.
-        import warnings
-        warnings.warn(f"CTA-pair GEMM launch refused (code {rc}); using the single-CTA tcgen05 kernel")
-        set_gemm_pair(False)
+        pairs_refused(rc)
     rc = lib().ell_gemm_bf16(_p(a), _p(b), _p(out), _p(bias), c_int(M), c_int(N), c_int(K), c_int(a.shape[1]),
                              c_int(b.shape[1]), c_int(N), c_int(1 if a_mn else 0), c_int(1 if b_mn else 0),
                              c_int(out_mode), c_int(bn), _p(err_flag(a.device)), _stream())

@@ -2,7 +2,7 @@
 and the tcgen05 GEMM / attention) for bf16 and fp32 CUDA tensors; the signatures are those of ``ops.infer``."""
 from __future__ import annotations
 
-from ctypes import c_float, c_int, c_longlong
+from ctypes import addressof, c_float, c_int, c_longlong
 
 import torch
 
@@ -195,6 +195,37 @@ def relu2_scaled(x, z):
     _check(lib().ell_relu2_scaled(_p(x), _p(z), _p(out), c_int(n), c_int(F), c_int(_rows(x, "x")), c_int(z.stride(0)),
                                   _bf(x.dtype), _stream()), "relu2_scaled")
     return out
+
+
+# ---- the layers of a decoder -----------------------------------------------------------------------
+_STEP_PARTS = ("", "rmsnorm_fwd", "gemm", "rope_append", "attention", "swiglu_fwd")
+_STEP_NO_PAIRS = -1000
+
+
+def decoder_step(x, layers, norm, sizes, meta, fresh, max_len, eps, scale):
+    """The normed rows behind the layers of a step (``csrc/decoder_step.cu``).  ``layers``: per layer the addresses of the weights (qkv,
+    o, gate and up, down, both norms), of its keys and values and of its rotary tables, and the rows of these; ``sizes``: query heads,
+    key heads, head size, feed-forward width.  The caller has looked the operands over and keeps them alive."""
+    T, W = x.shape
+    one = meta["one_token"]
+    flat = [v for l in layers for v in l]
+    table = (c_longlong * len(flat))(*flat)
+    y = torch.empty_like(x)
+    words = [addressof(table), x.data_ptr(), norm.data_ptr(), y.data_ptr(), 0, meta["position_ids"].data_ptr(),
+             meta["row_start"].data_ptr(), meta["kv_base"].data_ptr(), meta["kv_len"].data_ptr(), meta["cu_seqlens"].data_ptr(),
+             err_flag(x.device).data_ptr(), len(layers), T, W, *sizes, fresh, max_len, 0 if one else meta["cu_seqlens"].numel() - 1,
+             1 if one else meta["max_seqlen"], cu.gemm_pair_enabled(), 0, 0]
+    args = (c_longlong * len(words))(*words)
+    for _ in range(2):
+        work = torch.empty(lib().ell_decoder_step_work(args), dtype=torch.uint8, device=x.device)
+        args[4] = work.data_ptr()
+        rc = lib().ell_decoder_step(args, c_float(eps), c_float(scale), _stream())
+        if rc != _STEP_NO_PAIRS:
+            break
+        cu.pairs_refused(rc)
+        args[-3] = 0
+    _check(rc, f"decoder_step ({_STEP_PARTS[args[-1]]})" if rc else "decoder_step", args[-2])
+    return y
 
 
 # ---- attention -----------------------------------------------------------------------------------

@@ -10,7 +10,7 @@ from __future__ import annotations
 import torch
 import torch.nn.functional as F
 
-from . import _adjacent_alias
+from . import _adjacent_alias, get_backend, get_gemm_backend
 from . import reference_infer as ref
 
 _ROWS = 32              # recurrent state rows (key channels) are padded to a multiple of this
@@ -188,6 +188,30 @@ def relu2_scaled(x, z):
     if _kern(x):
         return _cu().relu2_scaled(x, z)
     return (torch.sigmoid(z).unsqueeze(-1) * torch.relu(x.float()) ** 2).to(x.dtype)
+
+
+# ---- the layers of a decoder in one call -----------------------------------------------------------
+_STEP_INTS = ("position_ids", "row_start", "kv_base", "kv_len", "cu_seqlens")
+
+
+def decoder_step_ok(x, meta):
+    """Whether ``decoder_step`` takes the rows ``x [T, W]`` and the index of the step."""
+    if not (x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and x.is_contiguous() and not x.data_ptr() & 15 and
+            get_backend() == "b200" and get_gemm_backend() == "tcgen05" and x.shape[0] > 0 and x.shape[1] % 8 == 0 and x.shape[1] <= 8192):
+        return False
+    if meta.get("tree_mask") is not None or not _cu().cu.nothing_to_record():
+        return False
+    for name in _STEP_INTS:
+        t = meta.get(name)
+        if t is None or t.dtype != torch.int32 or not t.is_cuda or not t.is_contiguous() or \
+                (t.numel() != x.shape[0] and name != "cu_seqlens"):
+            return False
+    return True
+
+
+def decoder_step(x, layers, norm, sizes, meta, fresh, max_len, eps, scale):
+    """Rows ``x`` through ``layers`` (addresses, see ``cuda_infer.decoder_step``) and the norm behind them."""
+    return _cu().decoder_step(x, layers, norm.detach(), sizes, meta, fresh, max_len, eps, scale)
 
 
 # ---- attention -----------------------------------------------------------------------------------

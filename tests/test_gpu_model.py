@@ -206,3 +206,120 @@ def test_what_the_recorded_functions_refuse_is_refused_without_gradients():
                     torch.func.vmap(f)(x)
                 with pytest.raises(RuntimeError), torch.autograd.forward_ad.dual_level():
                     f(torch.autograd.forward_ad.make_dual(x[0], torch.ones_like(x[0])))
+
+
+def _llama(width, heads, kv, ff, layers=2, **more):
+    from easyllm_b200.models.hf_models import CausalLM, arch_from_hf_config
+    cfg = {"model_type": "llama", "vocab_size": 512, "hidden_size": width, "intermediate_size": ff, "num_hidden_layers": layers,
+           "num_attention_heads": heads, "num_key_value_heads": kv, **more}
+    torch.manual_seed(0)
+    with torch.device("cuda"):
+        return CausalLM(arch_from_hf_config(cfg), dtype=torch.bfloat16).eval()
+
+
+def _steps(model, monkeypatch, counts, natively, capacity=512):
+    """Prompts that start, prompts that go on and one token each: everything that comes out or is kept, launches, and how many of the
+    steps one call issued."""
+    import easyllm_b200.ops.cuda as cu
+    from easyllm_b200.ops import infer
+    taken = []
+    step = infer.decoder_step
+    with monkeypatch.context() as m:
+        m.setattr(infer, "decoder_step", lambda *a: taken.append(1) or step(*a))
+        if not natively:
+            m.setattr(infer, "decoder_step_ok", lambda *a: False)
+        gen = torch.Generator().manual_seed(3)
+        state = model.new_state(len(counts), capacity)
+        slots = [state.open() for _ in counts]
+        before, out = cu.LAUNCHES, []
+        for n in (counts, counts, [1] * len(counts)):
+            h, meta = model.step(state, slots, [torch.randint(0, 512, (c,), generator=gen).cuda() for c in n])
+            out.append(model.logits(h[meta["last_rows"].cuda()]))
+            out.append(h)
+    cu.check_err_flag()
+    return out + [t for c in state.layers for t in (c.k, c.v)], cu.LAUNCHES - before, len(taken)
+
+
+# rows on both sides of the lines between the products: matrix-vector, few rows, single CTAs, CTA pairs (and the gated one)
+@pytest.mark.parametrize("counts", [[1], [3, 2], [16], [17], [77], [200, 57], [256], [1999, 1, 130]])
+@pytest.mark.parametrize("width,heads,kv,ff", [(1024, 8, 2, 2816), (256, 4, 4, 704), (768, 16, 16, 1024)])
+def test_layers_of_a_step_issued_by_one_call_give_the_bits_of_the_modules(width, heads, kv, ff, counts, monkeypatch):
+    _need_gpu()
+    model = _llama(width, heads, kv, ff)
+    a, la, na = _steps(model, monkeypatch, counts, True)
+    b, lb, nb = _steps(model, monkeypatch, counts, False)
+    assert (na, nb) == (3, 0) and la == lb
+    assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+def test_a_changed_module_of_a_step_is_called(monkeypatch):
+    """Hooks, replaced or adapted modules, biases, tables without rotation: the modules' own forward runs, with the same result."""
+    _need_gpu()
+    from torch import nn
+    want = _steps(_llama(256, 4, 2, 512), monkeypatch, [9, 4], True)[0]
+
+    def hooked(m, calls):
+        m.model.layers[1].mlp.up_proj.register_forward_hook(lambda *_: calls.append(1))
+        return m.model.layers[1].mlp
+
+    def replaced(m, calls):
+        class Own(nn.Linear):
+            def forward(self, x):
+                return super().forward(x)
+        lin = m.model.layers[0].self_attn.o_proj
+        lin.__class__ = Own
+
+    def patched(m, calls):
+        norm = m.model.layers[0].input_layernorm
+        forward = norm.forward
+        norm.forward = lambda *a: calls.append(1) or forward(*a)
+
+    def everywhere(m, calls):
+        handle = nn.modules.module.register_module_forward_hook(lambda *_: calls.append(1))
+        handles.append(handle)
+
+    handles = []
+    for change, called in ((hooked, False), (replaced, False), (patched, True), (everywhere, True)):
+        model, calls = _llama(256, 4, 2, 512), []
+        change(model, calls)
+        try:
+            got, _, taken = _steps(model, monkeypatch, [9, 4], True)
+        finally:
+            for h in handles:
+                h.remove()
+        assert taken == 0 and bool(calls) == called, change
+        assert all(torch.equal(x, y) for x, y in zip(got, want)), change
+    for more in ({"attention_bias": True}, {"model_type": "baichuan2-13b"}):
+        assert _steps(_llama(256, 4, 4, 512, **more), monkeypatch, [9, 4], True)[2] == 0
+    with torch.no_grad():                            # weights apart: they are copied together for the call, as before
+        model = _llama(256, 4, 2, 512)
+        model.fuse_weights = lambda: None
+        assert _steps(model, monkeypatch, [9, 4], True)[2] == 0
+
+
+def test_a_refused_launch_on_pairs_is_repeated_without(monkeypatch):
+    """The call comes back with the code of a refusal: the step is issued again on single CTAs, with a warning, and stays there."""
+    _need_gpu()
+    import easyllm_b200.ops.cuda as cu
+    import easyllm_b200.ops.cuda_infer as ci
+    model = _llama(512, 4, 2, 1024)
+    cu.set_gemm_pair(False)
+    try:
+        want = _steps(model, monkeypatch, [256], True)[0]
+        cu.set_gemm_pair(True)
+        real = cu.lib()
+
+        class Refusing:
+            def __getattr__(self, name):
+                return getattr(real, name)
+
+            def ell_decoder_step(self, args, *rest):
+                return ci._STEP_NO_PAIRS if args[len(args) - 3] else real.ell_decoder_step(args, *rest)
+
+        monkeypatch.setattr(ci, "lib", lambda: Refusing())
+        with pytest.warns(UserWarning, match="refused"):
+            got = _steps(model, monkeypatch, [256], True)[0]
+        assert not cu.gemm_pair_enabled()
+        assert all(torch.equal(x, y) for x, y in zip(got, want))
+    finally:
+        cu.set_gemm_pair(True)
