@@ -453,7 +453,8 @@ class DecoderLayer(nn.Module):
         if n1 is None or n2 is None or None in mats:
             return None
         cos, sin = at.rotary.get(int(meta["max_position"]), k.device)
-        return (*mats, n1.data_ptr(), n2.data_ptr(), k.data_ptr(), v.data_ptr(), cos.data_ptr(), sin.data_ptr(), cos.shape[0])
+        return (*mats, n1.data_ptr(), n2.data_ptr(), k.data_ptr(), v.data_ptr(), cos.data_ptr(), sin.data_ptr(), cos.shape[0],
+                k.shape[0] * k.shape[1])
 
 
 def _block_norm(a: HFArch, dtype):

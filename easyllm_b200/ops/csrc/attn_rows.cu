@@ -569,11 +569,11 @@ attn_latent_kernel(const __grid_constant__ CUtensorMap tmK, const AttnRowsArgs a
     }
 }
 
-// ---- bf16 rows over cached keys on mma.sync ------------------------------------------------------------
+// ---- bf16 rows over cached keys on matrix instructions ------------------------------------------------------------
 // Decoding reads every cached key and value once for a few query rows: bound by those bytes, if the arithmetic keeps up.
 // On the FMA pipe it did not (230 us for 64 rows x 2048 keys x 8 key heads, 537 MB, which take 83; 115 here); and a continued prompt
-// read its whole context once per token (1060 us for 301 tokens of two sequences over 3000, 115 here).  Here a tile of 16 rows is the consecutive tokens of one
-// sequence times the query heads of one key head, and m16n8k16 does the products:
+// read its whole context once per token (1060 us for 301 tokens of two sequences over 3000).  Here a tile of rows is the consecutive
+// tokens of one sequence times the query heads of one key head, and matrix instructions do the products:
 //   scores  exact bf16 products, fp32 sums, scale and bias applied in fp32
 //   values  the fp32 weights go in as three bf16 parts, so they keep their 24 bits.  With two parts, in turn for one accumulator at
 //           a time, 64 rows x 2048 keys took 136 us; with three, several accumulators taking turns, 125
@@ -582,12 +582,10 @@ attn_latent_kernel(const __grid_constant__ CUtensorMap tmK, const AttnRowsArgs a
 //                     softmax, accumulators and a ring of cp.async stages of its own; no barrier until their results meet.
 //                     Rows on the M side took 977 instructions a unit and 232 registers, and stayed at 162 us, bound by
 //                     the latency of eight warps an SM.
-//   attn_tile_kernel  more rows (continued prompts): a warp owns 16 of the CTA's 64 rows, tiles of 64 keys are shared
+//   attn_tile_kernel  more rows (continued prompts): 128 of them on tcgen05, see there
 // Ranges of keys and their merge are those of attn_rows_kernel.
 constexpr int kAtThreads = 128, kAtKRow = 256, kAtStages = 3;      // bytes of a key / value row in shared memory (up to 128)
 constexpr int kAtHeads = 16;                                       // most query heads of a CTA
-constexpr int kAtTile = 64, kAtUnit = 32, kAtRows = 64;            // attn_tile_kernel: keys of a stage, of a softmax step; rows
-constexpr int kAtStage = 2 * kAtTile * kAtKRow, kAtSmem = kAtStages * kAtStage;
 constexpr int kAfKeys = 16, kAfStage = 2 * kAfKeys * kAtKRow;      // attn_few_kernel: keys of a warp's unit
 constexpr int kAfSmem = 4 * kAtStages * kAfStage;
 
@@ -612,104 +610,17 @@ __device__ __forceinline__ void split_bf16(float x, float y, uint32_t (&p)[3]) {
   }
 }
 
-// What a thread keeps of its rows g and g + 8 (g = lane / 4).
-struct AtRows {
-  float m[2], l[2];                 // maximum; this lane's share of the sum
-  int first[2], end[2];             // keys the row sees, counted from the sequence's first row
-  float slope[2];
-};
-
-template <int UK>
-__device__ __forceinline__ void at_unit(const uint8_t* ks, const uint8_t* vs, int key0, bool mask, bool bias, float scale,
-                                        int ksteps, int vtiles, const uint32_t (&q)[8][4], AtRows& r, float (&acc)[16][4]) {
-  const int lane = threadIdx.x & 31, quad = lane >> 3, l8 = lane & 7, t = lane & 3;
-  float s[UK / 8][4];
+// The same by truncation: eight of the 24 bits a part.  Without the conversions, which share the unit of the exponential.
+__device__ __forceinline__ void cut_bf16(float x, float y, uint32_t (&p)[3]) {
 #pragma unroll
-  for (int n = 0; n < UK / 8; ++n)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) s[n][i] = 0.f;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    if (k < ksteps) {
-#pragma unroll
-      for (int n = 0; n < UK / 16; ++n) {
-        uint32_t b[4];
-        ldsm4(b, ks + at_place(n * 16 + (quad >> 1) * 8 + l8, k * 2 + (quad & 1)));
-        mma_bf16(s[2 * n], q[k], b[0], b[1]);
-        mma_bf16(s[2 * n + 1], q[k], b[2], b[3]);
-      }
-    }
-  }
-  float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-  for (int n = 0; n < UK / 8; ++n)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int h = i >> 1, key = key0 + n * 8 + 2 * t + (i & 1);
-      float x = s[n][i] * scale;
-      if (bias) x += r.slope[h] * (float)(key - (r.end[h] - 1));
-      if (mask && (key < r.first[h] || key >= r.end[h])) x = -INFINITY;
-      s[n][i] = x;
-      mx[h] = fmaxf(mx[h], x);
-    }
-  float al[2];
-  bool grew = false;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
-    mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
-    const float m = fmaxf(r.m[h], mx[h]);
-    grew |= m > r.m[h];
-    al[h] = m == -INFINITY ? 1.f : expf(r.m[h] - m);               // no key yet: nothing to rescale
-    r.m[h] = m;
-    r.l[h] *= al[h];
-  }
-  if (__any_sync(0xffffffffu, grew)) {
-#pragma unroll
-    for (int n = 0; n < 16; ++n) {
-      acc[n][0] *= al[0];
-      acc[n][1] *= al[0];
-      acc[n][2] *= al[1];
-      acc[n][3] *= al[1];
-    }
-  }
-#pragma unroll
-  for (int n = 0; n < UK / 8; ++n)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int h = i >> 1;
-      s[n][i] = r.m[h] == -INFINITY ? 0.f : expf(s[n][i] - r.m[h]);
-      r.l[h] += s[n][i];
-    }
-#pragma unroll
-  for (int k = 0; k < UK / 16; ++k) {
-    uint32_t w[3][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      uint32_t p[3];
-      split_bf16(s[2 * k + (i >> 1)][2 * (i & 1)], s[2 * k + (i >> 1)][2 * (i & 1) + 1], p);
-#pragma unroll
-      for (int x = 0; x < 3; ++x) w[x][i] = p[x];
-    }
-#pragma unroll
-    for (int n = 0; n < 8; n += 2) {
-      uint32_t b[2][4];
-#pragma unroll
-      for (int y = 0; y < 2; ++y)
-        if (n + y < vtiles) ldsm4_t(b[y], vs + at_place(k * 16 + (quad & 1) * 8 + l8, (n + y) * 2 + (quad >> 1)));
-#pragma unroll
-      for (int x = 0; x < 3; ++x)                      // products of one accumulator wait for one another: four take turns
-#pragma unroll
-        for (int y = 0; y < 2; ++y)
-          if (n + y < vtiles) {
-            mma_bf16(acc[2 * (n + y)], w[x], b[y][0], b[y][1]);
-            mma_bf16(acc[2 * (n + y) + 1], w[x], b[y][2], b[y][3]);
-          }
-    }
+  for (int i = 0; i < 3; ++i) {
+    p[i] = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+    x -= __uint_as_float(__float_as_uint(x) & 0xffff0000u);
+    y -= __uint_as_float(__float_as_uint(y) & 0xffff0000u);
   }
 }
 
-// One warp copies or four do: sixteen lanes take a row of KEYS keys and values, a 16-byte piece each.  Rows past the range are
+// Sixteen lanes of a warp take a row of KEYS keys and values, a 16-byte piece each.  Rows past the range are
 // zero-filled: their weight is 0, and 0 times what lies there must be 0.
 template <int KEYS, int THREADS>
 struct AtLoader {
@@ -1045,86 +956,335 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const __grid_co
   }
 }
 
-__global__ void __launch_bounds__(kAtThreads, 2) attn_tile_kernel(const __grid_constant__ AttnRowsArgs a, const int* __restrict__ cu, int tiles, int tt) {
-  chain_enter(cu);
-  extern __shared__ __align__(128) uint8_t atsm[];
+// ---- continued prompts on tcgen05 ----------------------------------------------------------------------
+// A CTA takes 128 rows (consecutive tokens of one sequence times the query heads of one key head) and a range of keys, in tiles of 64:
+//   warps 0-7  softmax: a thread owns a row, its TMEM lane, and half of a tile's keys (warps 4-7 the second half; the maxima meet in
+//              shared memory).  Fp32 weights go back to TMEM as three bf16 parts, so that the product with V keeps their 24 bits; O is
+//              rescaled where a maximum grew
+//   warp 8     issues: S = Q K^T (128 x 64), O += P_i V for the three parts (P from TMEM, V in place as an MN-major operand)
+//   warp 9     TMA: tiles of keys and values through a ring of two stages
+// TMEM columns: S 0-63, P_0 and P_1 over the scores that the threads have read, P_2 64-95, O 128-255.  That is half of TMEM, and 97 KB
+// of shared memory, so two CTAs share an SM: one's softmax runs beside the other's products.  Bound by the chain of a tile, from the
+// scores (8 products) through the softmax to the 12 products of its parts.  On mma.sync a warp owned 16 rows and walked its chain alone.
+// us, kernel and merge: 301 tokens of two sequences over 3000, 16 heads on 8, 114 -> 42; 512 tokens over 4096, 32 on 8, 519 -> 113; 512
+// over 1000 beside three of 16 tokens, 16 on 4, 100 -> 63; 17 over 3000 24 -> 16; 33 over 64, 32 on 8, 16 -> 11.  With four warps, a
+// row a thread, 48 and 126; with expf and conversions to bf16, which share a unit, in place of ex2 and truncation, 54 and 151.
+// Results are as far from 64 bits as before (the rounding to bf16, 1.65e-3); in fp32 in front of it 2.4e-6, where mma.sync had 1.6e-6.
+constexpr int kAtTile = 64, kAtRows = 128, kAtTileThreads = 320, kAtHalf = kAtTile / 2;
+constexpr int kAtQChunk = kAtRows * 128, kAtKvChunk = kAtTile * 128;     // [rows x 64 columns], 128-byte swizzle rows
+constexpr int kAtQBytes = 2 * kAtQChunk, kAtStage = 4 * kAtKvChunk;      // a stage: keys, values
+constexpr int kAtBars = kAtQBytes + 2 * kAtStage, kAtSmem = kAtBars + 1024 + 2560;
+constexpr int kAtErr = 15;
+constexpr float kLog2e = 1.4426950408889634f;
+
+struct AtShared {
+  uint64_t q_full, full[2], empty[2], s_full, p_full, o_full;
+  uint32_t tmem_base;
+  int gave_up;
+  float met[2][2][kAtRows];       // by turns: what the threads of a row have found in their half of the keys
+};
+static_assert(sizeof(AtShared) <= 2560, "");
+
+// Barrier of the two warps of 32 rows; whether any of their threads has failed.
+__device__ __forceinline__ bool at_pair_failed(int quad, bool failed) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "barrier.red.or.pred p, %2, 64, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(any) : "r"((uint32_t)failed), "r"(quad + 1) : "memory");
+  return any != 0;
+}
+
+__global__ void __launch_bounds__(kAtTileThreads, 2)
+attn_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ AttnRowsArgs a,
+                 const int* __restrict__ cu, int tiles, int tt) {
+  using namespace sm100;
+  extern __shared__ uint8_t atsm_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(atsm_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* kv = smem + kAtQBytes;
+  AtShared* sh = reinterpret_cast<AtShared*>(smem + kAtBars);
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  if (warp == 8) tmem_alloc<256>(&sh->tmem_base);
+  chain_next();
+  chain_wait(cu);
   AtTile T;
-  if (!T.init(a, cu, tiles, tt)) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, t = lane & 3;
-  const int ksteps = a.d / 16, vtiles = a.dv / 16, row0 = warp * 16;
-  const AtLoader<kAtTile, kAtThreads> loader(a, T.base, T.g, T.k0, T.k1, threadIdx.x);
-#pragma unroll
-  for (int i = 0; i < kAtStages - 1; ++i) loader.load(i, atsm + i * kAtStage);
-  uint32_t q[8][4];
-  AtRows r;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int m = min(row0 + gr + 8 * h, T.rows - 1), tok = T.token(m), head = T.head(m);      // rows past the end repeat the last
-    const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(a.q) + (size_t)tok * a.ldq + (size_t)head * a.d + 2 * t;
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-#pragma unroll
-      for (int c = 0; c < 2; ++c) q[k][2 * c + h] = k < ksteps ? *reinterpret_cast<const uint32_t*>(src + k * 16 + c * 8) : 0u;
-    r.end[h] = a.len[tok];
-    r.first[h] = max(0, r.end[h] - a.window);
-    r.slope[h] = a.slopes != nullptr ? a.slopes[head] : 0.f;
-    r.m[h] = -INFINITY;
-    r.l[h] = 0.f;
+  const bool any = T.init(a, cu, tiles, tt);
+  const int rows = any ? T.rows : 0, warps = any ? (rows + 31) / 32 : 1;  // groups of 32 rows
+  if (threadIdx.x == 0) {
+    mbar_init(&sh->q_full, 2 * warps);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&sh->full[i], 1);
+      mbar_init(&sh->empty[i], 1);
+    }
+    mbar_init(&sh->s_full, 1);
+    mbar_init(&sh->p_full, 2 * warps);
+    mbar_init(&sh->o_full, 1);
+    sh->gave_up = *(volatile int*)a.err;               // an earlier kernel already failed: do not wait on anything
+    fence_barrier_init();
   }
-  float acc[16][4];
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = sh->tmem_base;
+  volatile int* gave_up = &sh->gave_up;
+  const bool dead = *gave_up != 0;
+  const int n_tiles = any && T.k1 > T.k0 ? (T.k1 - T.k0 + kAtTile - 1) / kAtTile : 0;
+  const int kc = (a.d + 63) / 64, vc = (a.dv + 63) / 64;                // 64-column chunks of a key, of a value
+  auto fail = [&]() {
+    *gave_up = 1;
+    atomicCAS(a.err, 0, kAtErr);
+  };
+
+  if (!any || dead) {
+    // nothing was issued
+  } else if (warp == 9) {
+    if (lane == 0) {
+      for (int j = 0; j < n_tiles; ++j) {
+        const int s = j & 1, row = (int)T.base + T.k0 + j * kAtTile;    // rows past the tensor are zero-filled
+        if (!mbar_wait(&sh->empty[s], ((j >> 1) & 1) ^ 1, gave_up)) {
+          fail();
+          break;
+        }
+        mbar_expect_tx(&sh->full[s], (kc + vc) * kAtKvChunk);
+        uint8_t* st = kv + s * kAtStage;
+        for (int c = 0; c < kc; ++c) tma_load_3d(st + c * kAtKvChunk, &tmK, &sh->full[s], c * 64, T.g, row);
+        for (int c = 0; c < vc; ++c) tma_load_3d(st + (2 + c) * kAtKvChunk, &tmV, &sh->full[s], c * 64, T.g, row);
+      }
+    }
+  } else if (warp == 8) {
+    constexpr uint32_t idesc_s = make_idesc_bf16(128, kAtTile, false, false);
+    const uint32_t idesc_o = make_idesc_bf16(128, a.dv, false, true);
+    const uint32_t e = elect_one(), tm = __reduce_or_sync(0xffffffffu, tmem);
+    const uint64_t q_desc = make_smem_desc(smem_u32(smem), 16, 1024), k_desc = make_smem_desc(smem_u32(kv), 16, 1024);
+    const uint64_t v_desc = make_smem_desc(smem_u32(kv) + 2 * kAtKvChunk, kAtKvChunk, 1024);
+    const int ksteps = a.d / 16;
+    // The scores of a tile go over the parts of the one before: those products were issued earlier, and are taken in order.
+    auto scores = [&](int j) -> bool {
+      const int s = j & 1;
+      if (!mbar_wait_warp(&sh->full[s], (j >> 1) & 1, gave_up)) return false;
+      tc_fence_after();
+      const uint64_t kd = k_desc + s * (kAtStage >> 4);
+      if (ksteps == 8) {
 #pragma unroll
-  for (int n = 0; n < 16; ++n)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
-  const int n_tiles = T.k1 > T.k0 ? (T.k1 - T.k0 + kAtTile - 1) / kAtTile : 0;
-  for (int tile = 0; tile < n_tiles; ++tile) {
-    cp_async_wait<kAtStages - 2>();
-    __syncthreads();
-    loader.load(tile + kAtStages - 1, atsm + (tile + kAtStages - 1) % kAtStages * kAtStage);   // free since the step before
-    const uint8_t* ks = atsm + tile % kAtStages * kAtStage;
-    const uint8_t* vs = ks + kAtTile * kAtKRow;
-    if (row0 < T.rows) {
+        for (int k = 0; k < 8; ++k)
+          umma_bf16_warp(e, tm, q_desc + (((k >> 2) * kAtQChunk + (k & 3) * 32) >> 4), kd + (((k >> 2) * kAtKvChunk + (k & 3) * 32) >> 4),
+                         idesc_s, k != 0);
+      } else {
 #pragma unroll 1
-      for (int u = 0; u < kAtTile; u += kAtUnit) {
-        const int key = T.k0 + tile * kAtTile + u;
-        if (key >= T.k1) break;
-        const bool mask = key + kAtUnit > min(T.len0, T.k1) || key < T.last_first;
-        at_unit<kAtUnit>(ks + u * kAtKRow, vs + u * kAtKRow, key, mask, a.slopes != nullptr, a.scale, ksteps, vtiles, q, r, acc);
+        for (int k = 0; k < ksteps; ++k)
+          umma_bf16_warp(e, tm, q_desc + (((k >> 2) * kAtQChunk + (k & 3) * 32) >> 4), kd + (((k >> 2) * kAtKvChunk + (k & 3) * 32) >> 4),
+                         idesc_s, k != 0);
       }
+      umma_commit_warp(e, &sh->s_full);
+      return true;
+    };
+    bool ok = n_tiles == 0 || (mbar_wait_warp(&sh->q_full, 0, gave_up) && scores(0));
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      const int s = j & 1;
+      ok = mbar_wait_warp(&sh->p_full, j & 1, gave_up);
+      if (!ok) break;
+      tc_fence_after();
+      const uint64_t vd = v_desc + s * (kAtStage >> 4);
+#pragma unroll
+      for (int x = 0; x < 3; ++x)
+#pragma unroll
+        for (int k = 0; k < kAtTile / 16; ++k)
+          umma_bf16_ts_warp(e, tm + 128, tm + x * 32 + k * 8, vd + ((k * 2048) >> 4), idesc_o, (j | x | k) != 0);
+      umma_commit_warp(e, &sh->empty[s]);
+      if (j + 1 < n_tiles) ok = scores(j + 1);
+      else umma_commit_warp(e, &sh->o_full);
+    }
+    if (!ok && e) fail();
+  } else if ((warp & 3) < warps) {
+    const int quad = warp & 3, half = warp >> 2, row = quad * 32 + lane;
+    const int m = min(row, rows - 1), tok = T.token(m), head = T.head(m);                   // rows past the end repeat the last
+    {
+      const __nv_bfloat16* q = reinterpret_cast<const __nv_bfloat16*>(a.q);
+      const bool wide = a.ldq % 8 == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0;
+      const unsigned long long mine = reinterpret_cast<unsigned long long>(q + (size_t)tok * a.ldq + (size_t)head * a.d);
+      if (wide) {                                      // sixteen lanes a row, each warp half of the rows
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+          const int r = half * 16 + i + (lane >> 4), piece = lane & 15, at = quad * 32 + r;
+          const uint4* src = reinterpret_cast<const uint4*>(__shfl_sync(0xffffffffu, mine, r)) + piece;
+          if (piece * 8 < kc * 64)
+            *reinterpret_cast<uint4*>(smem + (piece >> 3) * kAtQChunk + at * 128 + (((piece ^ at) & 7) << 4)) =
+                piece * 8 < a.d ? *src : make_uint4(0, 0, 0, 0);
+        }
+      } else {
+#pragma unroll 4
+        for (int i = 0; i < 32; ++i) {
+          const int r = half * 16 + (i >> 1), word = (i & 1) * 32 + lane, at = quad * 32 + r, piece = word >> 2;
+          const uint32_t* src = reinterpret_cast<const uint32_t*>(__shfl_sync(0xffffffffu, mine, r)) + word;
+          if (word * 2 < kc * 64)
+            *reinterpret_cast<uint32_t*>(smem + (piece >> 3) * kAtQChunk + at * 128 + (((piece ^ at) & 7) << 4) + (word & 3) * 4) =
+                word * 2 < a.d ? *src : 0u;
+        }
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh->q_full);
+    }
+    const int end = a.len[tok], first = max(0, end - a.window);
+    const bool bias = a.slopes != nullptr;
+    const float slope = bias ? a.slopes[head] : 0.f;
+    const uint32_t t_row = tmem + ((uint32_t)(quad * 32) << 16), t_s = t_row + half * kAtHalf, t_p = t_row + half * (kAtHalf / 2);
+    const uint32_t t_o = t_row + 128;
+    const int o_end = min(a.dv, half * 64 + 64);       // this thread's columns of O: half * 64 .. o_end - 1
+    float mx = -INFINITY, l = 0.f;
+    bool failed = false;
+    for (int j = 0; j < n_tiles; ++j) {
+      // this also says that the products of the step before have been added: they were issued earlier
+      failed = !mbar_wait(&sh->s_full, j & 1, gave_up);
+      __syncwarp();
+      tc_fence_after();
+      uint32_t s[kAtHalf];
+      tmem_ld_32x32(t_s, s);
+      tmem_ld_wait();
+      const int key0 = T.k0 + j * kAtTile + half * kAtHalf;
+#pragma unroll
+      for (int i = 0; i < kAtHalf; ++i) s[i] = __float_as_uint(__uint_as_float(s[i]) * a.scale);
+      if (bias) {
+#pragma unroll
+        for (int i = 0; i < kAtHalf; ++i)
+          s[i] = __float_as_uint(fmaf(slope, (float)(key0 + i - (end - 1)), __uint_as_float(s[i])));
+      }
+      if (key0 + kAtHalf > min(T.len0, T.k1) || key0 < T.last_first) {
+        const int lo = first - key0, hi = end - 1 - key0;
+        uint32_t seen = hi < 0 ? 0u : 0xffffffffu >> (31 - min(hi, 31));
+        if (lo > 0) seen = lo > 31 ? 0u : seen & (0xffffffffu << lo);
+#pragma unroll
+        for (int i = 0; i < kAtHalf; ++i)
+          if (!(seen >> i & 1)) s[i] = 0xff800000u;    // -inf
+      }
+      float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int i = 0; i < kAtHalf; i += 8)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) m4[x] = fmax3(m4[x], __uint_as_float(s[i + 2 * x]), __uint_as_float(s[i + 2 * x + 1]));
+      const float here = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+      sh->met[j & 1][half][row] = here;
+      // both have read their scores too: the parts may go over them
+      tc_fence_before();
+      if (at_pair_failed(quad, failed)) {
+        failed = true;
+        break;
+      }
+      tc_fence_after();
+      const float now = fmaxf(mx, fmaxf(here, sh->met[j & 1][half ^ 1][row]));
+      if (__any_sync(0xffffffffu, now > mx)) {
+        const float al = now == -INFINITY ? 1.f : ex2_approx((mx - now) * kLog2e);           // no key yet: nothing to rescale
+        mx = now;
+        l *= al;
+        if (j > 0) {
+#pragma unroll 1
+          for (int c = half * 64; c < o_end; c += 32) {
+            uint32_t v[32];
+            tmem_ld_32x32(t_o + c, v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * al);
+            tmem_st_32x32(t_o + c, v);
+          }
+        }
+      }
+      const float ref = mx == -INFINITY ? 0.f : mx;    // no key yet: all weights 0
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int c = 0; c < kAtHalf; c += 16) {
+        uint32_t part[3][8];
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+          const float p0 = ex2_approx((__uint_as_float(s[c + i]) - ref) * kLog2e), p1 = ex2_approx((__uint_as_float(s[c + i + 1]) - ref) * kLog2e);
+          sum[i & 2] += p0;
+          sum[(i & 2) + 1] += p1;
+          uint32_t p[3];
+          cut_bf16(p0, p1, p);
+#pragma unroll
+          for (int x = 0; x < 3; ++x) part[x][i >> 1] = p[x];
+        }
+#pragma unroll
+        for (int x = 0; x < 3; ++x) tmem_st_32x8(t_p + x * 32 + c / 2, part[x]);
+      }
+      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh->p_full);
+    }
+    sh->met[n_tiles & 1][half][row] = l;
+    if (n_tiles > 0 && !failed) failed = !mbar_wait(&sh->o_full, 0, gave_up);
+    failed = at_pair_failed(quad, failed);
+    tc_fence_after();
+    if (failed) {
+      fail();
+    } else {
+      l += sh->met[n_tiles & 1][half ^ 1][row];
+      // Rows leave 32 columns at a time through the warp's own place in the stages, which nobody reads any more, so that a store
+      // covers neighbouring columns.
+      float* stage = reinterpret_cast<float*>(kv) + warp * 32 * 33;
+      float f = 1.f, *part = nullptr;
+      __nv_bfloat16* out = T.place(a, m, mx, l, f, part);
+      if (row < rows && half == 0 && part != nullptr) {
+        part[0] = mx;
+        part[1] = l;
+      }
+      const unsigned long long to = part != nullptr ? reinterpret_cast<unsigned long long>(part + 2) : reinterpret_cast<unsigned long long>(out);
+      const int n_rows = min(32, rows - quad * 32);
+      float probe = l * 0.f;                           // NaN once a value is not finite
+      for (int c = half * 64; c < o_end; c += 32) {
+        uint32_t v[32];
+        if (n_tiles > 0) {
+          tmem_ld_32x32(t_o + c, v);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = 0u;
+        }
+        const int cols = min(32, o_end - c);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const float x = i < cols ? __uint_as_float(v[i]) : 0.f;
+          probe = fmaf(x, 0.f, probe);
+          stage[lane * 33 + i] = x * f;
+        }
+        __syncwarp();
+        if (part != nullptr) {
+#pragma unroll 8
+          for (int r = 0; r < n_rows; ++r) {
+            float* dst = reinterpret_cast<float*>(__shfl_sync(0xffffffffu, to, r)) + c;
+            if (lane < cols) dst[lane] = stage[r * 33 + lane];
+          }
+        } else {
+#pragma unroll 4
+          for (int r = 0; r < n_rows; r += 2) {        // two rows a store, two columns a lane
+            const int rr = r + (lane >> 4), col = (lane & 15) * 2;
+            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(__shfl_sync(0xffffffffu, to, rr & 31)) + c + col;
+            if (rr < n_rows && col < cols)
+              *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(stage[rr * 33 + col], stage[rr * 33 + col + 1]);
+          }
+        }
+        __syncwarp();
+      }
+      // rows with values that are not finite, once both halves of them are written
+      sh->met[(n_tiles & 1) ^ 1][half][row] = not_finite(probe) ? 1.f : 0.f;
+      at_pair_failed(quad, false);
+      const bool odd_row = row < rows && half == 0 && sh->met[(n_tiles & 1) ^ 1][0][row] + sh->met[(n_tiles & 1) ^ 1][1][row] > 0.f;
+      for (uint32_t odd = __ballot_sync(0xffffffffu, odd_row); odd != 0; odd &= odd - 1) at_row_alone(a, T, quad * 32 + __ffs(odd) - 1);
     }
   }
-  uint32_t odd_rows = 0;                             // of the warp's sixteen
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    r.l[h] += __shfl_xor_sync(0xffffffffu, r.l[h], 1);
-    r.l[h] += __shfl_xor_sync(0xffffffffu, r.l[h], 2);
-    float probe = r.l[h] * 0.f;                      // NaN once a value is not finite
-#pragma unroll
-    for (int n = 0; n < 16; ++n) probe = fmaf(acc[n][2 * h], 0.f, fmaf(acc[n][2 * h + 1], 0.f, probe));
-    const uint32_t lanes = __ballot_sync(0xffffffffu, not_finite(probe));
-#pragma unroll
-    for (int x = 0; x < 8; ++x)
-      if (lanes >> 4 * x & 15) odd_rows |= 1u << (8 * h + x);
-    const int m = row0 + gr + 8 * h;
-    if (m >= T.rows) continue;
-    float f, *part;
-    __nv_bfloat16* out = T.place(a, m, r.m[h], r.l[h], f, part);
-    if (part != nullptr && t == 0) {
-      part[0] = r.m[h];
-      part[1] = r.l[h];
-    }
-#pragma unroll
-    for (int n = 0; n < 16; ++n) {
-      if (n < 2 * vtiles) {
-        const int c = n * 8 + 2 * t;
-        if (part != nullptr) *reinterpret_cast<float2*>(part + 2 + c) = make_float2(acc[n][2 * h], acc[n][2 * h + 1]);
-        else *reinterpret_cast<__nv_bfloat162*>(out + c) = __floats2bfloat162_rn(acc[n][2 * h] * f, acc[n][2 * h + 1] * f);
-      }
+  tc_fence_before();
+  __syncthreads();
+  if (*gave_up && !dead && threadIdx.x == 0) {         // copies and products still in flight end before their memory goes away
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) {
     }
   }
-  __syncwarp();
-  for (int x = 0; x < 16; ++x)
-    if (odd_rows >> x & 1 && row0 + x < T.rows) at_row_alone(a, T, row0 + x);
+  __syncthreads();
+  if (warp == 8) {
+    tc_fence_after();
+    tmem_dealloc<256>(tmem);
+  }
 }
 
 // How a call runs on these kernels: tokens and CTAs of a tile, ranges of keys.  One sequence per `cu` entry, or one token
@@ -1166,10 +1326,11 @@ static AtPlan at_plan(int n, int n_seq, int max_q, int H, int G, int d, int dv, 
   const long long ctas = (long long)(one ? n : n_seq * p.tiles) * G * groups;
   if (window > 0 && max_len > window) max_len = window;
   max_len += p.tt - 1;                                  // a tile's rows see windows that start apart
-  // the tiles of continued prompts differ in length, so they are dealt finer than the two CTAs that fit an SM
+  // Continued prompts: as many ranges as the two CTAs that fit an SM leave room for.  One CTA an SM or three, 301 tokens over 3000: 62 and
+  // 72 us where two took 54; 512 over 4096 219 and 193, 151; four, where tiles differ most (512 beside three of 16 tokens) 67, 87.
   const long long most = (max_len + 127) / 128;
   long long s = p.few ? at_ranges(ctas, most < kArMaxSplits ? most : kArMaxSplits, (double)max_len * (d + dv) * 2)
-                      : (4LL * kNumSMs + ctas - 1) / ctas;
+                      : 2LL * kNumSMs / ctas;
   if (s > most) s = most;
   if (s > kArMaxSplits) s = kArMaxSplits;
   p.splits = s < 1 ? 1 : (int)s;
@@ -1177,28 +1338,41 @@ static AtPlan at_plan(int n, int n_seq, int max_q, int H, int G, int d, int dv, 
   return p;
 }
 
+int make_tmap_bf16_2d(CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t outer, uint64_t row_stride_bytes,
+                      uint32_t box_inner, uint32_t box_outer);
+int make_tmap_bf16_heads(CUtensorMap* map, const void* ptr, uint64_t dim, uint64_t heads, uint64_t rows, uint64_t row_stride_bytes,
+                         uint32_t box_dim, uint32_t box_rows, uint64_t head_stride_bytes);
+
 template <typename Kernel>
-static int launch_at(Kernel kern, int smem, bool& configured, const AttnRowsArgs& a, const AtPlan& p, const int* cu, int n_seq,
-                     cudaStream_t stream) {
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
-  const int rep = a.H / a.G, groups = (rep + kAtHeads - 1) / kAtHeads;
-  const bool one = p.tt == 1;
-  dim3 grid(one ? a.n : n_seq * p.tiles, a.G * groups, p.splits);
+static int allow_smem(Kernel kern, int smem, bool& configured) {
+  if (configured) return 0;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  configured = e == cudaSuccess;
+  return (int)e;
+}
+static int launch_attn_cached(const AttnRowsArgs& a, const AtPlan& p, const int* cu, int n_seq, long long rows, cudaStream_t stream) {
+  static bool few8 = false, few16 = false, tile = false;
+  const int rep = a.H / a.G, nh = rep < kAtHeads ? rep : kAtHeads, groups = (rep + kAtHeads - 1) / kAtHeads;
+  if (p.tt == 1) cu = nullptr;
+  const dim3 grid(p.tt == 1 ? a.n : n_seq * p.tiles, a.G * groups, p.splits);
   if (grid.y > 65535) return -2;
-  launch_chained(kern, grid, kAtThreads, smem, stream, a, one ? nullptr : cu, p.tiles, p.tt);
+  int rc;
+  if (!p.few) {
+    CUtensorMap tk, tv;
+    rc = make_tmap_bf16_heads(&tk, a.k, a.d, a.G, rows, (uint64_t)a.ldk * 2, 64, kAtTile, 0);
+    if (!rc) rc = make_tmap_bf16_heads(&tv, a.v, a.dv, a.G, rows, (uint64_t)a.ldv * 2, 64, kAtTile, 0);
+    if (!rc) rc = allow_smem(attn_tile_kernel, kAtSmem, tile);
+    if (rc) return rc;
+    launch_chained(attn_tile_kernel, grid, kAtTileThreads, kAtSmem, stream, tk, tv, a, cu, p.tiles, p.tt);
+  } else if (p.tt * nh <= 8) {
+    if ((rc = allow_smem(attn_few_kernel<1>, kAfSmem, few8)) != 0) return rc;
+    launch_chained(attn_few_kernel<1>, grid, kAtThreads, kAfSmem, stream, a, cu, p.tiles, p.tt);
+  } else {
+    if ((rc = allow_smem(attn_few_kernel<2>, kAfSmem, few16)) != 0) return rc;
+    launch_chained(attn_few_kernel<2>, grid, kAtThreads, kAfSmem, stream, a, cu, p.tiles, p.tt);
+  }
   if (a.splits > 1) launch_chained(attn_rows_merge_kernel<__nv_bfloat16>, dim3(a.n, a.H), kArThreads, 0, stream, a);
   return launch_status();
-}
-static int launch_attn_tile(const AttnRowsArgs& a, const AtPlan& p, const int* cu, int n_seq, cudaStream_t stream) {
-  static bool few8 = false, few16 = false, tile = false;
-  if (!p.few) return launch_at(attn_tile_kernel, kAtSmem, tile, a, p, cu, n_seq, stream);
-  const int rep = a.H / a.G;
-  return p.tt * (rep < kAtHeads ? rep : kAtHeads) <= 8 ? launch_at(attn_few_kernel<1>, kAfSmem, few8, a, p, cu, n_seq, stream)
-                                                       : launch_at(attn_few_kernel<2>, kAfSmem, few16, a, p, cu, n_seq, stream);
 }
 
 static int al_mt(int H) { return H > 16 ? 2 : 1; }
@@ -1212,9 +1386,6 @@ static int attn_latent_splits(int n, int H, int max_len) {
   if (s > kArMaxSplits) s = kArMaxSplits;
   return s < 1 ? 1 : (int)s;
 }
-
-int make_tmap_bf16_2d(CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t outer, uint64_t row_stride_bytes,
-                      uint32_t box_inner, uint32_t box_outer);
 
 template <int MT>
 static int launch_attn_latent(const AttnRowsArgs& a, long long rows, cudaStream_t stream) {
@@ -1291,26 +1462,26 @@ ELL_API long long ell_attn_rows_scratch(int n, int H, int G, int d, int dv, int 
 // Rows of ldq / ldk / ldv elements; max_len bounds len[] (it sets the number of ranges, longer rows would be cut).
 // window: keys a row sees (<= 0: all).  gate: rows of ldg elements of the activation type, or null.
 // cu [n_seq + 1] (or null): rows cu[i] .. cu[i + 1] - 1 are consecutive tokens of one sequence, with one base and lengths that
-// grow by one; max_q bounds their number.
+// grow by one; max_q bounds their number.  kv_rows: rows of k and v.
 ELL_API int ell_attn_rows(const void* q, const void* k, const void* v, void* out, float* part, const int* base,
                           const int* len, const float* sink, const float* slopes, const void* gate, int n, int H, int G,
                           int d, int dv, int ldq, int ldk, int ldv, int ldg, int max_len, int window, float scale,
-                          const int* cu, int n_seq, int max_q, int is_bf16, cudaStream_t stream) {
+                          const int* cu, int n_seq, int max_q, long long kv_rows, int is_bf16, int* err, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (H % G || dv > 8 * kArThreads || H > 65535) return -2;
   const AtPlan p = at_plan(n, cu != nullptr ? n_seq : 0, max_q, H, G, d, dv, max_len, window, is_bf16);
   if (window <= 0) window = 0x7fffffff;
   if (max_len > window) max_len = window;
-  AttnRowsArgs a{q, k, v, out, part, base, len, sink, slopes, n, H, G, d, dv, ldq, ldk, ldv, 1, 0, scale, window, gate, ldg, nullptr, 0};
+  AttnRowsArgs a{q, k, v, out, part, base, len, sink, slopes, n, H, G, d, dv, ldq, ldk, ldv, 1, 0, scale, window, gate, ldg, err, 0};
   const int esz = is_bf16 ? 2 : 4;
   const bool vec = (d * esz) % 16 == 0 && (dv * esz) % 16 == 0 && (ldk * esz) % 16 == 0 && (ldv * esz) % 16 == 0 &&
                    aligned_to(k, 16) && aligned_to(v, 16);
-  if (p.fits && vec && ldq % 2 == 0 && aligned_to(q, 4)) {
+  if (p.fits && vec && ldq % 2 == 0 && aligned_to(q, 4) && (p.few || kv_rows <= 0x7fffffff)) {
     a.splits = p.splits;
     a.range = p.range;
     a.all_ranges = p.tt > 1;
     if (a.splits > 1 && part == nullptr) return -2;
-    return launch_attn_tile(a, p, cu, n_seq, stream);
+    return launch_attn_cached(a, p, cu, n_seq, kv_rows, stream);
   }
   a.splits = attn_rows_splits(n, H, G, max_len);
   a.range = ((max_len + a.splits - 1) / a.splits + 63) / 64 * 64;
@@ -1338,7 +1509,7 @@ ELL_API int ell_attn_latent(const void* q, const void* k, void* out, float* part
   if (n <= 0) return 0;
   if (!(is_bf16 && attn_latent_fits(k, d, dv, ldq, ldk, H)))
     return ell_attn_rows(q, k, k, out, part, base, len, nullptr, nullptr, gate, n, H, 1, d, dv, ldq, ldk, ldk, ldg, max_len,
-                         window, scale, nullptr, 0, 1, is_bf16, stream);
+                         window, scale, nullptr, 0, 1, rows, is_bf16, err, stream);
   if (!aligned_to(q, 16) || !aligned_to(k, 16) || !aligned_to(out, 16) || rows > 0x7fffffff) return -2;
   if (window <= 0) window = 0x7fffffff;
   if (max_len > window) max_len = window;

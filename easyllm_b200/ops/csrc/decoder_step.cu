@@ -30,18 +30,18 @@ ELL_API int ell_flash_attn_fwd(const void* q, const void* k, const void* v, void
 ELL_API long long ell_attn_rows_scratch(int n, int H, int G, int d, int dv, int max_len, int window, int n_seq, int max_q, int is_bf16);
 ELL_API int ell_attn_rows(const void* q, const void* k, const void* v, void* out, float* part, const int* base, const int* len,
                           const float* sink, const float* slopes, const void* gate, int n, int H, int G, int d, int dv, int ldq, int ldk,
-                          int ldv, int ldg, int max_len, int window, float scale, const int* cu, int n_seq, int max_q, int is_bf16,
-                          cudaStream_t stream);
+                          int ldv, int ldg, int max_len, int window, float scale, const int* cu, int n_seq, int max_q,
+                          long long kv_rows, int is_bf16, int* err, cudaStream_t stream);
 
 namespace ell {
 
-// One layer: weights [(Hq + 2 Hk) D, W], [W, Hq D], [2 F, W] (gate first), [W, F], the norms' [W]; the cache's keys and values as rows
-// of Hk D; rotary tables fp32 [table_rows, D / 2].
+// One layer: weights [(Hq + 2 Hk) D, W], [W, Hq D], [2 F, W] (gate first), [W, F], the norms' [W]; the cache's keys and values as kv_rows
+// rows of Hk D; rotary tables fp32 [table_rows, D / 2].
 struct StepLayer {
   const void *qkv, *o, *gate_up, *down, *norm1, *norm2;
   void *kc, *vc;
   const float *cos, *sin;
-  long long table_rows;
+  long long table_rows, kv_rows;
 };
 struct StepArgs {
   const StepLayer* layers;
@@ -55,7 +55,7 @@ struct StepArgs {
   long long pairs;                // whether products may run on CTA pairs
   long long launches, failed;     // out: launches; the kind of launch that failed
 };
-static_assert(sizeof(StepLayer) == 11 * 8 && sizeof(StepArgs) == 25 * 8, "the caller lays them out as 64-bit words");
+static_assert(sizeof(StepLayer) == 12 * 8 && sizeof(StepArgs) == 25 * 8, "the caller lays them out as 64-bit words");
 enum StepPart { kStepNorm = 1, kStepProduct, kStepRotation, kStepAttention, kStepActivation };
 constexpr int kStepNoPairs = -1000;                  // a launch on CTA pairs was refused: the call is repeated without
 
@@ -143,7 +143,7 @@ static int step_layers(StepArgs& a, float eps, float scale, cudaStream_t stream)
     } else {
       ELL_STEP(kStepAttention, ell_attn_rows(qkv, l.kc, l.vc, att, at.ranges ? part : nullptr, a.kv_base, a.kv_len, nullptr, nullptr, nullptr, T, Hq, Hk, D, D,
                                              ld, Hk * D, Hk * D, 0, (int)a.max_len, 0, scale, a.n_seq ? a.cu : nullptr, (int)a.n_seq,
-                                             (int)a.max_q, 1, stream));
+                                             (int)a.max_q, l.kv_rows, 1, a.err, stream));
       a.launches += at.ranges;
     }
     ELL_STEP(kStepProduct, step_product(a, att, l.o, delta, W, Hq * D, stream));

@@ -204,7 +204,7 @@ _STEP_NO_PAIRS = -1000
 
 def decoder_step(x, layers, norm, sizes, meta, fresh, max_len, eps, scale):
     """The normed rows behind the layers of a step (``csrc/decoder_step.cu``).  ``layers``: per layer the addresses of the weights (qkv,
-    o, gate and up, down, both norms), of its keys and values and of its rotary tables, and the rows of these; ``sizes``: query heads,
+    o, gate and up, down, both norms), of its keys and values and of its rotary tables, and the rows of the tables and of the cache; ``sizes``: query heads,
     key heads, head size, feed-forward width.  The caller has looked the operands over and keeps them alive."""
     T, W = x.shape
     one = meta["one_token"]
@@ -270,8 +270,8 @@ def attention_rows(q, k, v, base, length, max_len, scale, sink=None, alibi_slope
                                _p(None if sink is None else _f32(sink, "sink")), _p(sl), _gate(gate, q)[0], c_int(T),
                                c_int(H), c_int(G), c_int(d), c_int(dv), c_int(_heads(q, "q")), c_int(_heads(k, "k")),
                                c_int(_heads(v, "v")), _gate(gate, q)[1], c_int(max_len), c_int(window or 0), c_float(scale),
-                               _p(cu_seqlens), c_int(n_seq), c_int(max_q), _bf(q.dtype), _stream()), "attn_rows",
-           2 if need else 1)
+                               _p(cu_seqlens), c_int(n_seq), c_int(max_q), c_longlong(min(k.shape[0], v.shape[0])), _bf(q.dtype),
+                               _p(err_flag(q.device)), _stream()), "attn_rows", 2 if need else 1)
     return out
 
 

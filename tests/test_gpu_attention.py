@@ -355,6 +355,29 @@ def test_values_that_are_not_finite_reach_the_rows_that_see_them(steps, past, H,
         assert (o[fine].double() - want[fine]).norm() <= 1.9e-3 * want[fine].norm()
 
 
+@pytest.mark.parametrize("offset,pad", [(0, 0), (2, 0), (0, 2)])
+@pytest.mark.parametrize("tokens,past,H,G,d,dv", [(17, 47, 1, 1, 128, 128), (32, 0, 1, 1, 64, 64), (33, 31, 1, 1, 80, 16), (127, 65, 2, 2, 128, 64),
+                                                  (43, 128, 3, 1, 128, 128), (42, 511, 3, 1, 32, 112), (9, 4000, 16, 1, 128, 128)])
+def test_rows_of_a_continued_prompt_fill_tiles_to_their_edges(tokens, past, H, G, d, dv, offset, pad):
+    """Groups of 32 rows and tiles of 128 that are filled, one short and one over, keys likewise; queries on 16-byte places and on none.
+    Bounds as for the rows above."""
+    from easyllm_b200.ops import infer as iops
+    torch.manual_seed(tokens + d)
+    dev, cap = "cuda", past + tokens + 3
+    k, v = (torch.randn(2 * cap, G, n, device=dev).bfloat16() for n in (d, dv))
+    ld = H * d + pad
+    flat = torch.randn(offset + 2 * tokens * ld, device=dev).bfloat16()
+    q = flat[offset:].view(2 * tokens, ld)[:, :H * d].unflatten(1, (H, d))
+    assert q.data_ptr() % 16 == 2 * offset
+    base, length = [0] * tokens + [cap] * tokens, [past + j + 1 for j in range(tokens)] * 2
+    b, n = (torch.tensor(x, dtype=torch.int32, device=dev) for x in (base, length))
+    cu = torch.tensor([0, tokens, 2 * tokens], dtype=torch.int32, device=dev)
+    want = _rows_exact(q, k, v, base, length, d ** -0.5, None, None, None, None)
+    o = iops.attention_rows(q, k, v, b, n, past + tokens, d ** -0.5, cu_seqlens=cu, max_q=tokens)
+    assert (o.double() - want).norm() <= 1.9e-3 * want.norm()
+    assert (o.double() - want).abs().max() <= 2.0 ** -8 * want.abs().max()
+
+
 @pytest.mark.parametrize("hq,hk", [(5, 5), (6, 2)])
 def test_heads_in_several_groups(cu, hq, hk):
     """So many tokens that the heads' CTAs come in several groups, the last one smaller: documents of 512 tokens alone (the same
