@@ -25,6 +25,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ... import ops
+from ...ops import decoder
 from ...ops import infer as iops
 from ...ops import reference as ref
 from ..layers import RotaryTables, alibi_slopes
@@ -427,6 +428,10 @@ class DecoderLayer(nn.Module):
         return self.self_attn.new_state(*a)
 
     def forward(self, delta, residual, meta, cache=None):
+        if cache is None and delta.is_cuda and delta.requires_grad and torch.is_grad_enabled():
+            plan = self._train_plan(delta, residual, meta)
+            if plan is not None:
+                return decoder.train_layer(delta, residual, *plan)
         if residual is None:
             h = delta
             n1 = self.input_layernorm(h)
@@ -434,6 +439,34 @@ class DecoderLayer(nn.Module):
             n1, h = self.input_layernorm(delta, residual)
         n2, h = self.post_attention_layernorm(self.self_attn(n1, meta, cache), h)
         return self.mlp(n2), h
+
+    def _train_plan(self, x, residual, meta):
+        """What ``decoder.train_layer`` needs of this layer for packed rows whose gradients are recorded, or None where it does not
+        stand for ``forward`` (modules replaced, adapted or hooked, weights without a ``main_grad``)."""
+        at, mlp = self._modules["self_attn"], self._modules["mlp"]
+        if not (_plain(at, Attention) and _plain(mlp, MLP)) or _global_hooks() or type(self) is not DecoderLayer:
+            return None
+        a, width, part, gate = at.a, x.shape[1], at._modules, mlp._modules
+        pos, row_start = meta["position_ids"], meta.get("row_start")
+        if not (decoder.rows_ok(x) and (residual is None or (decoder.rows_ok(residual) and residual.shape == x.shape))) or \
+                at.d != decoder.HEAD or a.qkv_bias or a.o_bias or (a.use_logn_attn and not self.training) or width % 8 or width > 8192 or \
+                not ops.attention_kernels_ok(x.dtype, at.d) or ops.get_gemm_backend() != "tcgen05" or ops.cuda.transforms_active() or \
+                any(t is None or t.dtype != torch.int32 or not t.is_cuda or not t.is_contiguous() or t.numel() != x.shape[0] for t in (pos, row_start)):
+            return None
+        hq, hk, d, ff = at.hq, at.hk, at.d, a.intermediate_size
+        eps = self._modules["input_layernorm"].eps
+        norms = [_norm_weight(self._modules[n], width, eps) for n in ("input_layernorm", "post_attention_layernorm")]
+        groups = [(width, (part["q_proj"], hq * d), (part["k_proj"], hk * d), (part["v_proj"], hk * d)), (hq * d, (part["o_proj"], width)),
+                  (width, (gate["gate_proj"], ff), (gate["up_proj"], ff)), (ff, (gate["down_proj"], width))]
+        if ff % 8 or None in norms or any(_adjacent_rows(*g) is None for g in groups):
+            return None
+        weights = [lin._parameters["weight"] for g in groups for lin, _ in g[1:]] + norms
+        if not all(w.requires_grad and getattr(w, "main_grad", None) is not None for w in weights):
+            return None
+        cos, sin = at.rotary.get(int(meta["max_position"]), x.device) if at.rotary is not None else (None, None)
+        slopes = ops.cuda._slopes(at.slopes, hq, x.device)
+        fused = [iops.fused_alias([lin._parameters["weight"] for lin, _ in g[1:]]) for g in groups] + [w.detach() for w in norms]
+        return decoder.TrainPlan(fused, hq, hk, ff, cos, sin, pos, row_start, slopes, eps, 1.0 / math.sqrt(d)), weights
 
     def addresses(self, width, meta, cache, eps):
         """What ``ops.infer.decoder_step`` needs to know of this layer, or None where it does not stand for ``forward``."""

@@ -627,6 +627,11 @@ def _attn_kernel_reason(dtype, head_dim):
     return None
 
 
+def attention_kernels_ok(dtype, head_dim):
+    """Whether attention in both directions runs on the sm_100a kernels."""
+    return _attn_kernel_reason(dtype, head_dim) is None and _cu()._FA_BWD == "kernel"
+
+
 def _pad_heads(t, D):
     """[T, H, d] → [T, H, D] with zero columns: scores and outputs of the padded columns are exactly zero, so the
     128-wide kernels serve smaller heads (their tiles are half empty, which only small test models pay)."""

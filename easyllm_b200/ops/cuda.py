@@ -40,8 +40,9 @@ def lib():
                               "(or __graft_entry__.build()) before using the CUDA ops")
         _lib = ctypes.CDLL(_LIB_PATH if os.path.exists(_LIB_PATH) else _SERVE_LIB_PATH)
         for name in ("ell_rmsnorm_bwd_scratch_elems", "ell_attn_rows_scratch", "ell_attn_latent_scratch",
-                     "ell_scan_chunks_work", "ell_decoder_step_work"):
-            getattr(_lib, name).restype = c_longlong
+                     "ell_scan_chunks_work", "ell_decoder_step_work", "ell_decoder_layer_kept", "ell_decoder_layer_work"):
+            if hasattr(_lib, name):            # the library of the serving kernels has no training step
+                getattr(_lib, name).restype = c_longlong
     return _lib
 
 

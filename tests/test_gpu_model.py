@@ -323,3 +323,117 @@ def test_a_refused_launch_on_pairs_is_repeated_without(monkeypatch):
         assert all(torch.equal(x, y) for x, y in zip(got, want))
     finally:
         cu.set_gemm_pair(True)
+
+
+def _train_layers(cfg, lens, natively, monkeypatch, change=None, freeze=(), drop=(), wrt=None, checkpointing=False):
+    """One micro-batch through a model with an optimizer's fp32 gradient buffer: loss, gradients, launches and layers issued by one call."""
+    import easyllm_b200.ops.cuda as cu
+    from easyllm_b200.models.hf_models import CausalLM, arch_from_hf_config
+    from easyllm_b200.ops import decoder
+    from easyllm_b200.optim.zero import ZeroOptimizer
+    torch.manual_seed(1)
+    with torch.device("cuda"):
+        model = CausalLM(arch_from_hf_config(cfg), dtype=torch.bfloat16).train()
+    for name, p in model.named_parameters():
+        p.requires_grad_(not any(f in name for f in freeze))
+    opt = ZeroOptimizer([(n, p) for n, p in model.named_parameters() if p.requires_grad], lr=1e-4, stage=0)
+    if change is not None:
+        change(model)
+    if checkpointing:
+        model.gradient_checkpointing_enable()
+    taken = []
+    layer = decoder.train_layer
+    with monkeypatch.context() as m:
+        m.setattr(decoder, "train_layer", lambda *a: taken.append(1) or layer(*a))
+        if not natively:
+            m.setattr(decoder, "rows_ok", lambda x: False)
+        gen, T, cu_seqlens = torch.Generator().manual_seed(2), sum(lens), torch.tensor([0] + lens).cumsum(0).int()
+        opt.zero_grad()
+        before = cu.LAUNCHES
+        loss = model(input_ids=torch.randint(0, 512, (1, T), generator=gen), labels=torch.randint(0, 512, (1, T), generator=gen),
+                     position_ids=torch.cat([torch.arange(n) for n in lens]).unsqueeze(0), cu_seqlens=cu_seqlens)["loss"]
+        for p in drop:
+            dict(model.named_parameters())[p].main_grad = None
+        if wrt is not None:
+            params = dict(model.named_parameters())
+            torch.autograd.grad(loss, [params[n] for n in wrt], allow_unused=True)
+        else:
+            loss.backward()
+            if not drop:                       # the optimizer adds gradients to the main_grad that it made
+                opt.accumulate_grads()
+    cu.check_err_flag()
+    grads = {n: (p.grad.float() if p.grad is not None else p.main_grad if getattr(p, "main_grad", None) is not None else None)
+             for n, p in model.named_parameters()}
+    return loss.detach(), grads, cu.LAUNCHES - before, len(taken)
+
+
+_TRAIN = {"model_type": "llama", "vocab_size": 512, "hidden_size": 512, "intermediate_size": 704, "num_hidden_layers": 3,
+          "num_attention_heads": 4, "num_key_value_heads": 2}
+
+
+def _same_gradients(a, b):
+    """Equal bits where the layers' own kernels made them; what lies in front of the first layer gets one rounding to bf16 less."""
+    for n in a:
+        assert (a[n] is None) == (b[n] is None), n
+        if a[n] is None:
+            continue
+        if "embed" in n:
+            assert (a[n] - b[n]).norm() <= 2.0 ** -8 * b[n].norm()
+        else:
+            assert torch.equal(a[n], b[n]), n
+
+
+@pytest.mark.parametrize("lens", [[1], [16], [5, 36], [200], [256], [257, 64], [2048, 3]])
+@pytest.mark.parametrize("more", [{}, {"num_key_value_heads": 4, "intermediate_size": 1000}, {"model_type": "baichuan2-13b"}])
+def test_layers_of_a_training_step_issued_by_one_call_give_the_bits_of_the_functions(lens, more, monkeypatch):
+    _need_gpu()
+    cfg = {**_TRAIN, **more}
+    la, ga, na, ta = _train_layers(cfg, lens, True, monkeypatch)
+    lb, gb, nb, tb = _train_layers(cfg, lens, False, monkeypatch)
+    assert (ta, tb) == (3, 0) and na == nb
+    assert torch.equal(la, lb)
+    _same_gradients(ga, gb)
+
+
+@pytest.mark.parametrize("kw,native", [
+    ({"checkpointing": True}, 6),                                           # recomputed in the backward pass
+    ({"freeze": ("layers.1.self_attn.q_proj",)}, 2),                        # a weight without a gradient: the layer's functions
+    ({"freeze": ("embed_tokens",)}, 2),                                     # nothing in front of the first layer records
+    ({"drop": ("model.layers.1.mlp.up_proj.weight", "model.layers.2.input_layernorm.weight")}, 3),   # gone between the passes
+    ({"wrt": ("model.embed_tokens.weight",)}, 3),                           # no weight of a layer is asked for: no products for them
+    ({"wrt": ("model.layers.1.mlp.down_proj.weight",)}, 3),
+])
+def test_layers_of_a_training_step_beside_the_usual_one(kw, native, monkeypatch):
+    _need_gpu()
+    la, ga, _, ta = _train_layers(_TRAIN, [40, 9], True, monkeypatch, **kw)
+    lb, gb, _, tb = _train_layers(_TRAIN, [40, 9], False, monkeypatch, **kw)
+    assert (ta, tb) == (native, 0)
+    assert torch.equal(la, lb)
+    if "drop" in kw:                                                        # bf16 gradients of autograd beside the fp32 ones
+        for n in kw["drop"]:
+            assert torch.equal(ga[n], gb[n]), n
+    _same_gradients(ga, gb)
+
+
+def test_a_changed_module_of_a_training_step_is_called(monkeypatch):
+    _need_gpu()
+    calls = []
+
+    def hooked(m):
+        m.model.layers[1].self_attn.o_proj.register_forward_hook(lambda *_: None)
+
+    def patched(m):
+        norm, forward = m.model.layers[0].post_attention_layernorm, m.model.layers[0].post_attention_layernorm.forward
+        norm.forward = lambda *a: calls.append(1) or forward(*a)
+
+    want = _train_layers(_TRAIN, [33], False, monkeypatch)
+    for change in (hooked, patched):
+        loss, grads, _, taken = _train_layers(_TRAIN, [33], True, monkeypatch, change=change)
+        assert taken == 2 and torch.equal(loss, want[0])
+        _same_gradients(grads, want[1])
+    assert calls
+    saved = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: saved.append(t.shape) or t.cpu(), lambda t: t.cuda()):
+        loss, grads, _, taken = _train_layers(_TRAIN, [33], True, monkeypatch)
+    assert taken == 3 and saved
+    _same_gradients(grads, want[1])
