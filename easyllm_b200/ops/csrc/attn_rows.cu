@@ -12,6 +12,8 @@
 //
 // Latent attention (one key row shared by all query heads, whose first dv columns are also the value, bf16) has a
 // kernel of its own, attn_latent_kernel: the products run on mma.sync m16n8k16 over a key tile that is read once.
+#include <algorithm>
+
 #include "sm100.cuh"
 #include "vec.cuh"
 
@@ -571,46 +573,33 @@ attn_latent_kernel(const __grid_constant__ CUtensorMap tmK, const AttnRowsArgs a
 
 // ---- bf16 rows over cached keys on matrix instructions ------------------------------------------------------------
 // Decoding reads every cached key and value once for a few query rows: bound by those bytes, if the arithmetic keeps up.
-// On the FMA pipe it did not (230 us for 64 rows x 2048 keys x 8 key heads, 537 MB, which take 83; 115 here); and a continued prompt
+// On the FMA pipe it did not (230 us for 64 rows x 2048 keys x 8 key heads, 537 MB, which take 83); and a continued prompt
 // read its whole context once per token (1060 us for 301 tokens of two sequences over 3000).  Here a tile of rows is the consecutive
 // tokens of one sequence times the query heads of one key head, and matrix instructions do the products:
 //   scores  exact bf16 products, fp32 sums, scale and bias applied in fp32
-//   values  the fp32 weights go in as three bf16 parts, so they keep their 24 bits.  With two parts, in turn for one accumulator at
-//           a time, 64 rows x 2048 keys took 136 us; with three, several accumulators taking turns, 125
-//   attn_few_kernel   up to 16 rows (decoding).  Keys are the M side of both products and rows the N side, so 8 rows cost
-//                     half of 16: S^T = K q^T, O^T = V^T P^T.  The four warps take units of 16 keys in turn, each with a
-//                     softmax, accumulators and a ring of cp.async stages of its own; no barrier until their results meet.
-//                     Rows on the M side took 977 instructions a unit and 232 registers, and stayed at 162 us, bound by
-//                     the latency of eight warps an SM.
+//   values  the fp32 weights go in as three bf16 parts, so they keep their 24 bits; several accumulators take turns, since the
+//           parts' products of one wait for one another
+//   attn_few_kernel   up to 16 rows (decoding), on mma.sync.  Keys are the M side of both products and rows the N side, so 8 rows
+//                     cost half of 16: S^T = K q^T, O^T = V^T P^T.  The four warps take units of 16 keys in turn, each with a softmax,
+//                     accumulators and a ring of three stages of its own, filled by TMA; no barrier until their results meet.
+//                     With 16 cp.async and their addresses a lane and unit, sizes known at run time only, expf and conversions a unit
+//                     took 687 instructions, five cycles each with two warps a scheduler, and 64 rows x 2100 keys x 8 key heads
+//                     116 us (4.7 TB/s); now 86 (6.5 TB/s, merge included).  8 rows x 4200 43 -> 28, one x 4000 x 4 10.0 -> 8.7.
+//                     Equal shares of all keys for every CTA, rows divided where a share ends: 92, 31 and 14.
 //   attn_tile_kernel  more rows (continued prompts): 128 of them on tcgen05, see there
 // Ranges of keys and their merge are those of attn_rows_kernel.
-constexpr int kAtThreads = 128, kAtKRow = 256, kAtStages = 3;      // bytes of a key / value row in shared memory (up to 128)
+constexpr int kAtThreads = 128;
 constexpr int kAtHeads = 16;                                       // most query heads of a CTA
-constexpr int kAfKeys = 16, kAfStage = 2 * kAfKeys * kAtKRow;      // attn_few_kernel: keys of a warp's unit
-constexpr int kAfSmem = 4 * kAtStages * kAfStage;
+constexpr int kAfKeys = 16, kAfChunk = kAfKeys * 128;              // keys of a warp's unit; bytes of 64 columns of them
+// All of a CTA's shared memory is in kAfSmem: two CTAs and the system's 1 KB each just fit a split of 196 KB.  112 bytes more took 228 KB,
+// which later kernels of the chain found their L1 cut down by (a decoding product of 6144 x 4096 13.6 -> 19.5 us).
+constexpr int kAfStage = 4 * kAfChunk, kAfStages = 3, kAfRing = 4 * kAfStages * kAfStage, kAfSmem = kAfRing + 1024;
+static_assert(2 * (kAfSmem + 1024) <= 196 * 1024, "");
+constexpr int kAfErr = 15;
+constexpr float kLog2e = 1.4426950408889634f;
 
-__device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, bool in) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
-               "r"(in ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ uint32_t at_place(int row, int piece) {       // 16-byte piece of a row, no bank conflicts in ldmatrix
-  return (uint32_t)(row * kAtKRow + ((piece ^ (row & 7)) << 4));
-}
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-// x and y as three bf16 parts each: 24 bits, nothing is lost
-__device__ __forceinline__ void split_bf16(float x, float y, uint32_t (&p)[3]) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    p[i] = pack_bf16(x, y);
-    x -= __uint_as_float(p[i] << 16);
-    y -= __uint_as_float(p[i] & 0xffff0000u);
-  }
-}
-
-// The same by truncation: eight of the 24 bits a part.  Without the conversions, which share the unit of the exponential.
+// x and y as three bf16 parts each, eight of their 24 bits a part: nothing is lost.  By truncation, since conversions share the unit of
+// the exponential.
 __device__ __forceinline__ void cut_bf16(float x, float y, uint32_t (&p)[3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
@@ -619,41 +608,6 @@ __device__ __forceinline__ void cut_bf16(float x, float y, uint32_t (&p)[3]) {
     y -= __uint_as_float(__float_as_uint(y) & 0xffff0000u);
   }
 }
-
-// Sixteen lanes of a warp take a row of KEYS keys and values, a 16-byte piece each.  Rows past the range are
-// zero-filled: their weight is 0, and 0 times what lies there must be 0.
-template <int KEYS, int THREADS>
-struct AtLoader {
-  const __nv_bfloat16 *kb, *vb;      // first row of the range
-  int piece, row_in, keys, ldk, ldv;
-  bool k_in, v_in;
-  __device__ __forceinline__ AtLoader(const AttnRowsArgs& a, size_t base, int g, int k0, int k1, int who) {
-    piece = who & 15;
-    row_in = who >> 4;
-    kb = reinterpret_cast<const __nv_bfloat16*>(a.k) + (base + k0) * a.ldk + (size_t)g * a.d + piece * 8;
-    vb = reinterpret_cast<const __nv_bfloat16*>(a.v) + (base + k0) * a.ldv + (size_t)g * a.dv + piece * 8;
-    keys = k1 - k0;
-    ldk = a.ldk;
-    ldv = a.ldv;
-    k_in = piece < a.d / 8;
-    v_in = piece < a.dv / 8;
-  }
-  __device__ __forceinline__ void load(int tile, uint8_t* stage) const {
-    const int first = tile * KEYS;
-    if (first < keys) {
-#pragma unroll
-      for (int i = 0; i < KEYS * 16 / THREADS; ++i) {
-        const int row = row_in + i * (THREADS / 16);
-        const bool in = first + row < keys;
-        const size_t at = in ? first + row : 0;
-        uint8_t* dst = stage + at_place(row, piece);
-        if (k_in) cp_async16_zfill(dst, kb + at * ldk, in);
-        if (v_in) cp_async16_zfill(dst + KEYS * kAtKRow, vb + at * ldv, in);
-      }
-    }
-    cp_async_commit();
-  }
-};
 
 // The tokens, heads and keys of a CTA.  blockIdx.x: tile of `tt` tokens of a sequence (cu null: one token each), y: key head
 // and group of its query heads, z: range of keys.
@@ -756,21 +710,61 @@ __device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
   return y;
 }
 
-// NB: groups of 8 rows.
-template <int NB>
-__global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const __grid_constant__ AttnRowsArgs a, const int* __restrict__ cu, int tiles, int tt) {
+struct AfRing {
+  uint64_t full[4][kAfStages];    // of a warp's stages
+  int gave_up;
+};
+static_assert(sizeof(AfRing) <= 128, "");
+// The stages start at a multiple of 1024; the barriers lie in what is left in front of them, or behind.
+__device__ __forceinline__ uint8_t* af_stages(uint8_t* raw) {
+  return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
+}
+__device__ __forceinline__ AfRing& af_ring(uint8_t* raw) {
+  uint8_t* stages = af_stages(raw);
+  return *reinterpret_cast<AfRing*>(stages - raw >= 128 ? raw : stages + kAfRing);
+}
+// NB: groups of 8 rows.  FULL: heads of 128.
+template <int NB, bool FULL>
+__global__ void __launch_bounds__(kAtThreads, 2)
+attn_few_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ AttnRowsArgs a,
+                const int* __restrict__ cu, int tiles, int tt) {
+  extern __shared__ __align__(128) uint8_t atsm_raw[];
+  uint8_t* atsm = af_stages(atsm_raw);
+  AfRing& ring = af_ring(atsm_raw);
+  if (threadIdx.x == 0) {
+    for (int w = 0; w < 4; ++w)
+      for (int i = 0; i < kAfStages; ++i) sm100::mbar_init(&ring.full[w][i], 1);
+    sm100::fence_barrier_init();
+    sm100::tma_prefetch_desc(&tmK);
+    sm100::tma_prefetch_desc(&tmV);
+    ring.gave_up = 0;
+  }
+  __syncthreads();
   chain_enter(cu);
-  extern __shared__ __align__(128) uint8_t atsm[];
   AtTile T;
   if (!T.init(a, cu, tiles, tt)) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, t = lane & 3, quad = lane >> 3, l8 = lane & 7;
-  const AtLoader<kAfKeys, 32> loader(a, T.base, T.g, T.k0, T.k1, lane);
-  uint8_t* ring = atsm + warp * kAfStage * kAtStages;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, gr = lane >> 2, t = lane & 3, quad = lane >> 3,
+            l8 = lane & 7;
+  uint8_t* stages = atsm + warp * kAfStage * kAfStages;
   const int n_units = T.k1 > T.k0 ? (T.k1 - T.k0 + kAfKeys - 1) / kAfKeys : 0;
+  const int mine = n_units > warp ? (n_units - warp + 3) / 4 : 0;       // units warp, warp + 4, ...
+  const int kc = FULL ? 2 : (a.d + 63) / 64, vc = FULL ? 2 : (a.dv + 63) / 64;
+  volatile int* gave_up = &ring.gave_up;
+  // rows past the range are other keys or zeros: their weight is 0 (and a row that is not finite is looked at again)
+  auto load = [&](int i) {
+    if (i < mine && lane == 0) {
+      const int s = i % kAfStages;
+      uint8_t* st = stages + s * kAfStage;
+      const int row = (int)T.base + T.k0 + (warp + 4 * i) * kAfKeys;
+      sm100::mbar_expect_tx(&ring.full[warp][s], (kc + vc) * kAfChunk);
+      for (int c = 0; c < kc; ++c) sm100::tma_load_3d(st + c * kAfChunk, &tmK, &ring.full[warp][s], c * 64, T.g, row);
+      for (int c = 0; c < vc; ++c) sm100::tma_load_3d(st + (2 + c) * kAfChunk, &tmV, &ring.full[warp][s], c * 64, T.g, row);
+    }
+  };
 #pragma unroll
-  for (int i = 0; i < kAtStages - 1; ++i) loader.load(warp + i * 4, ring + i * kAfStage);
+  for (int i = 0; i < kAfStages - 1; ++i) load(i);
 
-  const int ksteps = a.d / 16, vtiles = a.dv / 16;
+  const int ksteps = FULL ? 8 : a.d / 16, vtiles = FULL ? 8 : a.dv / 16;
   uint32_t q[NB][8][2];                              // B operand: row gr of the group
   float m[NB][2], l[NB][2], slope[NB][2];            // of rows 2 t, 2 t + 1: maximum, this lane's share of the sum
   int first[NB][2], end[NB][2];                      // keys they see
@@ -801,15 +795,14 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const __grid_co
       for (int i = 0; i < 4; ++i) acc[n][b][i] = 0.f;
 
   constexpr int kTogether = 4 / NB;
-  const uint32_t k_row = (quad & 1) * 8 + l8, v_row = (quad >> 1) * 8 + l8;          // & 7 = l8
-  int stage = 0;
-  for (int u = warp; u < n_units; u += 4) {
-    cp_async_wait<kAtStages - 2>();
-    __syncwarp();
-    loader.load(u + (kAtStages - 1) * 4, ring + (stage == 0 ? kAtStages - 1 : stage - 1) * kAfStage);   // free since the step before
-    const uint8_t* ks = ring + stage * kAfStage + k_row * kAtKRow;
-    const uint8_t* vs = ring + stage * kAfStage + kAfKeys * kAtKRow + v_row * kAtKRow;
-    stage = stage == kAtStages - 1 ? 0 : stage + 1;
+  const uint32_t k_row = ((quad & 1) * 8 + l8) * 128, v_row = ((quad >> 1) * 8 + l8) * 128 + 2 * kAfChunk;      // row & 7 = l8
+  bool failed = false;
+  for (int i = 0; i < mine; ++i) {
+    const int stage = i % kAfStages;
+    failed = !sm100::mbar_wait_warp(&ring.full[warp][stage], (i / kAfStages) & 1, gave_up);
+    if (failed) break;
+    load(i + kAfStages - 1);                           // over the unit before, which all lanes are done with (the fence and the votes)
+    const uint8_t *ks = stages + stage * kAfStage + k_row, *vs = stages + stage * kAfStage + v_row;
     float s[NB][4], s2[NB][4];                       // two chains of sums
 #pragma unroll
     for (int b = 0; b < NB; ++b)
@@ -819,12 +812,12 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const __grid_co
     for (int k = 0; k < 8; ++k) {
       if (k < ksteps) {
         uint32_t x[4];
-        ldsm4(x, ks + (((k * 2 + (quad >> 1)) ^ l8) << 4));
+        ldsm4(x, ks + (k >> 2) * kAfChunk + ((((k & 3) * 2 + (quad >> 1)) ^ l8) << 4));
 #pragma unroll
         for (int b = 0; b < NB; ++b) mma_bf16(k & 1 ? s2[b] : s[b], x, q[b][k][0], q[b][k][1]);
       }
     }
-    const int key0 = T.k0 + u * kAfKeys;
+    const int key0 = T.k0 + (warp + 4 * i) * kAfKeys;
     const bool mask = key0 + kAfKeys > min(T.len0, T.k1) || key0 < T.last_first;
     float al[NB][2];
     bool grew = false;
@@ -847,11 +840,11 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const __grid_co
         for (int o = 4; o <= 16; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         const float now = fmaxf(m[b][j], mx);
         grew |= now > m[b][j];
-        al[b][j] = now == -INFINITY ? 1.f : expf(m[b][j] - now);       // no key yet: nothing to rescale
+        al[b][j] = now == -INFINITY ? 1.f : sm100::ex2_approx((m[b][j] - now) * kLog2e);       // no key yet: nothing to rescale
         m[b][j] = now;
         const float ref = now == -INFINITY ? 0.f : now;
-        s[b][j] = expf(s[b][j] - ref);
-        s[b][j + 2] = expf(s[b][j + 2] - ref);
+        s[b][j] = sm100::ex2_approx((s[b][j] - ref) * kLog2e);
+        s[b][j + 2] = sm100::ex2_approx((s[b][j + 2] - ref) * kLog2e);
         l[b][j] = l[b][j] * al[b][j] + (s[b][j] + s[b][j + 2]);
       }
     }
@@ -868,7 +861,7 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const __grid_co
     for (int b = 0; b < NB; ++b)
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
-        split_bf16(s[b][2 * c], s[b][2 * c + 1], w[b][c]);
+        cut_bf16(s[b][2 * c], s[b][2 * c + 1], w[b][c]);
 #pragma unroll
         for (int x = 0; x < 3; ++x) w[b][c][x] = transpose_8x8(w[b][c][x]);
       }
@@ -878,7 +871,7 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const __grid_co
       uint32_t x[kTogether][4];
 #pragma unroll
       for (int y = 0; y < kTogether; ++y)
-        if (n + y < vtiles) ldsm4_t(x[y], vs + ((((n + y) * 2 + (quad & 1)) ^ l8) << 4));
+        if (n + y < vtiles) ldsm4_t(x[y], vs + ((n + y) >> 2) * kAfChunk + (((((n + y) & 3) * 2 + (quad & 1)) ^ l8) << 4));
 #pragma unroll
       for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -888,6 +881,8 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const __grid_co
             for (int b = 0; b < NB; ++b) mma_bf16(acc[n + y][b], x[y], w[b][0][i], w[b][1][i]);
           }
     }
+    sm100::fence_proxy_async_smem();                   // these reads before the copies that go over them
+    __syncwarp();
   }
 #pragma unroll
   for (int b = 0; b < NB; ++b)
@@ -896,8 +891,18 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_few_kernel(const __grid_co
 #pragma unroll
       for (int o = 4; o <= 16; o <<= 1) l[b][j] += __shfl_xor_sync(0xffffffffu, l[b][j], o);
 
-  cp_async_wait<0>();
+  if (failed) *gave_up = 1;
   __syncthreads();
+  if (*gave_up) {                                      // copies in flight land before the CTA ends
+    if (threadIdx.x == 0) {
+      atomicCAS(a.err, 0, kAfErr);
+      const unsigned long long t0 = sm100::globaltimer_ns();
+      while (sm100::globaltimer_ns() - t0 < 200000ull) {
+      }
+    }
+    __syncthreads();
+    return;
+  }
   float* stat = reinterpret_cast<float*>(atsm);      // [warp][16 rows] maximum | sum
   float* sums = stat + 128;                          // [warp][16 rows][ld]
   const int ld = a.dv + 8;
@@ -974,8 +979,6 @@ constexpr int kAtTile = 64, kAtRows = 128, kAtTileThreads = 320, kAtHalf = kAtTi
 constexpr int kAtQChunk = kAtRows * 128, kAtKvChunk = kAtTile * 128;     // [rows x 64 columns], 128-byte swizzle rows
 constexpr int kAtQBytes = 2 * kAtQChunk, kAtStage = 4 * kAtKvChunk;      // a stage: keys, values
 constexpr int kAtBars = kAtQBytes + 2 * kAtStage, kAtSmem = kAtBars + 1024 + 2560;
-constexpr int kAtErr = 15;
-constexpr float kLog2e = 1.4426950408889634f;
 
 struct AtShared {
   uint64_t q_full, full[2], empty[2], s_full, p_full, o_full;
@@ -999,7 +1002,7 @@ __global__ void __launch_bounds__(kAtTileThreads, 2)
 attn_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ AttnRowsArgs a,
                  const int* __restrict__ cu, int tiles, int tt) {
   using namespace sm100;
-  extern __shared__ uint8_t atsm_raw[];
+  extern __shared__ __align__(128) uint8_t atsm_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(atsm_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* kv = smem + kAtQBytes;
   AtShared* sh = reinterpret_cast<AtShared*>(smem + kAtBars);
@@ -1032,7 +1035,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
   const int kc = (a.d + 63) / 64, vc = (a.dv + 63) / 64;                // 64-column chunks of a key, of a value
   auto fail = [&]() {
     *gave_up = 1;
-    atomicCAS(a.err, 0, kAtErr);
+    atomicCAS(a.err, 0, kAfErr);
   };
 
   if (!any || dead) {
@@ -1293,20 +1296,22 @@ struct AtPlan {
   bool fits, few;
   int tt, tiles, splits, range;
 };
-// Ranges of decoding rows: the CTAs come in rounds of two an SM, and the last round takes as long as a full one, so the number of
-// ranges decides how much of it is idle.  A round reads its keys at 5 TB/s and costs 3 us besides, a merge 3.  Measured (us; 32 query
-// heads on 8 key heads, ranges 1 / 2 / 3 / 4): 48 sequences of 2048 keys 111 / 94 / 90 / 99, 64 of them 114 / 122 / 125 / 122, 24 of
-// 3000 82 / 88 / 66 / 74; 10 sequences of 2048 with 32 key heads 105 / 88 / 83 / 83.  A CTA an SM and fewer go in about one round: the
-// last range, which ends before the bound of the lengths, may be a few CTAs over it.  (That pays where the lengths stay below the
-// bound; with all rows at it, 4 sequences of 3000 with 16 key heads take 28 in 4 ranges and 33 in 5, 8 of 4096 with 8 take 37 and 51.)
+// Ranges of decoding rows.  A CTA draws 47 GB/s, all together 6.4 TB/s (136 of them), and two an SM are resident: full rounds of CTAs go at
+// the second rate, the last one at what its CTAs draw; a round costs 1.5 us besides, a merge 3.5.  The bound of the lengths may be
+// met by all rows, or by one where the mean is half of it: the sum of both decides.  Measured (us; ranges 1 / 2 / 3 / 4): 64 sequences of
+// 2100 keys, 32 query heads on 8, 86 / 95 / 98 / 98; 48 of 2048 73 / 69 / 71 / 73; 24 of 3000 48 / 56 / 54 / 55; 8 of 4200, 16 on 8, 49 / 31 / 28 /
+// 28 (5: 32); 10 of 2048, 32 on 32, 70 / 63 / 62 / 62; 40 of 64 to 4096, 16 on 4, 50 / 37 / 35 / 39; 16 of 100 in caches of 512 5 / 7 / 8 / 9.
 static int at_ranges(long long ctas, long long most, double bytes_of_cta) {
-  if (ctas <= kNumSMs) return (int)((2LL * kNumSMs + ctas / 2) / ctas < most ? (2LL * kNumSMs + ctas / 2) / ctas : most);
-  const double whole = bytes_of_cta * 2 * kNumSMs / 5e6;
+  constexpr double kAll = 6.4e6, kOne = 47e3;          // bytes a us
+  const long long resident = 2 * kNumSMs;
   int best = 1;
   double least = 1e30;
   for (int s = 1; s <= most; ++s) {
-    const long long rounds = (ctas * s + 2 * kNumSMs - 1) / (2 * kNumSMs);
-    const double us = rounds * (whole / s + 3.0) + (s > 1 ? 3.0 : 0.0);
+    const double b = bytes_of_cta / s;
+    const long long n = ctas * s, rounds = (n - 1) / resident, last = n - rounds * resident;
+    const double alike = rounds * (resident * b / kAll + 1.5) + std::max(last * b / kAll, b / kOne);
+    const double varied = std::max(n * b / 2 / kAll, b / kOne);
+    const double us = alike + varied + (s > 1 ? 7.0 : 0.0);
     if (us < least) {
       least = us;
       best = s;
@@ -1351,25 +1356,32 @@ static int allow_smem(Kernel kern, int smem, bool& configured) {
   return (int)e;
 }
 static int launch_attn_cached(const AttnRowsArgs& a, const AtPlan& p, const int* cu, int n_seq, long long rows, cudaStream_t stream) {
-  static bool few8 = false, few16 = false, tile = false;
   const int rep = a.H / a.G, nh = rep < kAtHeads ? rep : kAtHeads, groups = (rep + kAtHeads - 1) / kAtHeads;
   if (p.tt == 1) cu = nullptr;
   const dim3 grid(p.tt == 1 ? a.n : n_seq * p.tiles, a.G * groups, p.splits);
   if (grid.y > 65535) return -2;
-  int rc;
+  CUtensorMap tk, tv;
+  const int box = p.few ? kAfKeys : kAtTile;
+  int rc = make_tmap_bf16_heads(&tk, a.k, a.d, a.G, rows, (uint64_t)a.ldk * 2, 64, box, 0);
+  if (!rc) rc = make_tmap_bf16_heads(&tv, a.v, a.dv, a.G, rows, (uint64_t)a.ldv * 2, 64, box, 0);
+  if (rc) return rc;
   if (!p.few) {
-    CUtensorMap tk, tv;
-    rc = make_tmap_bf16_heads(&tk, a.k, a.d, a.G, rows, (uint64_t)a.ldk * 2, 64, kAtTile, 0);
-    if (!rc) rc = make_tmap_bf16_heads(&tv, a.v, a.dv, a.G, rows, (uint64_t)a.ldv * 2, 64, kAtTile, 0);
-    if (!rc) rc = allow_smem(attn_tile_kernel, kAtSmem, tile);
-    if (rc) return rc;
+    static bool tile = false;
+    if ((rc = allow_smem(attn_tile_kernel, kAtSmem, tile)) != 0) return rc;
     launch_chained(attn_tile_kernel, grid, kAtTileThreads, kAtSmem, stream, tk, tv, a, cu, p.tiles, p.tt);
-  } else if (p.tt * nh <= 8) {
-    if ((rc = allow_smem(attn_few_kernel<1>, kAfSmem, few8)) != 0) return rc;
-    launch_chained(attn_few_kernel<1>, grid, kAtThreads, kAfSmem, stream, a, cu, p.tiles, p.tt);
   } else {
-    if ((rc = allow_smem(attn_few_kernel<2>, kAfSmem, few16)) != 0) return rc;
-    launch_chained(attn_few_kernel<2>, grid, kAtThreads, kAfSmem, stream, a, cu, p.tiles, p.tt);
+    const bool full = a.d == 128 && a.dv == 128, small = p.tt * nh <= 8;
+#define ELL_FEW(NB_, FULL_)                                                                                                   \
+  if (small == (NB_ == 1) && full == FULL_) {                                                                                 \
+    static bool ready = false;                                                                                                \
+    if ((rc = allow_smem(attn_few_kernel<NB_, FULL_>, kAfSmem, ready)) != 0) return rc;                                       \
+    launch_chained(attn_few_kernel<NB_, FULL_>, grid, kAtThreads, kAfSmem, stream, tk, tv, a, cu, p.tiles, p.tt);              \
+  }
+    ELL_FEW(1, true)
+    ELL_FEW(1, false)
+    ELL_FEW(2, true)
+    ELL_FEW(2, false)
+#undef ELL_FEW
   }
   if (a.splits > 1) launch_chained(attn_rows_merge_kernel<__nv_bfloat16>, dim3(a.n, a.H), kArThreads, 0, stream, a);
   return launch_status();
@@ -1476,7 +1488,7 @@ ELL_API int ell_attn_rows(const void* q, const void* k, const void* v, void* out
   const int esz = is_bf16 ? 2 : 4;
   const bool vec = (d * esz) % 16 == 0 && (dv * esz) % 16 == 0 && (ldk * esz) % 16 == 0 && (ldv * esz) % 16 == 0 &&
                    aligned_to(k, 16) && aligned_to(v, 16);
-  if (p.fits && vec && ldq % 2 == 0 && aligned_to(q, 4) && (p.few || kv_rows <= 0x7fffffff)) {
+  if (p.fits && vec && ldq % 2 == 0 && aligned_to(q, 4) && kv_rows <= 0x7fffffff) {
     a.splits = p.splits;
     a.range = p.range;
     a.all_ranges = p.tt > 1;
