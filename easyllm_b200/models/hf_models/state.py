@@ -16,6 +16,7 @@ advanced on the device.
 """
 from __future__ import annotations
 
+import numpy as np
 import torch
 
 from ... import ops
@@ -122,20 +123,24 @@ class DecodeState:
         start = [self.lengths[s] for s in slots]
         self.reserve(max(p + c for p, c in zip(start, counts)))
         dev, S, T = self.device, len(slots), sum(counts)
-        cu = [0]
-        for c in counts:
-            cu.append(cu[-1] + c)
-        n = torch.tensor(counts)
-        sl, p0 = torch.tensor(slots), torch.tensor(start)
-        first = torch.tensor(cu[:-1])
-        pos = torch.arange(T) - torch.repeat_interleave(first - p0, n, output_size=T)
-        # one host buffer, one copy: sequence borders, slots, start positions | positions, first row of the sequence,
-        # row of its first key, keys
-        tok_slot = torch.repeat_interleave(sl, n, output_size=T)
-        rows = torch.repeat_interleave(first, n, output_size=T)
-        buf = torch.cat((torch.tensor(cu), sl, p0, pos, rows, tok_slot * self.capacity, pos + 1)).to(torch.int32)
-        if dev.type == "cuda":
-            buf = buf.pin_memory().to(dev, non_blocking=True)
+        # One host buffer, one copy: sequence borders, slots, start positions | positions, first row of the sequence, row of its first
+        # key, keys.  Filled through numpy, a microsecond an operation: a short prompt waits for it (75 us with tensors, 35 so; 77 tokens
+        # through 4 layers of 2048 450 -> 410).
+        buf = torch.empty(3 * S + 1 + 4 * T, dtype=torch.int32, pin_memory=dev.type == "cuda")
+        a = buf.numpy()
+        cu, tok = a[:S + 1], a[3 * S + 1:].reshape(4, T)
+        n = np.array(counts, dtype=np.int64)
+        cu[0] = 0
+        np.cumsum(n, out=cu[1:])
+        a[S + 1:2 * S + 1], a[2 * S + 1:3 * S + 1] = slots, start
+        seq = np.repeat(np.arange(S), n)
+        first = cu[:-1].astype(np.int64)
+        tok[1] = first[seq]
+        tok[0] = np.arange(T) - (first - np.array(start, dtype=np.int64))[seq]
+        tok[2] = (np.array(slots, dtype=np.int64) * self.capacity)[seq]
+        tok[3] = tok[0] + 1
+        last = torch.from_numpy(cu[1:].astype(np.int64) - 1)
+        buf = buf.to(dev, non_blocking=True)
         parts = buf.split([S + 1, S, S, T, T, T, T])
         for s, c in zip(slots, counts):
             self.lengths[s] += c if advance else 0
@@ -144,7 +149,7 @@ class DecodeState:
                 "row_start": parts[4], "kv_base": parts[5], "kv_len": parts[6], "max_seqlen": max(counts),
                 "max_position": max(p + c for p, c in zip(start, counts)), "batch": S, "fresh": fresh,
                 "one_token": T == S, "kv_capacity": self.capacity,
-                "last_rows": torch.tensor(cu[1:]) - 1}
+                "last_rows": last}
 
 
 class DecodeGraph:

@@ -158,3 +158,24 @@ def test_hf_inference_interactive_and_question_file(tmp_path):
     rows = [json.loads(l) for l in open(tmp_path / "out.jsonl")]
     assert [r["id"] for r in rows] == [0, 1] and rows[1]["input"] == "capital of France"
     assert [r["gold"] for r in rows] == ["2", "Paris"] and all(isinstance(r["answer"], str) for r in rows)
+
+
+def test_index_of_a_step():
+    """Borders, slots and, token by token, position, first row, first key row and keys, for steps of one and of several sequences."""
+    from easyllm_b200.models.hf_models.state import DecodeState
+    state = object.__new__(DecodeState)
+    state.device, state.capacity, state.layers, state.tokens = torch.device("cpu"), 512, [], None
+    state.lengths, state.free = [0] * 4, []
+    for slots, counts in (([2], [5]), ([0, 2, 3], [1, 300, 2]), ([3], [1]), ([1, 0], [1, 1]), ([2, 1, 0, 3], [1, 7, 1, 2])):
+        start = [state.lengths[s] for s in slots]
+        m = state.step_meta(slots, counts)
+        assert [state.lengths[s] for s in slots] == [p + c for p, c in zip(start, counts)]
+        cu = [sum(counts[:i]) for i in range(len(counts) + 1)]
+        tokens = [(i, j) for i, c in enumerate(counts) for j in range(c)]
+        want = {"cu_seqlens": cu, "seq_slot": slots, "seq_pos0": start, "position_ids": [start[i] + j for i, j in tokens],
+                "row_start": [cu[i] for i, _ in tokens], "kv_base": [slots[i] * state.capacity for i, _ in tokens],
+                "kv_len": [start[i] + j + 1 for i, j in tokens], "last_rows": [c - 1 for c in cu[1:]]}
+        for name, values in want.items():
+            assert m[name].tolist() == values and m[name].dtype == (torch.int64 if name == "last_rows" else torch.int32), name
+        assert (m["max_seqlen"], m["max_position"]) == (max(counts), max(p + c for p, c in zip(start, counts)))
+        assert (m["fresh"], m["one_token"]) == (not any(start), len(tokens) == len(slots))
