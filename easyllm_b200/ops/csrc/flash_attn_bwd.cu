@@ -457,7 +457,10 @@ struct FbItem {
   int valid, q0, h, kv_lo, n, max_start;       // n key tiles from kv_lo; max_start: document start of the tile's last row
 };
 struct FbQShared {
-  uint64_t q_full, q_empty, do_full, do_empty, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full, s_free, dp_full[2], ds_full, dq_full;
+  uint64_t q_full, q_empty, do_full, do_empty, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full, s_free, dp_full[2], dq_full;
+  // A barrier for even and one for odd steps: dP of a step is there before dS of the step before is waited for, so a warp may be done
+  // with a step while another still makes the one before.
+  uint64_t ds_full[2];
   uint64_t item_full[2], item_empty[2], claim, claimed;
   alignas(16) uint32_t response[4];
   FbItem item[2];
@@ -491,12 +494,12 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       mbar_init(&sh->v_full[s], 1);
       mbar_init(&sh->v_empty[s], 1);
       mbar_init(&sh->dp_full[s], 1);
+      mbar_init(&sh->ds_full[s], kFbSoftmaxWarps);
       mbar_init(&sh->item_full[s], 1);
       mbar_init(&sh->item_empty[s], 1 + 1 + kFbSoftmaxWarps);   // loader, MMA warp, softmax warps
     }
     mbar_init(&sh->s_full, 1);
     mbar_init(&sh->s_free, kFbSoftmaxWarps);
-    mbar_init(&sh->ds_full, kFbSoftmaxWarps);
     mbar_init(&sh->dq_full, 1);
     mbar_init(&sh->claim, 1);
     mbar_init(&sh->claimed, 1);
@@ -604,12 +607,12 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         ok = scores(i, true, warp_uniform(n == 1));
         for (int t = 0; warp_uniform(t < n) && ok; ++t) {
           const int s = g & 1;
-          const uint32_t ph = g & 1;
+          const uint32_t ph = (g >> 1) & 1;
           const bool more = warp_uniform(t + 1 < n);
           ++g;
           if (more) ok = scores(i, false, warp_uniform(t + 2 == n));
           // dQ += dS K
-          ok = ok && mbar_wait_warp(&sh->ds_full, ph, abort_flag);
+          ok = ok && mbar_wait_warp(&sh->ds_full[s], ph, abort_flag);
           if (!ok) break;
           tc_fence_after();
           const uint64_t b = k_mn + s * tile;
@@ -722,7 +725,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&sh->ds_full);
+        if (lane == 0) mbar_arrive(&sh->ds_full[g & 1]);
       }
       // ---------------- epilogue: 32 rows x 64 columns a warp, from groups 0 and 1 (the others go on) ----------------
       if (wg < 2) {

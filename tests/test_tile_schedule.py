@@ -268,3 +268,53 @@ def test_reduce_scatter_schedule_cannot_deadlock_across_ranks(cu, tp, M, N, resi
     ideal_rounds = -(-len(order[0][1]) // order[0][0])
     assert rnd + 1 <= ideal_rounds + 1, (rnd + 1, ideal_rounds)      # at most one round lost to waiting
     assert waits <= order[0][0] * tp, (waits, n_units)               # and only around the start
+
+
+def _orders_of_dq(n_barriers, n_steps, n_warps):
+    """Walk all orders in which the issuing warp and ``n_warps`` softmax warps of the queries kernel of the attention backward pass
+    (csrc/flash_attn_bwd.cu) may meet at their barriers; the steps whose dS a product read before every warp had written it."""
+    issuer = []
+    for g in range(n_steps):
+        if g == 0:
+            issuer += [("arrive", "s_full"), ("arrive", "dp_full0")]
+        if g + 1 < n_steps:                      # scores of the next step come before the wait for dS of this one
+            issuer += [("wait", "s_free", g & 1), ("arrive", "s_full"), ("arrive", f"dp_full{(g + 1) & 1}")]
+        issuer += [("wait", f"ds_full{g % n_barriers}", (g // n_barriers) & 1), ("read", g)]
+    warp = []
+    for g in range(n_steps):
+        warp += [("wait", "s_full", g & 1), ("arrive", "s_free"), ("wait", f"dp_full{g & 1}", (g >> 1) & 1), ("write", g),
+                 ("arrive", f"ds_full{g % n_barriers}")]
+    programs = [issuer] + [warp] * n_warps
+    need = {"s_free": n_warps, **{f"ds_full{i}": n_warps for i in range(n_barriers)}}
+    names = sorted({op[1] for p in (issuer, warp) for op in p if op[0] in ("wait", "arrive")})
+    at = {n: i for i, n in enumerate(names)}
+    bad, seen, todo, ended = set(), set(), [((0,) * len(programs), (0,) * len(names))], False
+    while todo:
+        pcs, arrived = state = todo.pop()        # arrivals since the start: the phase is their number over those of a phase
+        if state in seen:
+            continue
+        seen.add(state)
+        ended |= all(pc == len(p) for pc, p in zip(pcs, programs))
+        for i, (pc, p) in enumerate(zip(pcs, programs)):
+            if pc == len(p):
+                continue
+            op, after = p[pc], arrived
+            if op[0] == "wait" and (arrived[at[op[1]]] // need.get(op[1], 1)) & 1 == op[2]:
+                continue                         # the phase of this parity is not over
+            if op[0] == "arrive":
+                after = tuple(n + (j == at[op[1]]) for j, n in enumerate(arrived))
+            if op[0] == "read" and any(q <= warp.index(("write", op[1])) for q in pcs[1:]):
+                bad.add(op[1])
+            todo.append((pcs[:i] + (pc + 1,) + pcs[i + 1:], after))
+    assert ended
+    return bad
+
+
+def test_products_of_the_query_gradient_read_finished_operands():
+    import re
+    from easyllm_b200.ops import build
+    text = open([s for s in build.sources() if s.endswith("flash_attn_bwd.cu")][0]).read()
+    shared = re.search(r"struct FbQShared \{(.*?)\n\};", text, re.S).group(1)
+    n = int(re.search(r"\bds_full(?:\[(\d)\])?[,;]", shared).group(1) or 1)
+    assert _orders_of_dq(n, 5, 2) == set()
+    assert _orders_of_dq(1, 3, 2) != set()       # the model sees what one barrier lets through
