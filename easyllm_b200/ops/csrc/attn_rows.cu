@@ -1008,6 +1008,9 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
   AtShared* sh = reinterpret_cast<AtShared*>(smem + kAtBars);
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (warp == 8) tmem_alloc<256>(&sh->tmem_base);
+  tc_fence_before();
+  __syncthreads();                                     // the TMEM is this CTA's before the next kernel's CTAs come in
+  tc_fence_after();
   chain_next();
   chain_wait(cu);
   AtTile T;
@@ -1025,9 +1028,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     sh->gave_up = *(volatile int*)a.err;               // an earlier kernel already failed: do not wait on anything
     fence_barrier_init();
   }
-  tc_fence_before();
   __syncthreads();
-  tc_fence_after();
   const uint32_t tmem = sh->tmem_base;
   volatile int* gave_up = &sh->gave_up;
   const bool dead = *gave_up != 0;

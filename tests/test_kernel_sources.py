@@ -34,6 +34,21 @@ def test_every_restricted_pointer_goes_through_the_wait():
         assert set(pointers) <= set(passed), (path, kernel, set(pointers) - set(passed))
 
 
+def test_the_next_kernel_comes_in_after_the_allocation():
+    """In a kernel that holds TMEM all threads meet between the allocation, which one warp makes and may wait for, and the call that
+    lets the next kernel's CTAs in: they could take the TMEM that this kernel's CTA is still waiting for."""
+    seen = 0
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
+        text = re.sub(r"//[^\n]*", "", open(path).read())
+        for part in text.split("__global__")[1:]:
+            part = part.split("\n}\n")[0]
+            alloc, let_in = re.search(r"tmem_alloc\w*(<[^>]*>)?\(", part), re.search(r"chain_(next|enter)\(", part)
+            if alloc is not None and let_in is not None:
+                seen += 1
+                assert alloc.start() < let_in.start() and "__syncthreads();" in part[alloc.end():let_in.start()], (os.path.basename(path), part[:120])
+    assert seen >= 3
+
+
 def test_fast_math_sources_do_not_use_the_accurate_activations():
     """vec.cuh's activations are as accurate as the expf that the compiler's flags give them."""
     from easyllm_b200.ops import build
