@@ -255,6 +255,12 @@ class Attention(nn.Module):
                     "vq": QuantizedKV(slots, capacity, self.hk, self.dv, device, dtype), "len": 0}
         return KVRows(slots, capacity, self.hk, self.d, self.dv, device, dtype)
 
+    def rotates_only(self, hq, hk, d):
+        """Whether ``forward`` over cached rows is that of ``hq`` query heads on ``hk`` key heads of ``d``, keys and values alike, with
+        rotary positions, the usual scale and nothing besides: what a call for all layers of a step takes for granted."""
+        return (self.hq, self.hk, self.d, self.dv) == (hq, hk, d, d) and self.scale == 1.0 / math.sqrt(d) and self.sink is None and \
+            self.slopes is None and not self.a.use_logn_attn and isinstance(self.rotary, RotaryTables) and self.rotary.head_dim == d
+
     def _split(self, qkv):
         T, nq, nk = qkv.shape[0], self.hq * self.d, self.hk * self.d
         return (qkv[:, :nq].view(T, self.hq, self.d), qkv[:, nq:nq + nk].view(T, self.hk, self.d),
@@ -468,15 +474,18 @@ class DecoderLayer(nn.Module):
         fused = [iops.fused_alias([lin._parameters["weight"] for lin, _ in g[1:]]) for g in groups] + [w.detach() for w in norms]
         return decoder.TrainPlan(fused, hq, hk, ff, cos, sin, pos, row_start, slopes, eps, 1.0 / math.sqrt(d)), weights
 
-    def addresses(self, width, meta, cache, eps):
-        """What ``ops.infer.decoder_step`` needs to know of this layer, or None where it does not stand for ``forward``."""
+    def addresses(self, sizes, width, meta, cache, eps):
+        """What ``ops.infer.decoder_step`` needs to know of this layer, or None where it does not stand for ``forward`` with ``sizes``:
+        query heads, key heads, head size, feed-forward width, which the call takes once for all layers, as it does the scores' scale."""
         at, mlp = self._modules["self_attn"], self._modules["mlp"]
         if not (_plain(self, DecoderLayer) and _plain(at, Attention) and _plain(mlp, MLP) and type(cache) is KVRows):
             return None
-        hq, hk, d, ff = at.hq, at.hk, at.d, at.a.intermediate_size
+        hq, hk, d, ff = sizes
+        if not at.rotates_only(hq, hk, d):
+            return None
         part, k, v = at._modules, cache.k, cache.v
         if any(c.dtype != torch.bfloat16 or not c.is_cuda or not c.is_contiguous() or c.shape[2:] != (hk, d) or c.data_ptr() & 15
-               for c in (k, v)):
+               for c in (k, v)) or k.shape != v.shape:
             return None
         n1, n2 = (_norm_weight(self._modules[n], width, eps) for n in ("input_layernorm", "post_attention_layernorm"))
         mats = (_adjacent_rows(width, (part["q_proj"], hq * d), (part["k_proj"], hk * d), (part["v_proj"], hk * d)),
@@ -666,6 +675,7 @@ class CausalLM(nn.Module):
         are not those of that call."""
         a, layers, norm = self.arch, self.model.layers, self.model.norm
         d = a.head_dim
+        sizes = a.num_attention_heads, a.kv_heads, d, a.intermediate_size
         if a.position != "rope" or self.model.hybrid or a.use_logn_attn or a.qkv_bias or a.o_bias or d % 16 or d > 128 or len(layers) == 0 or \
                 len(caches) != len(layers) or _global_hooks() or not iops.decoder_step_ok(x, meta) or a.hidden_size != x.shape[1]:
             return None
@@ -674,13 +684,13 @@ class CausalLM(nn.Module):
             return None
         table = []
         for layer, cache in zip(layers, caches):
-            t = layer.addresses(x.shape[1], meta, cache, a.rms_norm_eps) if type(layer) is DecoderLayer else None
+            t = layer.addresses(sizes, x.shape[1], meta, cache, a.rms_norm_eps) if type(layer) is DecoderLayer else None
             if t is None:
                 return None
             table.append(t)
         fresh = bool(meta["fresh"]) and not meta["one_token"]
-        return iops.decoder_step(x, table, w, (a.num_attention_heads, a.kv_heads, d, a.intermediate_size), meta, fresh,
-                                 int(meta.get("kv_bound", meta["max_position"])), a.rms_norm_eps, layers[0].self_attn.scale)
+        return iops.decoder_step(x, table, w, sizes, meta, fresh, int(meta.get("kv_bound", meta["max_position"])), a.rms_norm_eps,
+                                 1.0 / math.sqrt(d))
 
     def forward(self, input_ids=None, attention_mask=None, labels=None, position_ids=None, cu_seqlens=None,
                 inputs_embeds=None, return_dict=True, **_):

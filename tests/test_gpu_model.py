@@ -297,6 +297,62 @@ def test_a_changed_module_of_a_step_is_called(monkeypatch):
         assert _steps(model, monkeypatch, [9, 4], True)[2] == 0
 
 
+def _fewer_query_heads(m):
+    from easyllm_b200.models.hf_models.modeling import Attention
+    m.model.layers[1].self_attn = _like(m, Attention(m.arch, torch.bfloat16, {"heads": 2, "kv_heads": 2, "dim": 64, "vdim": 64}))
+
+
+def _fewer_key_heads(m):
+    from easyllm_b200.models.hf_models.modeling import Attention
+    m.model.layers[0].self_attn = _like(m, Attention(m.arch, torch.bfloat16, {"heads": 4, "kv_heads": 1, "dim": 64, "vdim": 64}))
+
+
+def _own_scale(m):
+    from easyllm_b200.models.hf_models.modeling import Attention
+    m.model.layers[1].self_attn = _like(m, Attention(m.arch, torch.bfloat16, {"heads": 4, "kv_heads": 2, "dim": 64, "vdim": 64, "scale": 0.5}))
+
+
+def _sink(m):
+    from easyllm_b200.models.hf_models.modeling import Attention
+    m.model.layers[0].self_attn = _like(m, Attention(m.arch, torch.bfloat16, {"heads": 4, "kv_heads": 2, "dim": 64, "vdim": 64, "sink": True}))
+    with torch.no_grad():
+        m.model.layers[0].self_attn.sink.fill_(3.0)
+
+
+def _scale_of_the_first(m):
+    m.model.layers[0].self_attn.scale = 0.25
+
+
+def _no_positions(m):
+    m.model.layers[1].self_attn.slopes = torch.tensor([0.5, 0.25, 0.125, 0.0625])
+
+
+def _narrower_feed_forward(m):
+    import dataclasses
+    from easyllm_b200.models.hf_models.modeling import MLP
+    m.model.layers[1].mlp = _like(m, MLP(dataclasses.replace(m.arch, intermediate_size=256), torch.bfloat16))
+
+
+def _like(m, part):
+    part = part.to(m.lm_head.weight.device).eval()
+    torch.manual_seed(5)
+    part.apply(m._init)
+    return part
+
+
+_OTHER_LAYERS = [_fewer_query_heads, _fewer_key_heads, _own_scale, _sink, _scale_of_the_first, _no_positions, _narrower_feed_forward]
+
+
+@pytest.mark.parametrize("change", _OTHER_LAYERS)
+def test_a_layer_unlike_the_others_gives_the_result_of_its_modules(change, monkeypatch):
+    _need_gpu()
+    model = _llama(256, 4, 2, 512)
+    change(model)
+    got, _, taken = _steps(model, monkeypatch, [9, 4], True)
+    want = _steps(model, monkeypatch, [9, 4], False)[0]
+    assert taken == 0 and all(torch.equal(x, y) for x, y in zip(got, want))
+
+
 def test_a_refused_launch_on_pairs_is_repeated_without(monkeypatch):
     """The call comes back with the code of a refusal: the step is issued again on single CTAs, with a warning, and stays there."""
     _need_gpu()

@@ -179,3 +179,16 @@ def test_index_of_a_step():
             assert m[name].tolist() == values and m[name].dtype == (torch.int64 if name == "last_rows" else torch.int32), name
         assert (m["max_seqlen"], m["max_position"]) == (max(counts), max(p + c for p, c in zip(start, counts)))
         assert (m["fresh"], m["one_token"]) == (not any(start), len(tokens) == len(slots))
+
+
+def test_layers_that_a_call_for_all_layers_does_not_stand_for():
+    """Attention of other sizes, with another scale, a sink or a bias of the distance is not what the one call computes."""
+    from easyllm_b200.models.hf_models import CausalLM, arch_from_hf_config
+    from test_gpu_model import _OTHER_LAYERS
+    for change in [None] + _OTHER_LAYERS:
+        m = CausalLM(arch_from_hf_config({"model_type": "llama", "vocab_size": 64, "hidden_size": 256, "intermediate_size": 512,
+                                          "num_hidden_layers": 2, "num_attention_heads": 4, "num_key_value_heads": 2}), dtype=torch.bfloat16)
+        if change is not None:
+            change(m)
+        alike = all(layer.self_attn.rotates_only(4, 2, 64) for layer in m.model.layers)
+        assert alike == (change is None or change.__name__ == "_narrower_feed_forward"), change
