@@ -676,8 +676,9 @@ class CausalLM(nn.Module):
         a, layers, norm = self.arch, self.model.layers, self.model.norm
         d = a.head_dim
         sizes = a.num_attention_heads, a.kv_heads, d, a.intermediate_size
-        if a.position != "rope" or self.model.hybrid or a.use_logn_attn or a.qkv_bias or a.o_bias or d % 16 or d > 128 or len(layers) == 0 or \
-                len(caches) != len(layers) or _global_hooks() or not iops.decoder_step_ok(x, meta) or a.hidden_size != x.shape[1]:
+        if a.position != "rope" or self.model.hybrid or a.use_logn_attn or a.qkv_bias or a.o_bias or d % 16 or d > 128 or \
+                a.intermediate_size % 8 or len(layers) == 0 or len(caches) != len(layers) or _global_hooks() or \
+                not iops.decoder_step_ok(x, meta) or a.hidden_size != x.shape[1]:
             return None
         w = _norm_weight(norm, x.shape[1], a.rms_norm_eps)
         if w is None or not _plain(layers, nn.ModuleList):

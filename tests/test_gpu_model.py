@@ -353,6 +353,18 @@ def test_a_layer_unlike_the_others_gives_the_result_of_its_modules(change, monke
     assert taken == 0 and all(torch.equal(x, y) for x, y in zip(got, want))
 
 
+@pytest.mark.parametrize("width,heads,ff", [(256, 4, 1004), (256, 4, 700), (132, 2, 704), (240, 10, 704)])
+def test_sizes_that_the_kernels_do_not_take_are_served(width, heads, ff, monkeypatch):
+    """Feed-forward widths, rows and heads that are no multiples of 8 or 16: no call for all layers, but an answer, near fp32's."""
+    _need_gpu()
+    model = _llama(width, heads, heads, ff)
+    got, _, taken = _steps(model, monkeypatch, [9, 4], True)
+    want = _steps(model.float(), monkeypatch, [9, 4], False)[0]
+    assert taken == 0
+    for x, y in zip(got[:6:2], want[:6:2]):          # logits: a dozen roundings to bf16 on the way, 2^-9 each
+        assert (x.float() - y.float()).norm() <= 12 * 2.0 ** -9 * y.float().norm()
+
+
 def test_a_refused_launch_on_pairs_is_repeated_without(monkeypatch):
     """The call comes back with the code of a refusal: the step is issued again on single CTAs, with a warning, and stays there."""
     _need_gpu()
