@@ -395,7 +395,8 @@ class MLP(nn.Module):
 
 def _plain(m, cls):
     """Whether ``m`` is a ``cls`` itself whose call is its class's ``forward`` and nothing besides."""
-    return type(m) is cls and "forward" not in m.__dict__ and \
+    own = m.__dict__
+    return type(m) is cls and "forward" not in own and "_attend" not in own and "_split" not in own and \
         not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
 
 
@@ -450,7 +451,7 @@ class DecoderLayer(nn.Module):
         """What ``decoder.train_layer`` needs of this layer for packed rows whose gradients are recorded, or None where it does not
         stand for ``forward`` (modules replaced, adapted or hooked, weights without a ``main_grad``)."""
         at, mlp = self._modules["self_attn"], self._modules["mlp"]
-        if not (_plain(at, Attention) and _plain(mlp, MLP)) or _global_hooks() or type(self) is not DecoderLayer:
+        if not (_plain(at, Attention) and _plain(mlp, MLP)) or _global_hooks() or type(self) is not DecoderLayer or not _as_written():
             return None
         a, width, part, gate = at.a, x.shape[1], at._modules, mlp._modules
         pos, row_start = meta["position_ids"], meta.get("row_start")
@@ -497,6 +498,18 @@ class DecoderLayer(nn.Module):
         cos, sin = at.rotary.get(int(meta["max_position"]), k.device)
         return (*mats, n1.data_ptr(), n2.data_ptr(), k.data_ptr(), v.data_ptr(), cos.data_ptr(), sin.data_ptr(), cos.shape[0],
                 k.shape[0] * k.shape[1])
+
+
+# The methods that one call for a layer, or for all of them, stands for.
+_WRITTEN = [(cls, name, getattr(cls, name)) for cls, names in
+            ((DecoderLayer, "__call__ forward"), (Attention, "__call__ forward _attend _split"), (MLP, "__call__ forward"),
+             (RMSNorm, "__call__ forward"), (nn.Linear, "__call__ forward"), (nn.ModuleList, "__iter__"))
+            for name in names.split()]
+
+
+def _as_written():
+    """Whether the layers' classes have the methods they were written with (a program may put its own in their place)."""
+    return all(getattr(cls, name) is f for cls, name, f in _WRITTEN)
 
 
 def _block_norm(a: HFArch, dtype):
@@ -678,7 +691,7 @@ class CausalLM(nn.Module):
         sizes = a.num_attention_heads, a.kv_heads, d, a.intermediate_size
         if a.position != "rope" or self.model.hybrid or a.use_logn_attn or a.qkv_bias or a.o_bias or d % 16 or d > 128 or \
                 a.intermediate_size % 8 or len(layers) == 0 or len(caches) != len(layers) or _global_hooks() or \
-                not iops.decoder_step_ok(x, meta) or a.hidden_size != x.shape[1]:
+                not _as_written() or not iops.decoder_step_ok(x, meta) or a.hidden_size != x.shape[1]:
             return None
         w = _norm_weight(norm, x.shape[1], a.rms_norm_eps)
         if w is None or not _plain(layers, nn.ModuleList):

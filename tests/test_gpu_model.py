@@ -483,6 +483,23 @@ def test_layers_of_a_training_step_beside_the_usual_one(kw, native, monkeypatch)
     _same_gradients(ga, gb)
 
 
+@pytest.mark.parametrize("cls,name", [("Attention", "forward"), ("Attention", "_attend"), ("MLP", "forward"), ("RMSNorm", "forward"),
+                                      ("DecoderLayer", "__call__")])
+def test_a_method_put_in_the_place_of_a_classes_own_is_called(cls, name, monkeypatch):
+    _need_gpu()
+    from easyllm_b200.models.hf_models import modeling
+    want = _steps(_llama(256, 4, 2, 512), monkeypatch, [9, 4], False)[0]
+    loss = _train_layers(_TRAIN, [33], False, monkeypatch)[0]
+    own, calls = getattr(getattr(modeling, cls), name), []
+    monkeypatch.setattr(getattr(modeling, cls), name, lambda *a, **k: calls.append(1) or own(*a, **k))
+    got, _, taken = _steps(_llama(256, 4, 2, 512), monkeypatch, [9, 4], True)
+    assert taken == 0 and calls and all(torch.equal(x, y) for x, y in zip(got, want))
+    calls.clear()
+    got, _, _, taken = _train_layers(_TRAIN, [33], True, monkeypatch)
+    assert taken == 0 and torch.equal(got, loss)
+    assert calls or name == "_attend"                # of cached rows only
+
+
 def test_a_changed_module_of_a_training_step_is_called(monkeypatch):
     _need_gpu()
     calls = []
