@@ -22,6 +22,8 @@ ELL_API int ell_gemm_bf16(const void* A, const void* B, void* C, const void* bia
                           int a_mn, int b_mn, int out_mode, int bn_hint, int* err, cudaStream_t stream);
 ELL_API int ell_gemm_bf16_pair(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda, int ldb, int ldc,
                                int a_mn, int b_mn, int out_mode, int* err, cudaStream_t stream);
+ELL_API int ell_gemm_pair_route(int M, int N);
+ELL_API int ell_gemm_pair_refused(int rc);
 ELL_API int ell_gemm_glu_pair(const void* x, const void* W, void* out, const void* bias, int M, int F, int K, int ldx, int ldo, int act,
                               int* err, cudaStream_t stream);
 ELL_API int ell_flash_attn_fwd(const void* q, const void* k, const void* v, void* out, float* lse, const int* row_start, int T, int Hq,
@@ -52,25 +54,25 @@ struct StepArgs {
   long long n_layers, T, W, Hq, Hk, D, F;
   long long fresh;                // prompts that start here: attention within the batch; else over the cached rows
   long long max_len, n_seq, max_q;
+  long long gated;                // whether the gated product may run (on CTA pairs)
   long long pairs;                // whether products may run on CTA pairs
   long long launches, failed;     // out: launches; the kind of launch that failed
 };
-static_assert(sizeof(StepLayer) == 12 * 8 && sizeof(StepArgs) == 25 * 8, "the caller lays them out as 64-bit words");
+static_assert(sizeof(StepLayer) == 12 * 8 && sizeof(StepArgs) == 26 * 8, "the caller lays them out as 64-bit words");
 enum StepPart { kStepNorm = 1, kStepProduct, kStepRotation, kStepAttention, kStepActivation };
-constexpr int kStepNoPairs = -1000;                  // a launch on CTA pairs was refused: the call is repeated without
+// A launch on CTA pairs was refused: the call is repeated without any, or without the gated one alone.
+constexpr int kStepNoPairs = -1000, kStepNotGated = -1001;
 
-// Where the tiled product runs on CTA pairs; the same line as for single products.
-static bool use_pairs(const StepArgs& a, long long N) {
-  return a.pairs && a.T >= 256 && N >= 256 && (a.T % 256 == 0 || a.T >= 2048);
-}
-static int no_pairs(int rc) { return rc == -20 || rc == 9 || rc == 701 || rc == 912 ? kStepNoPairs : rc; }
+static bool use_pairs(const StepArgs& a, long long N) { return a.pairs && ell_gemm_pair_route((int)a.T, (int)N); }
+static bool use_gated(const StepArgs& a) { return a.gated && use_pairs(a, 2 * a.F); }
+static int refused(int rc, int instead) { return ell_gemm_pair_refused(rc) ? instead : rc; }
 
 // out [T, N] = x [T, K] w^T
 static int step_product(const StepArgs& a, const void* x, const void* w, void* out, long long N_, long long K_, cudaStream_t stream) {
   const int T = (int)a.T, N = (int)N_, K = (int)K_, route = ell_gemm_thin_route(T, N, K);
   if (route == 2) return ell_matvec(x, w, nullptr, out, 0, 0, 0, 1, T, N, K, K, N, 0, 0, 0, 1, stream);
   if (route) return ell_gemm_thin(x, w, out, nullptr, T, N, K, K, K, N, 0, 0, 0, 0, -1, a.err, stream);
-  if (use_pairs(a, N)) return no_pairs(ell_gemm_bf16_pair(x, w, out, nullptr, T, N, K, K, K, N, 0, 0, 0, a.err, stream));
+  if (use_pairs(a, N)) return refused(ell_gemm_bf16_pair(x, w, out, nullptr, T, N, K, K, K, N, 0, 0, 0, a.err, stream), kStepNoPairs);
   return ell_gemm_bf16(x, w, out, nullptr, T, N, K, K, K, N, 0, 0, 0, 0, a.err, stream);
 }
 
@@ -106,7 +108,7 @@ static StepWork step_work(const StepArgs& a) {
   const size_t end = at;
   at = shared;
   w.act = take(T * a.F * 2);
-  if (!use_pairs(a, 2 * a.F)) w.gate_up = take(T * 2 * a.F * 2);
+  if (!use_gated(a)) w.gate_up = take(T * 2 * a.F * 2);
   w.bytes = std::max(at, end);
   return w;
 }
@@ -149,8 +151,8 @@ static int step_layers(StepArgs& a, float eps, float scale, cudaStream_t stream)
     ELL_STEP(kStepProduct, step_product(a, att, l.o, delta, W, Hq * D, stream));
     d = delta;
     ELL_STEP(kStepNorm, add_norm(l.norm2, normed));
-    if (use_pairs(a, 2 * F)) {
-      ELL_STEP(kStepProduct, no_pairs(ell_gemm_glu_pair(normed, l.gate_up, act, nullptr, T, F, W, W, F, 1, a.err, stream)));
+    if (use_gated(a)) {
+      ELL_STEP(kStepProduct, refused(ell_gemm_glu_pair(normed, l.gate_up, act, nullptr, T, F, W, W, F, 1, a.err, stream), kStepNotGated));
     } else {
       ELL_STEP(kStepProduct, step_product(a, normed, l.gate_up, gate_up, 2 * F, W, stream));
       ELL_STEP(kStepActivation, ell_swiglu_fwd(gate_up, act, T, F, stream));
@@ -173,7 +175,8 @@ ELL_API long long ell_decoder_step_work(const long long* args) {
 
 // The normed rows y behind `n_layers` layers (norm, attention, norm, gated feed-forward; residual sums in bf16) for the T new rows x of
 // a step, whose keys and values go to the caches.  D a multiple of 16 up to 128, W and F multiples of 8, all on 16-byte boundaries.
-// args: the words of StepArgs.  kStepNoPairs: to be called again with `pairs` 0 (what it has written so far is written again).
+// args: the words of StepArgs.  kStepNoPairs, kStepNotGated: to be called again with `pairs`, or `gated`, 0 (what it has written so far is
+// written again).
 ELL_API int ell_decoder_step(long long* args, float eps, float scale, cudaStream_t stream) {
   StepArgs& a = *reinterpret_cast<StepArgs*>(args);
   a.launches = a.failed = 0;

@@ -20,6 +20,8 @@ ELL_API int ell_gemm_bf16(const void* A, const void* B, void* C, const void* bia
                           int a_mn, int b_mn, int out_mode, int bn_hint, int* err, cudaStream_t stream);
 ELL_API int ell_gemm_bf16_pair(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda, int ldb, int ldc,
                                int a_mn, int b_mn, int out_mode, int* err, cudaStream_t stream);
+ELL_API int ell_gemm_pair_route(int M, int N);
+ELL_API int ell_gemm_pair_refused(int rc);
 ELL_API int ell_flash_attn_fwd(const void* q, const void* k, const void* v, void* out, float* lse, const int* row_start, int T, int Hq,
                                int Hk, int d, int dv, int q_stride, int k_stride, int v_stride, float scale, const float* alibi_slopes,
                                const float* sink, int window, int* err, cudaStream_t stream);
@@ -51,15 +53,12 @@ static_assert(sizeof(TrainLayer) == 39 * 8, "the caller lays it out as 64-bit wo
 constexpr int kTrD = 128;                            // head size
 enum TrainPart { kTrNorm = 1, kTrProduct, kTrRotation, kTrAttention, kTrActivation };
 
-static bool tr_pairs(const TrainLayer& a, long long M, long long N) {
-  return a.pairs && M >= 256 && N >= 256 && (M % 256 == 0 || M >= 2048);
-}
 static int tr_product(TrainLayer& a, const void* x, const void* w, void* out, long long M_, long long N_, long long K_, int lda, int ldb,
                       int a_mn, int b_mn, int out_mode, cudaStream_t stream) {
   const int M = (int)M_, N = (int)N_, K = (int)K_;
-  if (tr_pairs(a, M, N)) {
+  if (a.pairs && ell_gemm_pair_route(M, N)) {
     const int rc = ell_gemm_bf16_pair(x, w, out, nullptr, M, N, K, lda, ldb, N, a_mn, b_mn, out_mode, a.err, stream);
-    if (rc != -20 && rc != 9 && rc != 701 && rc != 912) return rc;
+    if (!ell_gemm_pair_refused(rc)) return rc;
     a.pairs = 0;                                       // nothing was launched: on single CTAs from here on
   }
   return ell_gemm_bf16(x, w, out, nullptr, M, N, K, lda, ldb, N, a_mn, b_mn, out_mode, 0, a.err, stream);

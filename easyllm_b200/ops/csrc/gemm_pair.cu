@@ -1138,6 +1138,13 @@ ELL_API int ell_gemm_owned_tile_order(int rows_per_rank, int tiles_n, int tp, in
 // Rounds by which a rank's own tiles trail the peers' in the CTA-pair reduce-scatter, in quarter waves (0: default).
 ELL_API void ell_gemm_set_rs_lag(int quarter_waves) { ell::g_rs_lag_q = quarter_waves < 0 ? 0 : quarter_waves; }
 
+// Where a product of M rows and N columns runs on CTA pairs: at least one 256 x 256 tile, and rows that fill the second CTA's half.
+ELL_API int ell_gemm_pair_route(int M, int N) { return M >= 256 && N >= 256 && (M % 256 == 0 || M >= 2048); }
+
+// Whether a pair launch came back with the code of a launch that was refused (nothing ran, the error is not sticky): it cannot be
+// scheduled together (-20), invalid configuration (9), out of resources (701), invalid cluster size (912).
+ELL_API int ell_gemm_pair_refused(int rc) { return rc == -20 || rc == 9 || rc == 701 || rc == 912; }
+
 ELL_API int ell_gemm_pair_resident_clusters() { return ell::pair::resident_clusters(); }
 
 // Clusters the kernel would launch for `tiles` tiles when `resident` clusters fit on the device.

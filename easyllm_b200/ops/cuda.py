@@ -366,11 +366,6 @@ def set_gemm_pair(enabled):
     _GEMM_PAIR = bool(enabled)
 
 
-# launch-time refusals of a cluster launch (nothing ran, the error is not sticky): cannot co-schedule (-20), invalid
-# configuration (9), launch out of resources (701), invalid cluster size (912)
-_PAIR_LAUNCH_REFUSED = (-20, 9, 701, 912)
-
-
 def pairs_refused(rc):
     """The launch itself was refused (no device work was issued): this device cannot co-schedule the two-CTA cluster with the kernel's
     shared memory.  The single-CTA kernel is used from here on."""
@@ -379,8 +374,18 @@ def pairs_refused(rc):
     set_gemm_pair(False)
 
 
+@functools.lru_cache(maxsize=4096)
+def _pair_route(M, N):
+    return bool(lib().ell_gemm_pair_route(c_int(M), c_int(N)))
+
+
+def _pair_refused(rc):
+    """Whether a launch on CTA pairs came back refused: nothing ran, and the error is not sticky."""
+    return rc != 0 and bool(lib().ell_gemm_pair_refused(c_int(rc)))
+
+
 def _use_pair(M, N, bn):
-    return _GEMM_PAIR and bn == 0 and M >= 256 and N >= 256 and (M % 256 == 0 or M >= 2048)
+    return _GEMM_PAIR and bn == 0 and _pair_route(M, N)
 
 
 @functools.lru_cache(maxsize=4096)
@@ -448,7 +453,7 @@ def gemm(a, b, out=None, bias=None, a_mn=False, b_mn=False, out_mode=0, bn=0, pa
         rc = lib().ell_gemm_bf16_pair(_p(a), _p(b), _p(out), _p(bias), c_int(M), c_int(N), c_int(K), c_int(a.shape[1]),
                                       c_int(b.shape[1]), c_int(N), c_int(1 if a_mn else 0), c_int(1 if b_mn else 0),
                                       c_int(out_mode), _p(err_flag(a.device)), _stream())
-        if rc not in _PAIR_LAUNCH_REFUSED:
+        if not _pair_refused(rc):
             _check(rc, "gemm_bf16_pair")
             return out
         pairs_refused(rc)
@@ -476,7 +481,7 @@ def gemm_glu(x, w, bias, act):
     out = torch.empty(M, F, dtype=x.dtype, device=x.device)
     rc = lib().ell_gemm_glu_pair(_p(x), _p(w), _p(out), _p(bias), c_int(M), c_int(F), c_int(K), c_int(ldx), c_int(F),
                                  c_int({"silu": 1, "gelu_tanh": 2}[act]), _p(err_flag(x.device)), _stream())
-    if rc in _PAIR_LAUNCH_REFUSED:
+    if _pair_refused(rc):
         return None
     _check(rc, "gemm_glu_pair")
     return out

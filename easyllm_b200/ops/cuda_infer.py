@@ -51,7 +51,7 @@ def _gemm(x, ldx, w, bias, out, ldc, out_mode):
             c_int(0), c_int(out_mode))
     if cu._use_pair(M, N, 0):
         rc = lib().ell_gemm_bf16_pair(*args, _p(err_flag(x.device)), _stream())
-        if rc not in cu._PAIR_LAUNCH_REFUSED:
+        if not cu._pair_refused(rc):
             return _check(rc, "gemm_bf16_pair")
     _check(lib().ell_gemm_bf16(*args, c_int(0), _p(err_flag(x.device)), _stream()), "gemm_bf16")
 
@@ -199,7 +199,7 @@ def relu2_scaled(x, z):
 
 # ---- the layers of a decoder -----------------------------------------------------------------------
 _STEP_PARTS = ("", "rmsnorm_fwd", "gemm", "rope_append", "attention", "swiglu_fwd")
-_STEP_NO_PAIRS = -1000
+_STEP_NO_PAIRS, _STEP_NOT_GATED = -1000, -1001
 
 
 def decoder_step(x, layers, norm, sizes, meta, fresh, max_len, eps, scale):
@@ -214,16 +214,19 @@ def decoder_step(x, layers, norm, sizes, meta, fresh, max_len, eps, scale):
     words = [addressof(table), x.data_ptr(), norm.data_ptr(), y.data_ptr(), 0, meta["position_ids"].data_ptr(),
              meta["row_start"].data_ptr(), meta["kv_base"].data_ptr(), meta["kv_len"].data_ptr(), meta["cu_seqlens"].data_ptr(),
              err_flag(x.device).data_ptr(), len(layers), T, W, *sizes, fresh, max_len, 0 if one else meta["cu_seqlens"].numel() - 1,
-             1 if one else meta["max_seqlen"], cu.gemm_pair_enabled(), 0, 0]
+             1 if one else meta["max_seqlen"], 1, cu.gemm_pair_enabled(), 0, 0]
     args = (c_longlong * len(words))(*words)
-    for _ in range(2):
+    while True:
         work = torch.empty(lib().ell_decoder_step_work(args), dtype=torch.uint8, device=x.device)
         args[4] = work.data_ptr()
         rc = lib().ell_decoder_step(args, c_float(eps), c_float(scale), _stream())
-        if rc != _STEP_NO_PAIRS:
+        if rc == _STEP_NO_PAIRS and args[-3]:
+            cu.pairs_refused(rc)
+            args[-3] = 0
+        elif rc == _STEP_NOT_GATED and args[-4]:       # of this call: the plain product, as where a single layer's is refused
+            args[-4] = 0
+        else:
             break
-        cu.pairs_refused(rc)
-        args[-3] = 0
     _check(rc, f"decoder_step ({_STEP_PARTS[args[-1]]})" if rc else "decoder_step", args[-2])
     return y
 

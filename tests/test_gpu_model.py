@@ -393,6 +393,29 @@ def test_a_refused_launch_on_pairs_is_repeated_without(monkeypatch):
         cu.set_gemm_pair(True)
 
 
+def test_a_refused_gated_launch_leaves_the_others_on_pairs(monkeypatch):
+    """What the modules do: the plain product and the activation, and nothing is turned off."""
+    _need_gpu()
+    import easyllm_b200.ops.cuda as cu
+    import easyllm_b200.ops.cuda_infer as ci
+    model = _llama(512, 4, 2, 1024)
+    with monkeypatch.context() as m:
+        m.setattr(cu, "gemm_glu", lambda *a: None)
+        want = _steps(model, monkeypatch, [256], False)[0]
+    real = cu.lib()
+
+    class Refusing:
+        def __getattr__(self, name):
+            return getattr(real, name)
+
+        def ell_decoder_step(self, args, *rest):
+            return ci._STEP_NOT_GATED if args[len(args) - 4] and args[len(args) - 3] else real.ell_decoder_step(args, *rest)
+
+    monkeypatch.setattr(ci, "lib", lambda: Refusing())
+    got = _steps(model, monkeypatch, [256], True)[0]
+    assert cu.gemm_pair_enabled() and all(torch.equal(x, y) for x, y in zip(got, want))
+
+
 def _train_layers(cfg, lens, natively, monkeypatch, change=None, freeze=(), drop=(), wrt=None, checkpointing=False):
     """One micro-batch through a model with an optimizer's fp32 gradient buffer: loss, gradients, launches and layers issued by one call."""
     import easyllm_b200.ops.cuda as cu
