@@ -451,11 +451,14 @@ def moe_route(z, top, bias=None, softmax=False):
     return idx, w
 
 
+ROUTER_ROWS = 64        # of the router's weight that one launch takes
+
+
 def moe_router(h, w, experts, top, bias=None, softmax=False):
     """fp32 ``h wᵀ`` and the routing of its first ``experts`` columns in one launch: ``(z, (idx, scores))``; None where the kernel does
     not take the operands."""
     (T, W), N = h.shape, w.shape[0]
-    if h.dtype != torch.bfloat16 or w.dtype != h.dtype or N > 64 or top > 16 or W % 8 or not w.is_contiguous() or T == 0:
+    if h.dtype != torch.bfloat16 or w.dtype != h.dtype or N > ROUTER_ROWS or top > 16 or W % 8 or not w.is_contiguous() or T == 0:
         return None
     ldx = _rows(h, "h")
     if ldx % 8 or (h.data_ptr() | w.data_ptr()) & 15:

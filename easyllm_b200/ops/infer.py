@@ -327,7 +327,7 @@ def moe_router(h, weights, experts, top, bias=None, softmax=False):
     """Router logits ``z = h [W_1; W_2; ...]ᵀ`` in fp32, and the routing of the first ``experts`` of them (for the ``routed`` of the
     expert ops) where one kernel does both, else None."""
     no_grad_check(h, *weights)
-    if _kern(h):
+    if _kern(h) and sum(w.shape[0] for w in weights) <= _cu().ROUTER_ROWS:
         both = _cu().moe_router(h, fused(weights), experts, top, None if bias is None else bias.detach(), softmax)
         if both is not None:
             return both

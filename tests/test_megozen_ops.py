@@ -327,3 +327,22 @@ def test_row_plan_of_the_grouped_product(T, top, E):
     want_scale = torch.zeros(int(n_tiles) * 128)
     want_scale[rows] = w.flatten()
     assert torch.equal(scale[:int(n_tiles) * 128].cpu(), want_scale)
+
+
+@pytest.mark.gpu
+def test_a_router_that_is_too_wide_for_one_launch_is_put_together_once(monkeypatch):
+    """Experts and shared gate in memory of their own are copied together for the product: once, also where routing is a launch of its own."""
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    from easyllm_b200.ops import infer as iops
+    torch.manual_seed(0)
+    h = torch.randn(40, 256, device="cuda").bfloat16()
+    for experts, copies in ((60, 1), (70, 1)):
+        weights = [torch.randn(n, 256, device="cuda").bfloat16() for n in (experts, 1)]
+        made, cat = [], torch.cat
+        with monkeypatch.context() as m:
+            m.setattr(torch, "cat", lambda ts, *a: made.append(1) or cat(ts, *a))
+            z, routed = iops.moe_router(h, weights, experts, 2)
+        assert len(made) == copies and (routed is not None) == (experts < 64)
+        want = h.double() @ torch.cat(weights).double().t()
+        assert (z.double() - want).norm() <= 256 * 2.0 ** -24 * want.norm()
