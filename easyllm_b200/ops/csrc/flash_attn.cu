@@ -54,9 +54,9 @@ struct FaCfg {
   static constexpr int kQBytes = NC * kQChunk, kKBytes = NC * kKChunk;
   static constexpr int kVBytes = 2 * kKChunk;          // value heads of up to 128
   static constexpr int kOps = 2 * kQBytes + 2 * kKBytes + 2 * kVBytes;   // Q x2, K x2, V x2
-  static constexpr bool kStage = kOps + 32768 + 1024 + 640 <= 232448;      // room for the output rows on their way out
-  static constexpr int kBars = kOps + (kStage ? 32768 : 0);
+  static constexpr int kBars = kOps + 32768;           // between them the output rows on their way out
   static constexpr int kSmemBytes = kBars + 1024 + 640;
+  static_assert(kSmemBytes <= 232448, "");
   static constexpr int kFirst = KN > 64 ? 64 : 32;     // keys of the first part of P
 };
 constexpr float kFaRescaleThreshold = 8.0f;   // log2 units
@@ -501,55 +501,35 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (fa.gate != nullptr && row_valid)
         inv_l *= 1.f / (1.f + __expf(-__bfloat162float(fa.gate[(size_t)row * fa.ldg + h])));
       const bool write = row_valid && ok && !*abort_flag;
-      if constexpr (Cfg::kStage) {
-        // Through the warp's own 32 rows x 64 columns of shared memory and out by the TMA unit, which leaves out what lies past the
-        // tensor: a row at a time from registers touches 32 lines a store, 4000 cycles a tile.
-        uint8_t* stage = smem + Cfg::kOps + (warp - 4) * 4096;
-        const bool out_ok = __all_sync(0xffffffffu, ok && !*abort_flag);
+      // Through the warp's own 32 rows x 64 columns of shared memory and out by the TMA unit, which leaves out what lies past the
+      // tensor: a row at a time from registers touches 32 lines a store, 4000 cycles a tile.
+      uint8_t* stage = smem + Cfg::kOps + (warp - 4) * 4096;
+      const bool out_ok = __all_sync(0xffffffffu, ok && !*abort_flag);
 #pragma unroll 1
-        for (int c = 0; c < dv; c += 64) {
-          uint32_t v[64];
-          tmem_ld_32x32(t_o + c, v);
-          tmem_ld_32x32(t_o + c + 32, v + 32);
-          tmem_ld_wait();
-          if (lane == 0) tma_store_wait_read<0>();         // of the chunk, or the item, before
-          __syncwarp();
+      for (int c = 0; c < dv; c += 64) {
+        uint32_t v[64];
+        tmem_ld_32x32(t_o + c, v);
+        tmem_ld_32x32(t_o + c + 32, v + 32);
+        tmem_ld_wait();
+        if (lane == 0) tma_store_wait_read<0>();         // of the chunk, or the item, before
+        __syncwarp();
 #pragma unroll
-          for (int g = 0; g < 8; ++g) {
-            float f[8];
+        for (int g = 0; g < 8; ++g) {
+          float f[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(v[g * 8 + i]) * inv_l;
-            *reinterpret_cast<bf16x8*>(stage + lane * 128 + ((g ^ (lane & 7)) << 4)) = pack8(f);
-          }
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0 && out_ok) {
-            tma_store_3d(&tmO, stage, c, h, tile_first + quad * 32);
-            tma_store_commit();
-          }
+          for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(v[g * 8 + i]) * inv_l;
+          *reinterpret_cast<bf16x8*>(stage + lane * 128 + ((g ^ (lane & 7)) << 4)) = pack8(f);
         }
-      } else {
-        __nv_bfloat16* orow = fa.out + ((size_t)row * fa.Hq + h) * dv;
-#pragma unroll 1
-        for (int c = 0; c * 32 < dv; ++c) {
-          uint32_t v[32];
-          tmem_ld_32x32(t_o + c * 32, v);
-          tmem_ld_wait();
-          if (write) {
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              if (c * 32 + g * 8 >= dv) break;
-              float f[8];
-#pragma unroll
-              for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(v[g * 8 + i]) * inv_l;
-              *reinterpret_cast<bf16x8*>(orow + c * 32 + g * 8) = pack8(f);
-            }
-          }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && out_ok) {
+          tma_store_3d(&tmO, stage, c, h, tile_first + quad * 32);
+          tma_store_commit();
         }
       }
       if (write && fa.lse != nullptr) fa.lse[(size_t)h * fa.T + row] = m_used * 0.6931471805599453f + logf(l);
     }
-    if (Cfg::kStage && lane == 0) tma_store_wait_read<0>();
+    if (lane == 0) tma_store_wait_read<0>();
   }
 
   tc_fence_before();
