@@ -360,6 +360,14 @@ __device__ __forceinline__ void mma_bf16(float* c, const uint32_t* a, uint32_t b
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// The same with a sum that starts here.
+__device__ __forceinline__ void mma_bf16_first(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+
 template <int MT>
 __global__ void __launch_bounds__(kAlWarps * 32)
 attn_latent_kernel(const __grid_constant__ CUtensorMap tmK, const AttnRowsArgs a) {
@@ -577,15 +585,18 @@ attn_latent_kernel(const __grid_constant__ CUtensorMap tmK, const AttnRowsArgs a
 // read its whole context once per token (1060 us for 301 tokens of two sequences over 3000).  Here a tile of rows is the consecutive
 // tokens of one sequence times the query heads of one key head, and matrix instructions do the products:
 //   scores  exact bf16 products, fp32 sums, scale and bias applied in fp32
-//   values  the fp32 weights go in as three bf16 parts, so they keep their 24 bits; several accumulators take turns, since the
-//           parts' products of one wait for one another
+//   values  the fp32 weights go in as three bf16 parts, so they keep their 24 bits.  The products of a few keys start from zero, the small
+//           parts first, and are added to the sums in fp32: the tensor core cuts off what does not fit its accumulator, and a sum that
+//           stays in one drifts with its length
 //   attn_few_kernel   up to 16 rows (decoding), on mma.sync.  Keys are the M side of both products and rows the N side, so 8 rows
 //                     cost half of 16: S^T = K q^T, O^T = V^T P^T.  The four warps take units of 16 keys in turn, each with a softmax,
-//                     accumulators and a ring of three stages of its own, filled by TMA; no barrier until their results meet.
-//                     With 16 cp.async and their addresses a lane and unit, sizes known at run time only, expf and conversions a unit
-//                     took 687 instructions, five cycles each with two warps a scheduler, and 64 rows x 2100 keys x 8 key heads
-//                     116 us (4.7 TB/s); now 86 (6.5 TB/s, merge included).  8 rows x 4200 43 -> 28, one x 4000 x 4 10.0 -> 8.7.
-//                     Equal shares of all keys for every CTA, rows divided where a share ends: 92, 31 and 14.
+//                     sums and a ring of three stages of its own, filled by TMA; no barrier until their results meet.
+//                     Bound by the keys' and values' bytes.  us, merge included, one B200, keys larger than L2 (8 sequences: as large):
+//                     64 rows x 2100 keys x 8 key heads, 551 MB, 87 (6.3 TB/s); 8 x 4200 x 8 29.4; 10 x 2048 x 32 62; one x 4000 x 4 9.7.
+//                     With 16 cp.async and their addresses a lane and unit 117, 43, 82 and 10.6.  With ex2 of a rounded x log2(e) in
+//                     place of expf and sums that stay in the accumulators 86, 28.8, 60 and 9.5, but 1.1e-6 off 64 bits in front of the
+//                     rounding to bf16, and 3.3e-6 for values of one sign, where this is 2.1e-7 and 5e-8 (8 x 4200).  Equal shares of
+//                     all keys for every CTA, rows divided where a share ends: 92, 31 and 14 (the last for one x 4000).
 //   attn_tile_kernel  more rows (continued prompts): 128 of them on tcgen05, see there
 // Ranges of keys and their merge are those of attn_rows_kernel.
 constexpr int kAtThreads = 128;
@@ -803,6 +814,7 @@ attn_few_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     if (failed) break;
     load(i + kAfStages - 1);                           // over the unit before, which all lanes are done with (the fence and the votes)
     const uint8_t *ks = stages + stage * kAfStage + k_row, *vs = stages + stage * kAfStage + v_row;
+    const int key0 = T.k0 + (warp + 4 * i) * kAfKeys;
     float s[NB][4], s2[NB][4];                       // two chains of sums
 #pragma unroll
     for (int b = 0; b < NB; ++b)
@@ -817,10 +829,8 @@ attn_few_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
         for (int b = 0; b < NB; ++b) mma_bf16(k & 1 ? s2[b] : s[b], x, q[b][k][0], q[b][k][1]);
       }
     }
-    const int key0 = T.k0 + (warp + 4 * i) * kAfKeys;
     const bool mask = key0 + kAfKeys > min(T.len0, T.k1) || key0 < T.last_first;
     float al[NB][2];
-    bool grew = false;
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
 #pragma unroll
@@ -839,22 +849,13 @@ attn_few_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
 #pragma unroll
         for (int o = 4; o <= 16; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         const float now = fmaxf(m[b][j], mx);
-        grew |= now > m[b][j];
-        al[b][j] = now == -INFINITY ? 1.f : sm100::ex2_approx((m[b][j] - now) * kLog2e);       // no key yet: nothing to rescale
+        al[b][j] = now == -INFINITY ? 1.f : expf(m[b][j] - now);       // no key yet: nothing to rescale
         m[b][j] = now;
         const float ref = now == -INFINITY ? 0.f : now;
-        s[b][j] = sm100::ex2_approx((s[b][j] - ref) * kLog2e);
-        s[b][j + 2] = sm100::ex2_approx((s[b][j + 2] - ref) * kLog2e);
+        s[b][j] = expf(s[b][j] - ref);
+        s[b][j + 2] = expf(s[b][j + 2] - ref);
         l[b][j] = l[b][j] * al[b][j] + (s[b][j] + s[b][j + 2]);
       }
-    }
-    if (__any_sync(0xffffffffu, grew)) {
-#pragma unroll
-      for (int n = 0; n < 8; ++n)
-#pragma unroll
-        for (int b = 0; b < NB; ++b)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) acc[n][b][i] *= al[b][i & 1];
     }
     uint32_t w[NB][2][3];                            // weights as the B operand: keys 2 t .. of row gr
 #pragma unroll
@@ -872,14 +873,31 @@ attn_few_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
 #pragma unroll
       for (int y = 0; y < kTogether; ++y)
         if (n + y < vtiles) ldsm4_t(x[y], vs + ((n + y) >> 2) * kAfChunk + (((((n + y) & 3) * 2 + (quad & 1)) ^ l8) << 4));
+      float sum[kTogether][NB][4];
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
+      for (int i = 2; i >= 0; --i)
 #pragma unroll
         for (int y = 0; y < kTogether; ++y)
           if (n + y < vtiles) {
 #pragma unroll
-            for (int b = 0; b < NB; ++b) mma_bf16(acc[n + y][b], x[y], w[b][0][i], w[b][1][i]);
+            for (int b = 0; b < NB; ++b) {
+              if (i == 2) mma_bf16_first(sum[y][b], x[y], w[b][0][i], w[b][1][i]);
+              else mma_bf16(sum[y][b], x[y], w[b][0][i], w[b][1][i]);
+            }
           }
+#pragma unroll
+      for (int y = 0; y < kTogether; ++y)
+        if (n + y < vtiles) {
+#pragma unroll
+          for (int b = 0; b < NB; ++b)
+#pragma unroll
+            for (int i = 0; i < 4; i += 2) {
+              float* o = acc[n + y][b] + i;
+              const float2 v = sm100::ffma2(make_float2(o[0], o[1]), make_float2(al[b][0], al[b][1]), make_float2(sum[y][b][i], sum[y][b][i + 1]));
+              o[0] = v.x;
+              o[1] = v.y;
+            }
+        }
     }
     sm100::fence_proxy_async_smem();                   // these reads before the copies that go over them
     __syncwarp();

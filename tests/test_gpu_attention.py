@@ -326,6 +326,56 @@ def test_weights_of_cached_rows_keep_32_bits(steps, past, H, G):
     assert (o - want).norm() <= 2.4e-3 * want.norm()
 
 
+def _parts(x):
+    """fp64 ``x`` as three bf16 numbers, 24 bits of it."""
+    out = []
+    for _ in range(3):
+        out.append(x.bfloat16())
+        x = x - out[-1].double()
+    return out
+
+
+def _scores_of_keys(tokens, past, fill):
+    """One head whose scores are the first places of the keys, for sequences that go on with ``tokens`` tokens after ``past``; the new
+    tokens weigh nothing.  ``fill(i, k, v)``: the cached keys' scores and values of sequence i."""
+    dev, d, n = "cuda", 64, len(past)
+    cap = max(past) + tokens
+    k, v = torch.zeros(n * cap, 1, d, device=dev).bfloat16(), torch.zeros(n * cap, 1, d, device=dev).bfloat16()
+    q = torch.zeros(n * tokens, 1, d, device=dev).bfloat16()
+    q[:, :, 0] = 1
+    for i, p in enumerate(past):
+        own = slice(i * cap, i * cap + p)
+        fill(i, k[own, 0, 0], v[own, 0])
+        if tokens > 1:
+            k[i * cap + p:i * cap + p + tokens, 0, 0] = -300
+    base = [i * cap for i in range(n) for _ in range(tokens)]
+    length = [p + j + (tokens > 1) for p in past for j in range(tokens)]
+    kw = {"cu_seqlens": torch.arange(0, n * tokens + 1, tokens, device=dev, dtype=torch.int32), "max_q": tokens} if tokens > 1 else {}
+    return q, k, v, base, length, kw
+
+
+@pytest.mark.parametrize("tokens", [1, 5])
+def test_exponentials_of_cached_rows_keep_32_bits(tokens):
+    """Two weights, 1 and e^-x, whose values 1 and -e^x (24 bits of it, in three keys) cancel: what is left is the error of the weight.
+    expf is off by 2 units of 2^-23 at most; four products are cut, or rounded, at 2^-23 of the sum.  An exponential of base 2 of the
+    rounded product x log2(e) would be off by up to 2^-18 ln 2 where that product is above 64."""
+    from easyllm_b200.ops import infer as iops
+    scores = [-40 - 30 * i / 64 for i in range(64)]        # the parts of e^-70 are no denormal numbers
+
+    def fill(i, k, v):
+        k[:] = torch.tensor([0] + [scores[i]] * 3, device=k.device)
+        v[0] = 1
+        for j, p in enumerate(_parts(-torch.exp(-k[1].double()))):
+            v[1 + j] = p
+
+    q, k, v, base, length, kw = _scores_of_keys(tokens, [4] * 64, fill)
+    b, n = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in (base, length))
+    o = iops.attention_rows(q, k, v, b, n, max(length), 1.0, **kw).double()
+    want = _rows_exact(q, k, v, base, length, 1.0, None, None, None, None)
+    assert want.abs().max() < 2.0 ** -23
+    assert (o - want).abs().max() <= 6 * 2.0 ** -23
+
+
 @pytest.mark.parametrize("window", [None, 77])
 @pytest.mark.parametrize("steps,past,H,G", [([1, 1], [700, 63], 8, 2), ([3, 4], [130, 20], 8, 2), ([65, 40], [300, 25], 8, 2), ([2, 20], [2500, 30], 4, 4)])
 def test_values_that_are_not_finite_reach_the_rows_that_see_them(steps, past, H, G, window):
