@@ -607,7 +607,6 @@ constexpr int kAfKeys = 16, kAfChunk = kAfKeys * 128;              // keys of a 
 constexpr int kAfStage = 4 * kAfChunk, kAfStages = 3, kAfRing = 4 * kAfStages * kAfStage, kAfSmem = kAfRing + 1024;
 static_assert(2 * (kAfSmem + 1024) <= 196 * 1024, "");
 constexpr int kAfErr = 15;
-constexpr float kLog2e = 1.4426950408889634f;
 
 // x and y as three bf16 parts each, eight of their 24 bits a part: nothing is lost.  By truncation, since conversions share the unit of
 // the exponential.
@@ -981,42 +980,49 @@ attn_few_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
 
 // ---- continued prompts on tcgen05 ----------------------------------------------------------------------
 // A CTA takes 128 rows (consecutive tokens of one sequence times the query heads of one key head) and a range of keys, in tiles of 64:
-//   warps 0-7  softmax: a thread owns a row, its TMEM lane, and half of a tile's keys (warps 4-7 the second half; the maxima meet in
-//              shared memory).  Fp32 weights go back to TMEM as three bf16 parts, so that the product with V keeps their 24 bits; O is
-//              rescaled where a maximum grew
-//   warp 8     issues: S = Q K^T (128 x 64), O += P_i V for the three parts (P from TMEM, V in place as an MN-major operand)
-//   warp 9     TMA: tiles of keys and values through a ring of two stages
-// TMEM columns: S 0-63, P_0 and P_1 over the scores that the threads have read, P_2 64-95, O 128-255.  That is half of TMEM, and 97 KB
-// of shared memory, so two CTAs share an SM: one's softmax runs beside the other's products.  Bound by the chain of a tile, from the
-// scores (8 products) through the softmax to the 12 products of its parts.  On mma.sync a warp owned 16 rows and walked its chain alone.
-// us, kernel and merge: 301 tokens of two sequences over 3000, 16 heads on 8, 114 -> 42; 512 tokens over 4096, 32 on 8, 519 -> 113; 512
-// over 1000 beside three of 16 tokens, 16 on 4, 100 -> 63; 17 over 3000 24 -> 16; 33 over 64, 32 on 8, 16 -> 11.  With four warps, a
-// row a thread, 48 and 126; with expf and conversions to bf16, which share a unit, in place of ex2 and truncation, 54 and 151.
-// Results are as far from 64 bits as before (the rounding to bf16, 1.65e-3); in fp32 in front of it 2.4e-6, where mma.sync had 1.6e-6.
-constexpr int kAtTile = 64, kAtRows = 128, kAtTileThreads = 320, kAtHalf = kAtTile / 2;
+//   warps 0-7   softmax: a thread owns a row, its TMEM lane, and half of a tile's keys (warps 4-7 the second half; the maxima meet in
+//               shared memory).  Fp32 weights go back to TMEM as three bf16 parts, so that the product with V keeps their 24 bits
+//   warps 8-15  sums: a thread owns a row and half of its value columns in registers, and adds every tile's product to them in fp32
+//   warp 16     issues: S = Q K^T (128 x 64), O_tile = P_2 V + P_1 V + P_0 V (P from TMEM, V in place as an MN-major operand)
+//   warp 17     TMA: tiles of keys and values through a ring of four stages
+// TMEM columns: for even and odd tiles S 0-63, P_0 and P_1 over the scores that the threads have read, P_2 64-95 (128-223); O_tile
+// 256-383 and 384-511.
+// Every tile's product starts from zero, the small parts first, so that four products of it are cut at the tile's own size, and no
+// accumulator is read back to be rescaled.  512 tokens over 4096 keys, in fp32 in front of the rounding to bf16, against 64 bits: 3.2e-7, and
+// 1.1e-7 for values of one sign; with sums that stay in TMEM and ex2 of a rounded x log2(e) 7.3e-6 and 2.3e-5, with mma.sync's
+// accumulators 4.6e-6 and 4.8e-6.
+// One CTA an SM; bound by the softmax, 1.5 us a tile (its twenty products take 0.55).  us, kernel and merge, one B200: 301 tokens of two
+// sequences over 3000, 16 heads on 8, 41; 512 tokens over 4096, 32 on 8, 99; 512 over 1000 beside three of 16 tokens, 16 on 4, 33; 700 over
+// 2000, 16 on 16, 54; 17 over 3000, 32 on 8, 18; 33 over 64 10.4; 64 over 1200, 16 heads of 64, 17.6.  Two CTAs an SM with 256 columns and 97 KB
+// each, whose sums stayed in TMEM: 40, 106, 45, 54, 19, 9.5 and 15.3; a warp for 16 rows on mma.sync: 134, 466, 74, 150, 39, 10.8 and 20.8.
+constexpr int kAtTile = 64, kAtRows = 128, kAtTileThreads = 576, kAtHalf = kAtTile / 2, kAtStages = 4;
 constexpr int kAtQChunk = kAtRows * 128, kAtKvChunk = kAtTile * 128;     // [rows x 64 columns], 128-byte swizzle rows
 constexpr int kAtQBytes = 2 * kAtQChunk, kAtStage = 4 * kAtKvChunk;      // a stage: keys, values
-constexpr int kAtBars = kAtQBytes + 2 * kAtStage, kAtSmem = kAtBars + 1024 + 2560;
+constexpr int kAtBars = kAtQBytes + kAtStages * kAtStage, kAtSmem = kAtBars + 1024 + 6144;
+constexpr int kAtIssueWarp = 16, kAtLoadWarp = 17;
 
 struct AtShared {
-  uint64_t q_full, full[2], empty[2], s_full, p_full, o_full;
+  uint64_t q_full, full[kAtStages], empty[kAtStages], s_full[2], p_full[2], o_full[2], o_free[2], al_full[4], done;
   uint32_t tmem_base;
   int gave_up;
   float met[2][2][kAtRows];       // by turns: what the threads of a row have found in their half of the keys
+  // Factor of the sums before a tile.  Four tiles: scores of tile j + 4 come after the product of j + 2, and that after the sums of j.
+  float al[4][kAtRows];
+  float stat[2][kAtRows];         // maximum and sum of a row in the end
 };
-static_assert(sizeof(AtShared) <= 2560, "");
+static_assert(sizeof(AtShared) <= 6144, "");
 
 // Barrier of the two warps of 32 rows; whether any of their threads has failed.
-__device__ __forceinline__ bool at_pair_failed(int quad, bool failed) {
+__device__ __forceinline__ bool at_pair_failed(int id, bool failed) {
   uint32_t any;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
       "barrier.red.or.pred p, %2, 64, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(any) : "r"((uint32_t)failed), "r"(quad + 1) : "memory");
+      : "=r"(any) : "r"((uint32_t)failed), "r"(id) : "memory");
   return any != 0;
 }
 
-__global__ void __launch_bounds__(kAtTileThreads, 2)
+__global__ void __launch_bounds__(kAtTileThreads, 1)
 attn_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ AttnRowsArgs a,
                  const int* __restrict__ cu, int tiles, int tt) {
   using namespace sm100;
@@ -1025,7 +1031,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
   uint8_t* kv = smem + kAtQBytes;
   AtShared* sh = reinterpret_cast<AtShared*>(smem + kAtBars);
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  if (warp == 8) tmem_alloc<256>(&sh->tmem_base);
+  if (warp == kAtIssueWarp) tmem_alloc<512>(&sh->tmem_base);
   tc_fence_before();
   __syncthreads();                                     // the TMEM is this CTA's before the next kernel's CTAs come in
   tc_fence_after();
@@ -1036,13 +1042,18 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
   const int rows = any ? T.rows : 0, warps = any ? (rows + 31) / 32 : 1;  // groups of 32 rows
   if (threadIdx.x == 0) {
     mbar_init(&sh->q_full, 2 * warps);
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < kAtStages; ++i) {
       mbar_init(&sh->full[i], 1);
       mbar_init(&sh->empty[i], 1);
     }
-    mbar_init(&sh->s_full, 1);
-    mbar_init(&sh->p_full, 2 * warps);
-    mbar_init(&sh->o_full, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&sh->s_full[i], 1);
+      mbar_init(&sh->p_full[i], 2 * warps);
+      mbar_init(&sh->o_full[i], 1);
+      mbar_init(&sh->o_free[i], 2 * warps);
+    }
+    for (int i = 0; i < 4; ++i) mbar_init(&sh->al_full[i], warps);
+    mbar_init(&sh->done, warps);
     sh->gave_up = *(volatile int*)a.err;               // an earlier kernel already failed: do not wait on anything
     fence_barrier_init();
   }
@@ -1059,11 +1070,11 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 
   if (!any || dead) {
     // nothing was issued
-  } else if (warp == 9) {
+  } else if (warp == kAtLoadWarp) {
     if (lane == 0) {
       for (int j = 0; j < n_tiles; ++j) {
-        const int s = j & 1, row = (int)T.base + T.k0 + j * kAtTile;    // rows past the tensor are zero-filled
-        if (!mbar_wait(&sh->empty[s], ((j >> 1) & 1) ^ 1, gave_up)) {
+        const int s = j % kAtStages, row = (int)T.base + T.k0 + j * kAtTile;    // rows past the tensor are zero-filled
+        if (!mbar_wait(&sh->empty[s], ((j / kAtStages) & 1) ^ 1, gave_up)) {
           fail();
           break;
         }
@@ -1073,51 +1084,56 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         for (int c = 0; c < vc; ++c) tma_load_3d(st + (2 + c) * kAtKvChunk, &tmV, &sh->full[s], c * 64, T.g, row);
       }
     }
-  } else if (warp == 8) {
+  } else if (warp == kAtIssueWarp) {
     constexpr uint32_t idesc_s = make_idesc_bf16(128, kAtTile, false, false);
     const uint32_t idesc_o = make_idesc_bf16(128, a.dv, false, true);
     const uint32_t e = elect_one(), tm = __reduce_or_sync(0xffffffffu, tmem);
     const uint64_t q_desc = make_smem_desc(smem_u32(smem), 16, 1024), k_desc = make_smem_desc(smem_u32(kv), 16, 1024);
     const uint64_t v_desc = make_smem_desc(smem_u32(kv) + 2 * kAtKvChunk, kAtKvChunk, 1024);
     const int ksteps = a.d / 16;
-    // The scores of a tile go over the parts of the one before: those products were issued earlier, and are taken in order.
+    // The scores of a tile go over the parts of the one two before: those products were issued earlier, and are taken in order.
     auto scores = [&](int j) -> bool {
-      const int s = j & 1;
-      if (!mbar_wait_warp(&sh->full[s], (j >> 1) & 1, gave_up)) return false;
+      const int s = j % kAtStages;
+      if (!mbar_wait_warp(&sh->full[s], (j / kAtStages) & 1, gave_up)) return false;
       tc_fence_after();
       const uint64_t kd = k_desc + s * (kAtStage >> 4);
+      const uint32_t dst = tm + (j & 1) * 128;
       if (ksteps == 8) {
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          umma_bf16_warp(e, tm, q_desc + (((k >> 2) * kAtQChunk + (k & 3) * 32) >> 4), kd + (((k >> 2) * kAtKvChunk + (k & 3) * 32) >> 4),
+          umma_bf16_warp(e, dst, q_desc + (((k >> 2) * kAtQChunk + (k & 3) * 32) >> 4), kd + (((k >> 2) * kAtKvChunk + (k & 3) * 32) >> 4),
                          idesc_s, k != 0);
       } else {
 #pragma unroll 1
         for (int k = 0; k < ksteps; ++k)
-          umma_bf16_warp(e, tm, q_desc + (((k >> 2) * kAtQChunk + (k & 3) * 32) >> 4), kd + (((k >> 2) * kAtKvChunk + (k & 3) * 32) >> 4),
+          umma_bf16_warp(e, dst, q_desc + (((k >> 2) * kAtQChunk + (k & 3) * 32) >> 4), kd + (((k >> 2) * kAtKvChunk + (k & 3) * 32) >> 4),
                          idesc_s, k != 0);
       }
-      umma_commit_warp(e, &sh->s_full);
+      umma_commit_warp(e, &sh->s_full[j & 1]);
       return true;
     };
     bool ok = n_tiles == 0 || (mbar_wait_warp(&sh->q_full, 0, gave_up) && scores(0));
+    if (ok && n_tiles > 1) ok = scores(1);
     for (int j = 0; j < n_tiles && ok; ++j) {
-      const int s = j & 1;
-      ok = mbar_wait_warp(&sh->p_full, j & 1, gave_up);
+      const int s = j % kAtStages, b = j & 1;
+      const uint32_t ph = (j >> 1) & 1;
+      ok = mbar_wait_warp(&sh->p_full[b], ph, gave_up) && (j < 2 || mbar_wait_warp(&sh->o_free[b], ph ^ 1, gave_up));
       if (!ok) break;
       tc_fence_after();
       const uint64_t vd = v_desc + s * (kAtStage >> 4);
+      const uint32_t dst = tm + 256 + b * 128, p = tm + b * 128;
 #pragma unroll
-      for (int x = 0; x < 3; ++x)
+      for (int x = 2; x >= 0; --x)
 #pragma unroll
         for (int k = 0; k < kAtTile / 16; ++k)
-          umma_bf16_ts_warp(e, tm + 128, tm + x * 32 + k * 8, vd + ((k * 2048) >> 4), idesc_o, (j | x | k) != 0);
+          umma_bf16_ts_warp(e, dst, p + x * 32 + k * 8, vd + ((k * 2048) >> 4), idesc_o, x != 2 || k != 0);
       umma_commit_warp(e, &sh->empty[s]);
-      if (j + 1 < n_tiles) ok = scores(j + 1);
-      else umma_commit_warp(e, &sh->o_full);
+      umma_commit_warp(e, &sh->o_full[b]);
+      if (j + 2 < n_tiles) ok = scores(j + 2);
     }
     if (!ok && e) fail();
-  } else if ((warp & 3) < warps) {
+  } else if ((warp & 3) < warps && warp < 8) {
+    // ------------------------------- softmax -------------------------------
     const int quad = warp & 3, half = warp >> 2, row = quad * 32 + lane;
     const int m = min(row, rows - 1), tok = T.token(m), head = T.head(m);                   // rows past the end repeat the last
     {
@@ -1151,17 +1167,16 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     const bool bias = a.slopes != nullptr;
     const float slope = bias ? a.slopes[head] : 0.f;
     const uint32_t t_row = tmem + ((uint32_t)(quad * 32) << 16), t_s = t_row + half * kAtHalf, t_p = t_row + half * (kAtHalf / 2);
-    const uint32_t t_o = t_row + 128;
-    const int o_end = min(a.dv, half * 64 + 64);       // this thread's columns of O: half * 64 .. o_end - 1
     float mx = -INFINITY, l = 0.f;
     bool failed = false;
     for (int j = 0; j < n_tiles; ++j) {
-      // this also says that the products of the step before have been added: they were issued earlier
-      failed = !mbar_wait(&sh->s_full, j & 1, gave_up);
+      const uint32_t turn = (j & 1) * 128;
+      // this also says that the products of two tiles before have been made: they were issued earlier
+      failed = !mbar_wait(&sh->s_full[j & 1], (j >> 1) & 1, gave_up);
       __syncwarp();
       tc_fence_after();
       uint32_t s[kAtHalf];
-      tmem_ld_32x32(t_s, s);
+      tmem_ld_32x32(t_s + turn, s);
       tmem_ld_wait();
       const int key0 = T.k0 + j * kAtTile + half * kAtHalf;
 #pragma unroll
@@ -1188,28 +1203,20 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
       sh->met[j & 1][half][row] = here;
       // both have read their scores too: the parts may go over them
       tc_fence_before();
-      if (at_pair_failed(quad, failed)) {
+      if (at_pair_failed(quad + 1, failed)) {
         failed = true;
         break;
       }
       tc_fence_after();
       const float now = fmaxf(mx, fmaxf(here, sh->met[j & 1][half ^ 1][row]));
-      if (__any_sync(0xffffffffu, now > mx)) {
-        const float al = now == -INFINITY ? 1.f : ex2_approx((mx - now) * kLog2e);           // no key yet: nothing to rescale
-        mx = now;
-        l *= al;
-        if (j > 0) {
-#pragma unroll 1
-          for (int c = half * 64; c < o_end; c += 32) {
-            uint32_t v[32];
-            tmem_ld_32x32(t_o + c, v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * al);
-            tmem_st_32x32(t_o + c, v);
-          }
-        }
+      const float al = now == mx ? 1.f : expf(mx - now);                     // no key yet: nothing to rescale
+      if (half == 0) {
+        sh->al[j & 3][row] = al;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh->al_full[j & 3]);
       }
+      mx = now;
+      l *= al;
       const float ref = mx == -INFINITY ? 0.f : mx;    // no key yet: all weights 0
       float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -1217,7 +1224,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         uint32_t part[3][8];
 #pragma unroll
         for (int i = 0; i < 16; i += 2) {
-          const float p0 = ex2_approx((__uint_as_float(s[c + i]) - ref) * kLog2e), p1 = ex2_approx((__uint_as_float(s[c + i + 1]) - ref) * kLog2e);
+          const float p0 = expf(__uint_as_float(s[c + i]) - ref), p1 = expf(__uint_as_float(s[c + i + 1]) - ref);
           sum[i & 2] += p0;
           sum[(i & 2) + 1] += p1;
           uint32_t p[3];
@@ -1226,25 +1233,60 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
           for (int x = 0; x < 3; ++x) part[x][i >> 1] = p[x];
         }
 #pragma unroll
-        for (int x = 0; x < 3; ++x) tmem_st_32x8(t_p + x * 32 + c / 2, part[x]);
+        for (int x = 0; x < 3; ++x) tmem_st_32x8(t_p + turn + x * 32 + c / 2, part[x]);
       }
       l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&sh->p_full);
+      if (lane == 0) mbar_arrive(&sh->p_full[j & 1]);
     }
     sh->met[n_tiles & 1][half][row] = l;
-    if (n_tiles > 0 && !failed) failed = !mbar_wait(&sh->o_full, 0, gave_up);
-    failed = at_pair_failed(quad, failed);
-    tc_fence_after();
-    if (failed) {
+    if (at_pair_failed(quad + 1, failed)) {
+      fail();
+    } else if (half == 0) {
+      sh->stat[0][row] = mx;
+      sh->stat[1][row] = l + sh->met[n_tiles & 1][1][row];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh->done);
+    }
+  } else if ((warp & 3) < warps && warp < 16) {
+    // ------------------------------- sums -------------------------------
+    const int quad = warp & 3, half = (warp - 8) >> 2, row = quad * 32 + lane;
+    const uint32_t t_o = tmem + ((uint32_t)(quad * 32) << 16) + 256 + half * 64;
+    const int mine = min(64, a.dv - half * 64);        // this thread's columns (none: not above 0)
+    float acc[64];
+#pragma unroll
+    for (int i = 0; i < 64; ++i) acc[i] = 0.f;
+    bool failed = false;
+    for (int j = 0; j < n_tiles; ++j) {
+      failed = !mbar_wait_warp(&sh->al_full[j & 3], (j >> 2) & 1, gave_up) || !mbar_wait_warp(&sh->o_full[j & 1], (j >> 1) & 1, gave_up);
+      if (failed) break;
+      tc_fence_after();
+      const float al = sh->al[j & 3][row];
+#pragma unroll
+      for (int c = 0; c < 64; c += 16) {
+        if (c < mine) {
+          uint32_t v[16];
+          tmem_ld_32x16(t_o + (j & 1) * 128 + c, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) acc[c + i] = fmaf(acc[c + i], al, __uint_as_float(v[i]));
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh->o_free[j & 1]);
+    }
+    failed = failed || !mbar_wait_warp(&sh->done, 0, gave_up);
+    if (at_pair_failed(quad + 5, failed)) {
       fail();
     } else {
-      l += sh->met[n_tiles & 1][half ^ 1][row];
       // Rows leave 32 columns at a time through the warp's own place in the stages, which nobody reads any more, so that a store
       // covers neighbouring columns.
-      float* stage = reinterpret_cast<float*>(kv) + warp * 32 * 33;
+      const int m = min(row, rows - 1);
+      const float mx = sh->stat[0][row], l = sh->stat[1][row];
+      float* stage = reinterpret_cast<float*>(kv) + (warp - 8) * 32 * 33;
       float f = 1.f, *part = nullptr;
       __nv_bfloat16* out = T.place(a, m, mx, l, f, part);
       if (row < rows && half == 0 && part != nullptr) {
@@ -1254,44 +1296,38 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
       const unsigned long long to = part != nullptr ? reinterpret_cast<unsigned long long>(part + 2) : reinterpret_cast<unsigned long long>(out);
       const int n_rows = min(32, rows - quad * 32);
       float probe = l * 0.f;                           // NaN once a value is not finite
-      for (int c = half * 64; c < o_end; c += 32) {
-        uint32_t v[32];
-        if (n_tiles > 0) {
-          tmem_ld_32x32(t_o + c, v);
-          tmem_ld_wait();
-        } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = 0u;
-        }
-        const int cols = min(32, o_end - c);
+      for (int c0 = 0; c0 < 64; c0 += 32) {
+        if (c0 < mine) {
+          const int cols = min(32, mine - c0), c = half * 64 + c0;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const float x = i < cols ? __uint_as_float(v[i]) : 0.f;
-          probe = fmaf(x, 0.f, probe);
-          stage[lane * 33 + i] = x * f;
-        }
-        __syncwarp();
-        if (part != nullptr) {
+          for (int i = 0; i < 32; ++i) {
+            probe = fmaf(acc[c0 + i], 0.f, probe);
+            stage[lane * 33 + i] = acc[c0 + i] * f;
+          }
+          __syncwarp();
+          if (part != nullptr) {
 #pragma unroll 8
-          for (int r = 0; r < n_rows; ++r) {
-            float* dst = reinterpret_cast<float*>(__shfl_sync(0xffffffffu, to, r)) + c;
-            if (lane < cols) dst[lane] = stage[r * 33 + lane];
-          }
-        } else {
+            for (int r = 0; r < n_rows; ++r) {
+              float* dst = reinterpret_cast<float*>(__shfl_sync(0xffffffffu, to, r)) + c;
+              if (lane < cols) dst[lane] = stage[r * 33 + lane];
+            }
+          } else {
 #pragma unroll 4
-          for (int r = 0; r < n_rows; r += 2) {        // two rows a store, two columns a lane
-            const int rr = r + (lane >> 4), col = (lane & 15) * 2;
-            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(__shfl_sync(0xffffffffu, to, rr & 31)) + c + col;
-            if (rr < n_rows && col < cols)
-              *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(stage[rr * 33 + col], stage[rr * 33 + col + 1]);
+            for (int r = 0; r < n_rows; r += 2) {      // two rows a store, two columns a lane
+              const int rr = r + (lane >> 4), col = (lane & 15) * 2;
+              __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(__shfl_sync(0xffffffffu, to, rr & 31)) + c + col;
+              if (rr < n_rows && col < cols)
+                *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(stage[rr * 33 + col], stage[rr * 33 + col + 1]);
+            }
           }
+          __syncwarp();
         }
-        __syncwarp();
       }
       // rows with values that are not finite, once both halves of them are written
-      sh->met[(n_tiles & 1) ^ 1][half][row] = not_finite(probe) ? 1.f : 0.f;
-      at_pair_failed(quad, false);
-      const bool odd_row = row < rows && half == 0 && sh->met[(n_tiles & 1) ^ 1][0][row] + sh->met[(n_tiles & 1) ^ 1][1][row] > 0.f;
+      sh->met[0][half][row] = not_finite(probe) ? 1.f : 0.f;
+      at_pair_failed(quad + 5, false);
+      const bool odd_row = row < rows && half == 0 && sh->met[0][0][row] + sh->met[0][1][row] > 0.f;
       for (uint32_t odd = __ballot_sync(0xffffffffu, odd_row); odd != 0; odd &= odd - 1) at_row_alone(a, T, quad * 32 + __ffs(odd) - 1);
     }
   }
@@ -1303,9 +1339,9 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     }
   }
   __syncthreads();
-  if (warp == 8) {
+  if (warp == kAtIssueWarp) {
     tc_fence_after();
-    tmem_dealloc<256>(tmem);
+    tmem_dealloc<512>(tmem);
   }
 }
 
@@ -1338,6 +1374,23 @@ static int at_ranges(long long ctas, long long most, double bytes_of_cta) {
   }
   return best;
 }
+// Ranges of continued prompts.  A CTA an SM takes 1.5 us a tile of 64 keys and 5 beside them; the ranges' sums are written and read once
+// at 3 TB/s, and their merge is a launch of 4.5 us.  Measured, us (ranges 1 / 2 / 3 / 4 / 6): 301 tokens of two sequences over 3000, 16 heads on
+// 8 (48 CTAs), 74 / 50 / 42 / 60 / 52; 512 tokens over 4096, 32 on 8 (128), 100 / 130 / 138 / 148 / 161; 700 over 2000, 16 on 16 (96), 54 / 75 /
+// 69 / 77 / 87; 17 over 3000, 32 on 8 (8), 71 / 44 / 34 / 28 / 24, with 18 20.
+static int at_tile_ranges(long long ctas, long long most, int max_len, double bytes) {
+  int best = 1;
+  double least = 1e30;
+  for (int s = 1; s <= most; ++s) {
+    const long long rounds = (ctas * s + kNumSMs - 1) / kNumSMs, tiles = ((max_len + s - 1) / s + kAtTile - 1) / kAtTile;
+    const double us = rounds * (tiles * 1.5 + 5) + (s > 1 ? 4.5 + bytes * s / 3e6 : 0.0);
+    if (us < least) {
+      least = us;
+      best = s;
+    }
+  }
+  return best;
+}
 static AtPlan at_plan(int n, int n_seq, int max_q, int H, int G, int d, int dv, int max_len, int window, bool is_bf16) {
   AtPlan p{};
   p.fits = is_bf16 && d % 16 == 0 && dv % 16 == 0 && d <= 128 && dv <= 128 && d > 0 && dv > 0;
@@ -1350,14 +1403,15 @@ static AtPlan at_plan(int n, int n_seq, int max_q, int H, int G, int d, int dv, 
   const long long ctas = (long long)(one ? n : n_seq * p.tiles) * G * groups;
   if (window > 0 && max_len > window) max_len = window;
   max_len += p.tt - 1;                                  // a tile's rows see windows that start apart
-  // Continued prompts: as many ranges as the two CTAs that fit an SM leave room for.  One CTA an SM or three, 301 tokens over 3000: 62 and
-  // 72 us where two took 54; 512 over 4096 219 and 193, 151; four, where tiles differ most (512 beside three of 16 tokens) 67, 87.
-  const long long most = (max_len + 127) / 128;
-  long long s = p.few ? at_ranges(ctas, most < kArMaxSplits ? most : kArMaxSplits, (double)max_len * (d + dv) * 2)
-                      : 2LL * kNumSMs / ctas;
-  if (s > most) s = most;
-  if (s > kArMaxSplits) s = kArMaxSplits;
-  p.splits = s < 1 ? 1 : (int)s;
+  const long long most = std::min<long long>((max_len + 127) / 128, kArMaxSplits);
+  long long s;
+  if (p.few) {
+    s = at_ranges(ctas, most, (double)max_len * (d + dv) * 2);
+  } else {                                              // no more tiles than the tokens fill, and one a sequence that is not full
+    const long long filled = std::min<long long>((long long)n_seq * p.tiles, n / p.tt + n_seq);
+    s = at_tile_ranges(filled * G * groups, most, max_len, (double)n * H * (dv + 2) * 8);
+  }
+  p.splits = (int)s;
   p.range = ((max_len + p.splits - 1) / p.splits + 63) / 64 * 64;
   return p;
 }

@@ -354,7 +354,7 @@ def _scores_of_keys(tokens, past, fill):
     return q, k, v, base, length, kw
 
 
-@pytest.mark.parametrize("tokens", [1, 5])
+@pytest.mark.parametrize("tokens", [1, 5, 17, 40])
 def test_exponentials_of_cached_rows_keep_32_bits(tokens):
     """Two weights, 1 and e^-x, whose values 1 and -e^x (24 bits of it, in three keys) cancel: what is left is the error of the weight.
     expf is off by 2 units of 2^-23 at most; four products are cut, or rounded, at 2^-23 of the sum.  An exponential of base 2 of the
@@ -374,6 +374,34 @@ def test_exponentials_of_cached_rows_keep_32_bits(tokens):
     want = _rows_exact(q, k, v, base, length, 1.0, None, None, None, None)
     assert want.abs().max() < 2.0 ** -23
     assert (o - want).abs().max() <= 6 * 2.0 ** -23
+
+
+@pytest.mark.parametrize("tokens,sequences", [(33, 160), (128, 148), (40, 3)])
+def test_sums_of_a_continued_prompt_round_every_tile(tokens, sequences):
+    """3000 positive values and one that takes their sum away again: what is left is the error of the sum.  A tile of 64 keys is four
+    products of the weights' first parts, each cut at 2^-23 of it, and is added to the sum with half of that; the weights are off by 2^-22
+    at most.  Sums that stay in the tensor core's accumulators are cut 12 times a tile, 2e-5 over 47 tiles."""
+    from easyllm_b200.ops import infer as iops
+    torch.manual_seed(tokens)
+    last = 3
+
+    def fill(i, k, v):
+        n = k.numel() - last
+        k[:n] = -torch.rand(n, device=k.device)
+        v[:n] = (torch.rand(n, v.shape[1], device=k.device) + 0.5).bfloat16()
+        total = torch.exp(k[:n].double()) @ v[:n].double()
+        for j, p in enumerate(_parts(-total)):
+            v[n + j] = p
+        sums.append((total, torch.exp(k.double()).sum()))
+
+    sums = []
+    q, k, v, base, length, kw = _scores_of_keys(tokens, [3000] * sequences, fill)
+    b, n = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in (base, length))
+    o = iops.attention_rows(q, k, v, b, n, max(length), 1.0, **kw).double()[::tokens, 0]
+    want = _rows_exact(q[::tokens], k, v, base[::tokens], length[::tokens], 1.0, None, None, None, None)[:, 0]
+    total, weights = torch.stack([t for t, _ in sums]), torch.stack([w for _, w in sums])
+    off = ((o - want) * weights[:, None] / total).abs()
+    assert off.max() <= (4 + 47 / 2 + 2) * 2.0 ** -23 and off.mean() <= 8 * 2.0 ** -23
 
 
 @pytest.mark.parametrize("window", [None, 77])
