@@ -760,7 +760,7 @@ attn_few_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
   const int mine = n_units > warp ? (n_units - warp + 3) / 4 : 0;       // units warp, warp + 4, ...
   const int kc = FULL ? 2 : (a.d + 63) / 64, vc = FULL ? 2 : (a.dv + 63) / 64;
   volatile int* gave_up = &ring.gave_up;
-  // rows past the range are other keys or zeros: their weight is 0 (and a row that is not finite is looked at again)
+  // rows past the range are whatever lies there: their weight is 0, and their values are cleared
   auto load = [&](int i) {
     if (i < mine && lane == 0) {
       const int s = i % kAfStages;
@@ -814,6 +814,13 @@ attn_few_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     load(i + kAfStages - 1);                           // over the unit before, which all lanes are done with (the fence and the votes)
     const uint8_t *ks = stages + stage * kAfStage + k_row, *vs = stages + stage * kAfStage + v_row;
     const int key0 = T.k0 + (warp + 4 * i) * kAfKeys;
+    if (key0 + kAfKeys > T.k1) {                       // 0 times what a former sequence left behind the end must be 0
+      uint8_t* left = stages + stage * kAfStage + 2 * kAfChunk + (T.k1 - key0) * 128;
+      const int pieces = (key0 + kAfKeys - T.k1) * 8;
+      for (int c = 0; c < vc; ++c)
+        for (int p = lane; p < pieces; p += 32) *reinterpret_cast<uint4*>(left + c * kAfChunk + p * 16) = make_uint4(0, 0, 0, 0);
+      __syncwarp();
+    }
     float s[NB][4], s2[NB][4];                       // two chains of sums
 #pragma unroll
     for (int b = 0; b < NB; ++b)
@@ -1236,6 +1243,16 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         for (int x = 0; x < 3; ++x) tmem_st_32x8(t_p + turn + x * 32 + c / 2, part[x]);
       }
       l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      const int behind = T.k0 + (j + 1) * kAtTile - T.k1;
+      if (behind > 0) {                                // rows past the range: 0 times what a former sequence left there must be 0
+        const int s = j % kAtStages;
+        failed = failed || !mbar_wait(&sh->full[s], (j / kAtStages) & 1, gave_up);
+        uint8_t* left = kv + s * kAtStage + 2 * kAtKvChunk + (kAtTile - behind) * 128;
+        for (int c = 0; c < vc; ++c)
+          for (int p = (half * warps + quad) * 32 + lane; p < behind * 8; p += 64 * warps)
+            *reinterpret_cast<uint4*>(left + c * kAtKvChunk + p * 16) = make_uint4(0, 0, 0, 0);
+        fence_proxy_async_smem();
+      }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();

@@ -404,6 +404,28 @@ def test_sums_of_a_continued_prompt_round_every_tile(tokens, sequences):
     assert off.max() <= (4 + 47 / 2 + 2) * 2.0 ** -23 and off.mean() <= 8 * 2.0 ** -23
 
 
+@pytest.mark.parametrize("steps,past,H,G", [([1] * 3, [700, 63, 64], 8, 2), ([3, 4], [130, 20], 4, 1), ([65, 40], [300, 25], 8, 2), ([17], [15], 1, 1)])
+def test_what_lies_behind_the_end_of_a_sequence_costs_nothing(steps, past, H, G):
+    """Slots are used again: infinities and NaN that an earlier sequence left behind the end give the bits that zeros there give (rows that
+    come out not finite are summed again key by key, in another order, in many times the time)."""
+    from easyllm_b200.ops import infer as iops
+    torch.manual_seed(sum(steps))
+    dev, d, cap = "cuda", 128, 1024
+    q = torch.randn(sum(steps), H, d, device=dev).bfloat16()
+    k, v = (torch.randn(len(steps) * cap, G, d, device=dev).bfloat16() for _ in "kv")
+    base = [i * cap for i, n in enumerate(steps) for _ in range(n)]
+    length = [p + j + 1 for n, p in zip(steps, past) for j in range(n)]
+    b, n = (torch.tensor(x, dtype=torch.int32, device=dev) for x in (base, length))
+    kw = {"cu_seqlens": torch.tensor([0] + steps, device=dev).cumsum(0).int(), "max_q": max(steps)} if max(steps) > 1 else {}
+    out = []
+    for left in (0.0, float("nan"), float("inf")):
+        for i, (new, p) in enumerate(zip(steps, past)):
+            k[i * cap + p + new:(i + 1) * cap] = left
+            v[i * cap + p + new:(i + 1) * cap] = left
+        out.append(iops.attention_rows(q, k, v, b, n, max(length), d ** -0.5, **kw))
+    assert bool(out[0].isfinite().all()) and torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
+
+
 @pytest.mark.parametrize("window", [None, 77])
 @pytest.mark.parametrize("steps,past,H,G", [([1, 1], [700, 63], 8, 2), ([3, 4], [130, 20], 8, 2), ([65, 40], [300, 25], 8, 2), ([2, 20], [2500, 30], 4, 4)])
 def test_values_that_are_not_finite_reach_the_rows_that_see_them(steps, past, H, G, window):
