@@ -606,7 +606,7 @@ constexpr int kAfKeys = 16, kAfChunk = kAfKeys * 128;              // keys of a 
 // which later kernels of the chain found their L1 cut down by (a decoding product of 6144 x 4096 13.6 -> 19.5 us).
 constexpr int kAfStage = 4 * kAfChunk, kAfStages = 3, kAfRing = 4 * kAfStages * kAfStage, kAfSmem = kAfRing + 1024;
 static_assert(2 * (kAfSmem + 1024) <= 196 * 1024, "");
-constexpr int kAfErr = 15;
+constexpr int kAfErr = 18;
 
 // x and y as three bf16 parts each, eight of their 24 bits a part: nothing is lost.  By truncation, since conversions share the unit of
 // the exponential.

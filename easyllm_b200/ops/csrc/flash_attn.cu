@@ -75,7 +75,7 @@ struct FaShared {
   int abort_flag;
 };
 
-enum FaErr { kFaErrProducer = 11, kFaErrMma = 12, kFaErrSoftmax = 13, kFaErrItems = 14 };
+enum FaErr { kFaErrProducer = 11, kFaErrMma = 12, kFaErrSoftmax = 13, kFaErrItems = 17 };
 
 // Tile plan of the forward kernel, __host__ __device__ so that ell_flash_fwd_plan can run the same arithmetic on the
 // host for a CPU test.  A query tile starting at row `first` walks key tiles of kFaN keys from kv_lo (the document

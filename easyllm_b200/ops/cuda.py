@@ -99,7 +99,9 @@ def check_err_flag():
     if v:
         f.zero_()
         raise KernelError(f"a kernel gave up a bounded wait (code {v}: 1 producer, 2 mma, 3 epilogue, 4 communication "
-                          "role, 5 peer flag; 11-15 the same roles of the CTA-pair GEMM; 21 cross-entropy exchange; "
+                          "role, 5 peer flag; 11-13, 15 the same roles of the CTA-pair GEMM, 11-13 also of the attention's forward pass and "
+                          "17 its work items; 14 latent attention over cached rows, 18 attention over cached rows; 21-24 the attention's "
+                          "backward pass, 21 also the cross-entropy exchange; "
                           "31 a token id outside the embedding table; 32 a position outside the rotary tables; "
                           "41 a scan over chunks; "
                           "6 / 16 a tile index outside a fused kernel's buffers)")

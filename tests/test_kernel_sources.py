@@ -59,6 +59,15 @@ def test_fast_math_sources_do_not_use_the_accurate_activations():
             assert not any(f + "(" in text for f in ("silu_f", "sigmoid_f", "gelu_tanh_f")), base
 
 
+def test_attention_kernels_of_a_model_report_codes_of_their_own():
+    """One word takes the code of the wait that ran out: within a model's attention kernels a code says which."""
+    codes = {}
+    for name in ("flash_attn", "flash_attn_bwd", "attn_rows"):
+        for code in re.findall(r"k(?:Fa|Fb|Al|Af)Err\w* = (\d+)", open(os.path.join(CSRC, name + ".cu")).read()):
+            assert codes.setdefault(code, name) == name and code not in ("1", "2", "3", "4", "5", "6", "15", "16", "31", "32", "41")
+    assert len(codes) == 10
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("rows", [1, 37, 300])
 def test_operands_updated_in_place_keep_their_order(rows):
