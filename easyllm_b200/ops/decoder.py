@@ -122,6 +122,9 @@ def _runs(node):
 def _main_grads(weights):
     """The fp32 ``main_grad`` of ``weights`` as one tensor, or None where they are missing or apart."""
     gs = [getattr(w, "main_grad", None) for w in weights]
+    for g, w in zip(gs, weights):              # what a product is not added to
+        if g is not None and w.dim() == 2 and (g.dtype != torch.float32 or not g.is_contiguous() or g.shape != w.shape):
+            raise ValueError(f"main_grad {tuple(g.shape)} {g.dtype}: expected contiguous fp32 of the weight's shape {tuple(w.shape)}")
     if any(g is None or g.dtype != torch.float32 or not g.is_contiguous() or g.shape != w.shape or g.data_ptr() & 15 for g, w in zip(gs, weights)):
         return None
     return gs[0] if len(gs) == 1 else _adjacent_alias(gs)

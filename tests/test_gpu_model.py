@@ -523,6 +523,19 @@ def test_a_method_put_in_the_place_of_a_classes_own_is_called(cls, name, monkeyp
     assert calls or name == "_attend"                # of cached rows only
 
 
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("make", [lambda g: g.bfloat16(), lambda g: g.clone().t().contiguous().t()])
+def test_a_gradient_buffer_that_a_product_is_not_added_to_is_refused(make, native, monkeypatch):
+    _need_gpu()
+
+    def other(m):
+        w = m.model.layers[1].mlp.down_proj.weight
+        w.main_grad = make(w.main_grad)
+
+    with pytest.raises(ValueError):
+        _train_layers(_TRAIN, [33], native, monkeypatch, change=other)
+
+
 def test_a_changed_module_of_a_training_step_is_called(monkeypatch):
     _need_gpu()
     calls = []

@@ -59,6 +59,13 @@ def test_fast_math_sources_do_not_use_the_accurate_activations():
             assert not any(f + "(" in text for f in ("silu_f", "sigmoid_f", "gelu_tanh_f")), base
 
 
+def test_accurate_sources_use_no_approximate_exponential():
+    from easyllm_b200.ops import build
+    for base in build.ACCURATE_SOURCES:
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, base + ".cu")).read())
+        assert not re.search(r"ex2_approx|ex2\.approx|__expf|__exp10f|exp2_poly|tanh\.approx", text), base
+
+
 def test_attention_kernels_of_a_model_report_codes_of_their_own():
     """One word takes the code of the wait that ran out: within a model's attention kernels a code says which."""
     codes = {}
