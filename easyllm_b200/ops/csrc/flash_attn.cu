@@ -17,9 +17,9 @@
 // The two tiles run on their own and so fall into alternation: one's softmax (2300 cycles a step, 1024 of them the special-function
 // unit's) beside the other's products (2 x 512).  What this replaced kept P in shared memory, whose bandwidth the two operands and P
 // filled, issued from one lane's branch (90 to 210 cycles a product that takes 65, see sm100.cuh), and left the SM empty between
-// items: start, masked diagonal, 4000 cycles of row-wise stores.  us, one B200, L2 flushed, before -> now: 4096 tokens, 32 heads 194 ->
-// 146 (0.94 PFLOP/s); 8 documents of 512, 32 heads on 8 93 -> 41; 3001 tokens in 7 documents, 16 on 4 54 -> 31; 77 tokens 14.6 -> 12.3
-// (launch included); latent keys of 128 + 64, 4096 tokens, 32 heads, a window of 1024 199 -> 136.
+// items: start, masked diagonal, 4000 cycles of row-wise stores.  us, one B200, inputs not in L2, before -> now: 4096 tokens, 32 heads
+// 196 -> 153 (0.90 PFLOP/s); 8 documents of 512, 32 heads on 8 92 -> 40; 3001 tokens in 7 documents, 16 on 4 54 -> 32; 77 tokens 15.3 -> 11.3
+// (launch included); latent keys of 128 + 64, 4096 tokens, 32 heads, a window of 1024 181 -> 118.
 // A single warp that took whichever tile could go cost 500 cycles a turn of its loop in looking around (4096 tokens 165 us).
 // Documents: row_start[t] is the first token of the document that token t belongs to; key j is
 // visible to query i iff row_start[i] <= j <= i, so tiles may straddle document boundaries.

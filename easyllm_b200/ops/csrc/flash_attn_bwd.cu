@@ -10,7 +10,7 @@
 // step (five products take 2560), 64 KB of fp32 went through shared memory twice a step, and dQ came out in the order the CTAs
 // ended.  Here P, dP and dS stay in TMEM, as operands of the products with them, and the chain of a step is the softmax threads' own work.
 //
-// 384 threads:
+// 640 threads:
 //   warp 0      TMA loads
 //   warp 1      issues the products (the whole warp walks the loop, see sm100.cuh)
 //   warp 2      statistics of the query tile (keys kernel) / work items (queries kernel)
@@ -22,11 +22,11 @@
 // Queries kernel: CTAs take (128-query tile, head) items as they get free; lanes are queries, columns keys.  TMEM: S 0-127, dP | dS of
 //   even steps 128-255, of odd steps 256-383, dQ 384-511.
 // What bounds them: of 3250 cycles a step in the keys kernel 1550 are the P pass (1024 of them the special-function unit's), 750 the dS
-// pass, the rest hand-overs and TMEM loads; products take 2048.  us, one B200, L2 flushed, row sums included, before -> now: 4096
-// tokens, 32 heads 585 -> 477; 8 documents of 512, 32 heads on 8 216 -> 171; 3001 tokens in 7 documents, 16 on 4 107 -> 93; 200 tokens,
-// 8 heads 38 -> 28.  Exponentials of a quarter of the columns on the FMA pipe: keys kernel 250 us, queries kernel 221; not worth
+// pass, the rest hand-overs and TMEM loads; products take 2048.  us, one B200, inputs not in L2, row sums included, before -> now: 4096
+// tokens, 32 heads 587 -> 482; 8 documents of 512, 32 heads on 8 216 -> 171; 3001 tokens in 7 documents, 16 on 4 114 -> 99; 200 tokens,
+// 8 heads 38 -> 30.  Exponentials of a quarter of the columns on the FMA pipe: keys kernel 250 us, queries kernel 221; not worth
 // their error of 7e-5.
-// dS and P^T of a thread's columns go over its own columns of dP and S only: those of the other group may not have been read yet.
+// dS and P^T of a thread's columns go over its own columns of dP and S only: those of another group may not have been read yet.
 // The transposed operands (dO, Q, K as [k x n]) are read in place with MN-major descriptors, so nothing is transposed in memory.
 // Every wait is bounded; on expiry the CTA records an error code, lets go of everything, frees its TMEM and returns.
 //

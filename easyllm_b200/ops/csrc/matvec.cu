@@ -460,8 +460,8 @@ __global__ void __launch_bounds__(256) moe_down_kernel(const T* __restrict__ hid
 // top + k); tile_expert[i] is the expert of row tile i, *n_tiles their number, pos[slot] the row of a slot, row_scale[row] its score
 // (rows of the padding: 0), xs[pos[slot]] = h[token].
 // A CTA takes a range of slots and counts for itself, over all slots, the rows of every expert and those before its range: reading the
-// indexes 148 times (30 kB for 3777 tokens, top 2) costs less than a plan made by one CTA and a launch that waits for it.  3777
-// tokens of 2048: 20 us in two launches -> 12; 64 tokens 6.6 -> 4.
+// indexes up to 296 times (30 kB for 3777 tokens, top 2) costs less than a plan made by one CTA and a launch that waits for it.  3777
+// tokens of 2048: 20 us in two launches -> 11.5; 64 tokens 6.6 -> 4.6.
 constexpr int kGatherThreads = 512;
 __global__ void __launch_bounds__(kGatherThreads) moe_gather_kernel(const uint4* __restrict__ h, uint4* __restrict__ xs,
                                                                      const int* __restrict__ idx, const float* __restrict__ wgt,

@@ -6,6 +6,7 @@ Cases: gemm_nt, gemm_nt_n4096, gemm_dgrad, gemm_wgrad, gemm_ag, gemm_rs, gemm_ar
 the prefix gemm_pair_ (CTA-pair kernel) plus gemm_pair_agk (gather of the reduction rows into the weight-gradient
 GEMM) and gemm_pair_ce (LM head with the cross-entropy epilogue), flash_fwd, flash_bwd, rmsnorm_fwd, rmsnorm_bwd,
 swiglu, rope, adam, ce, attn_latent (decoding, 64 sequences of 4096 tokens, 32 heads over a latent of 512 + 64),
+attn_decode (64 sequences of 2100 keys), attn_continue (151 tokens each of two sequences over 3000 keys),
 flash_latent (one prompt of 4096 tokens, keys of 128 + 64, a window of 1024).
 Inputs are larger than L2 (126 MB) where the op is memory-bound but hold well under a few GB,
 so a full-section profiler capture of 1-3 launches ends by itself in a minute or two.
@@ -112,6 +113,16 @@ def main():
         base = torch.arange(0, 64 * 4096, 4096, dtype=torch.int32, device="cuda")
         ln = torch.full((64,), 4096, dtype=torch.int32, device="cuda")
         fn = lambda: ci.attention_latent(q, rows, 512, base, ln, 4096, 0.07)          # noqa: E731
+    elif c in ("attn_decode", "attn_continue"):
+        from . import cuda_infer as ci
+        n, new, length, heads, groups = (64, 1, 2100, 32, 8) if c == "attn_decode" else (2, 151, 3000, 16, 8)
+        k, v = (torch.randn(n * 3072, groups, 128, **bf) for _ in "kv")
+        q = torch.randn(n * new, heads, 128, **bf)
+        i32 = dict(dtype=torch.int32, device="cuda")
+        base = torch.arange(0, n * 3072, 3072, **i32).repeat_interleave(new)
+        ln = torch.arange(length - new + 1, length + 1, **i32).repeat(n)
+        cus = torch.arange(0, n * new + 1, new, **i32) if new > 1 else None
+        fn = lambda: ci.attention_rows(q, k, v, base, ln, length, 128 ** -0.5, cu_seqlens=cus, max_q=new)   # noqa: E731
     elif c == "flash_latent":
         from . import cuda_infer as ci
         z = torch.randn(4096, 32 * 192 + 576, **bf); kv = torch.randn(4096, 32 * 256, **bf)
