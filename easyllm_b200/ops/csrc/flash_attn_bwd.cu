@@ -810,7 +810,7 @@ int make_tmap_bf16_heads(CUtensorMap* map, const void* ptr, uint64_t dim, uint64
 using namespace ell;
 
 // q [T, Hq, 128], k / v [T, Hk, 128] (row strides q_stride / kv_stride elements, views into a packed QKV
-// buffer are fine); out, dout [T, Hq, 128] contiguous; lse [Hq, T] from the forward.
+// buffer are fine); out, dout [T, Hq, 128] contiguous, on 16-byte places; lse [Hq, T] from the forward.
 // Outputs: dq [T, Hq, 128] (row stride dq_stride), dk / dv [T, Hk, 128] (row stride dkv_stride) - views into
 // one packed dQKV buffer are fine.  Scratch: delta fp32 [Hq, T],
 // dkv_acc fp32 [2, T, Hk*128] (GQA only, may be null: used when the head group is split over CTAs).
@@ -820,7 +820,7 @@ ELL_API int ell_flash_attn_bwd(const void* q, const void* k, const void* v, cons
                                int dkv_stride, float scale, const float* alibi_slopes, int* err, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (Hq % Hk) return -2;
-  if ((dq_stride % 8) || (dkv_stride % 8)) return -3;
+  if ((dq_stride % 8) || (dkv_stride % 8) || ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(dout)) & 15)) return -3;
   const int n_kt = (T + kFbTile - 1) / kFbTile;
   // few kv heads and a short sequence leave SMs idle: split each query-head group over CTAs
   const int nsplit = (Hq > Hk && dkv_acc != nullptr && Hk * n_kt < 2 * kNumSMs) ? Hq / Hk : 1;

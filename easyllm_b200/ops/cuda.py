@@ -672,6 +672,8 @@ def flash_attn_bwd(do, q, k, v, out, lse, row_start, scale, dq=None, dk=None, dv
         raise RuntimeError("libeasyllm_b200.so was built without ell_flash_attn_bwd")
     do = do.contiguous()
     out = out.contiguous()
+    if out.data_ptr() & 15:                    # read 16 bytes at a time
+        out = out.clone()
     if dq is None:
         dq = torch.empty(T, Hq, D, dtype=torch.bfloat16, device=q.device)
         dk = torch.empty(T, Hk, D, dtype=torch.bfloat16, device=q.device)

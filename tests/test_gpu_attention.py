@@ -158,6 +158,19 @@ def test_attention_backward_against_64_bits(cu, lens, Hq, Hk):
         assert (a.double() - b.grad).norm().item() < bound, name
 
 
+def test_attention_backward_of_results_on_no_16_byte_place(cu):
+    """The row sums read the results 16 bytes at a time; a copy of them that starts elsewhere gives the same gradients."""
+    torch.manual_seed(2)
+    T, H = 70, 2
+    q, k, v, do = (torch.randn(T, H, 128, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+    rs = torch.zeros(T, dtype=torch.int32, device="cuda")
+    out, lse = cu.flash_attn_fwd(q, k, v, rs, 128 ** -0.5)
+    moved = torch.empty(out.numel() + 4, device="cuda", dtype=torch.bfloat16)[4:].view_as(out).copy_(out)
+    assert moved.data_ptr() % 16 == 8
+    for a, b in zip(cu.flash_attn_bwd(do, q, k, v, out, lse, rs, 128 ** -0.5), cu.flash_attn_bwd(do, q, k, v, moved, lse, rs, 128 ** -0.5)):
+        assert torch.equal(a, b)
+
+
 def test_flash_packed_autograd_matches_library(cu):
     from easyllm_b200 import ops
     torch.manual_seed(3)
